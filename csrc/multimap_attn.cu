@@ -19,8 +19,9 @@
 //                          per-row RMS norm without a weight (v optional), q times a factor that grows with the position.
 // b200_multimap_attn       per-token attention in fp32 arithmetic over a 16-bit or 32-bit cache; prompt pieces and decoded
 //                          tokens take the same path: a vector kernel (16-byte row chunks, the heads of a KV group share the
-//                          K/V reads, `nsplit` key ranges + a merge kernel for few tokens with many keys) and a scalar one
-//                          (a warp per (token, head)) for row sizes that are not whole chunks.
+//                          K/V reads, `nsplit` key ranges + a merge kernel for few tokens with many keys), its tensor-core
+//                          form for bf16 rows of 64 or 128, and a scalar one (a warp per (token, head)) for row sizes that are
+//                          not whole chunks.
 #include "common.cuh"
 #include "mma_sync.cuh"
 
@@ -410,6 +411,43 @@ multimap_attn_kernel(const T* __restrict__ q, const T* __restrict__ ck, const T*
     if (d < Dv) orow[d] = from_f32<T>(res[a] * mult);
   }
 }
+// The four warps' (max, sum, acc[Dv]) of up to HB heads, left in shared memory as [4][HB][Dv + 2], are merged: the final row when
+// there is one map and one range of keys, else a row of `part` for the merge kernel.
+template <typename T>
+__device__ __forceinline__ void merge_warps(const float* sm, int HB, int nh, int h0, int t, int m, int split, int nsplit, int H, int M, int Dv,
+                                            T* __restrict__ out, long long ldo, float* __restrict__ part, float post,
+                                            const b200_attn_opts& opt) {
+  const int LDW = Dv + 2;
+  const bool direct = M == 1 && nsplit == 1;
+  for (int i = threadIdx.x; i < nh * Dv; i += blockDim.x) {
+    const int hh = i / Dv, d = i % Dv;
+    const int h = h0 + hh;
+    float mt = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) mt = fmaxf(mt, sm[(w * HB + hh) * LDW]);
+    float lt = 0.f, at = 0.f;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      const float* ws = sm + (w * HB + hh) * LDW;
+      if (ws[0] != -INFINITY) {
+        const float e = exp2f(ws[0] - mt);
+        lt += ws[1] * e;
+        at += ws[2 + d] * e;
+      }
+    }
+    if (direct) {
+      float f = post;
+      if (opt.sink) lt += exp2f(opt.sink[h] * kLog2e - mt);
+      if (opt.gate) f *= sigmoid_f(opt.gate[(long long)t * opt.ld_gate + h]);
+      out[(long long)t * ldo + (long long)h * Dv + d] = from_f32<T>(lt > 0.f ? at / lt * f : 0.f);
+    } else {
+      float* pr = part + ((((long long)t * H + h) * M + m) * nsplit + split) * LDW;
+      if (d == 0) { pr[0] = mt; pr[1] = lt; }
+      pr[2 + d] = at;
+    }
+  }
+}
+
 // Vector variant (D and Dv whole 16-byte chunks, at most 32 chunks each): a CTA owns one token, up to HB query heads of one
 // KV group, ONE map and one range of the visible keys (blockIdx.z = range * M + map). A lane is (key sub-index, chunk): the
 // CP lanes of a group read the key row of the map and the value row of one key with one 16-byte load each; scores are
@@ -573,36 +611,215 @@ multimap_attn_vec_kernel(const T* __restrict__ q, const T* __restrict__ ck, cons
     }
   }
   __syncthreads();
-  const bool direct = M == 1 && nsplit == 1;
-  for (int i = threadIdx.x; i < nh * Dv; i += blockDim.x) {
-    const int hh = i / Dv, d = i % Dv;
-    const int h = h0 + hh;
-    float mt = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < 4; ++w) mt = fmaxf(mt, sm[(w * HB + hh) * LDW]);
-    float lt = 0.f, at = 0.f;
-#pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      const float* ws = sm + (w * HB + hh) * LDW;
-      if (ws[0] != -INFINITY) {
-        const float e = exp2f(ws[0] - mt);
-        lt += ws[1] * e;
-        at += ws[2 + d] * e;
-      }
-    }
-    if (direct) {
-      float f = post;
-      if (opt.sink) lt += exp2f(opt.sink[h] * kLog2e - mt);
-      if (opt.gate) f *= sigmoid_f(opt.gate[(long long)t * opt.ld_gate + h]);
-      out[(long long)t * ldo + (long long)h * Dv + d] = from_f32<T>(lt > 0.f ? at / lt * f : 0.f);
-    } else {
-      float* pr = part + ((((long long)t * H + h) * M + m) * nsplit + split) * LDW;
-      if (d == 0) { pr[0] = mt; pr[1] = lt; }
-      pr[2 + d] = at;
-    }
-  }
+  merge_warps<T>(sm, HB, nh, h0, t, m, split, nsplit, H, M, Dv, out, ldo, part, post, opt);
 }
 
+// bf16 pools with rows of 64 or 128 (decode batches): the same split of the work — a CTA owns one token, up to ROWS heads of one KV
+// group, one map and one range of the visible keys — on mma.sync. The vector kernel above is bound by its instructions (for
+// every key and head eight FMAs, four shuffles and an exponential per lane), not by the bytes it reads. Here the heads of a
+// group are the 16 rows of the tensor-core tile and a warp walks its own tiles of 16 keys: S = Q K^T straight from the bf16
+// pool, P as the sum of two bf16 numbers (p and what rounding took from it: 2^-17 of p, far below the rounding of the
+// result), two products with V. Every warp fetches its tiles by itself, kDmStages in turn with cp.async, so nothing but
+// a warp barrier sits in the loop and 16 KiB of each warp are on their way (two CTAs of four warps per SM: 128 KiB, three
+// times what the memory's latency asks for).
+// 64 sequences at contexts of 3300 - 4000, 16 heads over 4 KV groups of 128 (484 MB of keys and values): 410 us in the vector
+// kernel (1.2 TB/s), 87 us here (5.6 TB/s).
+constexpr int kDmKeys = 16, kDmStages = 3;
+
+template <int D, int DV, int ROWS>
+__global__ void __launch_bounds__(128, 2)
+multimap_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ ck, const __nv_bfloat16* __restrict__ cv,
+                           const int* __restrict__ pos, const int* __restrict__ slot, const int* __restrict__ table, int max_blocks,
+                           __nv_bfloat16* __restrict__ out, long long ldo, float* __restrict__ part, int H, int G, int M, int bs_log2,
+                           float scale, int window, int keep_first, int nsplit, float post, const b200_attn_opts opt) {
+  constexpr int CK = D / 8, CV = DV / 8;                 // 16-byte chunks of a key / value row
+  constexpr uint32_t kStage = kDmKeys * (D + DV) * 2;
+  extern __shared__ __align__(16) float sm[];            // [4 warps][stages][16 keys][D | DV], then the warps' results
+  const int t = blockIdx.x;
+  const int rep = H / G;
+  const int passes = (rep + ROWS - 1) / ROWS;
+  const int g = blockIdx.y / passes;
+  const int h0 = g * rep + (blockIdx.y % passes) * ROWS;
+  const int nh = min(ROWS, g * rep + rep - h0);
+  const int split = blockIdx.z / M, m = blockIdx.z % M;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int p = pos[t];
+  const int* trow = table + (long long)slot[t] * max_blocks;
+  const int lo = first_seen(p, window, opt.chunk);
+  const int n1 = window > 0 ? min(max(keep_first, 0), lo) : 0;
+  const int total = n1 + (p + 1 - lo);
+  int i_lo = 0, i_hi = total;
+  if (nsplit > 1) {
+    const int chunk = ((total + nsplit - 1) / nsplit + 63) / 64 * 64;
+    i_lo = split * chunk;
+    i_hi = min(total, i_lo + chunk);
+  }
+  const bool capped = opt.softcap > 0.f;
+  const float sl2 = capped ? scale / opt.softcap : scale * kLog2e;
+  const float cap2 = opt.softcap * kLog2e;
+
+  uint32_t qa[D / 16][4];                                // the heads' queries as A fragments; rows past nh are zero
+#pragma unroll
+  for (int k = 0; k < D / 16; ++k)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int r = (lane >> 2) + (j & 1) * 8, c = k * 16 + (j >> 1) * 8 + 2 * (lane & 3);
+      qa[k][j] = r < nh ? *reinterpret_cast<const uint32_t*>(q + (((long long)t * H + h0 + r) * M + m) * D + c) : 0u;
+    }
+  const uint32_t sbase = smem_u32(sm) + warp * kDmStages * kStage;
+  const int bs_mask = (1 << bs_log2) - 1;
+  const int n_tiles = i_hi > i_lo ? (i_hi - i_lo + kDmKeys - 1) / kDmKeys : 0;
+  const int nt = n_tiles > warp ? (n_tiles - warp + 3) / 4 : 0;
+  // lanes 0 .. 15 hold the pool rows of the keys of the tile to be fetched next: its page numbers are read one tile ahead
+  int row_k = -1, row_v = -1;
+  auto lookup = [&](int tile) {
+    const int i = i_lo + (tile * 4 + warp) * kDmKeys + (lane & 15);
+    row_k = row_v = -1;
+    if (tile < nt && i < i_hi) {
+      const int kp = i < n1 ? i : lo + (i - n1);
+      const int blk = trow[kp >> bs_log2];
+      row_v = ((blk * G + g) << bs_log2) + (kp & bs_mask);
+      row_k = (((blk * G + g) * M + m) << bs_log2) + (kp & bs_mask);
+    }
+  };
+  auto fetch = [&](int stage) {                           // keys that are not there (row -1) arrive as zeros
+    const uint32_t dk = sbase + stage * kStage, dv = dk + kDmKeys * D * 2;
+#pragma unroll
+    for (int j = 0; j < kDmKeys * CK / 32; ++j) {
+      const int c = lane + 32 * j, r = c / CK, cc = c % CK;
+      const int pr = __shfl_sync(0xffffffffu, row_k, r);
+      cp_async16_zfill(dk + r * (D * 2) + ((cc ^ (r & 7)) << 4), ck + (long long)max(pr, 0) * D + cc * 8, pr >= 0);
+    }
+#pragma unroll
+    for (int j = 0; j < kDmKeys * CV / 32; ++j) {
+      const int c = lane + 32 * j, r = c / CV, cc = c % CV;
+      const int pr = __shfl_sync(0xffffffffu, row_v, r);
+      cp_async16_zfill(dv + r * (DV * 2) + ((cc ^ (r & 7)) << 4), cv + (long long)max(pr, 0) * DV + cc * 8, pr >= 0);
+    }
+  };
+  lookup(0);
+#pragma unroll
+  for (int x = 0; x < kDmStages - 1; ++x) {
+    if (x < nt) fetch(x);
+    cp_async_commit();
+    lookup(x + 1);
+  }
+  float o[DV / 8][4];
+#pragma unroll
+  for (int n = 0; n < DV / 8; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
+  float mx[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+  int stage = 0;
+  for (int tile = 0; tile < nt; ++tile) {
+    cp_async_wait<kDmStages - 2>();
+    __syncwarp();                                         // the tile is there for every lane, and the one before it is read
+    if (tile + kDmStages - 1 < nt) fetch(stage == 0 ? kDmStages - 1 : stage - 1);
+    cp_async_commit();
+    lookup(tile + kDmStages);
+    const uint32_t sk = sbase + stage * kStage, sv = sk + kDmKeys * D * 2;
+    stage = stage + 1 == kDmStages ? 0 : stage + 1;
+    float s[2][4];
+#pragma unroll
+    for (int n = 0; n < 2; ++n) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
+#pragma unroll
+    for (int k = 0; k < D / 16; k += 2)
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        const int r = n * 8 + (lane & 7), c = k * 2 + (lane >> 3);
+        uint32_t b0, b1, b2, b3;
+        ldsm_x4(sk + r * (D * 2) + ((c ^ (r & 7)) << 4), b0, b1, b2, b3);
+        mma_bf16_16816(s[n], qa[k][0], qa[k][1], qa[k][2], qa[k][3], b0, b1);
+        mma_bf16_16816(s[n], qa[k + 1][0], qa[k + 1][1], qa[k + 1][2], qa[k + 1][3], b2, b3);
+      }
+    const int left = i_hi - (i_lo + (tile * 4 + warp) * kDmKeys);       // keys of this tile inside the range
+    float top[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float x = s[n][j] * sl2;
+        if (capped) x = cap2 * tanh_ex2(x);
+        if (n * 8 + 2 * (lane & 3) + (j & 1) >= left) x = -INFINITY;
+        s[n][j] = x;
+        top[j >> 1] = fmaxf(top[j >> 1], x);
+      }
+    uint32_t hi[4], res[4];                               // P as A fragments: rounded to bf16, and what the rounding left
+    bool moved = false;
+    float ms[2], r_[2];
+#pragma unroll
+    for (int x = 0; x < ROWS / 8; ++x) {
+      top[x] = fmaxf(top[x], __shfl_xor_sync(0xffffffffu, top[x], 1));
+      top[x] = fmaxf(top[x], __shfl_xor_sync(0xffffffffu, top[x], 2));
+      const float mn = fmaxf(mx[x], top[x]);
+      ms[x] = mn == -INFINITY ? 0.f : mn;
+      r_[x] = ex2_approx(mx[x] - ms[x]);
+      moved |= mn != mx[x];
+      mx[x] = mn;
+    }
+    if (__any_sync(0xffffffffu, moved)) {
+#pragma unroll
+      for (int x = 0; x < ROWS / 8; ++x) {
+        l[x] *= r_[x];
+#pragma unroll
+        for (int n = 0; n < DV / 8; ++n) { o[n][2 * x] *= r_[x]; o[n][2 * x + 1] *= r_[x]; }
+      }
+    }
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        if (x < ROWS / 8) {
+          const float p0 = ex2_approx(s[n][2 * x] - ms[x < ROWS / 8 ? x : 0]), p1 = ex2_approx(s[n][2 * x + 1] - ms[x < ROWS / 8 ? x : 0]);
+          l[x] += p0 + p1;
+          const uint32_t w = pack_bf16x2(p0, p1);
+          const float2 f = unpack_bf16x2(w);
+          hi[n * 2 + x] = w;
+          res[n * 2 + x] = pack_bf16x2(p0 - f.x, p1 - f.y);
+        } else hi[n * 2 + x] = res[n * 2 + x] = 0u;
+      }
+#pragma unroll
+    for (int n = 0; n < DV / 8; n += 2) {
+      const int r = lane & 15, c = n + (lane >> 4);
+      uint32_t b0, b1, b2, b3;
+      ldsm_x4_trans(sv + r * (DV * 2) + ((c ^ (r & 7)) << 4), b0, b1, b2, b3);
+      mma_bf16_16816(o[n], hi[0], hi[1], hi[2], hi[3], b0, b1);
+      mma_bf16_16816(o[n + 1], hi[0], hi[1], hi[2], hi[3], b2, b3);
+      mma_bf16_16816(o[n], res[0], res[1], res[2], res[3], b0, b1);
+      mma_bf16_16816(o[n + 1], res[0], res[1], res[2], res[3], b2, b3);
+    }
+  }
+  cp_async_wait<0>();
+  __syncthreads();                                        // every warp is done with its tiles: their place takes the results
+  constexpr int LDW = DV + 2;
+#pragma unroll
+  for (int x = 0; x < ROWS / 8; ++x) {
+    l[x] += __shfl_xor_sync(0xffffffffu, l[x], 1);
+    l[x] += __shfl_xor_sync(0xffffffffu, l[x], 2);
+    const int hh = (lane >> 2) + 8 * x;
+    if (hh < nh) {
+      float* w = sm + (warp * ROWS + hh) * LDW;
+      if ((lane & 3) == 0) { w[0] = mx[x]; w[1] = l[x]; }
+#pragma unroll
+      for (int n = 0; n < DV / 8; ++n) *reinterpret_cast<float2*>(w + 2 + n * 8 + 2 * (lane & 3)) = make_float2(o[n][2 * x], o[n][2 * x + 1]);
+    }
+  }
+  __syncthreads();
+  merge_warps<__nv_bfloat16>(sm, ROWS, nh, h0, t, m, split, nsplit, H, M, DV, out, ldo, part, post, opt);
+}
+
+template <int D, int DV, int ROWS>
+static int launch_decode_mma(const void* q, const void* ck, const void* cv, const int* pos, const int* slot, const int* table, int max_blocks,
+                             void* out, long long ldo, float* part, int tokens, int H, int G, int M, int bs_log2, float scale, int window,
+                             int keep_first, int nsplit, float post, const b200_attn_opts& opt, cudaStream_t st) {
+  const size_t tiles = (size_t)4 * kDmStages * kDmKeys * (D + DV) * 2, rows = (size_t)4 * ROWS * (DV + 2) * 4;
+  const size_t smem = tiles > rows ? tiles : rows;
+  auto kern = multimap_decode_mma_kernel<D, DV, ROWS>;
+  if (smem > 48 * 1024) B200_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int passes = (H / G + ROWS - 1) / ROWS;
+  kern<<<dim3(tokens, G * passes, nsplit * M), 128, smem, st>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)ck, (const __nv_bfloat16*)cv, pos, slot,
+      table, max_blocks, (__nv_bfloat16*)out, ldo, part, H, G, M, bs_log2, scale, window, keep_first, nsplit, post, opt);
+  B200_LAUNCH_CHECK();
+  return 0;
+}
 // one warp per (token, head): merges the key ranges of every map, then the combination and the norm
 template <typename T>
 __global__ void __launch_bounds__(128)
@@ -774,6 +991,22 @@ B200_API int b200_multimap_attn_ex(const void* q, const void* ck, const void* cv
       const bool direct = M == 1 && nsplit == 1;
       if ((long long)G * passes > 65535 || nsplit * M > 65535) return B200_ERR_TOO_LARGE;
       if (!direct && !part) return B200_ERR_BAD_SHAPE;
+      if (dtype == B200_DT_BF16 && (D == 64 || D == 128) && (Dv == 64 || Dv == 128)) {
+        // the instances of the tensor-core kernel; pool rows are counted in 32 bits there, which 2^31 rows of 128 bytes never reach
+#define DM(DD, DVV)                                                                                                            \
+  (rep <= 8 ? launch_decode_mma<DD, DVV, 8>(q, ck, cv, pos, slot, table, max_blocks, out, ldo, part, tokens, H, G, M, bs_log2, scale, window, \
+                                            keep_first, nsplit, post, opt, st)                                                 \
+            : launch_decode_mma<DD, DVV, 16>(q, ck, cv, pos, slot, table, max_blocks, out, ldo, part, tokens, H, G, M, bs_log2, scale, window, \
+                                             keep_first, nsplit, post, opt, st))
+        const int rc = D == 64 ? (Dv == 64 ? DM(64, 64) : DM(64, 128)) : (Dv == 64 ? DM(128, 64) : DM(128, 128));
+#undef DM
+        if (rc) return rc;
+        if (!direct)
+          multimap_attn_merge_kernel<__nv_bfloat16><<<(unsigned)(((long long)tokens * H + 3) / 4), 128, 0, st>>>(
+              part, (__nv_bfloat16*)out, ldo, H, (long long)tokens * H, M, Dv, nsplit, combine, lambda, post, eps, opt);
+        B200_LAUNCH_CHECK();
+        return 0;
+      }
       dim3 grid(tokens, G * passes, nsplit * M);
       const size_t smem = (size_t)4 * HB * (Dv + 2) * sizeof(float);
 #define MMV2(T, HBV, VCV)                                                                                                    \

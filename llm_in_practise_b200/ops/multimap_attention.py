@@ -232,7 +232,11 @@ def multimap_attention(q: torch.Tensor, cache_k: torch.Tensor, cache_v: torch.Te
         if chunk > 0:
             seen = min(seen, chunk)
         nsplit = 1
-        if seen > 2 * _SPLIT_KEYS and T * G < 296:
+        if q.dtype == torch.bfloat16 and D in (64, 128) and Dv in (64, 128):
+            # the tensor-core decode kernel: as many CTAs as fit the 148 SMs at once, two each (64 sequences of 4000 keys, 4 groups: 87 us
+            # with 2 ranges, 90 with 3, 95 with 5); a range below 128 keys would not fill a CTA's four warps twice
+            nsplit = max(1, min(32, seen // 128, -(-296 // (T * G * M))))
+        elif seen > 2 * _SPLIT_KEYS and T * G < 296:
             nsplit = min(32, -(-seen // _SPLIT_KEYS), max(1, 592 // (T * G)))
         part = torch.empty(T * H * M * nsplit * (Dv + 2), dtype=torch.float32, device=q.device) if nsplit * M > 1 else None
         fn = nv.proto("b200_multimap_attn_ex", [vp, vp, vp, vp, vp, vp, i32, vp, i64, vp, i32, i32, i32, i32, i32, i32, i32, f32, i32, i32,
