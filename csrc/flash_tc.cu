@@ -1,47 +1,68 @@
-// K4 on the 5th-generation tensor cores: causal flash-attention forward with tcgen05.mma, S, P and O in TMEM, Q / K / V
-// tiles brought in by TMA straight out of the fused qkv projection (no head transposes, GQA by column offset), online
-// softmax by four warps whose threads each own ONE query row (TMEM lane = row, so row max and row sum need no shuffles).
+// K4 on the 5th-generation tensor cores: flash-attention forward with tcgen05.mma, S, P and O in TMEM, Q / K / V tiles brought in
+// by TMA in place (no head transposes, GQA by column offset), online softmax by four warps whose threads each own ONE query
+// row (TMEM lane = row, so row max and row sum need no shuffles).
 //
-//   CTA = (128-query tile, head, batch); 256 threads: warps 0-3 softmax, warp 4 TMA producer, warp 5 tcgen05 issuer (the
-//   whole warp runs the issue loop, elect.sync picks the lane: descriptors stay in uniform registers).
-//   TMEM (256 columns, two CTAs per SM): S(even j) [0, 64), S(odd j) [64, 128), O [128, 256).
-//   per 64-key block j:   S_j = Q K_j^T          (M 128 x N 64 x K 128, 8 UMMAs), issued one block AHEAD of the softmax
+//   CTA = 128 query rows; 256 threads: warps 0-3 softmax, warp 4 TMA producer, warp 5 tcgen05 issuer (the whole warp runs the
+//   issue loop, elect.sync picks the lane: descriptors stay in uniform registers).
+//   TMEM (256 columns, two CTAs per SM): S(even j) [0, 64), S(odd j) [64, 128), O [128, 128 + D).
+//   per 64-key block j:   S_j = Q K_j^T          (M 128 x N 64 x K D), issued one block AHEAD of the softmax
 //                         softmax warps: tcgen05.ld S_j (64 registers), running max, P = exp2(S c - m c) -> 16 bit,
 //                                        written over S_j in TMEM (tcgen05.st, two values per column)
-//                         O += P V_j             (M 128 x N 128 x K 64, 4 UMMAs, A operand from TMEM, V MN-major in place)
+//                         O += P V_j             (M 128 x N D x K 64, A operand from TMEM, V MN-major in place)
 //   O never leaves TMEM during the loop: the running max is only raised when a row's new max exceeds it by more than
 //   2^8 (exponents stay representable either way), and only then is O read, scaled and written back — a rare event
 //   after the first blocks of a row. The tensor pipe therefore sees QK(j+1), PV(j), QK(j+2), ... back to back while the
 //   softmax warps work on block j, and the second resident CTA fills the remaining bubbles.
-//   B200_FLASH_TC_PSMEM=1 selects the variant that hands P over through a 128B-swizzled shared-memory tile instead.
 //
-// Replaces the mma.sync kernel of flash_attn.cu for head_dim 128 forward passes (training forward, prefill); that
-// kernel stays for other head sizes, dropout and the backward pass. Reference call sites: SDPA behind
-// nn.MultiheadAttention (LLM_Distributed_Trainning/PyTorch/ddp_basics/ddp_gpt_wikitext2.py:89-96) and HF Qwen3 attention
-// (Fine-Tuning/qwen3-14b-qlora-dist-deepspeed.py:95-107).
+// One kernel, three ways to find the rows (MODE):
+//   dense    B sequences of S rows of the fused qkv projection; tile = 128 positions of one head
+//   varlen   sequences packed back to back (cu_seqlens on the device); tiles past a sequence's end leave at once
+//   paged    pieces of at most 64 rows (b200_multimap_attn_mma's tiles) over a paged cache. The two halves of the 128 rows are
+//            two heads of one KV group, so short pieces fill the tensor-core tile and their keys are fetched once for both;
+//            where a group's heads are odd in number they are two neighbouring tiles of one run and head. A 64-key block is
+//            one TMA box per page (page numbers read one block ahead), blocks that neither the window nor the kept first
+//            tokens reach are never fetched; sink, cap, chunks, gate as in multimap_attn_mma.cu
+// Rows of K and V past the last key of a sequence belong to somebody else (or were never written): their scores are masked, and
+// their V rows are zeroed in shared memory before the product, so that not even a NaN there reaches this sequence.
+//
+// Replaces the mma.sync kernels of flash_attn.cu (other head sizes, dropout and the backward pass stay there) and
+// multimap_attn_mma.cu (other sizes, two maps). Measured against them, bf16: six packed prompts of 77 - 2048 tokens, 32 / 8 heads
+// of 128: 237 -> 109 us; pages of 64, 16 / 4 heads of 128, pieces of 2048 and 700 (at 512) tokens beside two that decode:
+// 170 -> 57 us, window of 1024: 127 -> 44, chunks with capped scores: 194 -> 69, 8 / 8 heads: 101 -> 48; dense, 8 x 1000 tokens,
+// 16 / 8 heads of 64, forward and backward: 487 -> 457. Packed prompts too short to fill a tile take the same time in both.
+// Reference call sites: SDPA behind nn.MultiheadAttention (LLM_Distributed_Trainning/PyTorch/ddp_basics/ddp_gpt_wikitext2.py:89-96),
+// HF Qwen3 attention (Fine-Tuning/qwen3-14b-qlora-dist-deepspeed.py:95-107).
 #include "common.cuh"
 #include "tma_host.h"
 #include "../include/b200_ops.h"
 
-#include <stdio.h>
-#include <stdlib.h>
-
 namespace b200 {
 
-constexpr int kTcBM = 128, kTcBN = 64, kTcD = 128;
+constexpr int kTcBM = 128, kTcBN = 64;
 constexpr int kTcThreads = 256;
-constexpr uint32_t kTcQBytes = 32768, kTcKVStage = 16384, kTcPBytes = 16384;
-constexpr uint32_t kTcSmemQ = 0, kTcSmemK = 32768, kTcSmemV = 65536, kTcSmemP = 98304, kTcSmemBar = 114688;
-constexpr uint32_t kTcSmemBytes = kTcSmemBar + 256;
 constexpr uint32_t kTcTmemCols = 256, kTcTmemO = 128;
+constexpr float kTcLog2e = 1.4426950408889634f;
+enum { kTcDense = 0, kTcVarlen = 1, kTcPaged = 2 };
+
+// shared memory: Q [128 rows] as D / 64 swizzled halves of 16 KiB, two stages of K and of V [64 rows] as halves of 8 KiB, barriers
+template <int D> struct TcSmem {
+  static constexpr uint32_t kHalves = D / 64, kStage = 8192 * kHalves;
+  static constexpr uint32_t kQ = 0, kK = 16384 * kHalves, kV = kK + 2 * kStage, kBar = kV + 2 * kStage, kBytes = kBar + 128;
+};
 
 struct FlashTcParams {
   void* out;
   float* lse;         // [B, H, S] natural-log log-sum-exp of the scaled scores (what the backward kernel reads), may be null
-  int B, S, H, Hkv;
+  const int* cu;      // varlen: sequence b is rows [cu[b], cu[b + 1])
+  int S, H, Hkv;
   long long out_rs;   // elements between output rows
-  float scale_log2;   // softmax scale * log2(e)
-  int causal, is_bf16;
+  float scale_log2;   // softmax scale * log2(e) (capped: cap * log2(e))
+  int causal;
+  // paged
+  const int *tiles, *tile_of, *table;   // tile_of (odd head groups): (run, place in the run, tiles of the run, its first tile)
+  int max_blocks, bs_log2, window, keep_first;
+  float cin, post;    // capped: scores become tanh(cin q . k) before they are scaled
+  b200_attn_opts opt;
 };
 
 __device__ __forceinline__ float ex2f(float x) {
@@ -50,18 +71,8 @@ __device__ __forceinline__ float ex2f(float x) {
   return y;
 }
 
-// D[tmem] (+)= A[tmem] * B[smem desc]: the A operand (P, 16-bit, row = lane, two k values per column) comes from TMEM.
-__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// The same instructions issued from CONVERGED warp code (every lane of the issuing warp runs the loop, elect.sync picks the
-// lane): descriptors stay in uniform registers. From inside `if (lane == 0)` each UTCHMMA costs two R2UR moves and a
+// tcgen05.mma issued from CONVERGED warp code (every lane of the issuing warp runs the loop, elect.sync picks the lane):
+// descriptors stay in uniform registers. From inside `if (lane == 0)` each UTCHMMA costs two R2UR moves and a
 // divergence loop — more cycles than a 128 x 64 x 16 product spends on the tensor pipe.
 __device__ __forceinline__ void umma_f16_w(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -72,6 +83,7 @@ __device__ __forceinline__ void umma_f16_w(uint32_t tmem_d, uint64_t adesc, uint
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// the A operand (P, 16-bit, row = lane, two k values per column) comes from TMEM
 __device__ __forceinline__ void umma_f16_ts_w(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
@@ -95,35 +107,76 @@ __device__ __forceinline__ uint32_t pack16(float a, float b) {
   return *reinterpret_cast<const uint32_t*>(&hh);
 }
 
-// PT: P goes to the PV product through TMEM (over S); otherwise through the shared-memory tile at kTcSmemP.
-template <bool BF16, bool PT>
+// tanh for capped scores: by its power series where every score of the warp is small (|x| <= 1/4: the next term is below 3e-9 of x),
+// else 1 - 2 / (1 + e^(2x)) on the hardware's exponential (a few 1e-7 absolute)
+__device__ __forceinline__ float tanh_small(float x) {
+  const float y = x * x;
+  return x * fmaf(y, fmaf(y, fmaf(y, fmaf(y, 62.f / 2835.f, -17.f / 315.f), 2.f / 15.f), -1.f / 3.f), 1.f);
+}
+__device__ __forceinline__ float tanh_any(float x) { return 1.f - __fdividef(2.f, 1.f + ex2f(x * 2.8853900817779268f)); }
+
+template <int MODE, int D, bool BF16, bool CAP>
 __global__ void __launch_bounds__(kTcThreads, 2)
-flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm, const FlashTcParams p) {
+flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
+                    const FlashTcParams p) {
+  using L = TcSmem<D>;
+  constexpr int kHalves = L::kHalves;
   extern __shared__ __align__(1024) uint8_t smem_tc[];
   const uint32_t sbase = smem_u32(smem_tc);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // heavy (late) query tiles first: under the causal mask tile t has t + 1 times the work of tile 0
-  const int qt = (int)gridDim.x - 1 - (int)blockIdx.x;
-  const int h = blockIdx.y, b = blockIdx.z;
-  const int S = p.S;
-  const int q0 = qt * kTcBM;
-  const int hk = h / (p.H / p.Hkv);
-  const int qcol = h * kTcD, kcol = (p.H + hk) * kTcD, vcol = (p.H + p.Hkv + hk) * kTcD;
-  const int row_base = b * S;
-  const int kv_end = p.causal ? min(S, q0 + kTcBM) : S;
-  const int nblk = (kv_end + kTcBN - 1) / kTcBN;
 
-  const uint32_t bar = sbase + kTcSmemBar;
-  const uint32_t q_full = bar, kv_full0 = bar + 8, kv_empty0 = bar + 24, s_full0 = bar + 40, s_free0 = bar + 56,
-                 p_full = bar + 72, o_done = bar + 80, tmem_slot = bar + 96;
-  if (threadIdx.x == 0) {
-    if (sbase & 1023u) { printf("flash_tc: shared memory base is not 1024-byte aligned\n"); __trap(); }
-    tma_prefetch_desc(&tm);
-    mbar_init(q_full, 1);
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(kv_full0 + 8 * s, 1); mbar_init(kv_empty0 + 8 * s, 1);
-      mbar_init(s_full0 + 8 * s, 1); mbar_init(s_free0 + 8 * s, 4);
+  // ---- where this CTA's rows and keys are ----
+  int h = blockIdx.y, hk, row_base, q0, limit;            // limit: keys of the sequence; q0: position of row 0; row_base: its row 0
+  int nit, nA = 0, bB = 0;                                // key blocks: [0, nA), then bB, bB + 1, ...
+  int nrows = kTcBM, low_max = 0, keepW = 0;
+  bool solo = false;                                      // paged: the second half of the rows is the same head's next tile
+  const int* trow = nullptr;
+  auto low_of = [&](int pos) {
+    return p.opt.chunk > 0 ? pos / p.opt.chunk * p.opt.chunk : (p.window > 0 ? max(0, pos + 1 - p.window) : 0);
+  };
+  if (MODE == kTcPaged) {
+    const int tile = (int)gridDim.x - 1 - (int)blockIdx.x, rep = p.H / p.Hkv;
+    const int* tl = p.tiles + 4 * tile;
+    row_base = tl[0]; nrows = tl[1]; q0 = tl[2];
+    solo = rep & 1;
+    if (solo) {
+      const int place = p.tile_of[4 * tile + 1];
+      if (place & 1) return;                              // the tile before it takes both
+      if (place + 1 < p.tile_of[4 * tile + 2]) nrows += tl[5];
+      hk = h / rep;
+    } else {
+      hk = h / (rep / 2);
+      h *= 2;
     }
+    trow = p.table + (long long)tl[3] * p.max_blocks;
+    limit = q0 + nrows;
+    const int lo0 = low_of(q0);
+    keepW = p.window > 0 ? max(p.keep_first, 0) : 0;
+    nA = (min(keepW, lo0) + kTcBN - 1) / kTcBN;
+    bB = max(lo0 / kTcBN, nA);
+    nit = nA + (limit + kTcBN - 1) / kTcBN - bB;
+    low_max = low_of(q0 + (solo ? kTcBM : kTcBN) - 1);
+  } else {
+    // heavy (late) query tiles first: under the causal mask tile t has t + 1 times the work of tile 0
+    const int qt = (int)gridDim.x - 1 - (int)blockIdx.x, b = blockIdx.z;
+    hk = h / (p.H / p.Hkv);
+    row_base = MODE == kTcVarlen ? p.cu[b] : b * p.S;
+    limit = MODE == kTcVarlen ? p.cu[b + 1] - row_base : p.S;
+    q0 = qt * kTcBM;
+    if (MODE == kTcVarlen && q0 >= limit) return;
+    const int kv_end = p.causal ? min(limit, q0 + kTcBM) : limit;
+    nit = (kv_end + kTcBN - 1) / kTcBN;
+  }
+  auto block_of = [&](int it) { return MODE == kTcPaged ? (it < nA ? it : bB + (it - nA)) : it; };
+
+  const uint32_t bar = sbase + L::kBar;
+  const uint32_t q_full = bar, kv_full0 = bar + 8, kv_empty0 = bar + 24, s_full0 = bar + 40, p_full = bar + 56, o_done = bar + 64,
+                 tmem_slot = bar + 80;
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&tq);
+    if (MODE == kTcPaged) { tma_prefetch_desc(&tk); tma_prefetch_desc(&tv); }
+    mbar_init(q_full, 1);
+    for (int s = 0; s < 2; ++s) { mbar_init(kv_full0 + 8 * s, 1); mbar_init(kv_empty0 + 8 * s, 1); mbar_init(s_full0 + 8 * s, 1); }
     mbar_init(p_full, 4);
     mbar_init(o_done, 1);
     fence_mbar_init();
@@ -136,20 +189,53 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm, const FlashTcParams 
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
 
   if (warp == 4) {
+    // ---- Q: D / 64 column halves, each 128 rows (two 64-row boxes stacked = one K-major 128B-swizzled tile) ----
     if (lane == 0) {
-      // ---- Q: two 64-column halves, each 128 rows (two 64-row boxes stacked = one K-major 128B-swizzled tile) ----
-      mbar_arrive_expect_tx(q_full, kTcQBytes);
-      for (int half = 0; half < 2; ++half)
-        for (int rb = 0; rb < 2; ++rb)
-          tma_load_2d(sbase + kTcSmemQ + half * 16384 + rb * 8192, &tm, q_full, qcol + half * 64, row_base + q0 + rb * 64);
-      for (int j = 0; j < nblk; ++j) {
+      mbar_arrive_expect_tx(q_full, 16384 * kHalves);
+      for (int half = 0; half < kHalves; ++half)
+        for (int rb = 0; rb < 2; ++rb) {
+          const int col = (MODE == kTcPaged && !solo ? h + rb : h) * D + half * 64;
+          const int row = MODE == kTcPaged ? row_base + (solo ? rb * 64 : 0) : row_base + q0 + rb * 64;
+          tma_load_2d(sbase + L::kQ + half * 16384 + rb * 8192, &tq, q_full, col, row);
+        }
+    }
+    if (MODE == kTcPaged) {
+      // a block is `pieces` boxes of `psize` rows; lane i looks up and fetches piece i, its page number one block ahead
+      const int psl = min(p.bs_log2, 6), psize = 1 << psl, pieces = kTcBN >> psl;
+      auto row_of = [&](int it) {
+        const int kp = block_of(it) * kTcBN + lane * psize;
+        return (it < nit && lane < pieces && kp < limit)
+                   ? ((trow[kp >> p.bs_log2] * p.Hkv + hk) << p.bs_log2) + (kp & ((1 << p.bs_log2) - 1)) : -1;
+      };
+      int row = row_of(0);
+      for (int it = 0; it < nit; ++it) {
+        const int s = it & 1;
+        const int n = min(pieces, (limit - block_of(it) * kTcBN + psize - 1) >> psl);
+        if (lane == 0) {
+          mbar_wait(kv_empty0 + 8 * s, (((uint32_t)it >> 1) & 1u) ^ 1u);
+          mbar_arrive_expect_tx(kv_full0 + 8 * s, (uint32_t)(n * psize * 128 * 2 * kHalves));
+        }
+        __syncwarp();
+        if (row >= 0) {
+#pragma unroll
+          for (int half = 0; half < kHalves; ++half) {
+            const uint32_t dst = sbase + s * L::kStage + half * 8192 + lane * psize * 128;
+            tma_load_2d(dst + L::kK, &tk, kv_full0 + 8 * s, half * 64, row);
+            tma_load_2d(dst + L::kV, &tv, kv_full0 + 8 * s, half * 64, row);
+          }
+        }
+        row = row_of(it + 1);
+      }
+    } else if (lane == 0) {
+      const int kcol = (p.H + hk) * D, vcol = (p.H + p.Hkv + hk) * D;
+      for (int j = 0; j < nit; ++j) {
         const int s = j & 1;
         mbar_wait(kv_empty0 + 8 * s, (((uint32_t)j >> 1) & 1u) ^ 1u);
-        mbar_arrive_expect_tx(kv_full0 + 8 * s, 2 * kTcKVStage);
+        mbar_arrive_expect_tx(kv_full0 + 8 * s, 2 * L::kStage);
         const int r = row_base + j * kTcBN;
-        for (int half = 0; half < 2; ++half) {
-          tma_load_2d(sbase + kTcSmemK + s * kTcKVStage + half * 8192, &tm, kv_full0 + 8 * s, kcol + half * 64, r);
-          tma_load_2d(sbase + kTcSmemV + s * kTcKVStage + half * 8192, &tm, kv_full0 + 8 * s, vcol + half * 64, r);
+        for (int half = 0; half < kHalves; ++half) {
+          tma_load_2d(sbase + L::kK + s * L::kStage + half * 8192, &tk, kv_full0 + 8 * s, kcol + half * 64, r);
+          tma_load_2d(sbase + L::kV + s * L::kStage + half * 8192, &tv, kv_full0 + 8 * s, vcol + half * 64, r);
         }
       }
     }
@@ -160,14 +246,14 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm, const FlashTcParams 
       constexpr uint32_t kLoK = (16u >> 4) << 16, kLoMN = (8192u >> 4) << 16;
       auto desc = [](uint32_t lo) { return ((uint64_t)kHi << 32) | (uint64_t)lo; };
       const uint32_t idesc_qk = make_idesc_f16(kTcBM, kTcBN, BF16, false, false);
-      const uint32_t idesc_pv = make_idesc_f16(kTcBM, kTcD, BF16, false, true);
+      const uint32_t idesc_pv = make_idesc_f16(kTcBM, D, BF16, false, true);
       const uint32_t tS = tmem_base, tO = tmem_base + kTcTmemO;
-      const uint32_t qlo = ((sbase + kTcSmemQ) >> 4) | kLoK, plo = ((sbase + kTcSmemP) >> 4) | kLoK;
+      const uint32_t qlo = ((sbase + L::kQ) >> 4) | kLoK;
       auto issue_qk = [&](int j) {
         const int s = j & 1;
-        const uint32_t klo = ((sbase + kTcSmemK + s * kTcKVStage) >> 4) | kLoK;
+        const uint32_t klo = ((sbase + L::kK + s * L::kStage) >> 4) | kLoK;
 #pragma unroll
-        for (int half = 0; half < 2; ++half)
+        for (int half = 0; half < kHalves; ++half)
 #pragma unroll
           for (int ks = 0; ks < 4; ++ks)
             umma_f16_w(tS + s * kTcBN, desc(qlo + half * (16384u >> 4) + ks * 2u), desc(klo + half * (8192u >> 4) + ks * 2u),
@@ -178,24 +264,20 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm, const FlashTcParams 
       mbar_wait_spin(kv_full0, 0);
       tc_fence_after();
       issue_qk(0);
-      for (int j = 0; j < nblk; ++j) {
+      for (int j = 0; j < nit; ++j) {
         const int s = j & 1;
-        if (j + 1 < nblk) {
+        if (j + 1 < nit) {
           mbar_wait_spin(kv_full0 + 8 * ((j + 1) & 1), ((uint32_t)(j + 1) >> 1) & 1u);
-          // S buffer (j+1)&1 last held block j-1. PT: P(j-1) sat in it and PV(j-1) was issued before this UMMA, the pipe
-          // runs in order. Otherwise: the softmax warps have pulled S(j-1) into registers.
-          if (!PT && j >= 1) mbar_wait_spin(s_free0 + 8 * ((j + 1) & 1), ((uint32_t)(j - 1) >> 1) & 1u);
+          // S buffer (j+1)&1 last held block j-1: P(j-1) sat in it and PV(j-1) was issued before this UMMA, the pipe runs in order
           tc_fence_after();
           issue_qk(j + 1);
         }
         mbar_wait_spin(p_full, (uint32_t)j & 1u);               // P(j) is written (and O rescaled where a row needed it)
         tc_fence_after();
-        const uint32_t vlo = ((sbase + kTcSmemV + s * kTcKVStage) >> 4) | kLoMN;
+        const uint32_t vlo = ((sbase + L::kV + s * L::kStage) >> 4) | kLoMN;
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks) {
-          if (PT) umma_f16_ts_w(tO, tS + s * kTcBN + ks * 8, desc(vlo + ks * (2048u >> 4)), idesc_pv, (j | ks) ? 1u : 0u);
-          else umma_f16_w(tO, desc(plo + ks * 2u), desc(vlo + ks * (2048u >> 4)), idesc_pv, (j | ks) ? 1u : 0u);
-        }
+        for (int ks = 0; ks < 4; ++ks)
+          umma_f16_ts_w(tO, tS + s * kTcBN + ks * 8, desc(vlo + ks * (2048u >> 4)), idesc_pv, (j | ks) ? 1u : 0u);
         umma_commit_w(o_done);
         umma_commit_w(kv_empty0 + 8 * s);
       }
@@ -204,31 +286,47 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm, const FlashTcParams 
     // ================= softmax: thread = query row =================
     const int q = warp;                             // TMEM lane quarter this warp may touch (warp index mod 4)
     const int r = q * 32 + lane;                    // row inside the tile
-    const int grow = q0 + r;                        // position in the sequence
+    const int rr = MODE == kTcPaged && !solo ? (r & 63) : r;      // two heads: rows 64 .. 127 are the second one's
+    const int grow = q0 + rr;                       // position in the sequence
     const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
     const uint32_t tS = tmem_base + lane_addr, tO = tmem_base + lane_addr + kTcTmemO;
     const float sl = p.scale_log2;
-    const int lim = p.causal ? min(grow, S - 1) : S - 1;      // last visible key of this row
+    const int lim = (MODE == kTcPaged || p.causal) ? min(grow, limit - 1) : limit - 1;      // last visible key of this row
+    const int low = MODE == kTcPaged ? low_of(grow) : 0;                                    // first one, besides kept tokens
     float m_ref = -INFINITY, l = 0.f;
     uint32_t v[64];
-    for (int j = 0; j < nblk; ++j) {
-      const int kv0 = j * kTcBN, sb = j & 1;
-      const bool need_mask = (p.causal && kv0 + kTcBN - 1 > q0) || (kv0 + kTcBN > S);
+    for (int j = 0; j < nit; ++j) {
+      const int kv0 = block_of(j) * kTcBN, sb = j & 1;
+      const bool need_mask = MODE == kTcPaged ? (kv0 + kTcBN - 1 > q0 || (kv0 < low_max && kv0 + kTcBN - 1 >= keepW))
+                                              : ((p.causal && kv0 + kTcBN - 1 > q0) || (kv0 + kTcBN > limit));
       mbar_wait_warp(s_full0 + 8 * sb, ((uint32_t)j >> 1) & 1u);
       tc_fence_after();
       tmem_ld_32x32(tS + sb * kTcBN, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
       tmem_ld_32x32(tS + sb * kTcBN + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[32]));
       tmem_ld_wait();
-      if (!PT) {
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(s_free0 + 8 * sb);
+      if (CAP) {
+        float big = 0.f;
+#pragma unroll
+        for (int i = 0; i < 64; ++i) {
+          const float x = __uint_as_float(v[i]) * p.cin;
+          big = fmaxf(big, fabsf(x));
+          v[i] = __float_as_uint(x);
+        }
+        if (__any_sync(0xffffffffu, big > 0.25f)) {
+#pragma unroll
+          for (int i = 0; i < 64; ++i) v[i] = __float_as_uint(tanh_any(__uint_as_float(v[i])));
+        } else {                                          // small scores: the series takes fewer cycles than two special functions
+#pragma unroll
+          for (int i = 0; i < 64; ++i) v[i] = __float_as_uint(tanh_small(__uint_as_float(v[i])));
+        }
       }
       float mx = -INFINITY;
       if (need_mask) {
 #pragma unroll
-        for (int i = 0; i < 64; ++i)
-          if (kv0 + i > lim) v[i] = 0xff800000u;    // -inf
+        for (int i = 0; i < 64; ++i) {
+          const int kp = kv0 + i;
+          if (MODE == kTcPaged ? (kp > lim || (kp < low && kp >= keepW)) : kp > lim) v[i] = 0xff800000u;    // -inf
+        }
       }
 #pragma unroll
       for (int i = 0; i < 64; ++i) mx = fmaxf(mx, __uint_as_float(v[i]));
@@ -239,19 +337,18 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm, const FlashTcParams 
       if (raise) { alpha = ex2f(m_ref - m_new); m_ref = m_new; }
       const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
       const bool any_raise = j > 0 && __any_sync(0xffffffffu, raise);
-      // PV(j-1) complete: O is stable (and the shared P tile is free). A parity wait tells phase c from c + 1, not from
-      // c + 2, and S(j) only proves PV(j-2) complete: a warp that skipped this wait for a while is still safe here (o_done has
-      // completed j - 1 or j phases), but it must not reach the wait after the loop two phases behind, where the parity of
-      // "PV(nblk-3) done" reads as "PV(nblk-1) done" and O would be taken before the last two products. So the last block
-      // always waits.
-      if (j > 0 && (!PT || any_raise || j == nblk - 1)) {
+      // PV(j-1) complete: O is stable. A parity wait tells phase c from c + 1, not from c + 2, and S(j) only proves PV(j-2)
+      // complete: a warp that skipped this wait for a while is still safe here (o_done has completed j - 1 or j phases), but
+      // it must not reach the wait after the loop two phases behind, where the parity of "PV(nit-3) done" reads as
+      // "PV(nit-1) done" and O would be taken before the last two products. So the last block always waits.
+      if (j > 0 && (any_raise || j == nit - 1)) {
         mbar_wait_warp(o_done, (uint32_t)(j - 1) & 1u);
         tc_fence_after();
       }
       if (any_raise) {
         uint32_t o[32];
 #pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < D / 32; ++c) {
           tmem_ld_32x32(tO + c * 32, o);
           tmem_ld_wait();
 #pragma unroll
@@ -262,47 +359,44 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm, const FlashTcParams 
       l *= alpha;
       float rs0 = 0.f, rs1 = 0.f;
       const float nm = -m_use;
-      if (PT) {
-        uint32_t w[32];
+      uint32_t w[32];
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const float p0 = ex2f(fmaf(__uint_as_float(v[2 * i]), sl, nm)), p1 = ex2f(fmaf(__uint_as_float(v[2 * i + 1]), sl, nm));
-          rs0 += p0; rs1 += p1;
-          w[i] = pack16<BF16>(p0, p1);
-        }
-        tmem_st_32x32(tS + sb * kTcBN, w);
-        tmem_st_wait();
-        tc_fence_before();
-      } else {
-        const uint32_t prow = sbase + kTcSmemP + (uint32_t)r * 128u;
-#pragma unroll
-        for (int g = 0; g < 8; ++g) {
-          uint32_t o[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int i0 = g * 8 + e * 2;
-            const float p0 = ex2f(fmaf(__uint_as_float(v[i0]), sl, nm)), p1 = ex2f(fmaf(__uint_as_float(v[i0 + 1]), sl, nm));
-            rs0 += p0; rs1 += p1;
-            o[e] = pack16<BF16>(p0, p1);
-          }
-          asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(prow + (((uint32_t)g ^ ((uint32_t)r & 7u)) << 4)),
-                       "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
-        }
-        if (any_raise) tmem_st_wait();
-        tc_fence_before();
-        fence_proxy_async_smem();                        // generic-proxy stores -> visible to tcgen05.mma
+      for (int i = 0; i < 32; ++i) {
+        const float p0 = ex2f(fmaf(__uint_as_float(v[2 * i]), sl, nm)), p1 = ex2f(fmaf(__uint_as_float(v[2 * i + 1]), sl, nm));
+        rs0 += p0; rs1 += p1;
+        w[i] = pack16<BF16>(p0, p1);
       }
+      tmem_st_32x32(tS + sb * kTcBN, w);
+      if (kv0 + kTcBN > limit) {                          // the sequence's last block: V rows that are not its own become zeros
+        mbar_wait_warp(kv_full0 + 8 * sb, ((uint32_t)j >> 1) & 1u);
+        for (int i = threadIdx.x; i < (kv0 + kTcBN - limit) * 8 * kHalves; i += 128) {
+          const int row = limit - kv0 + i / (8 * kHalves), c = i % (8 * kHalves);
+          asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(sbase + L::kV + sb * L::kStage + (c >> 3) * 8192 + row * 128 + (c & 7) * 16),
+                       "r"(0) : "memory");
+        }
+        fence_proxy_async_smem();                         // generic-proxy stores -> visible to tcgen05.mma
+      }
+      tmem_st_wait();
+      tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full);
       l += rs0 + rs1;
     }
     // ---- finish: O / l -> 16 bit through shared memory (the Q tile is dead: every QK product has completed) ----
-    mbar_wait_warp(o_done, (uint32_t)(nblk - 1) & 1u);
+    mbar_wait_warp(o_done, (uint32_t)(nit - 1) & 1u);
     tc_fence_after();
-    const float inv = l > 0.f ? 1.f / l : 0.f;
-    const uint32_t orow = sbase + kTcSmemQ + (uint32_t)r * 256u;
+    const int head = MODE == kTcPaged && !solo ? h + (r >> 6) : h;
+    const bool live = MODE == kTcPaged ? rr < nrows : grow < limit;
+    if (MODE == kTcPaged && p.opt.sink) l += ex2f(p.opt.sink[head] * kTcLog2e - m_ref);   // no key: not scaled, not capped
+    float inv = l > 0.f ? 1.f / l : 0.f;
+    if (MODE == kTcPaged) {
+      inv *= p.post;
+      if (p.opt.gate && live) inv /= 1.f + expf(-p.opt.gate[(long long)(row_base + rr) * p.opt.ld_gate + head]);
+    }
+    constexpr int CH = D / 8;                             // 16-byte chunks of an output row
+    const uint32_t orow = sbase + L::kQ + (uint32_t)r * (D * 2u);
 #pragma unroll 1
-    for (int c = 0; c < 4; ++c) {
+    for (int c = 0; c < D / 32; ++c) {
       uint32_t o[32];
       tmem_ld_32x32(tO + c * 32, o);
       tmem_ld_wait();
@@ -313,22 +407,26 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm, const FlashTcParams 
         for (int e = 0; e < 4; ++e)
           w[e] = pack16<BF16>(__uint_as_float(o[g * 8 + e * 2]) * inv, __uint_as_float(o[g * 8 + e * 2 + 1]) * inv);
         const uint32_t chunk = (uint32_t)(c * 4 + g);
-        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(orow + ((chunk ^ ((uint32_t)r & 15u)) << 4)), "r"(w[0]),
+        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(orow + ((chunk ^ ((uint32_t)r & (CH - 1u))) << 4)), "r"(w[0]),
                      "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
       }
     }
-    if (p.lse && grow < S) p.lse[((long long)b * p.H + h) * S + grow] = m_ref * 0.6931471805599453f + __logf(l);
+    if (MODE == kTcDense && p.lse && live)
+      p.lse[((long long)blockIdx.z * p.H + h) * p.S + grow] = m_ref * 0.6931471805599453f + __logf(l);
     __syncwarp();
-    // each warp copies ITS 32 rows out (written by its own lanes): 16 lanes cover the 256 bytes of a row
-    uint16_t* obase = reinterpret_cast<uint16_t*>(p.out) + (long long)h * kTcD;
+    // each warp copies ITS 32 rows out (written by its own lanes): CH lanes cover the bytes of a row
+    uint16_t* obase = reinterpret_cast<uint16_t*>(p.out);
 #pragma unroll 4
-    for (int it = 0; it < 16; ++it) {
-      const int rr = q * 32 + it * 2 + (lane >> 4), chunk = lane & 15;
+    for (int it = 0; it < CH; ++it) {
+      const int row = q * 32 + it * (32 / CH) + lane / CH, chunk = lane % CH;
       uint32_t w0, w1, w2, w3;
       asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w0), "=r"(w1), "=r"(w2), "=r"(w3)
-                   : "r"(sbase + kTcSmemQ + (uint32_t)rr * 256u + (((uint32_t)chunk ^ ((uint32_t)rr & 15u)) << 4)));
-      if (q0 + rr < S)
-        *reinterpret_cast<uint4*>(obase + (long long)(row_base + q0 + rr) * p.out_rs + chunk * 8) = make_uint4(w0, w1, w2, w3);
+                   : "r"(sbase + L::kQ + (uint32_t)row * (D * 2u) + (((uint32_t)chunk ^ ((uint32_t)row & (CH - 1u))) << 4)));
+      const int rw = MODE == kTcPaged && !solo ? (row & 63) : row;
+      const bool keep = MODE == kTcPaged ? rw < nrows : q0 + rw < limit;
+      const long long at = (long long)(MODE == kTcPaged ? row_base + rw : row_base + q0 + rw) * p.out_rs +
+                           (MODE == kTcPaged && !solo ? h + (row >> 6) : h) * D + chunk * 8;
+      if (keep) *reinterpret_cast<uint4*>(obase + at) = make_uint4(w0, w1, w2, w3);
     }
   }
   tc_fence_before();
@@ -339,48 +437,114 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm, const FlashTcParams 
   }
 }
 
+template <int MODE, int D, bool BF16, bool CAP>
+static int launch_tc(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FlashTcParams& p, dim3 grid, cudaStream_t st) {
+  auto kern = flash_fwd_tc_kernel<MODE, D, BF16, CAP>;
+  static bool attr = false;
+  if (!attr) {
+    B200_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcSmem<D>::kBytes));
+    attr = true;
+  }
+  kern<<<grid, kTcThreads, TcSmem<D>::kBytes, st>>>(tq, tk, tv, p);
+  B200_LAUNCH_CHECK();
+  return 0;
+}
+
+// rows [rows, cols] of 16-bit values, boxes of 64 columns
+static int rows_map(CUtensorMap* tm, const void* base, uint64_t cols, uint64_t rows, uint32_t box_rows) {
+  uint64_t dims[2] = {cols, rows}, str[1] = {cols * 2};
+  uint32_t box[2] = {64, box_rows};
+  return make_tensor_map(tm, base, 2, 2, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+// autograd's backward threads have no current driver context until a runtime call binds the primary one; the tensor-map encode
+// is a driver entry point
+static int bind_device() {
+  int dev = 0;
+  B200_CHECK(cudaGetDevice(&dev));
+  B200_CHECK(cudaSetDevice(dev));
+  return 0;
+}
+
+template <int MODE>
+static int fused_qkv(const void* qkv, long long rows, FlashTcParams& p, int D, int dtype, dim3 grid, void* stream) {
+  if (int rc = bind_device()) return rc;
+  CUtensorMap tm;
+  if (int rc = rows_map(&tm, qkv, (uint64_t)(p.H + 2 * p.Hkv) * D, (uint64_t)rows, 64)) return rc;
+  cudaStream_t st = (cudaStream_t)stream;
+  const bool bf = dtype == B200_DT_BF16;
+  if (D == 64) return bf ? launch_tc<MODE, 64, true, false>(tm, tm, tm, p, grid, st) : launch_tc<MODE, 64, false, false>(tm, tm, tm, p, grid, st);
+  return bf ? launch_tc<MODE, 128, true, false>(tm, tm, tm, p, grid, st) : launch_tc<MODE, 128, false, false>(tm, tm, tm, p, grid, st);
+}
+
 }  // namespace b200
 using namespace b200;
 
-// Causal (or full) attention forward on the tcgen05 path. head_dim 128, 16-bit, no dropout. qkv [B*S, (H + 2 Hkv) * 128],
-// out [B*S, H * 128], lse [B, H, S] or NULL. Returns B200_ERR_UNSUPPORTED for shapes it does not cover (the caller then
+static int tc_check(const void* qkv, const void* out, int B, int S, int H, int Hkv, int D, int dtype) {
+  if ((D != 64 && D != 128) || (dtype != B200_DT_BF16 && dtype != B200_DT_FP16)) return B200_ERR_UNSUPPORTED;
+  if (B < 1 || S < 1 || H < 1 || Hkv < 1 || H % Hkv) return B200_ERR_BAD_SHAPE;
+  if (H > 65535 || B > 65535) return B200_ERR_UNSUPPORTED;
+  if ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(out)) & 15) return B200_ERR_BAD_ALIGN;
+  return 0;
+}
+
+// Causal (or full) attention forward on the tcgen05 path. head_dim 64 or 128, 16-bit, no dropout. qkv [B*S, (H + 2 Hkv) * D],
+// out [B*S, H * D], lse [B, H, S] or NULL. Returns B200_ERR_UNSUPPORTED for shapes it does not cover (the caller then
 // takes b200_flash_attn_fwd).
 B200_API int b200_flash_attn_fwd_tc(const void* qkv, void* out, float* lse, int B, int S, int H, int Hkv, int D, int causal,
                                     float scale, int dtype, void* stream) {
-  if (D != kTcD || (dtype != B200_DT_BF16 && dtype != B200_DT_FP16)) return B200_ERR_UNSUPPORTED;
-  if (B < 1 || S < 1 || H < 1 || Hkv < 1 || H % Hkv) return B200_ERR_BAD_SHAPE;
-  if ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(out)) & 15) return B200_ERR_BAD_ALIGN;
-  // autograd's backward threads have no current driver context until a runtime call binds the primary one; the tensor-map
-  // encode below is a driver entry point
-  { int dev = 0; B200_CHECK(cudaGetDevice(&dev)); B200_CHECK(cudaSetDevice(dev)); }
-  const long long W = (long long)(H + 2 * Hkv) * kTcD;
-  CUtensorMap tm;
-  {
-    uint64_t dims[2] = {(uint64_t)W, (uint64_t)B * (uint64_t)S}, str[1] = {(uint64_t)W * 2};
-    uint32_t box[2] = {64, 64};
-    if (int rc = make_tensor_map(&tm, qkv, 2, 2, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
-  }
+  if (int rc = tc_check(qkv, out, B, S, H, Hkv, D, dtype)) return rc;
   FlashTcParams p = {};
-  p.out = out; p.lse = lse; p.B = B; p.S = S; p.H = H; p.Hkv = Hkv; p.out_rs = (long long)H * kTcD;
-  p.scale_log2 = scale * 1.4426950408889634f; p.causal = causal; p.is_bf16 = dtype == B200_DT_BF16;
-  static const bool psmem = [] { const char* e = getenv("B200_FLASH_TC_PSMEM"); return e && atoi(e) != 0; }();
-  static bool attr = false;
-  if (!attr) {
-    B200_CHECK(cudaFuncSetAttribute(flash_fwd_tc_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmemBytes));
-    B200_CHECK(cudaFuncSetAttribute(flash_fwd_tc_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmemBytes));
-    B200_CHECK(cudaFuncSetAttribute(flash_fwd_tc_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmemBytes));
-    B200_CHECK(cudaFuncSetAttribute(flash_fwd_tc_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmemBytes));
-    attr = true;
-  }
-  dim3 grid((S + kTcBM - 1) / kTcBM, H, B);
+  p.out = out; p.lse = lse; p.S = S; p.H = H; p.Hkv = Hkv; p.out_rs = (long long)H * D;
+  p.scale_log2 = scale * kTcLog2e; p.causal = causal;
+  return fused_qkv<kTcDense>(qkv, (long long)B * S, p, D, dtype, dim3((S + kTcBM - 1) / kTcBM, H, B), stream);
+}
+
+// The packed form (see b200_flash_attn_varlen_fwd): `tokens` rows hold n_seqs sequences back to back, the longest of max_seqlen rows.
+B200_API int b200_flash_attn_varlen_fwd_tc(const void* qkv, void* out, const int* cu_seqlens, long long tokens, int n_seqs, int max_seqlen,
+                                           int H, int Hkv, int D, int causal, float scale, int dtype, void* stream) {
+  if (int rc = tc_check(qkv, out, n_seqs, max_seqlen, H, Hkv, D, dtype)) return rc;
+  if (!cu_seqlens || tokens < 1) return B200_ERR_BAD_SHAPE;
+  FlashTcParams p = {};
+  p.out = out; p.cu = cu_seqlens; p.S = max_seqlen; p.H = H; p.Hkv = Hkv; p.out_rs = (long long)H * D;
+  p.scale_log2 = scale * kTcLog2e; p.causal = causal;
+  return fused_qkv<kTcVarlen>(qkv, tokens, p, D, dtype, dim3((max_seqlen + kTcBM - 1) / kTcBM, H, n_seqs), stream);
+}
+
+// Prompt pieces over a paged cache, one map, key and value rows of one size (arguments as in b200_multimap_attn_mma_ex; `tokens`: rows
+// of q, `pool_rows`: rows of the pools, blocks * G * block_size; `tile_of` as described above, wanted where H / G is odd).
+// B200_ERR_UNSUPPORTED: the caller takes the mma.sync kernel.
+B200_API int b200_paged_attn_tc(const void* q, long long tokens, const void* ck, const void* cv, long long pool_rows, const int* tiles,
+                                const int* tile_of, int n_tiles, const int* table, int max_blocks, void* out, long long ldo, int H, int G,
+                                int D, int block_size, float scale, int window, int keep_first, float post, const b200_attn_opts* opts,
+                                int dtype, void* stream) {
+  if (n_tiles <= 0) return 0;
+  if (int rc = tc_check(q, out, 1, 1, H, G, D, dtype)) return rc;
+  const b200_attn_opts opt = opts ? *opts : b200_attn_opts{};
+  if (opt.chunk < 0 || (opt.chunk > 0 && window > 0) || !(opt.softcap >= 0.f) || !(scale > 0.f)) return B200_ERR_UNSUPPORTED;
+  const int rep = H / G;
+  if ((rep & 1) && !tile_of) return B200_ERR_UNSUPPORTED;
+  if (((reinterpret_cast<uintptr_t>(ck) | reinterpret_cast<uintptr_t>(cv)) & 15) || ldo % 8 || pool_rows > 0x7fffffffLL) return B200_ERR_UNSUPPORTED;
+  FlashTcParams p = {};
+  while ((1 << p.bs_log2) < block_size) ++p.bs_log2;
+  if ((1 << p.bs_log2) != block_size || block_size < 8) return B200_ERR_UNSUPPORTED;      // a swizzled box starts on a group of 8 rows
+  if (int rc = bind_device()) return rc;
+  CUtensorMap tq, tk, tv;
+  const uint32_t box = block_size < 64 ? block_size : 64;
+  if (int rc = rows_map(&tq, q, (uint64_t)H * D, (uint64_t)tokens, 64)) return rc;
+  if (int rc = rows_map(&tk, ck, (uint64_t)D, (uint64_t)pool_rows, box)) return rc;
+  if (int rc = rows_map(&tv, cv, (uint64_t)D, (uint64_t)pool_rows, box)) return rc;
+  const bool capped = opt.softcap > 0.f;
+  p.out = out; p.out_rs = ldo; p.H = H; p.Hkv = G; p.causal = 1; p.tiles = tiles; p.tile_of = tile_of; p.table = table; p.max_blocks = max_blocks;
+  p.window = window; p.keep_first = keep_first; p.post = post; p.opt = opt;
+  p.scale_log2 = (capped ? opt.softcap : scale) * kTcLog2e;
+  p.cin = capped ? scale / opt.softcap : 1.f;
+  const dim3 grid(n_tiles, rep & 1 ? H : H / 2);
   cudaStream_t st = (cudaStream_t)stream;
-  if (psmem) {
-    if (p.is_bf16) flash_fwd_tc_kernel<true, false><<<grid, kTcThreads, kTcSmemBytes, st>>>(tm, p);
-    else flash_fwd_tc_kernel<false, false><<<grid, kTcThreads, kTcSmemBytes, st>>>(tm, p);
-  } else {
-    if (p.is_bf16) flash_fwd_tc_kernel<true, true><<<grid, kTcThreads, kTcSmemBytes, st>>>(tm, p);
-    else flash_fwd_tc_kernel<false, true><<<grid, kTcThreads, kTcSmemBytes, st>>>(tm, p);
-  }
-  B200_LAUNCH_CHECK();
-  return 0;
+  const bool bf = dtype == B200_DT_BF16;
+#define TC_PAGED(DD)                                                                                                           \
+  (capped ? (bf ? launch_tc<kTcPaged, DD, true, true>(tq, tk, tv, p, grid, st) : launch_tc<kTcPaged, DD, false, true>(tq, tk, tv, p, grid, st)) \
+          : (bf ? launch_tc<kTcPaged, DD, true, false>(tq, tk, tv, p, grid, st) : launch_tc<kTcPaged, DD, false, false>(tq, tk, tv, p, grid, st)))
+  return D == 64 ? TC_PAGED(64) : TC_PAGED(128);
+#undef TC_PAGED
 }

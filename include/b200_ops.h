@@ -393,11 +393,21 @@ int b200_flash_attn_bwd(const void* qkv, const void* out, const void* dout, cons
                         float* dqkv32, void* dqkv, int B, int S, int H, int Hkv, int D, int causal, float scale,
                         float dropout_p, unsigned long long seed, int dtype, void* stream);
 /* The same forward on the 5th-generation tensor cores (csrc/flash_tc.cu): tcgen05.mma for Q K^T and P V with both
- * accumulators in TMEM, Q / K / V tiles by TMA straight from qkv, one softmax thread per query row. head_dim 128, 16-bit
+ * accumulators in TMEM, Q / K / V tiles by TMA straight from qkv, one softmax thread per query row. head_dim 64 or 128, 16-bit
  * dtypes, no dropout; returns B200_ERR_UNSUPPORTED for anything else (callers then use b200_flash_attn_fwd). B * S rows
- * of qkv must be addressable as one 2-D tensor map (row stride (H + 2 Hkv) * 128 elements, 16-byte aligned base). */
+ * of qkv must be addressable as one 2-D tensor map (row stride (H + 2 Hkv) * D elements, 16-byte aligned base). */
 int b200_flash_attn_fwd_tc(const void* qkv, void* out, float* lse, int B, int S, int H, int Hkv, int D, int causal,
                            float scale, int dtype, void* stream);
+/* The packed form (arguments as in b200_flash_attn_varlen_fwd; tokens: rows of qkv) and prompt pieces over a paged cache (one map,
+ * D = Dv, arguments as in b200_multimap_attn_mma_ex; tokens: rows of q, pool_rows: blocks * G * block_size;
+ * tile_of [n_tiles, 4] = (run, place in the run, tiles of the run, its first tile), wanted where H / G is odd), head_dim 64 or 128. */
+int b200_flash_attn_varlen_fwd_tc(const void* qkv, void* out, const int* cu_seqlens, long long tokens, int n_seqs, int max_seqlen, int H,
+                                  int Hkv, int D, int causal, float scale, int dtype, void* stream);
+struct b200_attn_opts;
+int b200_paged_attn_tc(const void* q, long long tokens, const void* ck, const void* cv, long long pool_rows, const int* tiles,
+                       const int* tile_of, int n_tiles, const int* table, int max_blocks, void* out, long long ldo, int H, int G, int D,
+                       int block_size, float scale, int window, int keep_first, float post, const struct b200_attn_opts* opts, int dtype,
+                       void* stream);
 
 /* Backward on the same tensor cores (csrc/flash_bwd_tc.cu): a dK/dV pass (K, V resident per 64-key block, query tiles
  * stream) and a dQ pass (Q, dO resident per 128-row tile, key blocks stream), every product a tcgen05.mma with TMEM

@@ -11,7 +11,7 @@ import torch
 
 from . import _native as nv
 
-vp, i32, f32, u64 = ctypes.c_void_p, ctypes.c_int, ctypes.c_float, ctypes.c_ulonglong
+vp, i32, i64, f32, u64 = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float, ctypes.c_ulonglong
 
 
 def flash_supported(qkv: torch.Tensor, head_dim: int) -> bool:
@@ -25,7 +25,7 @@ _TC_BWD = __import__("os").environ.get("B200_FLASH_TC_BWD", "1") != "0"
 def _fwd(qkv, B, S, H, Hkv, D, causal, scale, want_lse=True, dropout_p=0.0, seed=0):
     out = torch.empty(B * S, H * D, dtype=qkv.dtype, device=qkv.device)
     lse = torch.empty(B, H, S, dtype=torch.float32, device=qkv.device) if want_lse else None
-    if _TC and D == 128 and dropout_p == 0.0:
+    if _TC and D in (64, 128) and dropout_p == 0.0:
         # tcgen05 / TMEM / TMA forward (csrc/flash_tc.cu); the mma.sync kernel below keeps the other head sizes and dropout
         ft = nv.proto("b200_flash_attn_fwd_tc", [vp, vp, vp, i32, i32, i32, i32, i32, i32, f32, i32, vp])
         rc = ft(nv.ptr(qkv), nv.ptr(out), nv.ptr(lse), B, S, H, Hkv, D, int(causal), float(scale), nv.dtype_code(qkv.dtype),
@@ -98,6 +98,15 @@ def flash_attention_varlen(qkv: torch.Tensor, cu_seqlens: torch.Tensor, max_seql
         return torch.cat(outs, 0)
     qkv = qkv.contiguous()
     out = torch.empty(qkv.shape[0], H * D, dtype=qkv.dtype, device=qkv.device)
+    if _TC and D in (64, 128):
+        ft = nv.proto("b200_flash_attn_varlen_fwd_tc", [vp, vp, vp, i64, i32, i32, i32, i32, i32, i32, f32, i32, vp])
+        rc = ft(nv.ptr(qkv), nv.ptr(out), nv.ptr(cu_seqlens), qkv.shape[0], n, int(max_seqlen), H, Hkv, D, int(causal), float(scale),
+                nv.dtype_code(qkv.dtype), nv.stream())
+        if rc == 0:
+            nv.count_launch()
+            return out
+        if rc != nv.ERR_UNSUPPORTED:
+            nv.check(rc, "flash_attn_varlen_fwd_tc")
     fn = nv.proto("b200_flash_attn_varlen_fwd", [vp, vp, vp, i32, i32, i32, i32, i32, i32, f32, i32, vp])
     nv.check(fn(nv.ptr(qkv), nv.ptr(out), nv.ptr(cu_seqlens), n, int(max_seqlen), H, Hkv, D, int(causal), float(scale),
                 nv.dtype_code(qkv.dtype), nv.stream()), "flash_attn_varlen_fwd")

@@ -218,6 +218,17 @@ def multimap_attention(q: torch.Tensor, cache_k: torch.Tensor, cache_v: torch.Te
         if (pieces is not None and pieces.longest >= 8 and q.dtype == torch.bfloat16 and D % 8 == 0 and Dv % 8 == 0
                 and max(D, Dv) <= _MMA_MAX and scale > 0
                 and BS & (BS - 1) == 0 and out.stride(0) % 2 == 0 and out.data_ptr() % 4 == 0 and os.environ.get("B200_PAGED_MMA", "1") != "0"):
+            if M == 1 and D == Dv and D in (64, 128) and BS >= 8 and out.stride(0) % 8 == 0 and \
+                    (out.data_ptr() | q.data_ptr()) % 16 == 0 and nv.has("b200_paged_attn_tc"):
+                ft = nv.proto("b200_paged_attn_tc", [vp, i64, vp, vp, i64, vp, vp, i32, vp, i32, vp, i64, i32, i32, i32, i32, f32, i32, i32, f32, vp, i32, vp])
+                rc = ft(nv.ptr(q), T, nv.ptr(cache_k), nv.ptr(cache_v), cache_k.shape[0] * G * BS, nv.ptr(pieces.tiles),
+                        nv.ptr(pieces.tile_of), pieces.n_tiles, nv.ptr(table), table.shape[1], nv.ptr(out), out.stride(0), H, G, D, BS,
+                        float(scale), int(window), int(keep_first), float(post), opts, nv.dtype_code(q.dtype), nv.stream())
+                if rc == 0:
+                    nv.count_launch()
+                    return out
+                if rc != nv.ERR_UNSUPPORTED:
+                    nv.check(rc, "paged_attn_tc")
             fn = nv.proto("b200_multimap_attn_mma_ex", [vp, vp, vp, vp, i32, vp, i32, vp, i64, i32, i32, i32, i32, i32, i32, f32, i32, i32, i32,
                                                         f32, f32, f32, vp, i32, vp])
             nv.check(fn(nv.ptr(q), nv.ptr(cache_k), nv.ptr(cache_v), nv.ptr(pieces.tiles), pieces.n_tiles, nv.ptr(table),

@@ -58,3 +58,78 @@ def test_decode_batches(H, G, M, D, Dv, opt, BS):
     for max_pos in (0, 776):                                       # without and with the keys cut into ranges
         got = multimap_attention(q.cuda(), *map(dev, args), max_pos=max_pos, **{k: dev(v) for k, v in kw.items()})
         close(got, want)
+
+
+@pytest.mark.parametrize("H,G,D", [(4, 2, 128), (8, 2, 64), (10, 2, 64), (2, 2, 128), (3, 1, 128)])
+@pytest.mark.parametrize("opt", ["none", "window", "chunk"])
+@pytest.mark.parametrize("BS", [8, 16, 64, 128])
+def test_prompt_pieces(H, G, D, opt, BS):
+    """Pieces that start and end anywhere in pages and 64-key blocks, single tokens beside them, keys past the end that are NaN."""
+    from llm_in_practise_b200.inference.ragged import make_pieces
+    runs = [(65, 0), (1, 130), (9, 63), (130, 200), (64, 64), (1, 0)]                # (tokens, first position)
+    ck, cv, table, g = pools([n + p for n, p in runs], G, 1, D, D, BS)
+    pos = torch.cat([torch.arange(p, p + n) for n, p in runs]).to(torch.int32)
+    slot = torch.cat([torch.full((n,), i) for i, (n, _) in enumerate(runs)]).to(torch.int32)
+    T = pos.numel()
+    for i, (n, p) in enumerate(runs):                                                # what lies behind a sequence in its last page
+        if (n + p) % BS:
+            ck[table[i, (n + p) // BS], :, (n + p) % BS:] = float("nan")
+            cv[table[i, (n + p) // BS], :, (n + p) % BS:] = float("nan")
+    q = torch.randn(T, H * D, generator=g).to(torch.bfloat16)
+    kw = {}
+    if opt == "window":
+        kw = dict(window=70, keep_first=3, sink=torch.randn(H, generator=g))
+    if opt == "chunk":
+        kw = dict(chunk=100, softcap=5.0, gate=torch.randn(T, H, generator=g), post=0.7)
+    args = (ck, cv, table, pos, slot, H, G, 1, D, D, D ** -0.5)
+    want = multimap_attention(q, *args, **kw)
+    dev = lambda v: v.cuda() if isinstance(v, torch.Tensor) else v                                  # noqa: E731
+    firsts = [sum(n for n, _ in runs[:i]) for i in range(len(runs))]
+    pieces = make_pieces([(f, n, p, i) for i, (f, (n, p)) in enumerate(zip(firsts, runs))], "cuda")
+    wide = torch.zeros(T, H * D + 8, dtype=torch.bfloat16, device="cuda")
+    for out in (None, wide[:, :H * D]):
+        got = multimap_attention(q.cuda(), *map(dev, args), pieces=pieces, max_pos=329, out=out, **{k: dev(v) for k, v in kw.items()})
+        # here P is rounded to bf16 before the product (as in the mma.sync kernel): 2^-9 of every term, which averages out over the
+        # sum to well below 2^-9 of the largest value; the bound grants it in full
+        close(got, want, vmax=16.0)
+
+
+@pytest.mark.parametrize("H,Hkv,D", [(4, 2, 128), (6, 6, 64), (4, 1, 64)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("causal", [True, False])
+def test_packed_prompts(H, Hkv, D, dtype, causal):
+    """Lengths at the edges of key blocks and query tiles; a NaN in the sequence behind must not reach the one in front."""
+    from llm_in_practise_b200.ops.flash import flash_attention_varlen
+    lens = [1, 63, 64, 65, 128, 129, 200, 7]
+    g = torch.Generator().manual_seed(3)
+    qkv = torch.randn(sum(lens), (H + 2 * Hkv) * D, generator=g).to(dtype)
+    qkv[-7:] = float("nan")
+    cu = torch.tensor([0] + lens, dtype=torch.int32).cumsum(0).to(torch.int32)
+    want = flash_attention_varlen(qkv, cu, max(lens), H, Hkv, D, D ** -0.5, causal)
+    got = flash_attention_varlen(qkv.cuda(), cu.cuda(), max(lens), H, Hkv, D, D ** -0.5, causal)
+    close(got[:-7], want[:-7], vmax=16.0)
+    assert torch.isnan(got[-7:]).all()
+
+
+@pytest.mark.parametrize("B,S,H,Hkv,D", [(2, 1, 2, 1, 64), (3, 65, 2, 2, 64), (2, 129, 4, 2, 64), (1, 300, 6, 2, 128), (2, 256, 3, 3, 64)])
+@pytest.mark.parametrize("causal", [True, False])
+def test_fused_qkv_forward(B, S, H, Hkv, D, causal):
+    """Forward with the log-sum-exp the backward reads; a batch entry whose last rows are NaN leaves the ones beside it alone."""
+    from llm_in_practise_b200.ops.attention import _ref_attention
+    from llm_in_practise_b200.ops.flash import _fwd
+    g = torch.Generator().manual_seed(4)
+    qkv = torch.randn(B * S, (H + 2 * Hkv) * D, generator=g).to(torch.bfloat16)
+    want = _ref_attention(qkv, B, S, H, Hkv, D, causal, 0, D ** -0.5)
+    got, lse = _fwd(qkv.cuda(), B, S, H, Hkv, D, causal, D ** -0.5)
+    close(got, want, vmax=16.0)
+    t = qkv.double().view(B, S, H + 2 * Hkv, D)
+    k = t[:, :, H:H + Hkv].repeat_interleave(H // Hkv, 2)
+    sc = torch.einsum("bqhd,bkhd->bhqk", t[:, :, :H], k) * D ** -0.5
+    if causal:
+        sc = sc.masked_fill(~torch.ones(S, S, dtype=torch.bool).tril(), float("-inf"))
+    # products of bf16 numbers are exact in fp32, a sum of D of them is good to D 2^-24 of its terms: 1e-5 at these sizes
+    assert (lse.double().cpu() - torch.logsumexp(sc, -1)).abs().max().item() < 1e-4
+    if B > 1:
+        qkv[-S:] = float("nan")
+        again, _ = _fwd(qkv.cuda(), B, S, H, Hkv, D, causal, D ** -0.5)
+        assert torch.equal(again[:-S], got[:-S])
