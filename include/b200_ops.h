@@ -673,6 +673,12 @@ int b200_linear_scan(const float* q, long long ldq, const float* k, long long ld
                      long long ldg, const float* beta, long long ldb, const float* decay, float* state, const int* runs,
                      const int* pos, const int* slot, int n_runs, float* o, int H, int G, int D, int Dv, int mode, int act,
                      int ones, void* stream);
+/* Mode 3 of it over prompts, 64 tokens at a time (csrc/delta_chunk.cu): D 64 or 128, Dv % 16 == 0, 16-byte aligned rows; ws holds
+ * b200_delta_chunk_workspace floats. B200_ERR_UNSUPPORTED otherwise. */
+long long b200_delta_chunk_workspace(int tokens, int n_runs, int H);
+int b200_delta_chunk_scan(const float* q, long long ldq, const float* k, long long ldk, const float* v, long long ldv, const float* g,
+                          long long ldg, const float* beta, long long ldb, float* state, const int* runs, int n_runs, float* o, float* ws,
+                          int tokens, int H, int G, int D, int Dv, void* stream);
 /* Capped log gates of an mLSTM and their running maximum (mstate fp32 [rows, H]): a = exp(f + m - m'), b = exp(i - m'),
  * e = exp(-m'), all fp32 [tokens, H]; gi / gf fp32 rows of stride ldi / ldf holding one column per head. */
 int b200_mlstm_gates(const float* gi, long long ldi, const float* gf, long long ldf, const float* bi, const float* bf, float cap,

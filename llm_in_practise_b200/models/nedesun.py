@@ -243,7 +243,7 @@ class NedesunLayer(nn.Module):
         q, k, v = qkv[:, :G * D], qkv[:, G * D:2 * G * D], qkv[:, 2 * G * D:]
         a, b = self.cols(main, tail, "right.a"), self.cols(main, tail, "right.b")
         delta_gates(q, k, a, b, self.dt_bias, self.A_log, G, H, D, D ** -0.5, UNIT_EPS)
-        o = linear_scan(q, k, v, state[0], pos, slot, runs, n_runs, H, G, D, Dv, "head_delta", g=a, beta=b)
+        o = linear_scan(q, k, v, state[0], pos, slot, runs, n_runs, H, G, D, Dv, "head_delta", g=a, beta=b, pieces=pieces)
         z = scan_readout(o, H, Dv, self.mix_norm, H, eps, dt, post=self.cols(main, tail, "right.g"), post_act="silu")
         return left, linear_exact(z, self.right_o, out_dtype=torch.float32)
 

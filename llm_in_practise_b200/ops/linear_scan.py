@@ -165,8 +165,8 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.
     ``g`` = a and ``beta`` = b, both fp32 [T, H], and so does "head_delta" its decay and beta; "channel" takes ``g`` fp32
     [T, H * D] and optionally the bonus ``u`` fp32 [H, D]. ``act``: silu on q, k and v as they are read. ``ones``: every head of v gets
     one more column, all ones — ``Dv`` counts it, v itself has ``Dv - 1`` columns per head — so the state's last column
-    accumulates the decayed b k alone and o's last column is its product with q. ``pieces`` (``inference.ragged.Pieces``,
-    mode "channel"): runs of several tiles are walked tile by tile in parallel, see ``csrc/linear_scan.cu``."""
+    accumulates the decayed b k alone and o's last column is its product with q. ``pieces`` (``inference.ragged.Pieces``):
+    mode "channel" walks runs of several tiles tile by tile in parallel; "head_delta" sees from it how long the runs are."""
     T = q.shape[0]
     o = torch.empty(T, H * Dv, dtype=torch.float32, device=q.device)
     delta = mode in ("delta", "head_delta")
@@ -192,6 +192,10 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.
                     opt("run_tiles"), longest, nv.ptr(pos), nv.ptr(slot), nv.ptr(o), H, G, D, Dv, nv.stream()), "channel_scan")
         nv.count_launch(3 if tiled else 1)
         return o
+    if (nv.use_native(q) and mode == "head_delta" and runs is not None and D in (64, 128) and Dv % 16 == 0 and not act and not ones
+            and nv.has("b200_delta_chunk_scan") and _chunks_pay(T, n_runs, pieces, H, G, D, Dv)):
+        if _delta_chunks(q, k, v, g, beta, state, runs, n_runs, o, H, G, D, Dv):
+            return o
     if nv.use_native(q):
         fn = nv.proto("b200_linear_scan", [vp, i64, vp, i64, vp, i64, vp, i64, vp, i64, vp, vp, vp, vp, vp, i32, vp, i32, i32, i32,
                                            i32, i32, i32, i32, vp])
@@ -231,6 +235,34 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.
             ov[t] = torch.einsum("hde,hd->he", S, qf[t])
         state[s] = S
     return o
+
+
+def _chunks_pay(T: int, n_runs: int, pieces, H: int, G: int, D: int, Dv: int) -> bool:
+    """Whether prompts of the delta rule with one decay per head take less time 64 tokens at a time (csrc/delta_chunk.cu) than token by
+    token. Both as measured (us): the walk moves 0.24 per token of the longest run, or, with more (run, head, 16 columns) than about
+    320 (445 for keys of 64) at once, in proportion; a chunk is 6.5 (4.8) on one of 148 SMs, after the inverses. One run of 2048 tokens,
+    16 heads of 128: 225 against 502; three of 150: 74 against 56. Without ``pieces`` the runs count as equally long."""
+    blocks = H * (Dv // 16)
+    longest, tiles = (pieces.longest, pieces.n_tiles) if pieces is not None else (T / max(n_runs, 1), T / 64 + n_runs)
+    walk = 0.24 * max(longest, T * blocks / (320 if D == 128 else 445))
+    chunks = 17 * max(1.0, tiles * G / 200) + (6.5 if D == 128 else 4.8) * max(longest / 64, tiles * blocks / 148)
+    return chunks < 0.9 * walk
+
+
+def _delta_chunks(q, k, v, g, beta, state, runs, n_runs, o, H, G, D, Dv) -> bool:
+    """Mode "head_delta" over the runs of a step in chunks of 64 tokens; False: rows the kernels do not take."""
+    T = q.shape[0]
+    size = nv.lib().b200_delta_chunk_workspace
+    size.restype = i64
+    ws = torch.empty(size(T, n_runs, H), dtype=torch.float32, device=q.device)
+    fn = nv.proto("b200_delta_chunk_scan", [vp, i64, vp, i64, vp, i64, vp, i64, vp, i64, vp, vp, i32, vp, vp, i32, i32, i32, i32, i32, vp])
+    rc = fn(nv.ptr(q), q.stride(0), nv.ptr(k), k.stride(0), nv.ptr(v), v.stride(0), nv.ptr(g), g.stride(0), nv.ptr(beta), beta.stride(0),
+            nv.ptr(state), nv.ptr(runs), n_runs, nv.ptr(o), nv.ptr(ws), T, H, G, D, Dv, nv.stream())
+    if rc == nv.ERR_UNSUPPORTED:
+        return False
+    nv.check(rc, "delta_chunk_scan")
+    nv.count_launch(2 * max(1, -(-(T // 64 + n_runs) // 128)))
+    return True
 
 
 def mlstm_gates(gi: torch.Tensor, gf: torch.Tensor, bi: torch.Tensor, bf: torch.Tensor, cap: float, mstate: torch.Tensor,

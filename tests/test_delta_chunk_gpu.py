@@ -1,0 +1,55 @@
+"""The delta rule in chunks of 64 tokens against the recurrence in float64, at the edges of chunks, runs and windows of chunks."""
+import pytest
+import torch
+
+from llm_in_practise_b200.ops import linear_scan as scan_mod
+from llm_in_practise_b200.ops.linear_scan import linear_scan
+
+pytestmark = pytest.mark.gpu
+
+
+def walk(q, k, v, state, runs, H, G, D, Dv, a, b):
+    q, k, v, a, b, state = (t.double() for t in (q, k, v, a, b, state))
+    o, rep = torch.zeros(q.shape[0], H, Dv, dtype=torch.float64, device=q.device), H // G
+    q, k = (t.reshape(-1, G, D).repeat_interleave(rep, 1) for t in (q, k))
+    for first, n, p0, s in runs:
+        S = state[s].clone() if p0 > 0 else torch.zeros_like(state[s])
+        for t in range(first, first + n):
+            S = S * a[t].view(H, 1, 1)
+            u = b[t].view(H, 1) * (v[t].view(H, Dv) - torch.einsum("hde,hd->he", S, k[t]))
+            S = S + k[t][:, :, None] * u[:, None, :]
+            o[t] = torch.einsum("hde,hd->he", S, q[t])
+        state[s] = S
+    return o.reshape(-1, H * Dv), state
+
+
+@pytest.mark.parametrize("lens,H,G,D,Dv", [
+    ([64], 2, 1, 64, 16), ([65, 17, 63], 4, 4, 128, 48), ([1, 130, 1, 200], 4, 2, 128, 32), ([300], 6, 1, 64, 64),
+    ([64, 128, 90], 20, 4, 128, 128),                     # more (run, head, column block)s than SMs
+    ([8300, 40], 1, 1, 64, 16),                           # more chunks than one window of 128
+])
+@pytest.mark.parametrize("decay", [(0.9, 1.0), (0.0, 1.0), (1e-6, 1e-3)])
+def test_chunks(lens, H, G, D, Dv, decay, monkeypatch):
+    g = torch.Generator(device="cuda").manual_seed(7)
+    T, C = sum(lens), 2 * G * D + H * Dv
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)                                   # noqa: E731
+    x = rnd(T, C + 4)                                     # strided rows, as a slice of a projection
+    q, k, v = x[:, :G * D], x[:, G * D:2 * G * D], x[:, 2 * G * D:C]
+    for t in (q, k):
+        t /= t.reshape(T, G, D).norm(dim=-1).repeat_interleave(D, 1) + 1e-6
+    a = torch.rand(T, H, device="cuda", generator=g) * (decay[1] - decay[0]) + decay[0]
+    a[0] = 0.0
+    b = torch.rand(T, H, device="cuda", generator=g)
+    runs, at = [], 0
+    for i, n in enumerate(lens):
+        runs.append([at, n, 0 if i % 2 == 0 else 5 + i, i])
+        at += n
+    state = rnd(len(lens), H, D, Dv)
+    want_o, want_s = walk(q, k, v, state, runs, H, G, D, Dv, a, b)
+    pos = slot = torch.zeros(T, dtype=torch.int32, device="cuda")
+    monkeypatch.setattr(scan_mod, "_chunks_pay", lambda *a: True)      # these sizes are for the edges, not for the clock
+    o = linear_scan(q, k, v, state, pos, slot, torch.tensor(runs, dtype=torch.int32, device="cuda"), len(lens), H, G, D, Dv, "head_delta", g=a, beta=b)
+    # unit keys, beta < 1: nothing grows. A value is a sum over at most D keys and 64 tokens, each term rounded a few times: D + 64
+    # roundings of 2^-24 of the largest value on the way, four times over for the solve and the carried state
+    for got, want in ((o, want_o), (state, want_s)):
+        assert ((got.double() - want).abs().max() / want.abs().max()).item() < 4 * (D + 64) * 2.0 ** -24
