@@ -133,3 +133,26 @@ def test_fused_qkv_forward(B, S, H, Hkv, D, causal):
         qkv[-S:] = float("nan")
         again, _ = _fwd(qkv.cuda(), B, S, H, Hkv, D, causal, D ** -0.5)
         assert torch.equal(again[:-S], got[:-S])
+
+
+@pytest.mark.parametrize("B,S,H,Hkv", [(2, 1, 2, 1), (2, 64, 3, 3), (1, 65, 4, 2), (2, 129, 4, 1), (1, 300, 6, 2)])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("causal", [True, False])
+def test_fused_qkv_backward(B, S, H, Hkv, D, causal):
+    """Gradient of the fused projection at the edges of key blocks, query tiles and groups of heads, against float64 autograd."""
+    from llm_in_practise_b200.ops.flash import flash_attention
+    g = torch.Generator(device="cuda").manual_seed(5)
+    qkv = torch.randn(B * S, (H + 2 * Hkv) * D, device="cuda", generator=g).to(torch.bfloat16).requires_grad_()
+    go = torch.randn(B * S, H * D, device="cuda", generator=g).to(torch.bfloat16)
+    flash_attention(qkv, B, S, H, Hkv, D, causal, D ** -0.5).backward(go)
+    x = qkv.detach().double().requires_grad_()
+    t = x.view(B, S, H + 2 * Hkv, D).transpose(1, 2)
+    q, k, v = t[:, :H], t[:, H:H + Hkv].repeat_interleave(H // Hkv, 1), t[:, H + Hkv:].repeat_interleave(H // Hkv, 1)
+    sc = q @ k.transpose(-1, -2) * D ** -0.5
+    if causal:
+        sc = sc.masked_fill(~torch.ones(S, S, dtype=torch.bool, device="cuda").tril(), float("-inf"))
+    (sc.softmax(-1) @ v).transpose(1, 2).reshape(B * S, H * D).backward(go.double())
+    # P, dS, the forward's output behind delta and the result are rounded to bf16 (2^-9 each, independent): four times their root sum
+    for lo, hi in ((0, H * D), (H * D, (H + Hkv) * D), ((H + Hkv) * D, (H + 2 * Hkv) * D)):
+        a, b = qkv.grad[:, lo:hi].double(), x.grad[:, lo:hi]
+        assert (a - b).norm() <= 4 * 2 * 2.0 ** -9 * b.norm() + 2.0 ** -9 * go.double().norm() * (S == 1)
