@@ -62,7 +62,8 @@ def _stream_k_workspace(device: torch.device) -> Optional[torch.Tensor]:
         return None
     if torch.cuda.is_current_stream_capturing():
         return _sk_workspaces.get((device.index, "graph"))       # None: captured without stream-K
-    key = (device.index, torch.cuda.current_stream(device).cuda_stream)
+    index = device.index if device.index is not None else torch._C._cuda_getDevice()
+    key = (index, torch._C._cuda_getCurrentRawStream(index))
     ws = _sk_workspaces.get(key)
     if ws is None:
         fn = nv.lib().b200_gemm_workspace_bytes
