@@ -467,6 +467,241 @@ gemv_mma_kernel(const GemvParams p) {
   }
 }
 
+// element e of a tile's sums, in the order of the MMA's accumulators, to y
+template <bool BF16> __device__ __forceinline__ void ws_store(const GemvParams& p, long long row0, int e, float s) {
+  const int ln = (e & 127) >> 2, i = e & 3;
+  const long long row = row0 + (ln >> 2) + ((i & 2) ? 8 : 0);
+  const int tok = (e >> 7) * 8 + 2 * (ln & 3) + (i & 1);
+  if (row >= p.N || tok >= p.M) return;
+  if (p.bias) s += BF16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.bias)[row]) : __half2float(reinterpret_cast<const __half*>(p.bias)[row]);
+  if (BF16) reinterpret_cast<__nv_bfloat16*>(p.y)[(long long)tok * p.y_rs + row] = __float2bfloat16_rn(s);
+  else reinterpret_cast<__half*>(p.y)[(long long)tok * p.y_rs + row] = __float2half_rn(s);
+}
+
+// ---- integer codes, at most 16 tokens, groups of whole 128-wide chunks (POST above) --------------------------------------------
+// What bounds the kernel above here is not HBM but the load pipe (84 wavefronts per chunk of 16 x 128 weights, 32 of them for scales
+// fetched four bytes at a time from a row each) and the 286 instructions per warp and chunk. So
+//   * a unit of work is four chunks of 16 rows: their scales and zeros are two 16-byte pieces per row, copied by one cp.async of the
+//     warp a unit ahead, and what addresses cost is shared by four chunks,
+//   * the activations are laid out in shared memory once, in the order of the MMA's lanes (zero rows past M, pairs as the codes have
+//     them): no permutes, no predicates, and 16-byte reads without bank conflicts,
+//   * sum_k x of a chunk belongs to the activations, not to the weights: formed once, in fp32, instead of by an MMA per tile,
+//   * one CTA of 16 warps per SM deals the units of all its tiles to its warps in turn, and a warp requests a chunk of its next unit
+//     as it takes one of this unit, across the ends of tiles: 64 KB per SM are always on their way,
+//   * a cluster of `split` CTAs shares a tile's k: a slice of the activations then fits where all of them do not, and short matrices
+//     fill the last wave. The parts meet once, at the end, through distributed shared memory, in the order of the ranks.
+// Device time with cold caches, 8 tokens: N 24576, K 4096: 31.7 -> 24.7 us (8.7 at the rate of HBM; 1.6 instructions per cycle, a
+// quarter of the time goes into the activations and the first loads); K 17408, N 5120: 42 -> 26; 16 tokens, N 24576: 57 -> 33.
+// Requesting everything through a ring of cp.async instead of registers gave the same with 244 instructions per chunk; barriers once
+// per four rounds gave nothing.
+constexpr int kWsWarps = 16, kWsScales = 2 * 512;        // per warp: two units of 16 rows x (4 scales + 4 zeros)
+
+template <int TG> constexpr long long ws_smem(long long chunks, long long acc_tiles) {
+  return chunks * TG * (2048 + 32) + kWsWarps * kWsScales + 2 * kWsWarps * TG * 512 + (1 + acc_tiles) * TG * 512;
+}
+
+template <bool BF16, int TG>
+__global__ void __launch_bounds__(kWsWarps * 32, 1)
+w4_units_kernel(const GemvParams p, const int split) {
+  extern __shared__ __align__(128) unsigned char ws_sm[];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int r = blockIdx.x % split, cl = blockIdx.x / split, ncl = gridDim.x / split;
+  const int nch = p.K / 128, nun = (nch + 3) / 4;         // slices of k are whole units
+  const int c0 = nun * r / split * 4, cnt = min(nch, nun * (r + 1) / split * 4) - c0;
+  const int cmax = (nun + split - 1) / split * 4;
+  unsigned char* xs = ws_sm;                              // [cmax][TG][4][32 lanes] 16 bytes
+  float* xsum = reinterpret_cast<float*>(xs + cmax * TG * 2048);          // [cmax][TG][8]
+  float* scales = xsum + cmax * TG * 8 + warp * (kWsScales / 4);          // [2][scale, zero][16 rows][4 chunks]
+  float* red = xsum + cmax * TG * 8 + kWsWarps * (kWsScales / 4);         // [2][16 warps][TG * 128]
+  float* carry = red + 2 * kWsWarps * TG * 128;           // the sums of a tile that goes on in the next round
+  float* acc = carry + TG * 128;
+  const long long ntiles = (p.N + 15) / 16;
+  const int T = (int)((ntiles - 1 - cl) / ncl) + 1;       // the grid has no more clusters than tiles
+  const int upt = (cnt + 3) / 4;                          // units of a tile
+  const long long U = (long long)T * upt;
+  const int gpr = p.K / p.group;
+  const bool sv = p.group == 128 && gpr % 4 == 0 &&
+                  !((reinterpret_cast<uintptr_t>(p.scale) | reinterpret_cast<uintptr_t>(p.zs)) & 15);
+  const float* const sbase = lane < 16 ? p.scale : p.zs;  // this lane copies the scales or the zeros of a row
+
+  auto ask_scales = [&](int buf, long long row0, int c) {
+    if (!sbase) return;
+    const float* s = sbase + min(row0 + (lane & 15), p.N - 1) * gpr;
+    float* d = scales + buf * 128 + lane * 4;
+    if (sv) cp_async16(d, s + c0 + c);
+    else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (c + j < cnt) {
+          const int k = (c0 + c + j) * 128;
+          cp_async4(d + j, s + (p.gshift >= 0 ? k >> p.gshift : k / p.group));
+        }
+    }
+  };
+  uint4 wa[4], wb[4];
+  const uint8_t *pa = nullptr, *pb = nullptr;             // rows g and g + 8 of the next unit
+  int left = 0;                                           // and the chunks it has
+  auto aim = [&](long long u, int buf) {
+    const int tl = (int)(u / upt), c = (int)(u - (long long)tl * upt) * 4;
+    const long long row0 = (cl + (long long)tl * ncl) * 16;
+    const uint8_t* w = reinterpret_cast<const uint8_t*>(p.w) + (c0 + c) * 64 + t * 16;
+    pa = w + min(row0 + g, p.N - 1) * (p.K / 2);
+    pb = w + min(row0 + g + 8, p.N - 1) * (p.K / 2);
+    left = cnt - c;
+    ask_scales(buf, row0, c);
+  };
+  if (!sbase) {
+    *reinterpret_cast<float4*>(scales + lane * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
+    *reinterpret_cast<float4*>(scales + 128 + lane * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  if (warp < U) {
+    aim(warp, 0);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (j < left) { wa[j] = ld_nc_v4(pa + j * 64); wb[j] = ld_nc_v4(pb + j * 64); }
+  }
+  cp_async_commit();
+
+  // ---- the activations of this CTA's chunks, and their sums
+  for (int u = warp; u < cnt * TG; u += kWsWarps) {
+    const int c = u / TG, tok = (u - c * TG) * 8 + g;
+    uint4 v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = make_uint4(0, 0, 0, 0);
+    if (tok < p.M) {
+      const uint4* px = reinterpret_cast<const uint4*>(p.x + (long long)tok * p.x_rs + (c0 + c) * 128 + t * 32);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[i] = __ldg(px + i);
+    }
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t w[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float2 f;
+        if (BF16) f = unpack_bf16x2(w[j]);
+        else f = __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
+        s += f.x + f.y;
+      }
+      *reinterpret_cast<uint4*>(xs + ((u * 4 + i) * 32 + lane) * 16) =
+          make_uint4(__byte_perm(w[0], w[2], 0x5410), __byte_perm(w[0], w[2], 0x7632), __byte_perm(w[1], w[3], 0x5410), __byte_perm(w[1], w[3], 0x7632));
+    }
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    if (t == 0) xsum[u * 8 + g] = s;
+  }
+  __syncthreads();
+
+  uint32_t magic = BF16 ? 0x43004300u : 0x64006400u, mask = 0x000F000Fu;
+  asm volatile("" : "+r"(magic), "+r"(mask));            // both stay in registers (one LOP3 per pair of codes)
+  const float b0 = (BF16 ? 128.f : 1024.f) + p.lin_off;
+  const int rounds = (int)((U + kWsWarps - 1) / kWsWarps);
+  int part = warp % upt;                                  // of this warp's unit in its tile
+  for (int rd = 0; rd < rounds; ++rd) {
+    const long long u = (long long)rd * kWsWarps + warp;
+    float* rb = red + (rd & 1) * kWsWarps * TG * 128;     // the other buffer may still be read
+    if (u < U) {
+      cp_async_wait<0>();
+      __syncwarp();                                       // the other lanes' scales are there, and nobody reads those of the unit before
+      float Aa[4], Ab[4], za[4], zb[4];
+      const float* sc = scales + (rd & 1) * 128;
+      *reinterpret_cast<float4*>(Aa) = *reinterpret_cast<const float4*>(sc + g * 4);
+      *reinterpret_cast<float4*>(Ab) = *reinterpret_cast<const float4*>(sc + g * 4 + 32);
+      *reinterpret_cast<float4*>(za) = *reinterpret_cast<const float4*>(sc + g * 4 + 64);
+      *reinterpret_cast<float4*>(zb) = *reinterpret_cast<const float4*>(sc + g * 4 + 96);
+      const int c = part * 4, here = cnt - c;
+      left = 0;
+      if (u + kWsWarps < U) aim(u + kWsWarps, (rd + 1) & 1);
+      cp_async_commit();
+      float sum[TG][4];
+#pragma unroll
+      for (int tg = 0; tg < TG; ++tg)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sum[tg][i] = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t wA[4] = {wa[j].x, wa[j].y, wa[j].z, wa[j].w}, wB[4] = {wb[j].x, wb[j].y, wb[j].z, wb[j].w};
+        if (j < left) { wa[j] = ld_nc_v4(pa + j * 64); wb[j] = ld_nc_v4(pb + j * 64); }
+        if (j < here) {
+          const unsigned char* xc = xs + (c + j) * TG * 2048 + lane * 16;
+          float c1[TG][4], c2[TG][4];                     // two independent chains
+#pragma unroll
+          for (int tg = 0; tg < TG; ++tg)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) c1[tg][i] = c2[tg][i] = 0.f;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const uint32_t a0 = and_or(wA[q] >> 4, mask, magic), a1 = and_or(wA[q], mask, magic);
+            const uint32_t a2 = and_or(wA[q] >> 12, mask, magic), a3 = and_or(wA[q] >> 8, mask, magic);
+            const uint32_t d0 = and_or(wB[q] >> 4, mask, magic), d1 = and_or(wB[q], mask, magic);
+            const uint32_t d2 = and_or(wB[q] >> 12, mask, magic), d3 = and_or(wB[q] >> 8, mask, magic);
+#pragma unroll
+            for (int tg = 0; tg < TG; ++tg) {
+              const uint4 xv = *reinterpret_cast<const uint4*>(xc + (tg * 4 + q) * 512);
+              mma16816<BF16>(c1[tg], a0, d0, a1, d1, xv.x, xv.y);
+              mma16816<BF16>(c2[tg], a2, d2, a3, d3, xv.z, xv.w);
+            }
+          }
+          const float A = Aa[j] * p.lin_a, B = Ab[j] * p.lin_a, zA = za[j], zB = zb[j];
+#pragma unroll
+          for (int tg = 0; tg < TG; ++tg) {               // lin_a scale (code - lin_off) - zs, over the chunk's sums
+            const float2 sx = *reinterpret_cast<const float2*>(xsum + ((c + j) * TG + tg) * 8 + 2 * t);
+            sum[tg][0] = fmaf(A, fmaf(-b0, sx.x, c1[tg][0] + c2[tg][0]), fmaf(-zA, sx.x, sum[tg][0]));
+            sum[tg][1] = fmaf(A, fmaf(-b0, sx.y, c1[tg][1] + c2[tg][1]), fmaf(-zA, sx.y, sum[tg][1]));
+            sum[tg][2] = fmaf(B, fmaf(-b0, sx.x, c1[tg][2] + c2[tg][2]), fmaf(-zB, sx.x, sum[tg][2]));
+            sum[tg][3] = fmaf(B, fmaf(-b0, sx.y, c1[tg][3] + c2[tg][3]), fmaf(-zB, sx.y, sum[tg][3]));
+          }
+        }
+      }
+      part = (part + kWsWarps) % upt;
+#pragma unroll
+      for (int tg = 0; tg < TG; ++tg)
+        *reinterpret_cast<float4*>(rb + (warp * TG + tg) * 128 + lane * 4) = make_float4(sum[tg][0], sum[tg][1], sum[tg][2], sum[tg][3]);
+    }
+    __syncthreads();
+    // the round's units, in order, by a group of warps that changes from round to round
+    const int e = threadIdx.x - (rd % (kWsWarps / (4 * TG))) * TG * 128;
+    if (e >= 0 && e < TG * 128) {
+      const long long u0 = (long long)rd * kWsWarps;
+      const int n = (int)min((long long)kWsWarps, U - u0);
+      int tl = (int)(u0 / upt), up = (int)(u0 - (long long)tl * upt);
+      float s = up ? carry[e] : 0.f;
+      float v[kWsWarps];
+#pragma unroll
+      for (int w = 0; w < kWsWarps; ++w) v[w] = w < n ? rb[w * TG * 128 + e] : 0.f;
+#pragma unroll
+      for (int w = 0; w < kWsWarps; ++w) {
+        if (w < n) {
+          s += v[w];
+          if (++up == upt) {
+            if (split == 1) ws_store<BF16>(p, (cl + (long long)tl * ncl) * 16, e, s);
+            else acc[tl * TG * 128 + e] = s;
+            s = 0.f; up = 0; ++tl;
+          }
+        }
+      }
+      carry[e] = s;
+    }
+  }
+  if (split == 1) return;
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  for (int i = r * kWsWarps * 32 + threadIdx.x; i < T * TG * 128; i += split * kWsWarps * 32) {
+    float s = 0.f;
+    for (int w = 0; w < split; ++w) {
+      uint32_t a;
+      float v;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(acc + i)), "r"(w));
+      asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+      s += v;
+    }
+    ws_store<BF16>(p, (cl + (long long)(i / (TG * 128)) * ncl) * 16, i % (TG * 128), s);
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // peers read this CTA's parts until here
+}
+
 template <bool BF16, bool W4, int TG, int MINB, bool LIN = false, bool POST = false>
 static cudaError_t launch_gemv_one(const GemvParams& p_in, cudaStream_t st, int batch = 1) {
   GemvParams p = p_in;
@@ -491,14 +726,82 @@ static cudaError_t launch_gemv_one(const GemvParams& p_in, cudaStream_t st, int 
   return launch_pdl(gemv_mma_kernel<BF16, W4, TG, MINB, LIN, POST>, dim3(grid, batch), 256, smem, st, p);
 }
 
+// How a product is cut: the cluster size whose longest CTA has the least to do (chunks of weights, and the activations it lays out
+// first), among those whose slice of the activations fits. False: none does. A pass over a chunk costs about what two chunks' layout
+// of eight tokens does, a cluster's start and end as much as 64. Measured, 8 tokens (us, split 1 / 2 / 4): N 24576, K 4096: 24.5 / 25.7 /
+// 26.7; N 4096, K 12288: 19.3 / 18.4 / 17.3; N 5120, K 17408: - / 28.8 / 25.7 (33 clusters of four are resident, not 37).
+template <bool BF16, int TG>
+static bool w4_units_launch(const GemvParams& p, cudaStream_t st, cudaError_t& err) {
+  auto kern = w4_units_kernel<BF16, TG>;
+  constexpr long long kMax = 227 * 1024;
+  // clusters that are resident at once (a GPC has no multiple of four SMs); a device property, found once
+  static const struct Resident {
+    int n[3];
+    Resident() {
+      n[0] = kNumSMs;
+      for (int i = 1; i < 3; ++i) {
+        n[i] = 0;
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = 1 << i; at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.gridDim = dim3(kNumSMs >> i << i); cfg.blockDim = dim3(kWsWarps * 32); cfg.dynamicSmemBytes = kMax;
+        cfg.attrs = &at; cfg.numAttrs = 1;
+        if (cudaFuncSetAttribute(w4_units_kernel<BF16, TG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMax) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n[i], w4_units_kernel<BF16, TG>, &cfg) != cudaSuccess) { n[i] = 0; (void)cudaGetLastError(); }
+      }
+    }
+  } resident;
+  const long long tiles = (p.N + 15) / 16;
+  const int nun = (p.K / 128 + 3) / 4;
+  int best = -1, best_smem = 0;
+  long long best_cost = 0;
+  for (int i = 0; i < 3 && (1 << i) <= nun; ++i) {
+    const int ncl = resident.n[i], cm = ((nun + (1 << i) - 1) >> i) * 4;
+    if (ncl < 1) continue;
+    const long long rounds = (tiles + ncl - 1) / ncl, smem = ws_smem<TG>(cm, i ? rounds : 0);
+    if (smem > kMax) continue;
+    const long long cost = cm * (rounds + 2 * TG) + (i ? 64 : 0);
+    if (best < 0 || cost < best_cost) { best = i; best_cost = cost; best_smem = (int)smem; }
+  }
+  if (best < 0) return false;
+  if ((err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMax)) != cudaSuccess) return true;
+  const long long ncl = resident.n[best];
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((tiles < ncl ? tiles : ncl) << best));
+  cfg.blockDim = dim3(kWsWarps * 32);
+  cfg.dynamicSmemBytes = best_smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  int na = 0;
+  if (best > 0) {
+    attr[na].id = cudaLaunchAttributeClusterDimension;
+    attr[na].val.clusterDim.x = 1 << best; attr[na].val.clusterDim.y = attr[na].val.clusterDim.z = 1;
+    ++na;
+  }
+  if (pdl_enabled()) {
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na].val.programmaticStreamSerializationAllowed = 1;
+    ++na;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = na;
+  err = cudaLaunchKernelEx(&cfg, kern, p, 1 << best);
+  return true;
+}
+
 template <bool BF16>
-static int launch_gemv_lin(const GemvParams& p, cudaStream_t st) {
+static int launch_gemv_lin(const GemvParams& p_in, cudaStream_t st) {
+  GemvParams p = p_in;
+  p.gshift = (p.group & (p.group - 1)) == 0 ? __builtin_ctz(p.group) : -1;
   cudaError_t e;
   // 2 CTAs per SM (128 registers, no spills): with 4 chunks x 2 rows x 16 B requested up front per lane that is 64 KB in
   // flight per SM, above the ~44 KB that 6.5 TB/s x ~1 us of DRAM latency asks of each of the 148 SMs
   static const bool post_off = [] { const char* e = getenv("B200_GEMV_POST"); return e && atoi(e) == 0; }();
   static const int minb8 = [] { const char* e = getenv("B200_GEMV_MINB8"); return e ? atoi(e) : 2; }();
   if (p.group % 128 == 0 && !post_off) {   // scale applied to the chunk sums (see POST above)
+    if (!p.fuse && p.M <= 8 && w4_units_launch<BF16, 1>(p, st, e)) return (int)e;
+    if (!p.fuse && p.M > 8 && p.M <= 16 && w4_units_launch<BF16, 2>(p, st, e)) return (int)e;
     if (p.M <= 8) e = minb8 >= 4 ? launch_gemv_one<BF16, true, 1, 3, true, true>(p, st) : launch_gemv_one<BF16, true, 1, 2, true, true>(p, st);
     else if (p.M <= 16) e = launch_gemv_one<BF16, true, 2, 2, true, true>(p, st);
     else if (p.M <= 32) e = launch_gemv_one<BF16, true, 4, 2, true, true>(p, st);
