@@ -1,6 +1,6 @@
 // Warp-level tensor-core and async-copy wrappers shared by the attention kernels that run on mma.sync (ragged pieces over
-// paged caches: their tiles are ragged and their head sizes arbitrary multiples of 16, which the tcgen05 kernels of this
-// library do not take).
+// paged caches whose head sizes are arbitrary multiples of 16 or whose maps are several; head sizes 64 and 128 with one map run on
+// tcgen05, flash_tc.cu).
 #pragma once
 
 #include "common.cuh"

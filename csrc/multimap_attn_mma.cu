@@ -13,8 +13,8 @@
 // The instances are built for whole multiples of 16; other D and Dv (multiples of 8) run in the next larger one with zero
 // columns in shared memory.
 //
-// tcgen05 is not used: tiles are ragged (1 .. 64 rows at any position), D and Dv are independent multiples of 16, and the
-// mask has two disjoint key ranges per row; the like kernel of the single-map paged attention makes the same choice.
+// tcgen05 is not used here: D and Dv are independent multiples of 16 and the maps share one pass over V. Pieces with one map and
+// D = Dv = 64 or 128 take the tcgen05 kernel of flash_tc.cu where its options allow (ops/multimap_attention.py).
 #include "common.cuh"
 #include "mma_sync.cuh"
 #include "../include/b200_ops.h"
