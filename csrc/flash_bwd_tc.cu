@@ -445,11 +445,12 @@ static int launch_bwd(const CUtensorMap& tmq, const CUtensorMap& tmd, const Flas
 using namespace b200;
 
 // dqkv [B*S, (H + 2 Hkv) * D] = gradient of the fused projection for dout [B*S, H * D] (16-bit). out / lse are the
-// forward's outputs (lse natural log, [B, H, S]); delta [B, H, S] is a caller-provided fp32 work buffer. head_dim 64 or 128, no
-// dropout; B200_ERR_UNSUPPORTED otherwise (callers then use b200_flash_attn_bwd).
+// forward's outputs (lse natural log, [B, H, S]); delta [B, H, S] is a caller-provided fp32 work buffer. head_dim 64 or 128, scale > 0,
+// no dropout; B200_ERR_UNSUPPORTED otherwise (callers then use b200_flash_attn_bwd).
 B200_API int b200_flash_attn_bwd_tc(const void* qkv, const void* out, const void* dout, const float* lse, float* delta, void* dqkv,
                                     int B, int S, int H, int Hkv, int D, int causal, float scale, int dtype, void* stream) {
-  if ((D != 64 && D != 128) || (dtype != B200_DT_BF16 && dtype != B200_DT_FP16)) return B200_ERR_UNSUPPORTED;
+  // scale > 0: scores are masked before they are multiplied by it (see flash_tc.cu); other scales are the mma.sync kernel's
+  if ((D != 64 && D != 128) || (dtype != B200_DT_BF16 && dtype != B200_DT_FP16) || !(scale > 0.f)) return B200_ERR_UNSUPPORTED;
   if (B < 1 || S < 1 || H < 1 || Hkv < 1 || H % Hkv) return B200_ERR_BAD_SHAPE;
   if ((S + kBwBM - 1) / kBwBM > 65535 || (long long)H * B > 0x7fffffffLL) return B200_ERR_UNSUPPORTED;
   if ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(dout) |

@@ -480,20 +480,22 @@ static int fused_qkv(const void* qkv, long long rows, FlashTcParams& p, int D, i
 }  // namespace b200
 using namespace b200;
 
-static int tc_check(const void* qkv, const void* out, int B, int S, int H, int Hkv, int D, int dtype) {
-  if ((D != 64 && D != 128) || (dtype != B200_DT_BF16 && dtype != B200_DT_FP16)) return B200_ERR_UNSUPPORTED;
+// The scale is above zero here: scores are masked before they are multiplied by it, and a masked one, minus infinity, would become NaN
+// (times 0) or plus infinity. The mma.sync kernels multiply first and take any scale.
+static int tc_check(const void* qkv, const void* out, int B, int S, int H, int Hkv, int D, float scale, int dtype) {
+  if ((D != 64 && D != 128) || (dtype != B200_DT_BF16 && dtype != B200_DT_FP16) || !(scale > 0.f)) return B200_ERR_UNSUPPORTED;
   if (B < 1 || S < 1 || H < 1 || Hkv < 1 || H % Hkv) return B200_ERR_BAD_SHAPE;
   if (H > 65535 || B > 65535) return B200_ERR_UNSUPPORTED;
   if ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(out)) & 15) return B200_ERR_BAD_ALIGN;
   return 0;
 }
 
-// Causal (or full) attention forward on the tcgen05 path. head_dim 64 or 128, 16-bit, no dropout. qkv [B*S, (H + 2 Hkv) * D],
+// Causal (or full) attention forward on the tcgen05 path. head_dim 64 or 128, 16-bit, no dropout, scale > 0. qkv [B*S, (H + 2 Hkv) * D],
 // out [B*S, H * D], lse [B, H, S] or NULL. Returns B200_ERR_UNSUPPORTED for shapes it does not cover (the caller then
 // takes b200_flash_attn_fwd).
 B200_API int b200_flash_attn_fwd_tc(const void* qkv, void* out, float* lse, int B, int S, int H, int Hkv, int D, int causal,
                                     float scale, int dtype, void* stream) {
-  if (int rc = tc_check(qkv, out, B, S, H, Hkv, D, dtype)) return rc;
+  if (int rc = tc_check(qkv, out, B, S, H, Hkv, D, scale, dtype)) return rc;
   FlashTcParams p = {};
   p.out = out; p.lse = lse; p.S = S; p.H = H; p.Hkv = Hkv; p.out_rs = (long long)H * D;
   p.scale_log2 = scale * kTcLog2e; p.causal = causal;
@@ -503,7 +505,7 @@ B200_API int b200_flash_attn_fwd_tc(const void* qkv, void* out, float* lse, int 
 // The packed form (see b200_flash_attn_varlen_fwd): `tokens` rows hold n_seqs sequences back to back, the longest of max_seqlen rows.
 B200_API int b200_flash_attn_varlen_fwd_tc(const void* qkv, void* out, const int* cu_seqlens, long long tokens, int n_seqs, int max_seqlen,
                                            int H, int Hkv, int D, int causal, float scale, int dtype, void* stream) {
-  if (int rc = tc_check(qkv, out, n_seqs, max_seqlen, H, Hkv, D, dtype)) return rc;
+  if (int rc = tc_check(qkv, out, n_seqs, max_seqlen, H, Hkv, D, scale, dtype)) return rc;
   if (!cu_seqlens || tokens < 1) return B200_ERR_BAD_SHAPE;
   FlashTcParams p = {};
   p.out = out; p.cu = cu_seqlens; p.S = max_seqlen; p.H = H; p.Hkv = Hkv; p.out_rs = (long long)H * D;
@@ -519,9 +521,9 @@ B200_API int b200_paged_attn_tc(const void* q, long long tokens, const void* ck,
                                 int D, int block_size, float scale, int window, int keep_first, float post, const b200_attn_opts* opts,
                                 int dtype, void* stream) {
   if (n_tiles <= 0) return 0;
-  if (int rc = tc_check(q, out, 1, 1, H, G, D, dtype)) return rc;
+  if (int rc = tc_check(q, out, 1, 1, H, G, D, scale, dtype)) return rc;
   const b200_attn_opts opt = opts ? *opts : b200_attn_opts{};
-  if (opt.chunk < 0 || (opt.chunk > 0 && window > 0) || !(opt.softcap >= 0.f) || !(scale > 0.f)) return B200_ERR_UNSUPPORTED;
+  if (opt.chunk < 0 || (opt.chunk > 0 && window > 0) || !(opt.softcap >= 0.f)) return B200_ERR_UNSUPPORTED;
   const int rep = H / G;
   if ((rep & 1) && !tile_of) return B200_ERR_UNSUPPORTED;
   if (((reinterpret_cast<uintptr_t>(ck) | reinterpret_cast<uintptr_t>(cv)) & 15) || ldo % 8 || pool_rows > 0x7fffffffLL) return B200_ERR_UNSUPPORTED;

@@ -394,7 +394,7 @@ int b200_flash_attn_bwd(const void* qkv, const void* out, const void* dout, cons
                         float dropout_p, unsigned long long seed, int dtype, void* stream);
 /* The same forward on the 5th-generation tensor cores (csrc/flash_tc.cu): tcgen05.mma for Q K^T and P V with both
  * accumulators in TMEM, Q / K / V tiles by TMA straight from qkv, one softmax thread per query row. head_dim 64 or 128, 16-bit
- * dtypes, no dropout; returns B200_ERR_UNSUPPORTED for anything else (callers then use b200_flash_attn_fwd). B * S rows
+ * dtypes, scale > 0, no dropout; returns B200_ERR_UNSUPPORTED for anything else (callers then use b200_flash_attn_fwd). B * S rows
  * of qkv must be addressable as one 2-D tensor map (row stride (H + 2 Hkv) * D elements, 16-byte aligned base). */
 int b200_flash_attn_fwd_tc(const void* qkv, void* out, float* lse, int B, int S, int H, int Hkv, int D, int causal,
                            float scale, int dtype, void* stream);
@@ -412,7 +412,7 @@ int b200_paged_attn_tc(const void* q, long long tokens, const void* ck, const vo
 /* Backward on the same tensor cores (csrc/flash_bwd_tc.cu): a dK/dV pass (K, V resident per 128-key block, query tiles
  * stream) and a dQ pass (Q, dO resident per 128-row tile, key blocks stream), every product a tcgen05.mma with TMEM
  * accumulators; no atomics and no fp32 staging buffer (delta [B, H, S] is the only work buffer). head_dim 64 or 128, 16-bit,
- * no dropout; B200_ERR_UNSUPPORTED otherwise. */
+ * scale > 0, no dropout; B200_ERR_UNSUPPORTED otherwise. */
 int b200_flash_attn_bwd_tc(const void* qkv, const void* out, const void* dout, const float* lse, float* delta, void* dqkv,
                            int B, int S, int H, int Hkv, int D, int causal, float scale, int dtype, void* stream);
 

@@ -156,3 +156,35 @@ def test_fused_qkv_backward(B, S, H, Hkv, D, causal):
     for lo, hi in ((0, H * D), (H * D, (H + Hkv) * D), ((H + Hkv) * D, (H + 2 * Hkv) * D)):
         a, b = qkv.grad[:, lo:hi].double(), x.grad[:, lo:hi]
         assert (a - b).norm() <= 4 * 2 * 2.0 ** -9 * b.norm() + 2.0 ** -9 * go.double().norm() * (S == 1)
+
+
+def exact_fused(x, B, S, H, Hkv, D, causal, scale):
+    """Context [B * S, H * D] of the fused projection ``x`` in its own precision (float64 here), differentiable."""
+    t = x.view(B, S, H + 2 * Hkv, D).transpose(1, 2)
+    q, k, v = t[:, :H], t[:, H:H + Hkv].repeat_interleave(H // Hkv, 1), t[:, H + Hkv:].repeat_interleave(H // Hkv, 1)
+    sc = q @ k.transpose(-1, -2) * scale
+    if causal:
+        sc = sc.masked_fill(~torch.ones(S, S, dtype=torch.bool, device=x.device).tril(), float("-inf"))
+    return (sc.softmax(-1) @ v).transpose(1, 2).reshape(B * S, H * D)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("scale", [0.0, -0.1])
+def test_scale_not_positive(D, scale):
+    """Equal weights (scale 0) and reversed ones under the causal mask: a masked score stays minus infinity whatever it is multiplied by."""
+    from llm_in_practise_b200.ops.flash import flash_attention, flash_attention_varlen
+    B, S, H, Hkv = 2, 130, 4, 2
+    g = torch.Generator(device="cuda").manual_seed(6)
+    qkv = torch.randn(B * S, (H + 2 * Hkv) * D, device="cuda", generator=g).to(torch.bfloat16).requires_grad_()
+    go = torch.randn(B * S, H * D, device="cuda", generator=g).to(torch.bfloat16)
+    out = flash_attention(qkv, B, S, H, Hkv, D, True, scale)
+    out.backward(go)
+    x = qkv.detach().double().requires_grad_()
+    want = exact_fused(x, B, S, H, Hkv, D, True, scale)
+    want.backward(go.double())
+    close(out.detach(), want.detach().cpu(), vmax=16.0)
+    for lo, hi in ((0, H * D), (H * D, (H + Hkv) * D), ((H + Hkv) * D, (H + 2 * Hkv) * D)):
+        a, b = qkv.grad[:, lo:hi].double(), x.grad[:, lo:hi]       # the bound of test_fused_qkv_backward; exactly zero at scale 0
+        assert (a - b).norm() <= 4 * 2 * 2.0 ** -9 * b.norm()
+    cu = torch.tensor([0, S, 2 * S], dtype=torch.int32, device="cuda")
+    close(flash_attention_varlen(qkv.detach(), cu, S, H, Hkv, D, scale), want.detach().cpu(), vmax=16.0)
