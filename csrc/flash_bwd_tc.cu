@@ -163,7 +163,9 @@ __device__ __forceinline__ uint32_t bw_pack16(float a, float b) {
 }
 
 // MODE_Q false: dK / dV of one 128-key block (K, V resident, query tiles stream). MODE_Q true: dQ of one 128-row query tile
-// (Q, dO resident, key blocks stream). tmq: tensor map over qkv [B*S, W]; tmd: over dout [B*S, H*D]; both box {64, 64}.
+// (Q, dO resident, key blocks stream). tmq: tensor map over qkv [B, S, W]; tmd: over dout [B, S, H*D]; both box {64, 64, 1}. The
+// entry of the batch is a dimension of its own so that rows past its end arrive as zeros: with their scores masked alone, what lies
+// there (the next entry's rows) would still be multiplied by zero, and a NaN among it would arrive in the sums.
 template <bool BF16, bool MODE_Q, int D>
 __global__ void __launch_bounds__(kBwThreads, 1)
 flash_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CUtensorMap tmd, const FlashBwdTcParams p) {
@@ -221,9 +223,9 @@ flash_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_consta
       for (int half = 0; half < kHalves; ++half)
         for (int rb = 0; rb < 2; ++rb) {
           const uint32_t dst = sRes + half * 16384 + rb * 8192;
-          const int row = row_base + r0 + rb * 64;
-          tma_load_2d(dst, &tmq, res_full, (MODE_Q ? hq * D : kcol) + half * 64, row);
-          tma_load_2d(dst + L::kRes, MODE_Q ? &tmd : &tmq, res_full, (MODE_Q ? hq * D : vcol) + half * 64, row);
+          const int row = r0 + rb * 64;
+          tma_load_3d(dst, &tmq, res_full, (MODE_Q ? hq * D : kcol) + half * 64, row, b);
+          tma_load_3d(dst + L::kRes, MODE_Q ? &tmd : &tmq, res_full, (MODE_Q ? hq * D : vcol) + half * 64, row, b);
         }
       for (int n = 0; n < n_iter; ++n) {
         const int s = n % NST;
@@ -233,8 +235,8 @@ flash_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_consta
         mbar_arrive_expect_tx(st_full0 + 8 * s, L::kStage);
         const uint32_t dst = sRing + s * L::kStage;
         for (int half = 0; half < kHalves; ++half) {       // Q and dO, or K and V
-          tma_load_2d(dst + half * 8192, &tmq, st_full0 + 8 * s, (MODE_Q ? kcol : qh * D) + half * 64, row_base + row);
-          tma_load_2d(dst + L::kTile + half * 8192, MODE_Q ? &tmq : &tmd, st_full0 + 8 * s, (MODE_Q ? vcol : qh * D) + half * 64, row_base + row);
+          tma_load_3d(dst + half * 8192, &tmq, st_full0 + 8 * s, (MODE_Q ? kcol : qh * D) + half * 64, row, b);
+          tma_load_3d(dst + L::kTile + half * 8192, MODE_Q ? &tmq : &tmd, st_full0 + 8 * s, (MODE_Q ? vcol : qh * D) + half * 64, row, b);
         }
       }
     }
@@ -461,11 +463,11 @@ B200_API int b200_flash_attn_bwd_tc(const void* qkv, const void* out, const void
   const long long W = (long long)(H + 2 * Hkv) * D;
   CUtensorMap tmq, tmd;
   {
-    uint64_t dims[2] = {(uint64_t)W, (uint64_t)B * (uint64_t)S}, str[1] = {(uint64_t)W * 2};
-    uint32_t box[2] = {64, 64};
-    if (int rc = make_tensor_map(&tmq, qkv, 2, 2, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
-    uint64_t dims2[2] = {(uint64_t)H * D, (uint64_t)B * (uint64_t)S}, str2[1] = {(uint64_t)H * D * 2};
-    if (int rc = make_tensor_map(&tmd, dout, 2, 2, dims2, str2, box, CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
+    uint64_t dims[3] = {(uint64_t)W, (uint64_t)S, (uint64_t)B}, str[2] = {(uint64_t)W * 2, (uint64_t)W * 2 * S};
+    uint32_t box[3] = {64, 64, 1};
+    if (int rc = make_tensor_map(&tmq, qkv, 2, 3, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
+    uint64_t dims2[3] = {(uint64_t)H * D, (uint64_t)S, (uint64_t)B}, str2[2] = {(uint64_t)H * D * 2, (uint64_t)H * D * 2 * S};
+    if (int rc = make_tensor_map(&tmd, dout, 2, 3, dims2, str2, box, CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
   }
   FlashBwdTcParams p = {};
   p.dqkv = dqkv; p.lse = lse; p.delta = delta; p.B = B; p.S = S; p.H = H; p.Hkv = Hkv; p.W = W;

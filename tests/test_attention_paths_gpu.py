@@ -188,3 +188,24 @@ def test_scale_not_positive(D, scale):
         assert (a - b).norm() <= 4 * 2 * 2.0 ** -9 * b.norm()
     cu = torch.tensor([0, S, 2 * S], dtype=torch.int32, device="cuda")
     close(flash_attention_varlen(qkv.detach(), cu, S, H, Hkv, D, scale), want.detach().cpu(), vmax=16.0)
+
+
+@pytest.mark.parametrize("S", [1, 65, 129, 200])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("causal", [True, False])
+def test_backward_leaves_neighbours_alone(S, D, causal):
+    """The last tile of a batch entry ends inside the entry behind it: NaN there (queries, keys, values, gradient) must not arrive."""
+    from llm_in_practise_b200.ops.flash import flash_attention
+    H, Hkv = 4, 2
+    g = torch.Generator(device="cuda").manual_seed(7)
+    qkv = torch.randn(2 * S, (H + 2 * Hkv) * D, device="cuda", generator=g).to(torch.bfloat16)
+    go = torch.randn(2 * S, H * D, device="cuda", generator=g).to(torch.bfloat16)
+    grads = []
+    for poison in (False, True):
+        x, d = qkv.clone(), go.clone()
+        if poison:
+            x[S:], d[S:] = float("nan"), float("nan")
+        x.requires_grad_()
+        flash_attention(x, 2, S, H, Hkv, D, causal, D ** -0.5).backward(d)
+        grads.append(x.grad[:S])
+    assert torch.equal(*grads)
