@@ -26,6 +26,8 @@
 #include "mma_sync.cuh"
 
 #include <type_traits>
+
+#include <type_traits>
 #include "../include/b200_ops.h"
 
 #define B200_DISPATCH_T(dtype, ...)                                   \
@@ -624,7 +626,14 @@ multimap_attn_vec_kernel(const T* __restrict__ q, const T* __restrict__ ck, cons
 // times what the memory's latency asks for).
 // 64 sequences at contexts of 3300 - 4000, 16 heads over 4 KV groups of 128 (484 MB of keys and values): 410 us in the vector
 // kernel (1.2 TB/s), 87 us here (5.6 TB/s).
+// A value that is infinite would make NaN of the two terms (the second of P may be zero or negative); a warp whose sums hold a NaN at the
+// end walks its keys once more with such values left out of the second product: the first one alone says what they come to.
 constexpr int kDmKeys = 16, kDmStages = 3;
+
+// two bf16 numbers, those that are infinite or NaN replaced by zero
+__device__ __forceinline__ uint32_t finite_bf16x2(uint32_t w) {
+  return ((w & 0x7f80u) == 0x7f80u ? 0u : w & 0xffffu) | ((w & 0x7f800000u) == 0x7f800000u ? 0u : w & 0xffff0000u);
+}
 
 template <int D, int DV, int ROWS>
 __global__ void __launch_bounds__(128, 2)
@@ -697,97 +706,110 @@ multimap_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloa
       cp_async16_zfill(dv + r * (DV * 2) + ((cc ^ (r & 7)) << 4), cv + (long long)max(pr, 0) * DV + cc * 8, pr >= 0);
     }
   };
-  lookup(0);
+  float o[DV / 8][4], mx[2], l[2];
+  // AGAIN: the second walk over the same keys, see above
+  auto walk = [&](auto again) {
+    constexpr bool AGAIN = decltype(again)::value;
+    lookup(0);
 #pragma unroll
-  for (int x = 0; x < kDmStages - 1; ++x) {
-    if (x < nt) fetch(x);
-    cp_async_commit();
-    lookup(x + 1);
-  }
-  float o[DV / 8][4];
-#pragma unroll
-  for (int n = 0; n < DV / 8; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
-  float mx[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
-  int stage = 0;
-  for (int tile = 0; tile < nt; ++tile) {
-    cp_async_wait<kDmStages - 2>();
-    __syncwarp();                                         // the tile is there for every lane, and the one before it is read
-    if (tile + kDmStages - 1 < nt) fetch(stage == 0 ? kDmStages - 1 : stage - 1);
-    cp_async_commit();
-    lookup(tile + kDmStages);
-    const uint32_t sk = sbase + stage * kStage, sv = sk + kDmKeys * D * 2;
-    stage = stage + 1 == kDmStages ? 0 : stage + 1;
-    float s[2][4];
-#pragma unroll
-    for (int n = 0; n < 2; ++n) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
-#pragma unroll
-    for (int k = 0; k < D / 16; k += 2)
-#pragma unroll
-      for (int n = 0; n < 2; ++n) {
-        const int r = n * 8 + (lane & 7), c = k * 2 + (lane >> 3);
-        uint32_t b0, b1, b2, b3;
-        ldsm_x4(sk + r * (D * 2) + ((c ^ (r & 7)) << 4), b0, b1, b2, b3);
-        mma_bf16_16816(s[n], qa[k][0], qa[k][1], qa[k][2], qa[k][3], b0, b1);
-        mma_bf16_16816(s[n], qa[k + 1][0], qa[k + 1][1], qa[k + 1][2], qa[k + 1][3], b2, b3);
-      }
-    const int left = i_hi - (i_lo + (tile * 4 + warp) * kDmKeys);       // keys of this tile inside the range
-    float top[2] = {-INFINITY, -INFINITY};
-#pragma unroll
-    for (int n = 0; n < 2; ++n)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        float x = s[n][j] * sl2;
-        if (capped) x = cap2 * tanh_ex2(x);
-        if (n * 8 + 2 * (lane & 3) + (j & 1) >= left) x = -INFINITY;
-        s[n][j] = x;
-        top[j >> 1] = fmaxf(top[j >> 1], x);
-      }
-    uint32_t hi[4], res[4];                               // P as A fragments: rounded to bf16, and what the rounding left
-    bool moved = false;
-    float ms[2], r_[2];
-#pragma unroll
-    for (int x = 0; x < ROWS / 8; ++x) {
-      top[x] = fmaxf(top[x], __shfl_xor_sync(0xffffffffu, top[x], 1));
-      top[x] = fmaxf(top[x], __shfl_xor_sync(0xffffffffu, top[x], 2));
-      const float mn = fmaxf(mx[x], top[x]);
-      ms[x] = mn == -INFINITY ? 0.f : mn;
-      r_[x] = ex2_approx(mx[x] - ms[x]);
-      moved |= mn != mx[x];
-      mx[x] = mn;
+    for (int x = 0; x < kDmStages - 1; ++x) {
+      if (x < nt) fetch(x);
+      cp_async_commit();
+      lookup(x + 1);
     }
-    if (__any_sync(0xffffffffu, moved)) {
+#pragma unroll
+    for (int n = 0; n < DV / 8; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
+    mx[0] = mx[1] = -INFINITY;
+    l[0] = l[1] = 0.f;
+    int stage = 0;
+    for (int tile = 0; tile < nt; ++tile) {
+      cp_async_wait<kDmStages - 2>();
+      __syncwarp();                                         // the tile is there for every lane, and the one before it is read
+      if (tile + kDmStages - 1 < nt) fetch(stage == 0 ? kDmStages - 1 : stage - 1);
+      cp_async_commit();
+      lookup(tile + kDmStages);
+      const uint32_t sk = sbase + stage * kStage, sv = sk + kDmKeys * D * 2;
+      stage = stage + 1 == kDmStages ? 0 : stage + 1;
+      float s[2][4];
+#pragma unroll
+      for (int n = 0; n < 2; ++n) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
+#pragma unroll
+      for (int k = 0; k < D / 16; k += 2)
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+          const int r = n * 8 + (lane & 7), c = k * 2 + (lane >> 3);
+          uint32_t b0, b1, b2, b3;
+          ldsm_x4(sk + r * (D * 2) + ((c ^ (r & 7)) << 4), b0, b1, b2, b3);
+          mma_bf16_16816(s[n], qa[k][0], qa[k][1], qa[k][2], qa[k][3], b0, b1);
+          mma_bf16_16816(s[n], qa[k + 1][0], qa[k + 1][1], qa[k + 1][2], qa[k + 1][3], b2, b3);
+        }
+      const int left = i_hi - (i_lo + (tile * 4 + warp) * kDmKeys);       // keys of this tile inside the range
+      float top[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float x = s[n][j] * sl2;
+          if (capped) x = cap2 * tanh_ex2(x);
+          if (n * 8 + 2 * (lane & 3) + (j & 1) >= left) x = -INFINITY;
+          s[n][j] = x;
+          top[j >> 1] = fmaxf(top[j >> 1], x);
+        }
+      uint32_t hi[4], res[4];                               // P as A fragments: rounded to bf16, and what the rounding left
+      bool moved = false;
+      float ms[2], r_[2];
 #pragma unroll
       for (int x = 0; x < ROWS / 8; ++x) {
-        l[x] *= r_[x];
-#pragma unroll
-        for (int n = 0; n < DV / 8; ++n) { o[n][2 * x] *= r_[x]; o[n][2 * x + 1] *= r_[x]; }
+        top[x] = fmaxf(top[x], __shfl_xor_sync(0xffffffffu, top[x], 1));
+        top[x] = fmaxf(top[x], __shfl_xor_sync(0xffffffffu, top[x], 2));
+        const float mn = fmaxf(mx[x], top[x]);
+        ms[x] = mn == -INFINITY ? 0.f : mn;
+        r_[x] = ex2_approx(mx[x] - ms[x]);
+        moved |= mn != mx[x];
+        mx[x] = mn;
       }
-    }
+      if (__any_sync(0xffffffffu, moved)) {
 #pragma unroll
-    for (int x = 0; x < 2; ++x)
+        for (int x = 0; x < ROWS / 8; ++x) {
+          l[x] *= r_[x];
 #pragma unroll
-      for (int n = 0; n < 2; ++n) {
-        if (x < ROWS / 8) {
-          const float p0 = ex2_approx(s[n][2 * x] - ms[x < ROWS / 8 ? x : 0]), p1 = ex2_approx(s[n][2 * x + 1] - ms[x < ROWS / 8 ? x : 0]);
-          l[x] += p0 + p1;
-          const uint32_t w = pack_bf16x2(p0, p1);
-          const float2 f = unpack_bf16x2(w);
-          hi[n * 2 + x] = w;
-          res[n * 2 + x] = pack_bf16x2(p0 - f.x, p1 - f.y);
-        } else hi[n * 2 + x] = res[n * 2 + x] = 0u;
+          for (int n = 0; n < DV / 8; ++n) { o[n][2 * x] *= r_[x]; o[n][2 * x + 1] *= r_[x]; }
+        }
       }
 #pragma unroll
-    for (int n = 0; n < DV / 8; n += 2) {
-      const int r = lane & 15, c = n + (lane >> 4);
-      uint32_t b0, b1, b2, b3;
-      ldsm_x4_trans(sv + r * (DV * 2) + ((c ^ (r & 7)) << 4), b0, b1, b2, b3);
-      mma_bf16_16816(o[n], hi[0], hi[1], hi[2], hi[3], b0, b1);
-      mma_bf16_16816(o[n + 1], hi[0], hi[1], hi[2], hi[3], b2, b3);
-      mma_bf16_16816(o[n], res[0], res[1], res[2], res[3], b0, b1);
-      mma_bf16_16816(o[n + 1], res[0], res[1], res[2], res[3], b2, b3);
+      for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+          if (x < ROWS / 8) {
+            const float p0 = ex2_approx(s[n][2 * x] - ms[x < ROWS / 8 ? x : 0]), p1 = ex2_approx(s[n][2 * x + 1] - ms[x < ROWS / 8 ? x : 0]);
+            l[x] += p0 + p1;
+            const uint32_t w = pack_bf16x2(p0, p1);
+            const float2 f = unpack_bf16x2(w);
+            hi[n * 2 + x] = w;
+            res[n * 2 + x] = pack_bf16x2(p0 - f.x, p1 - f.y);
+          } else hi[n * 2 + x] = res[n * 2 + x] = 0u;
+        }
+#pragma unroll
+      for (int n = 0; n < DV / 8; n += 2) {
+        const int r = lane & 15, c = n + (lane >> 4);
+        uint32_t b0, b1, b2, b3;
+        ldsm_x4_trans(sv + r * (DV * 2) + ((c ^ (r & 7)) << 4), b0, b1, b2, b3);
+        mma_bf16_16816(o[n], hi[0], hi[1], hi[2], hi[3], b0, b1);
+        mma_bf16_16816(o[n + 1], hi[0], hi[1], hi[2], hi[3], b2, b3);
+        if (AGAIN) { b0 = finite_bf16x2(b0); b1 = finite_bf16x2(b1); b2 = finite_bf16x2(b2); b3 = finite_bf16x2(b3); }
+        mma_bf16_16816(o[n], res[0], res[1], res[2], res[3], b0, b1);
+        mma_bf16_16816(o[n + 1], res[0], res[1], res[2], res[3], b2, b3);
+      }
     }
-  }
-  cp_async_wait<0>();
+    cp_async_wait<0>();
+    bool odd = false;
+#pragma unroll
+    for (int n = 0; n < DV / 8; ++n)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) odd |= o[n][j] != o[n][j];
+    return __any_sync(0xffffffffu, odd);                  // the vote also ends every lane's reads of the tiles
+  };
+  if (walk(std::false_type{})) walk(std::true_type{});
   __syncthreads();                                        // every warp is done with its tiles: their place takes the results
   constexpr int LDW = DV + 2;
 #pragma unroll

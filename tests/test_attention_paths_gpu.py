@@ -209,3 +209,26 @@ def test_backward_leaves_neighbours_alone(S, D, causal):
         flash_attention(x, 2, S, H, Hkv, D, causal, D ** -0.5).backward(d)
         grads.append(x.grad[:S])
     assert torch.equal(*grads)
+
+
+@pytest.mark.parametrize("H,G,M,D,Dv", [(16, 4, 1, 128, 128), (12, 1, 1, 64, 64), (4, 2, 2, 64, 128)])
+def test_decode_values_not_finite(H, G, M, D, Dv):
+    """An infinite value weighted by a probability above zero is infinite, and it stays in its own column."""
+    rows = [1, 5, 70, 300]
+    ck, cv, table, g = pools(rows, G, M, D, Dv, 16)
+    inf = float("inf")
+    for i, n in enumerate(rows):                                   # (key, column, value): the first key, one inside and the last
+        for key, col, v in ((0, 0, inf), (n // 2, 3, -inf), (n - 1, Dv - 1, inf), (n // 3, 8, float("nan")), (0, 9, inf), (n - 1, 9, -inf)):
+            cv[table[i, key // 16], :, key % 16, col] = v
+    T = len(rows)
+    q = torch.randn(T, H * M * D, generator=g).to(torch.bfloat16)
+    pos, slot = torch.tensor([n - 1 for n in rows], dtype=torch.int32), torch.arange(T, dtype=torch.int32)
+    args = (ck, cv, table, pos, slot, H, G, M, D, Dv, D ** -0.5)
+    want = multimap_attention(q, *args).float()
+    dev = lambda v: v.cuda() if isinstance(v, torch.Tensor) else v                                  # noqa: E731
+    for max_pos in (0, 299):
+        got = multimap_attention(q.cuda(), *map(dev, args), max_pos=max_pos).float().cpu()
+        finite = want.isfinite()
+        assert torch.equal(got.isfinite(), finite)
+        assert torch.equal(got[~finite].nan_to_num(nan=0.0), want[~finite].nan_to_num(nan=0.0))
+        close(got[finite], want[finite])
