@@ -107,8 +107,8 @@ __device__ __forceinline__ uint32_t pack16(float a, float b) {
   return *reinterpret_cast<const uint32_t*>(&hh);
 }
 
-// tanh for capped scores: by its power series where every score of the warp is small (|x| <= 1/4: the next term is below 3e-9 of x),
-// else 1 - 2 / (1 + e^(2x)) on the hardware's exponential (a few 1e-7 absolute)
+// tanh for capped scores: by its power series where every score that the row sees in the block is small (|x| <= 1/4: the next term is
+// below 3e-9 of x), else 1 - 2 / (1 + e^(2x)) on the hardware's exponential (a few 1e-7 absolute)
 __device__ __forceinline__ float tanh_small(float x) {
   const float y = x * x;
   return x * fmaf(y, fmaf(y, fmaf(y, fmaf(y, 62.f / 2835.f, -17.f / 315.f), 2.f / 15.f), -1.f / 3.f), 1.f);
@@ -304,28 +304,39 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
       tmem_ld_32x32(tS + sb * kTcBN, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
       tmem_ld_32x32(tS + sb * kTcBN + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[32]));
       tmem_ld_wait();
+      // Keys the row does not see are taken out before the row chooses its form of tanh, and each row chooses for itself: its result
+      // must not depend on what lies behind the sequence, or in its window's other end, nor on the other rows of the tile.
+      auto hidden = [&](int kp) { return MODE == kTcPaged ? (kp > lim || (kp < low && kp >= keepW)) : kp > lim; };
       if (CAP) {
         float big = 0.f;
 #pragma unroll
-        for (int i = 0; i < 64; ++i) {
-          const float x = __uint_as_float(v[i]) * p.cin;
-          big = fmaxf(big, fabsf(x));
-          v[i] = __float_as_uint(x);
-        }
-        if (__any_sync(0xffffffffu, big > 0.25f)) {
+        for (int i = 0; i < 64; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * p.cin);
+        if (need_mask) {
 #pragma unroll
-          for (int i = 0; i < 64; ++i) v[i] = __float_as_uint(tanh_any(__uint_as_float(v[i])));
-        } else {                                          // small scores: the series takes fewer cycles than two special functions
+          for (int i = 0; i < 64; ++i)
+            if (hidden(kv0 + i)) v[i] = 0u;
+        }
+#pragma unroll
+        for (int i = 0; i < 64; ++i) big = fmaxf(big, fabsf(__uint_as_float(v[i])));
+        // Small scores: the series takes fewer cycles than two special functions. Only the warp's branches are decided together (its
+        // lanes stay in step for the TMEM accesses below); rows past the end of a short piece go along with the others.
+        const bool large = big > 0.25f, dead = MODE == kTcPaged && rr >= nrows;
+        if (!__any_sync(0xffffffffu, large && !dead)) {
 #pragma unroll
           for (int i = 0; i < 64; ++i) v[i] = __float_as_uint(tanh_small(__uint_as_float(v[i])));
+        } else if (__all_sync(0xffffffffu, large || dead)) {
+#pragma unroll
+          for (int i = 0; i < 64; ++i) v[i] = __float_as_uint(tanh_any(__uint_as_float(v[i])));
+        } else {
+#pragma unroll
+          for (int i = 0; i < 64; ++i) v[i] = __float_as_uint(large ? tanh_any(__uint_as_float(v[i])) : tanh_small(__uint_as_float(v[i])));
         }
       }
       float mx = -INFINITY;
       if (need_mask) {
 #pragma unroll
         for (int i = 0; i < 64; ++i) {
-          const int kp = kv0 + i;
-          if (MODE == kTcPaged ? (kp > lim || (kp < low && kp >= keepW)) : kp > lim) v[i] = 0xff800000u;    // -inf
+          if (hidden(kv0 + i)) v[i] = 0xff800000u;        // -inf
         }
       }
 #pragma unroll

@@ -152,30 +152,12 @@ multimap_attn_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat1
 #pragma unroll
         for (int n = 0; n < 8; ++n) mma_bf16_16816(s[n], qa[k][0], qa[k][1], qa[k][2], qa[k][3], b[n][0], b[n][1]);
       }
-      if (capped) {
-        float big = 0.f;
-#pragma unroll
-        for (int n = 0; n < 8; ++n)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) { s[n][j] *= cin; big = fmaxf(big, fabsf(s[n][j])); }
-        if (__any_sync(0xffffffffu, big > 0.25f)) {
-#pragma unroll
-          for (int n = 0; n < 8; ++n)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) s[n][j] = tanh_ex2(s[n][j]);
-        } else {                                          // small scores: the series takes fewer cycles than two special functions
-#pragma unroll
-          for (int n = 0; n < 8; ++n)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) s[n][j] = tanh_series(s[n][j]);
-        }
-      }
       // mask: key j is seen from position i iff j <= i and (j >= the low end of i's window or chunk, or j < keep_first). Blocks
       // wholly inside every row's range skip the test (uniform over the warp).
       const int k0 = kb * kK;
       const bool diag = k0 + kK - 1 > pos0 + warp * 16;
       const bool edge = k0 < low_w && k0 + kK - 1 >= keepW;
-      if (diag || edge) {
+      auto hide = [&](float with) {
         const int kbase = k0 + 2 * (lane & 3);
 #pragma unroll
         for (int n = 0; n < 8; ++n) {
@@ -183,10 +165,44 @@ multimap_attn_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat1
           for (int j = 0; j < 4; ++j) {
             const int kj = kbase + n * 8 + (j & 1), qi = qpos0 + (j >> 1) * 8;
             const bool seen = kj <= qi && (kj >= (j >> 1 ? low_b : low_a) || kj < keepW);
-            if (!seen) s[n][j] = -INFINITY;
+            if (!seen) s[n][j] = with;
           }
         }
+      };
+      if (capped) {
+        // each row chooses its form of tanh by the scores it sees: its result must not depend on other rows, or on rows behind the sequence
+        if (diag || edge) hide(0.f);
+        float big[2] = {0.f, 0.f};
+#pragma unroll
+        for (int n = 0; n < 8; ++n)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) { s[n][j] *= cin; big[j >> 1] = fmaxf(big[j >> 1], fabsf(s[n][j])); }
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          big[x] = fmaxf(big[x], __shfl_xor_sync(0xffffffffu, big[x], 1));
+          big[x] = fmaxf(big[x], __shfl_xor_sync(0xffffffffu, big[x], 2));
+        }
+        // small scores: the series takes fewer cycles than two special functions. Only the warp's branches are decided together: its lanes
+        // stay in step for the products below
+        const bool large[2] = {big[0] > 0.25f, big[1] > 0.25f};
+        if (!__any_sync(0xffffffffu, large[0] || large[1])) {
+#pragma unroll
+          for (int n = 0; n < 8; ++n)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) s[n][j] = tanh_series(s[n][j]);
+        } else if (__all_sync(0xffffffffu, large[0] && large[1])) {
+#pragma unroll
+          for (int n = 0; n < 8; ++n)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) s[n][j] = tanh_ex2(s[n][j]);
+        } else {
+#pragma unroll
+          for (int n = 0; n < 8; ++n)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) s[n][j] = large[j >> 1] ? tanh_ex2(s[n][j]) : tanh_series(s[n][j]);
+        }
       }
+      if (diag || edge) hide(-INFINITY);
       float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
       for (int n = 0; n < 8; ++n) {

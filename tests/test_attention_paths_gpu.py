@@ -232,3 +232,26 @@ def test_decode_values_not_finite(H, G, M, D, Dv):
         assert torch.equal(got.isfinite(), finite)
         assert torch.equal(got[~finite].nan_to_num(nan=0.0), want[~finite].nan_to_num(nan=0.0))
         close(got[finite], want[finite])
+
+
+@pytest.mark.parametrize("H,G,D", [(4, 2, 128), (3, 1, 64), (4, 2, 96)])
+def test_capped_rows_do_not_see_what_lies_behind(H, G, D):
+    """Which of the two forms of tanh a block's scores take must not depend on rows behind the sequence (large numbers or zeros there) nor on
+    the other rows of the tile. 96: the mma.sync kernel."""
+    from llm_in_practise_b200.inference.ragged import make_pieces
+    n, BS, cap = 70, 64, 1000.0                                    # scores of about 10: x = score / cap is small, its error times cap is not
+    ck, cv, table, g = pools([n], G, 1, D, D, BS)
+    q = torch.randn(n, H * D, generator=g).to(torch.bfloat16)
+    pos, slot = torch.arange(n, dtype=torch.int32), torch.zeros(n, dtype=torch.int32)
+    pieces = make_pieces([(0, n, 0, 0)], "cuda")
+    got = []
+    for behind in (0.0, 100.0):
+        ck[table[0, 1], :, n - BS:] = behind
+        got.append(multimap_attention(q.cuda(), ck.cuda(), cv.cuda(), table.cuda(), pos.cuda(), slot.cuda(), H, G, 1, D, D, 10 * D ** -0.5,
+                                      pieces=pieces, max_pos=n - 1, softcap=cap))
+    assert torch.equal(*got)
+    q[40] *= 64                                                    # one row with large scores leaves the others alone
+    again = multimap_attention(q.cuda(), ck.cuda(), cv.cuda(), table.cuda(), pos.cuda(), slot.cuda(), H, G, 1, D, D, 10 * D ** -0.5,
+                               pieces=pieces, max_pos=n - 1, softcap=cap)
+    others = torch.arange(n) != 40
+    assert torch.equal(again.cpu()[others], got[1].cpu()[others])
