@@ -255,3 +255,32 @@ def test_capped_rows_do_not_see_what_lies_behind(H, G, D):
                                pieces=pieces, max_pos=n - 1, softcap=cap)
     others = torch.arange(n) != 40
     assert torch.equal(again.cpu()[others], got[1].cpu()[others])
+
+
+@pytest.mark.parametrize("form,D", [("dense", 64), ("packed", 64), ("packed", 128), ("paged", 64), ("paged", 128)])
+def test_largest_weight_is_exact(form, D):
+    """Keys far below but for one in the first block and a somewhat larger one in the second, whose weight is then 1 in 16 bits too: the
+    first one's value is zero, so that the result is v / (1 + e^-d) with nothing rounded but the result."""
+    from llm_in_practise_b200.inference.ragged import make_pieces
+    from llm_in_practise_b200.ops.flash import flash_attention, flash_attention_varlen
+    H, S, dtype = 8, 128, torch.bfloat16
+    g = torch.Generator().manual_seed(8)
+    q, k = torch.zeros(S, H, D, dtype=dtype), torch.zeros(S, H, D, dtype=dtype)
+    v = torch.randn(S, H, D, generator=g).to(dtype)
+    d = torch.linspace(0.3, 5.0, H).to(dtype)                      # below 2^8 in weight
+    q[:, :, 0], k[:, :, 0] = 1.0, -100.0
+    k[3, :, 0], k[70, :, 0], v[3] = 0.0, d, 0.0
+    want = (v[70].double() / (1 + torch.exp(-d.double()))[:, None]).reshape(1, H * D)
+    qkv = torch.cat([q, k, v], 1).reshape(S, 3 * H * D).cuda()
+    if form == "dense":
+        got = flash_attention(qkv, 1, S, H, H, D, True, 1.0)
+    elif form == "packed":
+        got = flash_attention_varlen(qkv, torch.tensor([0, S], dtype=torch.int32, device="cuda"), S, H, H, D, 1.0)
+    else:
+        pos, slot = torch.arange(S, dtype=torch.int32, device="cuda"), torch.zeros(S, dtype=torch.int32, device="cuda")
+        page = lambda t: t.transpose(0, 1)[None].contiguous().cuda()                               # noqa: E731
+        got = multimap_attention(q.reshape(S, -1).cuda(), page(k), page(v), torch.zeros(1, 1, dtype=torch.int32, device="cuda"), pos, slot,
+                                 H, H, 1, D, D, 1.0, pieces=make_pieces([(0, S, 0, 0)], "cuda"), max_pos=S - 1)
+    got = got[70:].double().cpu()
+    half = 2.0 ** (torch.floor(torch.log2(want.abs())) - 8)        # half a step of bf16 at the result
+    assert ((got - want).abs() <= half * (1 + 2.0 ** -8)).all()    # 2^-8 of it: 2^-16 of the result, far above fp32's part
