@@ -209,6 +209,16 @@ __device__ __forceinline__ float gather4(const float4& v, int lane) {
   return z + __shfl_xor_sync(0xffffffffu, z, 4);
 }
 
+// Row t of a lower triangle times column c of X, in the layout of R and U: the columns above the diagonal are zero, and here they are not
+// multiplied either. dot_rows multiplies them, which is the same unless X holds an infinity or NaN: then it would reach rows, tokens, that
+// come before its own. So a chunk with such an R or U takes this one (a vote with the barriers that are there anyway).
+__device__ __forceinline__ float lower_dot(const float* row, const float* X, int t, int c) {
+  float s = 0.f;
+  for (int j = 0; j <= t; ++j) s = fmaf(row[j], X[pair_at(j >> 1, c) + (c & 1) * 2 + (j & 1)], s);
+  return s;
+}
+__device__ __forceinline__ bool not_finite(float x) { return !(fabsf(x) <= 3.402823466e38f); }
+
 // What limits the walk is shared memory, 128 bytes a cycle into registers against 128 FMAs: a tile of 4 x 4 outputs per thread would
 // take two bytes per FMA. So the small side of every product but the last stays in registers — S_0 with 16 rows of four columns in
 // every lane of every warp, R and U with eight — and a row of the other side costs one byte per FMA; the lanes' parts of
@@ -301,6 +311,7 @@ delta_chunk_scan_kernel(const DeltaChunkArgs p) {
     if (more) fetch_kvp(tile + 1, buf ^ 1);
     const float* Ks = sm + L::K + buf * kDcC * DP;
     const float* cs = sm + L::X + buf * 3 * kDcC;         // c | r_64 | beta
+    int odd = 0;                                          // an infinity or NaN among this thread's part of R, then of U
     // ---- [K; Q] S_0: a warp holds S_0 whole in registers, D / 8 rows of four columns per lane ----
     {
       float2 s0[D / 16][4];
@@ -325,6 +336,7 @@ delta_chunk_scan_kernel(const DeltaChunkArgs p) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             sk[i] = cs[2 * kDcC + t + i] * (sm[L::V + (buf * kDcC + t + i) * NC + cg] - cs[t + i] * sk[i]);
+            odd |= not_finite(sk[i]);
             if (!(lane & 4)) sm[L::O + (t + i) * NC + cg] = cs[t + i] * sq[i];
           }
         }
@@ -335,7 +347,7 @@ delta_chunk_scan_kernel(const DeltaChunkArgs p) {
         }
       }
     }
-    __syncthreads();
+    odd = __syncthreads_or(odd);
     if (more) fetch_q(tile + 1);
     // a lower triangle times [64, NC], the right side held in registers (eight rows of four columns per lane)
     float2 B[4][4];
@@ -356,6 +368,12 @@ delta_chunk_scan_kernel(const DeltaChunkArgs p) {
         dot_rows<8, 2>(sm + L::T + t * kDcCP + rl * 4, kDcCP, B, y);
 #pragma unroll
         for (int i = 0; i < 8; ++i) u[i] = gather4(y[i], lane);
+        if (odd) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) u[i] = lower_dot(sm + L::T + (t + i) * kDcCP, sm + L::R, t + i, cg);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) odd |= not_finite(u[i]);
       } else {
 #pragma unroll
         for (int i = 0; i < 8; ++i) u[i] = 0.f;
@@ -367,7 +385,7 @@ delta_chunk_scan_kernel(const DeltaChunkArgs p) {
         for (int i = 0; i < 8; i += 2) *reinterpret_cast<float2*>(sm + L::U + pair_at((t + i) / 2, cg) + (cg & 1) * 2) = make_float2(u[i], u[i + 1]);
       }
     }
-    __syncthreads();
+    odd = __syncthreads_or(odd);
     if (more) fetch_t(tile + 1);
     // ---- the read-out ----
     hold(sm + L::U);
@@ -380,6 +398,10 @@ delta_chunk_scan_kernel(const DeltaChunkArgs p) {
         float z[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) z[i] = gather4(y[i], lane);
+        if (odd) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) z[i] = lower_dot(sm + L::P + (buf * kDcC + t + i) * kDcCP, sm + L::U, t + i, cg);
+        }
         if (!(lane & 4)) {
 #pragma unroll
           for (int i = 0; i < 8; ++i)

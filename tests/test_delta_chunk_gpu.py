@@ -53,3 +53,26 @@ def test_chunks(lens, H, G, D, Dv, decay, monkeypatch):
     # roundings of 2^-24 of the largest value on the way, four times over for the solve and the carried state
     for got, want in ((o, want_o), (state, want_s)):
         assert ((got.double() - want).abs().max() / want.abs().max()).item() < 4 * (D + 64) * 2.0 ** -24
+
+
+@pytest.mark.parametrize("what,value", [("v", float("nan")), ("v", float("inf")), ("k", float("nan")), ("q", float("inf")), ("beta", float("nan")),
+                                        ("a", float("nan"))])
+@pytest.mark.parametrize("at", [5, 63, 100])
+def test_not_finite_stays_behind_its_token(what, value, at, monkeypatch):
+    """A NaN or infinity in one token reaches that token and the ones after it (of a value's column, of a head), never those before."""
+    g = torch.Generator(device="cuda").manual_seed(9)
+    n, H, G, D, Dv = 130, 4, 2, 64, 32
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)                                   # noqa: E731
+    q, k, v = rnd(n, G * D) * D ** -0.5, rnd(n, G * D) * D ** -0.5, rnd(n, H * Dv)
+    a, b = torch.rand(n, H, device="cuda", generator=g) * 0.5 + 0.5, torch.rand(n, H, device="cuda", generator=g)
+    {"v": v, "k": k, "q": q, "beta": b, "a": a}[what][at, 1] = value
+    runs, state = [[0, n, 3, 0]], rnd(1, H, D, Dv)
+    want_o, want_s = walk(q, k, v, state, runs, H, G, D, Dv, a, b)
+    pos = slot = torch.zeros(n, dtype=torch.int32, device="cuda")
+    monkeypatch.setattr(scan_mod, "_chunks_pay", lambda *a: True)
+    o = linear_scan(q, k, v, state, pos, slot, torch.tensor(runs, dtype=torch.int32, device="cuda"), 1, H, G, D, Dv, "head_delta", g=a, beta=b)
+    for got, want in ((o, want_o), (state, want_s)):
+        finite = want.isfinite()
+        assert torch.equal(got.isfinite(), finite)
+        # the bound of test_chunks
+        assert not finite.any() or ((got.double() - want)[finite].abs().max() / want[finite].abs().max()).item() < 4 * (D + 64) * 2.0 ** -24
