@@ -425,12 +425,9 @@ template <bool BF16, int D>
 static int launch_bwd(const CUtensorMap& tmq, const CUtensorMap& tmd, const FlashBwdTcParams& p, const void* out, const void* dout, float* delta,
                       cudaStream_t st) {
   constexpr int kSmem = (int)BwSmem<D>::kBytes;
-  static bool attr = false;
-  if (!attr) {
-    B200_CHECK(cudaFuncSetAttribute(flash_bwd_tc_kernel<BF16, false, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
-    B200_CHECK(cudaFuncSetAttribute(flash_bwd_tc_kernel<BF16, true, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
-    attr = true;
-  }
+  // per call: the attribute belongs to the current device, and a process may use several
+  B200_CHECK(cudaFuncSetAttribute(flash_bwd_tc_kernel<BF16, false, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+  B200_CHECK(cudaFuncSetAttribute(flash_bwd_tc_kernel<BF16, true, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
   const long long items = (long long)p.B * p.S * p.H;
   constexpr int per = 2 * 256 / (D / 8);
   flash_delta_tc_kernel<BF16, D><<<(unsigned)((items + per - 1) / per), 256, 0, st>>>((const uint16_t*)out, (const uint16_t*)dout, delta, items, p.S, p.H);

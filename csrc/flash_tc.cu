@@ -454,11 +454,8 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
 template <int MODE, int D, bool BF16, bool CAP>
 static int launch_tc(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FlashTcParams& p, dim3 grid, cudaStream_t st) {
   auto kern = flash_fwd_tc_kernel<MODE, D, BF16, CAP>;
-  static bool attr = false;
-  if (!attr) {
-    B200_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcSmem<D>::kBytes));
-    attr = true;
-  }
+  // per call: the attribute belongs to the current device, and a process may use several
+  B200_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcSmem<D>::kBytes));
   kern<<<grid, kTcThreads, TcSmem<D>::kBytes, st>>>(tq, tk, tv, p);
   B200_LAUNCH_CHECK();
   return 0;

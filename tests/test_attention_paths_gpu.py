@@ -284,3 +284,19 @@ def test_largest_weight_is_exact(form, D):
     got = got[70:].double().cpu()
     half = 2.0 ** (torch.floor(torch.log2(want.abs())) - 8)        # half a step of bf16 at the result
     assert ((got - want).abs() <= half * (1 + 2.0 ** -8)).all()    # 2^-8 of it: 2^-16 of the result, far above fp32's part
+
+
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="two GPUs in one process")
+def test_second_device():
+    """The opt-in to large shared memory belongs to a device: one process that uses two of them, one after the other."""
+    from llm_in_practise_b200.ops.flash import flash_attention, flash_attention_varlen
+    for D in (64, 128):
+        per = []
+        for dev in ("cuda:0", "cuda:1"):
+            with torch.cuda.device(dev):
+                x = torch.randn(130, 3 * 2 * D, generator=torch.Generator().manual_seed(9)).to(torch.bfloat16).to(dev).requires_grad_()
+                out = flash_attention(x, 1, 130, 2, 2, D, True, D ** -0.5)
+                out.backward(out.detach())
+                cu = torch.tensor([0, 130], dtype=torch.int32, device=dev)
+                per.append([t.cpu() for t in (out.detach(), x.grad, flash_attention_varlen(x.detach(), cu, 130, 2, 2, D, D ** -0.5))])
+        assert all(torch.equal(a, b) for a, b in zip(*per))
