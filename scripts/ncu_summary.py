@@ -50,8 +50,8 @@ def main():
     hdr, units = rows[0], rows[1]
     idx = {h: i for i, h in enumerate(hdr)}
     lines = [f"# {title}", "", f"Source report: `{rep}` (scratch, not tracked). Extracted with "
-             "`ncu -i <rep> --page raw --csv` by `scripts/ncu_summary.py`; capture flags "
-             "`--set full --clock-control none --import-source on`. Durations under ncu are NOT bench numbers.", ""]
+             "`ncu -i <rep> --page raw --csv` by `scripts/ncu_summary.py`. "
+             "Durations under ncu are NOT bench numbers.", ""]
     seen = {}
     for r in rows[2:]:
         name = r[idx["Kernel Name"]]
