@@ -1,7 +1,7 @@
-"""Reference arm of BASELINE config 2: the reference's OWN model code under torch DistributedDataParallel.
+"""Reference arm of the small pre-training runs: the reference's OWN model code under torch DistributedDataParallel.
 
-``baseline/_ref/`` holds unmodified copies of two reference files (``__graft_entry__.build()`` copies them from
-/root/reference; they are git-ignored and travel to the GPU box with the snapshot):
+``baseline/_ref/`` holds unmodified copies of two reference files (``__graft_entry__.build()`` copies them
+from the reference's tree; they are git-ignored):
 
     ddp_gpt_wikitext2.py   LLM_Distributed_Trainning/PyTorch/ddp_basics/ddp_gpt_wikitext2.py  (``GPTLike``, 65.97 M parameters)
     minigpt2_model.py      llm-demo/minigpt2/model.py                                         (``Config``, ``MiniGPT``)
@@ -10,7 +10,7 @@ The models are imported from those copies and trained exactly as ``ddp_gpt_wikit
 ``DistributedDataParallel(model, device_ids=[local_rank], output_device=local_rank, find_unused_parameters=False)``,
 ``optim.AdamW(lr=3e-4)``, ``nn.CrossEntropyLoss``, ``logits -> loss -> zero_grad -> backward -> step``, fp32, no AMP,
 no clipping. Only the data is synthetic (``[B, 256]`` random ids: wikitext is not reachable offline and the minigpt2
-corpus yields zero samples, SURVEY.md section 2.1-A). ``--amp bf16`` additionally times the same loop under
+corpus yields zero samples). ``--amp bf16`` additionally times the same loop under
 ``torch.autocast`` (not what the reference does; it is the stronger baseline for a bf16 framework).
 
 Nothing from ``llm_in_practise_b200`` is imported. Timing = CUDA events, barrier + synchronize on both sides, max over
@@ -30,7 +30,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 def _load(fname, modname):
     path = os.path.join(HERE, "_ref", fname)
     if not os.path.exists(path):
-        print(json.dumps({"impl": "reference", "unavailable": f"{path} is missing (run __graft_entry__.build() where /root/reference exists)"}))
+        print(json.dumps({"impl": "reference", "unavailable": f"{path} is missing (run __graft_entry__.build() where the reference's tree is present)"}))
         sys.exit(0)
     spec = importlib.util.spec_from_file_location(modname, path)
     mod = importlib.util.module_from_spec(spec)

@@ -2,7 +2,7 @@
 Fine-Tuning/qwen3-14b-qlora-dist-deepspeed.py (+ Fine-Tuning/ds_zero3_config.json).
 
 The stock script cannot run in this image: it imports peft, bitsandbytes, deepspeed and accelerate, none
-of which is installed or in /opt/wheelhouse, and /root/reference is not a pip-installable package. What
+of which is installed or available offline, and the reference is not a pip-installable package. What
 *is* in the image is the rest of that script's stack: torch 2.11 (cuBLAS, SDPA, NCCL) and transformers 5.5
 (``Qwen3ForCausalLM``, the class ``AutoModelForCausalLM`` resolves to). This file rebuilds the script's
 training step on exactly those libraries and nothing from ``llm_in_practise_b200``:
@@ -17,7 +17,7 @@ training step on exactly those libraries and nothing from ``llm_in_practise_b200
             ``fsdp2``: ``fully_shard`` per decoder layer + root (the ZeRO-3 equivalent: parameters sharded, all-gathered
             per layer in forward and backward, adapter gradients reduce-scattered), and ``ddp``: replicated base,
             ``DistributedDataParallel`` all-reduce of the adapter gradients (what the script degenerates to if DeepSpeed
-            leaves the quantised base replicated — SURVEY.md section 6)
+            leaves the quantised base replicated)
 
 Deviations from the stock script (all forced by the missing packages): the frozen base is bf16 instead of bitsandbytes
 NF4 (no dequantisation kernel in the step, 4x the bytes in the ZeRO-3 gather), the optimizer is fp32 AdamW instead of

@@ -1,4 +1,4 @@
-"""Reference arm of BASELINE config 5 and of the serving table: vLLM (the engine every serving recipe of the reference
+"""Reference arm of W4A16 inference and of the serving table: vLLM (the engine every serving recipe of the reference
 uses — ``vllm serve … --tensor-parallel-size T`` Quantization/README.md:175, Deployment/Ray/serve_run_examples/deepseek.py:26-34)
 on the same box, same model shape, random weights (``load_format="dummy"``), no tokenizer (token-id prompts).
 

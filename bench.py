@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Headline benchmark (BASELINE.json): Qwen3-14B QLoRA (NF4 base, LoRA r=8 on q_proj/v_proj, dropout 0.1,
+"""Headline benchmark: Qwen3-14B QLoRA (NF4 base, LoRA r=8 on q_proj/v_proj, dropout 0.1,
 8-bit AdamW) ZeRO-3 training throughput in tokens/s at 1/2/4/8 B200.
 
 Configuration = the reference's Fine-Tuning/qwen3-14b-qlora-dist-deepspeed.py + ds_zero3_config.json:
@@ -12,7 +12,7 @@ random-init weights of the Qwen3-14B architecture (no network for datasets or ch
         bench.py --gpus 8 --steps 10 --warmup 3
     python bench.py --impl reference ...     # the unmodified reference stack, if it can be installed
 
-Prints ONE JSON line on rank 0 (see the contract in the repo README / DESIGN.md).
+Prints ONE JSON line on rank 0 (its keys are described in the README).
 """
 from __future__ import annotations
 
@@ -108,7 +108,7 @@ class ClockSampler:
 
 def reference_arm(args):
     """``--impl reference``. The stock headline script (Fine-Tuning/qwen3-14b-qlora-dist-deepspeed.py) needs peft +
-    bitsandbytes + deepspeed + accelerate, which are neither installed nor in /opt/wheelhouse, and /root/reference has no
+    bitsandbytes + deepspeed + accelerate, which are neither installed nor available offline, and the reference has no
     setup.py / pyproject.toml to install. What runs instead is ``baseline/ref_headline.py``: the same training step on the
     part of the reference's stack that IS in the image (HF transformers ``Qwen3ForCausalLM`` + torch AdamW + torch
     FSDP2 / DDP over NCCL). It imports nothing from this repository's package and labels itself
@@ -316,7 +316,7 @@ def main():
                           "last_loss": last_loss}
         if stats:
             out["comm"] = stats
-        # second half of BASELINE.json's metric: exposed communication per optimizer step, max over ranks
+        # second half of the headline metric: exposed communication per optimizer step, max over ranks
         out["exposed_comm_ms"] = None if exposed is None else round(exposed, 3)
         print(json.dumps(out))
     if world > 1:

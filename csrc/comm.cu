@@ -5,7 +5,7 @@
 // ordering uses per-(channel, rank) epoch flags in symmetric memory: a rank publishes epoch e on
 // every peer with st.release.sys, and waits for all peers with ld.acquire.sys. Epochs only grow,
 // so flags never need resetting; every spin is bounded and traps with a message naming the
-// missing rank instead of hanging the GPU (SURVEY.md §5.3).
+// missing rank instead of hanging the GPU.
 //
 //   b200_allreduce      K-C1: two-shot all-reduce (avg) of a gradient bucket, in place, with the
 //                       1/world scale (and optional bf16 copy) fused. Replaces the c10d Reducer's

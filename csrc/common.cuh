@@ -2,8 +2,8 @@
 //
 // Everything here is inline PTX for Blackwell: mbarrier, TMA (cp.async.bulk.tensor),
 // tcgen05 (alloc / mma / commit / ld) and the proxy fences that glue them together.
-// There is no counterpart in the reference: it has no native code at all
-// (SURVEY.md §2.2); these wrap the instructions its dependency libraries would use.
+// There is no counterpart in the reference: it has no native code at
+// all; these wrap the instructions its dependency libraries would use.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -5,8 +5,8 @@
  * B200_ERR_* code (>= 10001). Nothing here synchronises the device. Entry points that need
  * temporary global memory take it from the caller (`scratch` / `workspace` arguments).
  *
- * Each declaration cites the reference call site (path:line under /root/reference) whose
- * library kernel it replaces; the reference itself contains no native code (SURVEY.md 2.2).
+ * Each declaration cites the reference call site (path:line within its project) whose
+ * library kernel it replaces; the reference itself contains no native code.
  */
 #ifndef B200_OPS_H_
 #define B200_OPS_H_

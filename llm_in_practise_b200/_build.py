@@ -4,7 +4,7 @@
                      (``-gencode arch=compute_100a,code=sm_100a -lineinfo``), C ABI in ``include/b200_ops.h``.
 ``libb200host.so`` — the host-side C++ runtime (safetensors reader, BPE tokenizer, CPU AdamW, ...).
 
-The reference has no build at all (it is pure Python, SURVEY.md §2.2); this replaces the
+The reference has no build at all (it is pure Python); this replaces the
 pip-installed native libraries it leans on. Nothing is JIT-compiled at run time: the .so files live
 under ``llm_in_practise_b200/_lib`` so they travel with the source tree.
 """

@@ -52,7 +52,7 @@ def build_messages(query: str, response: Optional[str] = None, system: str = "Yo
 def load_self_cognition(path: Optional[str] = None, name: str = "小马", author: str = "马哥教育") -> List[Dict[str, str]]:
     """Rows ``{"query", "response", "tag"}`` with the placeholders filled in."""
     cands = [path, os.environ.get("SELF_COGNITION_JSONL"),
-             "/root/reference/Fine-Tuning/LLaMA-Factory/self_cognition.jsonl"]
+             os.path.join(os.environ.get("LLM_IN_PRACTISE_DIR", "."), "Fine-Tuning/LLaMA-Factory/self_cognition.jsonl")]
     rows = []
     for p in cands:
         if p and os.path.exists(p):

@@ -8,7 +8,7 @@
 ``DistributedSampler``     deterministic permutation from (seed + epoch), padded to a multiple of world size, strided
                            per rank, ``set_epoch`` — same contract as torch's (ddp…:242-247,292-294).
 ``DataCollatorForLanguageModeling(mlm=False)``  labels = input_ids.clone(); labels[labels == pad] = -100 — the
-                           *effective* loss semantics of every Fine-Tuning/*.py script (SURVEY.md §2.1-D).
+                           *effective* loss semantics of every Fine-Tuning/*.py script.
 ``DataCollatorWithPadding``  dynamic right padding (+ ``pad_to_multiple_of``) — HF_Basics/trainer_demo.py:83.
 ``seed_worker`` / ``set_seed``  per-worker / per-rank seeding (…/temp/ddp_gpt_wikitext2.py:242-252,309).
 """

@@ -1,6 +1,6 @@
 """safetensors reader / writer (format: 8-byte little-endian header length, JSON header, raw
 little-endian tensor bytes) — byte-compatible with the ``safetensors`` wheel that HF
-``save_pretrained`` / ``from_pretrained`` use in the reference (SURVEY.md §5.4), implemented here so
+``save_pretrained`` / ``from_pretrained`` use in the reference, implemented here so
 checkpoints can be memory-mapped shard by shard without that (Rust) dependency.
 
 ``load_file`` memory-maps the file and returns zero-copy CPU tensors; ``safe_open`` gives lazy

@@ -1,4 +1,4 @@
-"""llm-demo: the two minimal GPTs (BASELINE configs 1 and 2).
+"""llm-demo: the two minimal GPTs.
 
 ``MiniGPT``   llm-demo/minigpt/model.py:5-32 — char-level, Embedding(V,64) + learned Embedding(16,64) positions,
               2 x nn.TransformerDecoderLayer(d_model=64, nhead=2, dropout=0.1) fed a zero "memory", Linear(64,V).

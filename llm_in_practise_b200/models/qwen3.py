@@ -55,7 +55,7 @@ class Qwen3Config:
         return cls(**{k: v for k, v in d.items() if k in keys})
 
 
-# Public checkpoint shapes (recalled, re-read config.json when real weights are used).
+# Public checkpoint shapes (from memory: re-read config.json when real weights are used).
 QWEN3_PRESETS: Dict[str, Qwen3Config] = {
     "qwen3-14b": Qwen3Config(hidden_size=5120, intermediate_size=17408, num_hidden_layers=40,
                              num_attention_heads=40, num_key_value_heads=8),

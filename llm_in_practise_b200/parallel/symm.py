@@ -9,7 +9,7 @@ grid-barrier counter.
 
 On CPU, or in a single-process run, the same objects degrade to ordinary tensors with a
 one-element pointer table, so engine code has one shape. The reference has no counterpart: all
-of its communication is implicit inside DDP / FSDP / DeepSpeed (SURVEY.md §2.5).
+of its communication is implicit inside DDP / FSDP / DeepSpeed.
 """
 from __future__ import annotations
 

@@ -4,7 +4,7 @@
               element in the high nibble; scale [N, K/g] fp32; zs = zero * scale or None for a fixed zero of 8).
 ``quantize_rtn``  round-to-nearest group quantiser (symmetric or asymmetric) — the arithmetic every other method ends in.
 
-Readers / writers (bit layouts reconstructed from the formats' public descriptions; SURVEY.md §5.4):
+Readers / writers (bit layouts reconstructed from the formats' public descriptions):
 * GPTQ (gptqmodel ``model.save``; Quantization/GPTQModel/quantize_qwen3_4b_gptq.py:16-46): ``qweight`` int32 [K/8, N]
   (8 nibbles per word along K, least-significant first), ``qzeros`` int32 [K/g, N/8] (nibbles along N, stored as
   zero - 1 in the classic v1 checkpoints), ``scales`` fp16 [K/g, N], ``g_idx`` int32 [K]; ``quantize_config.json``

@@ -124,7 +124,7 @@ def main(argv=None):
     ap.add_argument("--llamafactory_yaml", default=None, help="a LLaMA-Factory *_lora_sft.yaml: replaces --recipe")
     ap.add_argument("--model", default=None, help="HF checkpoint directory or preset name")
     ap.add_argument("--tokenizer", default=None, help="tokenizer directory (defaults to --model; byte tokenizer if none is found)")
-    ap.add_argument("--data", default=None, help="self_cognition.jsonl (default: the copy shipped with the reference tree)")
+    ap.add_argument("--data", default=None, help="self_cognition.jsonl (default: the file of that name under $LLM_IN_PRACTISE_DIR, else a small built-in set)")
     ap.add_argument("--name", default="小马")
     ap.add_argument("--author", default="马哥教育")
     ap.add_argument("--max_length", type=int, default=512)

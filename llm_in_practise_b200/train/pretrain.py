@@ -1,7 +1,7 @@
 """Hand-written pretraining loop with every feature the reference's GPT scripts use, behind one config.
 
 One function, ``run_pretraining(cfg)``, reproduces the behaviour of (reference files under
-``LLM_Distributed_Trainning/``; SURVEY.md §2.1 B and C):
+``LLM_Distributed_Trainning/``):
 
 * ``PyTorch/ddp_basics/ddp_gpt_wikitext{2,103}.py``            strategy="ddp"   (DistributedSampler + set_epoch, rank-0 logs,
                                                                 per-epoch mean loss all-reduce, ``.pth`` of the bare module)

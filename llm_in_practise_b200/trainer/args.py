@@ -1,4 +1,4 @@
-"""``TrainingArguments`` — every field the reference passes to HF's class, same names and defaults:
+"""``TrainingArguments`` — every field the reference passes to HF's class — same names and defaults:
 Fine-Tuning/qwen3-14b-qlora-dist-deepspeed.py:132-172, Fine-Tuning/qwen3-8b-lora-dist.py:137-173,
 HF_Basics/trainer_demo.py:86-107, HF_Basics/trainer_evaluate_demo.py:76-88, HF_Basics/accelerate_demo.py:88-90."""
 from __future__ import annotations

@@ -1,4 +1,4 @@
-"""Secondary training configurations of BASELINE.md section 2 (rows 2 and 3), timed like bench.py (CUDA events, barrier +
+"""Secondary training configurations (GPTLike / MiniGPT2 DDP, Qwen3-8B LoRA), timed like bench.py (CUDA events, barrier +
 synchronize on both sides, max over ranks, synthetic ids, random-init weights):
 
   --config gptlike-ddp    GPTLike-66M (6 layers, 12 heads, d 768, block 256, vocab 30522: the model of

@@ -43,5 +43,5 @@ for name, M, N, K, bmn in shapes:
     rows.append({"shape": name, "M": M, "N": N, "K": K, "b_mn": bmn, "b200_ms": round(t_mine, 4), "cublas_ms": round(t_ref, 4),
                  "b200_tflops": round(fl / t_mine / 1e9, 1), "cublas_tflops": round(fl / t_ref / 1e9, 1)})
     print(rows[-1], flush=True)
-os.makedirs("gpurun_out", exist_ok=True)
-json.dump(rows, open(f"gpurun_out/gemm_bench_ctas{os.environ.get('B200_GEMM_CTAS','auto')}.json", "w"), indent=1)
+os.makedirs("out", exist_ok=True)
+json.dump(rows, open(f"out/gemm_bench_ctas{os.environ.get('B200_GEMM_CTAS','auto')}.json", "w"), indent=1)

@@ -46,5 +46,5 @@ for name, out_f, in_f in shapes:
                      "cublas_bf16_only_ms": round(tc, 4), "fused_tflops": round(fl / tf / 1e9, 1), "unfused_tflops": round(fl / tu / 1e9, 1),
                      "cublas_tflops": round(fl / tc / 1e9, 1)})
         print(rows[-1], flush=True)
-os.makedirs("gpurun_out", exist_ok=True)
-json.dump(rows, open("gpurun_out/gemm_w4_bench.json", "w"), indent=1)
+os.makedirs("out", exist_ok=True)
+json.dump(rows, open("out/gemm_w4_bench.json", "w"), indent=1)

@@ -1,4 +1,4 @@
-"""W4A16 inference benchmark with tensor parallelism (BASELINE.md config 5): Qwen3-8B architecture, random-init weights,
+"""W4A16 inference benchmark with tensor parallelism: Qwen3-8B architecture, random-init weights,
 RTN W4A16 (group 128, symmetric: the GPTQ/compressed-tensors kernel layout), TP = WORLD_SIZE.
 
   torchrun --nproc-per-node T --master-addr 127.0.0.1 scripts/bench_infer_tp.py [--model qwen3-8b] [--batch 8] [--prompt 512] [--gen 64]

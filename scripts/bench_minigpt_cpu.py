@@ -1,4 +1,4 @@
-"""BASELINE config 1 on the CPU: the reference's llm-demo/minigpt/train.py (run unmodified, from a scratch directory) next
+"""The minigpt on the CPU: the reference's llm-demo/minigpt/train.py (run unmodified, from a scratch directory) next
 to `python -m llm_in_practise_b200.recipes.minigpt train` — wall time for the 200 epochs and the loss curve of both.
   python scripts/bench_minigpt_cpu.py [--epochs 200]"""
 import argparse, json, os, re, subprocess, sys, time
@@ -8,7 +8,7 @@ ap.add_argument("--epochs", type=int, default=200)
 ap.add_argument("--ref-dir", default="/root/reference/llm-demo/minigpt")
 a = ap.parse_args()
 root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-scratch = os.path.join(root, "gpurun_out", "minigpt_cpu")
+scratch = os.path.join(root, "out", "minigpt_cpu")
 os.makedirs(scratch, exist_ok=True)
 env = dict(os.environ, CUDA_VISIBLE_DEVICES="", PYTHONPATH=a.ref_dir + os.pathsep + root)
 

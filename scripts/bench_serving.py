@@ -1,6 +1,6 @@
 """Serving benchmark in the shape of the reference's published table (`vllm bench serve`, ShareGPT-like prompts, output
-length 256, 512 prompts, max-concurrency 8..256; LLM_on_Kubernetes/Inference_Platfrom/README.md:1504-1511, quoted in
-BASELINE.md section 1): mean / P99 TTFT, mean / P99 inter-token latency, requests/s and output tokens/s per concurrency.
+length 256, 512 prompts, max-concurrency 8..256; LLM_on_Kubernetes/Inference_Platfrom/README.md:1504-1511):
+mean / P99 TTFT, mean / P99 inter-token latency, requests/s and output tokens/s per concurrency.
 
 The engine is driven in-process (closed loop: a new request is submitted whenever one finishes, so `concurrency` requests
 are always in flight), Qwen3-8B architecture with random-init bf16 weights (the reference serves Qwen3-8B bf16), prompt
@@ -78,6 +78,6 @@ for C in a.concurrency:
     print(json.dumps(row), flush=True)
     del eng
     torch.cuda.empty_cache()
-os.makedirs("gpurun_out", exist_ok=True)
+os.makedirs("out", exist_ok=True)
 json.dump({"model": a.model, "weights": "W4A16 RTN g128" if a.w4 else "bf16", "mean_prompt_len": float(lens.mean()), "output_len": a.output_len,
-           "rows": rows}, open(f"gpurun_out/serving_{'w4' if a.w4 else 'bf16'}.json", "w"), indent=1)
+           "rows": rows}, open(f"out/serving_{'w4' if a.w4 else 'bf16'}.json", "w"), indent=1)

@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """Condense an ``.ncu-rep`` (read with ``ncu -i … --page raw --csv``) into the markdown summary kept under profiles/.
 
-usage: python scripts/ncu_summary.py gpurun_out/x.ncu-rep profiles/x.md ["title / what was run"]
+usage: python scripts/ncu_summary.py out/x.ncu-rep profiles/x.md ["title / what was run"]
 """
 import csv
 import io

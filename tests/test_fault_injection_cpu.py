@@ -1,4 +1,4 @@
-"""Failure handling under injected faults (SURVEY §5.3): a model call that raises inside the serving engine, a training run
+"""Failure handling under injected faults: a model call that raises inside the serving engine, a training run
 that dies mid-epoch, a rank that disappears from a collective."""
 import json
 import os

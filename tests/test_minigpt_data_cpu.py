@@ -1,4 +1,4 @@
-"""llm-demo counterparts (minigpt / minigpt2: config 1 of BASELINE.md), the data utilities, the GPTQModel-style front end and
+"""llm-demo counterparts (minigpt / minigpt2: the smallest configurations), the data utilities, the GPTQModel-style front end and
 the CPU AdamW of ZeRO-Offload — the pieces that only benchmarks exercised so far."""
 import os
 

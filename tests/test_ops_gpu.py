@@ -1,5 +1,5 @@
-"""Numerics of every CUDA kernel vs a plain PyTorch fp32 reference of the same op (SURVEY.md §4:
-"the oracle for every kernel is the plain torch expression the reference script executes")."""
+"""Numerics of every CUDA kernel vs a plain PyTorch fp32 reference of the same op: the oracle of every kernel is
+the plain torch expression that the reference's script executes."""
 import os
 
 import pytest

@@ -50,7 +50,7 @@ def test_lora_training_reduces_loss_cpu(tmp_path):
 
 
 def test_lora_param_count_matches_reference_numbers():
-    # SURVEY.md §6: r=8 on q_proj,v_proj -> 3 833 856 (Qwen3-8B) and 5 242 880 (Qwen3-14B)
+    # r=8 on q_proj,v_proj -> 3 833 856 (Qwen3-8B) and 5 242 880 (Qwen3-14B)
     for name, want in [("qwen3-8b", 3833856), ("qwen3-14b", 5242880)]:
         c = QWEN3_PRESETS[name]
         per_layer = 8 * (2 * c.hidden_size + c.num_attention_heads * c.head_dim + c.num_key_value_heads * c.head_dim)

@@ -101,8 +101,8 @@ def _suite(nproc, which, dump, port, env_extra=None):
     cmd = [sys.executable, "-m", "torch.distributed.run", "--nnodes=1", f"--nproc-per-node={nproc}", "--master-addr", "127.0.0.1",
            "--master-port", str(port), os.path.join(ROOT, "scripts", "check_multigpu.py"), "--suite", which, "--dump", dump]
     out = subprocess.run(cmd, capture_output=True, text=True, env=env, timeout=1500)
-    os.makedirs(os.path.join(ROOT, "gpurun_out"), exist_ok=True)
-    with open(os.path.join(ROOT, "gpurun_out", f"multigpu_suite_{which}_n{nproc}.log"), "w") as f:
+    os.makedirs(os.path.join(ROOT, "out"), exist_ok=True)
+    with open(os.path.join(ROOT, "out", f"multigpu_suite_{which}_n{nproc}.log"), "w") as f:
         f.write(out.stdout[-200000:] + "\n==== stderr ====\n" + out.stderr[-200000:])
     res = {}
     for ln in out.stdout.splitlines():
@@ -122,8 +122,8 @@ def runs(tmp_path_factory):
     d = tmp_path_factory.mktemp("mg")
     m = _suite(n, "multi", str(d / "multi"), 29651)
     s = _suite(1, "single", str(d / "single"), 29652, {"CHECK_TOTAL_RANKS": str(n)})
-    os.makedirs(os.path.join(ROOT, "gpurun_out"), exist_ok=True)
-    with open(os.path.join(ROOT, "gpurun_out", f"multigpu_suite_n{n}.json"), "w") as f:
+    os.makedirs(os.path.join(ROOT, "out"), exist_ok=True)
+    with open(os.path.join(ROOT, "out", f"multigpu_suite_n{n}.json"), "w") as f:
         json.dump({"world": n, "multi": m, "single": s}, f, indent=1)
     return {"n": n, "multi": m, "single": s, "dir": d}
 

@@ -1,5 +1,5 @@
 """ZeRO engine semantics on CPU/gloo with 2 processes: every stage must produce the same parameters
-as single-process training on the concatenated batch (SURVEY.md §4: multi-process CPU tests for
+as single-process training on the concatenated batch (multi-process CPU tests for
 wrapper semantics)."""
 import copy
 
