@@ -193,7 +193,7 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.
         nv.count_launch(3 if tiled else 1)
         return o
     if (nv.use_native(q) and mode == "head_delta" and runs is not None and D in (64, 128) and Dv % 16 == 0 and not act and not ones
-            and nv.has("b200_delta_chunk_scan") and _chunks_pay(T, n_runs, pieces, H, G, D, Dv)):
+            and _chunks_pay(T, n_runs, pieces, H, G, D, Dv)):
         if _delta_chunks(q, k, v, g, beta, state, runs, n_runs, o, H, G, D, Dv):
             return o
     if nv.use_native(q):
@@ -252,6 +252,8 @@ def _chunks_pay(T: int, n_runs: int, pieces, H: int, G: int, D: int, Dv: int) ->
 def _delta_chunks(q, k, v, g, beta, state, runs, n_runs, o, H, G, D, Dv) -> bool:
     """Mode "head_delta" over the runs of a step in chunks of 64 tokens; False: rows the kernels do not take."""
     T = q.shape[0]
+    if not nv.has("b200_delta_chunk_scan"):               # a library linked for a model without this mode
+        return False
     size = nv.lib().b200_delta_chunk_workspace
     size.restype = i64
     ws = torch.empty(size(T, n_runs, H), dtype=torch.float32, device=q.device)
