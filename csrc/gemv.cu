@@ -726,14 +726,16 @@ static cudaError_t launch_gemv_one(const GemvParams& p_in, cudaStream_t st, int 
   return launch_pdl(gemv_mma_kernel<BF16, W4, TG, MINB, LIN, POST>, dim3(grid, batch), 256, smem, st, p);
 }
 
+constexpr long long kWsMax = 227 * 1024;
+struct WsCut { int log2 = -1, smem = 0, clusters = 0; };  // log2 of the cluster size, -1: no slice of the activations fits
+
 // How a product is cut: the cluster size whose longest CTA has the least to do (chunks of weights, and the activations it lays out
-// first), among those whose slice of the activations fits. False: none does. A pass over a chunk costs about what two chunks' layout
-// of eight tokens does, a cluster's start and end as much as 64. Measured, 8 tokens (us, split 1 / 2 / 4): N 24576, K 4096: 24.5 / 25.7 /
-// 26.7; N 4096, K 12288: 19.3 / 18.4 / 17.3; N 5120, K 17408: - / 28.8 / 25.7 (33 clusters of four are resident, not 37).
+// first), among those whose slice of the activations fits. A pass over a chunk costs about what two chunks' layout of eight tokens
+// does, a cluster's start and end as much as 64. The weights of that cost come from three shapes at 8 tokens (us, split 1 / 2 / 4): N
+// 24576, K 4096: 24.5 / 25.7 / 26.7; N 4096, K 12288: 19.3 / 18.4 / 17.3; N 5120, K 17408: - / 28.8 / 25.7 (33 clusters of four are
+// resident, not 37); other shapes were not timed at every split.
 template <bool BF16, int TG>
-static bool w4_units_launch(const GemvParams& p, cudaStream_t st, cudaError_t& err) {
-  auto kern = w4_units_kernel<BF16, TG>;
-  constexpr long long kMax = 227 * 1024;
+static WsCut w4_units_cut(long long N, int K) {
   // clusters that are resident at once (a GPC has no multiple of four SMs); a device property, found once
   static const struct Resident {
     int n[3];
@@ -745,32 +747,40 @@ static bool w4_units_launch(const GemvParams& p, cudaStream_t st, cudaError_t& e
         cudaLaunchAttribute at;
         at.id = cudaLaunchAttributeClusterDimension;
         at.val.clusterDim.x = 1 << i; at.val.clusterDim.y = at.val.clusterDim.z = 1;
-        cfg.gridDim = dim3(kNumSMs >> i << i); cfg.blockDim = dim3(kWsWarps * 32); cfg.dynamicSmemBytes = kMax;
+        cfg.gridDim = dim3(kNumSMs >> i << i); cfg.blockDim = dim3(kWsWarps * 32); cfg.dynamicSmemBytes = kWsMax;
         cfg.attrs = &at; cfg.numAttrs = 1;
-        if (cudaFuncSetAttribute(w4_units_kernel<BF16, TG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMax) != cudaSuccess ||
+        if (cudaFuncSetAttribute(w4_units_kernel<BF16, TG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWsMax) != cudaSuccess ||
             cudaOccupancyMaxActiveClusters(&n[i], w4_units_kernel<BF16, TG>, &cfg) != cudaSuccess) { n[i] = 0; (void)cudaGetLastError(); }
       }
     }
   } resident;
-  const long long tiles = (p.N + 15) / 16;
-  const int nun = (p.K / 128 + 3) / 4;
-  int best = -1, best_smem = 0;
-  long long best_cost = 0;
+  const long long tiles = (N + 15) / 16;
+  const int nun = (K / 128 + 3) / 4;
+  WsCut cut;
+  long long best = 0;
   for (int i = 0; i < 3 && (1 << i) <= nun; ++i) {
     const int ncl = resident.n[i], cm = ((nun + (1 << i) - 1) >> i) * 4;
     if (ncl < 1) continue;
     const long long rounds = (tiles + ncl - 1) / ncl, smem = ws_smem<TG>(cm, i ? rounds : 0);
-    if (smem > kMax) continue;
+    if (smem > kWsMax) continue;
     const long long cost = cm * (rounds + 2 * TG) + (i ? 64 : 0);
-    if (best < 0 || cost < best_cost) { best = i; best_cost = cost; best_smem = (int)smem; }
+    if (cut.log2 < 0 || cost < best) { best = cost; cut.log2 = i; cut.smem = (int)smem; cut.clusters = (int)(tiles < ncl ? tiles : ncl); }
   }
+  return cut;
+}
+
+// False: no cut
+template <bool BF16, int TG>
+static bool w4_units_launch(const GemvParams& p, cudaStream_t st, cudaError_t& err) {
+  auto kern = w4_units_kernel<BF16, TG>;
+  const WsCut cut = w4_units_cut<BF16, TG>(p.N, p.K);
+  const int best = cut.log2;
   if (best < 0) return false;
-  if ((err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMax)) != cudaSuccess) return true;
-  const long long ncl = resident.n[best];
+  if ((err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWsMax)) != cudaSuccess) return true;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((tiles < ncl ? tiles : ncl) << best));
+  cfg.gridDim = dim3((unsigned)(cut.clusters << best));
   cfg.blockDim = dim3(kWsWarps * 32);
-  cfg.dynamicSmemBytes = best_smem;
+  cfg.dynamicSmemBytes = cut.smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
   int na = 0;
@@ -879,6 +889,16 @@ B200_API int b200_w4_gemv_linear(const void* x, const uint8_t* packed, const flo
   if (dtype == B200_DT_BF16) return launch_gemv_lin<true>(p, (cudaStream_t)stream);
   if (dtype == B200_DT_FP16) return launch_gemv_lin<false>(p, (cudaStream_t)stream);
   return B200_ERR_UNSUPPORTED;
+}
+
+// CTAs that share the k of a tile (1, 2 or 4) where b200_w4_gemv_linear deals units of chunks to warps, 0 where it takes the kernel
+// for any size
+B200_API int b200_w4_units_split(int M, long long N, int K, int group, int dtype) {
+  if (M < 1 || M > 16 || N < 1 || K < 128 || K % 128 || group < 128 || group % 128) return 0;
+  const bool bf = dtype == B200_DT_BF16;
+  const WsCut cut = M <= 8 ? (bf ? w4_units_cut<true, 1>(N, K) : w4_units_cut<false, 1>(N, K))
+                           : (bf ? w4_units_cut<true, 2>(N, K) : w4_units_cut<false, 2>(N, K));
+  return cut.log2 < 0 ? 0 : 1 << cut.log2;
 }
 
 // Row-parallel / plain projection with the fused tail (see GemvParams::fuse): kind 0 dense 16-bit weights, 1 4-bit codes

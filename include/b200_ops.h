@@ -438,6 +438,8 @@ int b200_w4_gemv_batched(const void* x, const uint8_t* packed, const float* scal
 int b200_w4_gemv_linear(const void* x, const uint8_t* packed, const float* scale, const float* zs, const void* bias, void* y,
                         int M, long long N, int K, int group, long long x_rs, long long y_rs, float lin_a, float lin_off,
                         int dtype, void* stream);
+/* CTAs that share the k of a tile (1, 2, 4) where that call deals units of chunks to warps, 0 where it takes the kernel for any size. */
+int b200_w4_units_split(int M, long long N, int K, int group, int dtype);
 
 /* K-C5 (decode flavour): a small-M projection whose launch also does what follows it in a decoder layer — the
  * tensor-parallel all-reduce of the row-parallel partial products (each rank writes its tiles into its half of a

@@ -7,6 +7,25 @@ from llm_in_practise_b200.ops.multimap_attention import multimap_attention
 
 pytestmark = pytest.mark.gpu
 
+@pytest.fixture
+def entries(monkeypatch):
+    """Names of the entry points that took a call (those that handed it back are not among them)."""
+    from llm_in_practise_b200.ops import _native as nv
+    names, real = set(), nv.proto
+
+    def proto(name, argtypes):
+        fn = real(name, argtypes)
+
+        def call(*args):
+            rc = fn(*args)
+            if rc == 0:
+                names.add(name)
+            return rc
+        return call
+    monkeypatch.setattr(nv, "proto", proto)
+    return names
+
+
 # Both sides round to bf16, whose neighbours are up to 2^-7 of a value apart: two roundings of nearly the same number differ by at
 # most one such step. What the kernels add on top (fp32 sums, 2^-17 of every probability, 2^-22 of every exponential) stays below
 # 2^-12 of the largest value; the bound has twice that.
@@ -63,7 +82,7 @@ def test_decode_batches(H, G, M, D, Dv, opt, BS):
 @pytest.mark.parametrize("H,G,D", [(4, 2, 128), (8, 2, 64), (10, 2, 64), (2, 2, 128), (3, 1, 128)])
 @pytest.mark.parametrize("opt", ["none", "window", "chunk"])
 @pytest.mark.parametrize("BS", [8, 16, 64, 128])
-def test_prompt_pieces(H, G, D, opt, BS):
+def test_prompt_pieces(H, G, D, opt, BS, entries):
     """Pieces that start and end anywhere in pages and 64-key blocks, single tokens beside them, keys past the end that are NaN."""
     from llm_in_practise_b200.inference.ragged import make_pieces
     runs = [(65, 0), (1, 130), (9, 63), (130, 200), (64, 64), (1, 0)]                # (tokens, first position)
@@ -92,12 +111,13 @@ def test_prompt_pieces(H, G, D, opt, BS):
         # here P is rounded to bf16 before the product (as in the mma.sync kernel): 2^-9 of every term, which averages out over the
         # sum to well below 2^-9 of the largest value; the bound grants it in full
         close(got, want, vmax=16.0)
+    assert entries == {"b200_paged_attn_tc"}
 
 
 @pytest.mark.parametrize("H,Hkv,D", [(4, 2, 128), (6, 6, 64), (4, 1, 64)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("causal", [True, False])
-def test_packed_prompts(H, Hkv, D, dtype, causal):
+def test_packed_prompts(H, Hkv, D, dtype, causal, entries):
     """Lengths at the edges of key blocks and query tiles; a NaN in the sequence behind must not reach the one in front."""
     from llm_in_practise_b200.ops.flash import flash_attention_varlen
     lens = [1, 63, 64, 65, 128, 129, 200, 7]
@@ -109,11 +129,12 @@ def test_packed_prompts(H, Hkv, D, dtype, causal):
     got = flash_attention_varlen(qkv.cuda(), cu.cuda(), max(lens), H, Hkv, D, D ** -0.5, causal)
     close(got[:-7], want[:-7], vmax=16.0)
     assert torch.isnan(got[-7:]).all()
+    assert entries == {"b200_flash_attn_varlen_fwd_tc"}
 
 
 @pytest.mark.parametrize("B,S,H,Hkv,D", [(2, 1, 2, 1, 64), (3, 65, 2, 2, 64), (2, 129, 4, 2, 64), (1, 300, 6, 2, 128), (2, 256, 3, 3, 64)])
 @pytest.mark.parametrize("causal", [True, False])
-def test_fused_qkv_forward(B, S, H, Hkv, D, causal):
+def test_fused_qkv_forward(B, S, H, Hkv, D, causal, entries):
     """Forward with the log-sum-exp the backward reads; a batch entry whose last rows are NaN leaves the ones beside it alone."""
     from llm_in_practise_b200.ops.attention import _ref_attention
     from llm_in_practise_b200.ops.flash import _fwd
@@ -133,12 +154,13 @@ def test_fused_qkv_forward(B, S, H, Hkv, D, causal):
         qkv[-S:] = float("nan")
         again, _ = _fwd(qkv.cuda(), B, S, H, Hkv, D, causal, D ** -0.5)
         assert torch.equal(again[:-S], got[:-S])
+    assert entries == {"b200_flash_attn_fwd_tc"}
 
 
 @pytest.mark.parametrize("B,S,H,Hkv", [(2, 1, 2, 1), (2, 64, 3, 3), (1, 65, 4, 2), (2, 129, 4, 1), (1, 300, 6, 2)])
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("causal", [True, False])
-def test_fused_qkv_backward(B, S, H, Hkv, D, causal):
+def test_fused_qkv_backward(B, S, H, Hkv, D, causal, entries):
     """Gradient of the fused projection at the edges of key blocks, query tiles and groups of heads, against float64 autograd."""
     from llm_in_practise_b200.ops.flash import flash_attention
     g = torch.Generator(device="cuda").manual_seed(5)
@@ -156,6 +178,7 @@ def test_fused_qkv_backward(B, S, H, Hkv, D, causal):
     for lo, hi in ((0, H * D), (H * D, (H + Hkv) * D), ((H + Hkv) * D, (H + 2 * Hkv) * D)):
         a, b = qkv.grad[:, lo:hi].double(), x.grad[:, lo:hi]
         assert (a - b).norm() <= 4 * 2 * 2.0 ** -9 * b.norm() + 2.0 ** -9 * go.double().norm() * (S == 1)
+    assert entries == {"b200_flash_attn_fwd_tc", "b200_flash_attn_bwd_tc"}
 
 
 def exact_fused(x, B, S, H, Hkv, D, causal, scale):
@@ -170,7 +193,7 @@ def exact_fused(x, B, S, H, Hkv, D, causal, scale):
 
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("scale", [0.0, -0.1])
-def test_scale_not_positive(D, scale):
+def test_scale_not_positive(D, scale, entries):
     """Equal weights (scale 0) and reversed ones under the causal mask: a masked score stays minus infinity whatever it is multiplied by."""
     from llm_in_practise_b200.ops.flash import flash_attention, flash_attention_varlen
     B, S, H, Hkv = 2, 130, 4, 2
@@ -188,6 +211,7 @@ def test_scale_not_positive(D, scale):
         assert (a - b).norm() <= 4 * 2 * 2.0 ** -9 * b.norm()
     cu = torch.tensor([0, S, 2 * S], dtype=torch.int32, device="cuda")
     close(flash_attention_varlen(qkv.detach(), cu, S, H, Hkv, D, scale), want.detach().cpu(), vmax=16.0)
+    assert entries == {"b200_flash_attn_fwd", "b200_flash_attn_bwd", "b200_flash_attn_varlen_fwd"}
 
 
 @pytest.mark.parametrize("S", [1, 65, 129, 200])

@@ -51,7 +51,7 @@ def test_rotation_of_vectors(T, n_q, n_k, n_v, D, normed, dtype):
     (5, 2056, "layer", True, torch.bfloat16, torch.float32),       # two per thread, the second with a remainder
     (7, 5120, "rms", True, torch.float16, torch.float16),
     (2, 8192, "layer", False, torch.bfloat16, torch.bfloat16),     # the widest row
-    (2, 8200, "rms", True, torch.bfloat16, torch.bfloat16),        # and the first that stays with the other kernels
+    (2, 8200, "rms", True, torch.bfloat16, torch.bfloat16),        # wider: the forward alone takes it
     (4, 4096, "rms", True, torch.float32, torch.float32),
 ])
 def test_row_norms(rows, cols, kind, res, dtype, wtype):

@@ -1,21 +1,28 @@
 """Decode products over 4-bit integer codes for at most 16 tokens: units of four chunks dealt to the warps, slices of k in clusters."""
+import ctypes
+
 import pytest
 import torch
 
+from llm_in_practise_b200.ops import _native as nv
 from llm_in_practise_b200.ops.w4 import w4_gemv
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("M,N,K,group,zeros,bias,dtype", [
-    (1, 8, 128, 128, True, False, torch.bfloat16),        # less than a tile, one chunk
-    (8, 40, 640, 128, True, True, torch.bfloat16),        # five chunks: a whole unit and one of a single chunk; scales not in fours
-    (9, 16 * 149, 1152, 384, False, False, torch.float16),  # more tiles than CTAs; a scale over three chunks
-    (16, 2000, 4224, 128, True, True, torch.float16),
-    (5, 4096, 12288, 128, True, False, torch.bfloat16),   # slices of k in a cluster
-    (13, 1000, 17408, 256, True, True, torch.bfloat16),   # 68 units over four slices
-    (16, 5120, 17408, 128, False, False, torch.bfloat16),
+@pytest.mark.parametrize("M,N,K,group,zeros,bias,dtype,split", [
+    (1, 8, 128, 128, True, False, torch.bfloat16, {1}),        # less than a tile, one chunk
+    (8, 40, 640, 128, True, True, torch.bfloat16, {1, 2}),     # five chunks: a whole unit and one of a single chunk; scales not in fours
+    (9, 16 * 149, 1152, 384, False, False, torch.float16, {1, 2, 4}),  # more tiles than CTAs; a scale over three chunks
+    (16, 2000, 4224, 128, True, True, torch.float16, {1, 2, 4}),
+    (5, 4096, 12288, 128, True, False, torch.bfloat16, {2, 4}),   # slices of k in a cluster
+    (13, 1000, 17408, 256, True, True, torch.bfloat16, {4}),   # 68 units over four slices
+    (16, 5120, 17408, 128, False, False, torch.bfloat16, {4}),
+    (8, 40, 65536, 128, True, False, torch.bfloat16, {0}),     # no slice of the activations fits: the kernel for any size
+    (17, 64, 1024, 128, True, False, torch.bfloat16, {0}),     # more tokens than this one takes
 ])
-def test_integer_codes(M, N, K, group, zeros, bias, dtype):
+def test_integer_codes(M, N, K, group, zeros, bias, dtype, split):
+    plan = nv.proto("b200_w4_units_split", [ctypes.c_int, ctypes.c_longlong, ctypes.c_int, ctypes.c_int, ctypes.c_int])
+    assert plan(M, N, K, group, nv.dtype_code(dtype)) in split
     gen = torch.Generator(device="cuda").manual_seed(N + K + M)
     rand = lambda *s: torch.randn(*s, generator=gen, device="cuda")
     x = rand(M, K).to(dtype)
