@@ -20,7 +20,7 @@
 // tf32 mma.sync takes as many cycles as the FMAs do. r_ij is a product taken from j upwards, the roundings a walk makes too;
 // sums of logarithms would lose digits to cancellation. Bound: the latency of the sums across lanes with two warps per scheduler
 // (44 % of the issue slots are used), then the FMA rate. One prompt of 2048 tokens, 16 heads of 128 x 128 over 4 q/k heads: 502 us token
-// by token, 18 + 207 here; 2048 and 513 tokens: 586 -> 285; error of the state against 64 bits 2e-7 both ways.
+// by token, 18 + 207 here; 2048 and 513 tokens: 586 -> 285 (6 more with the test for infinities and NaN); error of the state against 64 bits 2e-7 both ways.
 #include "common.cuh"
 #include "../include/b200_ops.h"
 
@@ -171,7 +171,7 @@ template <int D> struct DcSmem {                          // float offsets
 // with every other two pairs so that the eight lane groups of a warp read and write different banks
 __device__ __forceinline__ int pair_at(int pr, int c) { return pr * (2 * kDcNC) + (((c >> 1) ^ (pr >> 1 & 1)) << 2); }
 
-// NR rows' sums over 4 N2 elements (every eighth group of four, the lane's own) times four columns held as pairs of rows: with one warp per scheduler it is the rows beside one
+// NR rows' sums over 4 N2 elements (every eighth group of four, the lane's own) times four columns held as pairs of rows: with two warps per scheduler it is the rows beside one
 // another that keep the FMA pipe busy
 template <int NR, int N2>
 __device__ __forceinline__ void dot_rows(const float* rows, int stride, const float2 (&m)[2 * N2][4], float4 (&out)[NR]) {

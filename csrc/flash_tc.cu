@@ -24,11 +24,11 @@
 // Rows of K and V past the last key of a sequence belong to somebody else (or were never written): their scores are masked, and
 // their V rows are zeroed in shared memory before the product, so that not even a NaN there reaches this sequence.
 //
-// Replaces the mma.sync kernels of flash_attn.cu (other head sizes, dropout and the backward pass stay there) and
+// Takes the place of the mma.sync kernels of flash_attn.cu (other head sizes, other scales and dropout stay there) and
 // multimap_attn_mma.cu (other sizes, two maps). Measured against them, bf16: six packed prompts of 77 - 2048 tokens, 32 / 8 heads
-// of 128: 237 -> 109 us; pages of 64, 16 / 4 heads of 128, pieces of 2048 and 700 (at 512) tokens beside two that decode:
-// 170 -> 57 us, window of 1024: 127 -> 44, chunks with capped scores: 194 -> 69, 8 / 8 heads: 101 -> 48; dense, 8 x 1000 tokens,
-// 16 / 8 heads of 64, forward and backward: 487 -> 457. Packed prompts too short to fill a tile take the same time in both.
+// of 128: 237 -> 114 us, 16 / 8 heads of 64: 80 -> 57; pages of 64, 16 / 4 heads of 128, pieces of 2048 and 700 (at 512) tokens beside
+// two that decode: 171 -> 61 us, window of 1024: 128 -> 47, chunks with capped scores: 194 -> 82; eight packed prompts of 30 - 250
+// tokens (fp16): 19.1 -> 16.4.
 // Reference call sites: SDPA behind nn.MultiheadAttention (LLM_Distributed_Trainning/PyTorch/ddp_basics/ddp_gpt_wikitext2.py:89-96),
 // HF Qwen3 attention (Fine-Tuning/qwen3-14b-qlora-dist-deepspeed.py:95-107).
 #include "common.cuh"

@@ -625,7 +625,7 @@ multimap_attn_vec_kernel(const T* __restrict__ q, const T* __restrict__ ck, cons
 // a warp barrier sits in the loop and 16 KiB of each warp are on their way (two CTAs of four warps per SM: 128 KiB, three
 // times what the memory's latency asks for).
 // 64 sequences at contexts of 3300 - 4000, 16 heads over 4 KV groups of 128 (484 MB of keys and values): 410 us in the vector
-// kernel (1.2 TB/s), 87 us here (5.6 TB/s).
+// kernel (1.2 TB/s), 89 us here (5.4 TB/s); error of the result against 64 bits 0.00166 in both.
 // A value that is infinite would make NaN of the two terms (the second of P may be zero or negative); a warp whose sums hold a NaN at the
 // end walks its keys once more with such values left out of the second product: the first one alone says what they come to.
 constexpr int kDmKeys = 16, kDmStages = 3;

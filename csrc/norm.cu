@@ -275,8 +275,7 @@ norm_bwd_reg_kernel(const T* __restrict__ dy, const T* __restrict__ h, const WT*
   }
 }
 
-// vectors per thread and threads of the register kernel: one vector up to 256 of them, two up to 1024 (16-bit: 8192 columns); wider
-// rows stay with the kernel above
+// threads of the register kernel: one vector per thread up to 256 of them, two up to 1024 (16-bit: 8192 columns)
 static inline int reg_threads(int nvec, int nv) { return ((nvec + nv - 1) / nv + 31) / 32 * 32; }
 
 template <typename T, typename WT>
@@ -294,7 +293,7 @@ static int launch_norm_bwd(int layer_norm, const void* dy, const void* h, const 
                            const void* dres, void* dx, float* dwp, float* dbp, int rows, int cols, int grid,
                            cudaStream_t st) {
   const int nvec = cols / (16 / (int)sizeof(T));
-  if (!dwp && !dbp && nvec <= 1024) {
+  if (!dwp && !dbp) {                                       // at most 1024 vectors: wider rows are refused by the entry points
     constexpr int NV = MV == 1 ? 1 : 2;                     // MV 1: at most 256 vectors
     const int nt = reg_threads(nvec, NV);
     if (layer_norm)

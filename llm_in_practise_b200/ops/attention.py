@@ -2,8 +2,9 @@
 
 Two native paths share this front end:
 
-* ``flash`` (``csrc/flash_attn.cu``; 16-bit dtypes, head_dim 32 / 64 / 96 / 128, no window; probability dropout in-kernel): 64 x 64
-  tiles, online softmax forward, recomputing backward, no L x L tensor in memory in either direction.
+* ``flash`` (16-bit dtypes, head_dim 32 / 64 / 96 / 128, no window; ``csrc/flash_tc.cu`` and ``csrc/flash_bwd_tc.cu`` on tcgen05 for
+  64 and 128 without dropout, ``csrc/flash_attn.cu`` for the rest, probability dropout in-kernel): tiles, online softmax
+  forward, recomputing backward, no L x L tensor in memory in either direction.
 * ``tiled`` (always available): batched tcgen05 GEMMs (``csrc/gemm_tcgen05.cu``) around fused
   masked-softmax kernels (``csrc/loss.cu``); scores exist per (batch, head) as a transient.
 

@@ -1,4 +1,5 @@
-"""Flash attention (csrc/flash_attn.cu): forward keeps only the context and the row log-sum-exp, backward recomputes
+"""Flash attention (csrc/flash_tc.cu and csrc/flash_bwd_tc.cu on tcgen05 for heads of 64 and 128 with a scale above zero and no
+dropout, csrc/flash_attn.cu on mma.sync for the rest): forward keeps only the context and the row log-sum-exp, backward recomputes
 the probabilities tile by tile — no [B, H, S, S] tensor in either direction. Replaces the SDPA / flash-attn call behind
 HF Qwen3 (Fine-Tuning/qwen3-14b-qlora-dist-deepspeed.py:101-112) and the masked ``nn.MultiheadAttention`` of the GPT
 scripts (LLM_Distributed_Trainning/PyTorch/ddp_basics/ddp_gpt_wikitext2.py:92-96).
@@ -26,7 +27,7 @@ def _fwd(qkv, B, S, H, Hkv, D, causal, scale, want_lse=True, dropout_p=0.0, seed
     out = torch.empty(B * S, H * D, dtype=qkv.dtype, device=qkv.device)
     lse = torch.empty(B, H, S, dtype=torch.float32, device=qkv.device) if want_lse else None
     if _TC and D in (64, 128) and dropout_p == 0.0:
-        # tcgen05 / TMEM / TMA forward (csrc/flash_tc.cu); the mma.sync kernel below keeps the other head sizes and dropout
+        # tcgen05 / TMEM / TMA forward (csrc/flash_tc.cu); the mma.sync kernel below keeps the other head sizes, dropout and scales <= 0
         ft = nv.proto("b200_flash_attn_fwd_tc", [vp, vp, vp, i32, i32, i32, i32, i32, i32, f32, i32, vp])
         rc = ft(nv.ptr(qkv), nv.ptr(out), nv.ptr(lse), B, S, H, Hkv, D, int(causal), float(scale), nv.dtype_code(qkv.dtype),
                 nv.stream())

@@ -241,7 +241,8 @@ def _chunks_pay(T: int, n_runs: int, pieces, H: int, G: int, D: int, Dv: int) ->
     """Whether prompts of the delta rule with one decay per head take less time 64 tokens at a time (csrc/delta_chunk.cu) than token by
     token. Both as measured (us): the walk moves 0.24 per token of the longest run, or, with more (run, head, 16 columns) than about
     320 (445 for keys of 64) at once, in proportion; a chunk is 6.5 (4.8) on one of 148 SMs, after the inverses. One run of 2048 tokens,
-    16 heads of 128: 225 against 502; three of 150: 74 against 56. Without ``pieces`` the runs count as equally long."""
+    16 heads of 128: 225 against 502; three of 150: 74 against 56. The constants are fits to 16 heads and a few lengths; other head
+    counts rest on the proportions. Without ``pieces`` the runs count as equally long."""
     blocks = H * (Dv // 16)
     longest, tiles = (pieces.longest, pieces.n_tiles) if pieces is not None else (T / max(n_runs, 1), T / 64 + n_runs)
     walk = 0.24 * max(longest, T * blocks / (320 if D == 128 else 445))
@@ -250,7 +251,8 @@ def _chunks_pay(T: int, n_runs: int, pieces, H: int, G: int, D: int, Dv: int) ->
 
 
 def _delta_chunks(q, k, v, g, beta, state, runs, n_runs, o, H, G, D, Dv) -> bool:
-    """Mode "head_delta" over the runs of a step in chunks of 64 tokens; False: rows the kernels do not take."""
+    """Mode "head_delta" over the runs of a step in chunks of 64 tokens; False: rows the kernels do not take. The workspace is 33 KB per
+    chunk and head for at most 128 chunks at a time (136 MB at 32 heads), which the walk does without."""
     T = q.shape[0]
     if not nv.has("b200_delta_chunk_scan"):               # a library linked for a model without this mode
         return False
