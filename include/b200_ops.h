@@ -438,7 +438,15 @@ int b200_w4_gemv_batched(const void* x, const uint8_t* packed, const float* scal
 int b200_w4_gemv_linear(const void* x, const uint8_t* packed, const float* scale, const float* zs, const void* bias, void* y,
                         int M, long long N, int K, int group, long long x_rs, long long y_rs, float lin_a, float lin_off,
                         int dtype, void* stream);
-/* CTAs that share the k of a tile (1, 2, 4) where that call deals units of chunks to warps, 0 where it takes the kernel for any size. */
+/* The same product on tcgen05, for 17 to 64 tokens, groups of 128 and K a multiple of 512. `ws`: room for K x 32 (up to 32 tokens) or
+ * K x 64 16-bit values. B200_ERR_UNSUPPORTED: the caller takes the other. */
+int b200_w4_tc_linear(const void* x, const uint8_t* packed, const float* scale, const float* zs, const void* bias, void* y, void* ws,
+                      int M, long long N, int K, int group, long long x_rs, long long y_rs, float lin_a, float lin_off, int dtype,
+                      void* stream);
+/* CTAs that share the k of a tile (1, 2, 4) where that call is taken, 0 where it is refused. */
+int b200_w4_tc_split(int M, long long N, int K, int group);
+/* CTAs that share the k of a tile (1, 2, 4) where b200_w4_gemv_linear deals units of chunks to warps, 0 where it takes the kernel for any
+ * size. */
 int b200_w4_units_split(int M, long long N, int K, int group, int dtype);
 
 /* K-C5 (decode flavour): a small-M projection whose launch also does what follows it in a decoder layer — the

@@ -170,6 +170,22 @@ def linear_lut(lut) -> Optional[tuple]:
     return res
 
 
+def w4_tc(x, packed, scale, zs, N: int, K: int, group: int, lin, bias, y) -> bool:
+    """``w4_gemv`` of 17 to 64 tokens with integer codes (``lin`` = (a, off)) on tcgen05, into ``y``; False: a form that it does not take."""
+    M = x.shape[0]
+    if not 16 < M <= 64 or group != 128 or K % 512 or not nv.has("b200_w4_tc_linear"):
+        return False
+    ws = torch.empty(K * (32 if M <= 32 else 64), dtype=x.dtype, device=x.device)
+    fn = nv.proto("b200_w4_tc_linear", [vp, vp, vp, vp, vp, vp, vp, i32, i64, i32, i32, i64, i64, f32, f32, i32, vp])
+    rc = fn(nv.ptr(x), nv.ptr(packed), nv.ptr(scale), nv.ptr(zs), nv.ptr(bias), nv.ptr(y), nv.ptr(ws), M, N, K, group, x.stride(0),
+            y.stride(0), lin[0], lin[1], nv.dtype_code(x.dtype), nv.stream())
+    if rc == nv.ERR_UNSUPPORTED:
+        return False
+    nv.check(rc, "w4_tc_linear")
+    nv.count_launch(2)
+    return True
+
+
 def w4_gemv(x, packed, scale, zs, N: int, K: int, group: int, lut=None, bias=None) -> torch.Tensor:
     """y[m, :] = x[m, :] @ dequant(W)^T for 1 <= m <= 64 rows (decode / serving steps)."""
     M = x.shape[0]
@@ -182,8 +198,11 @@ def w4_gemv(x, packed, scale, zs, N: int, K: int, group: int, lut=None, bias=Non
     x = x.contiguous()
     y = torch.empty(M, N, dtype=x.dtype, device=x.device)
     lin = linear_lut(lut) if K % 128 == 0 else None
-    if lin is not None:   # integer codes: table-free conversion (csrc/gemv.cu, LIN)
-        f32 = ctypes.c_float
+    if lin is not None:   # integer codes: table-free conversion, on tcgen05 (csrc/w4_tc.cu) or for any size (csrc/gemv.cu, LIN)
+        # tcgen05 where the product is large enough that its two launches are not what takes the time (25.5 us on the host): 17 - 32
+        # tokens, N 12288, K 2048: 24.6 us on the mma.sync kernel and 25.4 here; N 4096, K 12288: 41 and 26; 64 tokens, N = K = 4096: 33 and 26
+        if M > 16 and N * K >= (1 << 25 if M <= 32 else 1 << 24) and w4_tc(x, packed, scale, zs, N, K, group, lin, bias, y):
+            return y
         fl = nv.proto("b200_w4_gemv_linear", [vp, vp, vp, vp, vp, vp, i32, i64, i32, i32, i64, i64, f32, f32, i32, vp])
         nv.check(fl(nv.ptr(x), nv.ptr(packed), nv.ptr(scale), nv.ptr(zs), nv.ptr(bias), nv.ptr(y), M, N, K, group,
                     x.stride(0), y.stride(0), lin[0], lin[1], nv.dtype_code(x.dtype), nv.stream()), "w4_gemv_linear")
