@@ -26,8 +26,8 @@
 //
 // Takes the place of the mma.sync kernels of flash_attn.cu (other head sizes, other scales and dropout stay there) and
 // multimap_attn_mma.cu (other sizes, two maps). Measured against them, bf16: six packed prompts of 77 - 2048 tokens, 32 / 8 heads
-// of 128: 237 -> 114 us, 16 / 8 heads of 64: 80 -> 57; pages of 64, 16 / 4 heads of 128, pieces of 2048 and 700 (at 512) tokens beside
-// two that decode: 171 -> 61 us, window of 1024: 128 -> 47, chunks with capped scores: 194 -> 82; eight packed prompts of 30 - 250
+// of 128: 237 -> 106 us, 16 / 8 heads of 64: 80 -> 57; pages of 64, 16 / 4 heads of 128, pieces of 2048 and 700 (at 512) tokens beside
+// two that decode: 171 -> 57 us, window of 1024: 128 -> 42, chunks with capped scores: 194 -> 80; eight packed prompts of 30 - 250
 // tokens (fp16): 19.1 -> 16.4.
 // Reference call sites: SDPA behind nn.MultiheadAttention (LLM_Distributed_Trainning/PyTorch/ddp_basics/ddp_gpt_wikitext2.py:89-96),
 // HF Qwen3 attention (Fine-Tuning/qwen3-14b-qlora-dist-deepspeed.py:95-107).
@@ -43,10 +43,14 @@ constexpr uint32_t kTcTmemCols = 256, kTcTmemO = 128;
 constexpr float kTcLog2e = 1.4426950408889634f;
 enum { kTcDense = 0, kTcVarlen = 1, kTcPaged = 2 };
 
-// shared memory: Q [128 rows] as D / 64 swizzled halves of 16 KiB, two stages of K and of V [64 rows] as halves of 8 KiB, barriers
+// shared memory: Q [128 rows] as D / 64 swizzled halves of 16 KiB, the rings of K and of V [64 rows] as halves of 8 KiB, barriers. K and V
+// have rings of their own: K's stage is free as soon as its scores are there, a whole block of softmax before V's. With one ring of two
+// stages for both, a block's keys were asked for when the product two blocks before had ended, and the softmax waited 500 of 2000 cycles for
+// its scores: 1 x 4096, 32 / 8 heads of 128: 160 -> 136 us (200 with the tiles of one head after another), window of 1024: 54 -> 46.
 template <int D> struct TcSmem {
   static constexpr uint32_t kHalves = D / 64, kStage = 8192 * kHalves;
-  static constexpr uint32_t kQ = 0, kK = 16384 * kHalves, kV = kK + 2 * kStage, kBar = kV + 2 * kStage, kBytes = kBar + 128;
+  static constexpr int NK = D == 64 ? 4 : 3, NV = D == 64 ? 4 : 2;      // two CTAs fit an SM
+  static constexpr uint32_t kQ = 0, kK = 16384 * kHalves, kV = kK + NK * kStage, kBar = kV + NV * kStage, kBytes = kBar + 192;
 };
 
 struct FlashTcParams {
@@ -64,6 +68,12 @@ struct FlashTcParams {
   b200_attn_opts opt;
 };
 
+// the largest of three (a NaN gives way, as in fmaxf)
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
 __device__ __forceinline__ float ex2f(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -118,7 +128,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
 flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
                     const FlashTcParams p) {
   using L = TcSmem<D>;
-  constexpr int kHalves = L::kHalves;
+  constexpr int kHalves = L::kHalves, NK = L::NK, NV = L::NV;
   // How far a row's maximum may run ahead of the one its weights refer to before O is scaled (an exponent of two). With none the largest
   // weight is 1 and has no rounding error, as in the mma.sync kernels: error of the result against 64 bits 0.00196 (six packed prompts,
   // bf16) and 0.00199 (pieces over pages); with a slack of 8 it was 0.00200 and 0.00206, at 108 and 57 us instead of 114 and 61. Dense
@@ -160,8 +170,10 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
     nit = nA + (limit + kTcBN - 1) / kTcBN - bB;
     low_max = low_of(q0 + (solo ? kTcBM : kTcBN) - 1);
   } else {
-    // heavy (late) query tiles first: under the causal mask tile t has t + 1 times the work of tile 0
-    const int qt = (int)gridDim.x - 1 - (int)blockIdx.x, b = blockIdx.z;
+    // The tile is the slowest grid dimension, heavy (late) query tiles of all heads and sequences first: under the causal mask tile t has
+    // t + 1 times the work of tile 0, and the short ones fill the end.
+    const int qt = (int)gridDim.z - 1 - (int)blockIdx.z, b = blockIdx.y;
+    h = blockIdx.x;
     hk = h / (p.H / p.Hkv);
     row_base = MODE == kTcVarlen ? p.cu[b] : b * p.S;
     limit = MODE == kTcVarlen ? p.cu[b + 1] - row_base : p.S;
@@ -173,14 +185,23 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
   auto block_of = [&](int it) { return MODE == kTcPaged ? (it < nA ? it : bB + (it - nA)) : it; };
 
   const uint32_t bar = sbase + L::kBar;
-  const uint32_t q_full = bar, kv_full0 = bar + 8, kv_empty0 = bar + 24, s_full0 = bar + 40, p_full = bar + 56, o_done = bar + 64,
-                 tmem_slot = bar + 80;
+  // P has two barriers: the softmax may be a block ahead of the issuing warp (S(j + 1) is asked for before V(j) and P(j) are waited for)
+  const uint32_t q_full = bar, s_full0 = bar + 8, p_full0 = bar + 24, o_done = bar + 40, tmem_slot = bar + 48;
+  auto k_full = [&](int j) { return bar + 56 + 8u * (j % NK); };
+  auto k_empty = [&](int j) { return bar + 56 + 8u * (NK + j % NK); };
+  auto v_full = [&](int j) { return bar + 56 + 8u * (2 * NK + j % NV); };
+  auto v_empty = [&](int j) { return bar + 56 + 8u * (2 * NK + NV + j % NV); };
+  auto k_phase = [&](int j) { return (uint32_t)(j / NK) & 1u; };
+  auto v_phase = [&](int j) { return (uint32_t)(j / NV) & 1u; };
+  auto k_at = [&](int j) { return sbase + L::kK + (uint32_t)(j % NK) * L::kStage; };
+  auto v_at = [&](int j) { return sbase + L::kV + (uint32_t)(j % NV) * L::kStage; };
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tq);
     if (MODE == kTcPaged) { tma_prefetch_desc(&tk); tma_prefetch_desc(&tv); }
     mbar_init(q_full, 1);
-    for (int s = 0; s < 2; ++s) { mbar_init(kv_full0 + 8 * s, 1); mbar_init(kv_empty0 + 8 * s, 1); mbar_init(s_full0 + 8 * s, 1); }
-    mbar_init(p_full, 4);
+    for (int s = 0; s < NK; ++s) { mbar_init(k_full(s), 1); mbar_init(k_empty(s), 1); }
+    for (int s = 0; s < NV; ++s) { mbar_init(v_full(s), 1); mbar_init(v_empty(s), 1); }
+    for (int s = 0; s < 2; ++s) { mbar_init(s_full0 + 8 * s, 1); mbar_init(p_full0 + 8 * s, 4); }
     mbar_init(o_done, 1);
     fence_mbar_init();
   }
@@ -210,35 +231,55 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
         return (it < nit && lane < pieces && kp < limit)
                    ? ((trow[kp >> p.bs_log2] * p.Hkv + hk) << p.bs_log2) + (kp & ((1 << p.bs_log2) - 1)) : -1;
       };
-      int row = row_of(0);
-      for (int it = 0; it < nit; ++it) {
-        const int s = it & 1;
-        const int n = min(pieces, (limit - block_of(it) * kTcBN + psize - 1) >> psl);
-        if (lane == 0) {
-          mbar_wait(kv_empty0 + 8 * s, (((uint32_t)it >> 1) & 1u) ^ 1u);
-          mbar_arrive_expect_tx(kv_full0 + 8 * s, (uint32_t)(n * psize * 128 * 2 * kHalves));
-        }
-        __syncwarp();
-        if (row >= 0) {
+      auto bytes_of = [&](int it) {
+        return (uint32_t)(min(pieces, (limit - block_of(it) * kTcBN + psize - 1) >> psl) * psize * 128 * kHalves);
+      };
+      // block it's keys, then the values of the block before it: a K stage is free long before a V stage
+      int row = row_of(0), row_v = -1;
+      for (int it = 0; it <= nit; ++it) {
+        if (it < nit) {
+          if (lane == 0) {
+            mbar_wait(k_empty(it), k_phase(it) ^ 1u);
+            mbar_arrive_expect_tx(k_full(it), bytes_of(it));
+          }
+          __syncwarp();
+          if (row >= 0) {
 #pragma unroll
-          for (int half = 0; half < kHalves; ++half) {
-            const uint32_t dst = sbase + s * L::kStage + half * 8192 + lane * psize * 128;
-            tma_load_2d(dst + L::kK, &tk, kv_full0 + 8 * s, half * 64, row);
-            tma_load_2d(dst + L::kV, &tv, kv_full0 + 8 * s, half * 64, row);
+            for (int half = 0; half < kHalves; ++half)
+              tma_load_2d(k_at(it) + half * 8192 + lane * psize * 128, &tk, k_full(it), half * 64, row);
           }
         }
-        row = row_of(it + 1);
+        const int next = row_of(it + 1);
+        if (it > 0) {
+          const int j = it - 1;
+          if (lane == 0) {
+            mbar_wait(v_empty(j), v_phase(j) ^ 1u);
+            mbar_arrive_expect_tx(v_full(j), bytes_of(j));
+          }
+          __syncwarp();
+          if (row_v >= 0) {
+#pragma unroll
+            for (int half = 0; half < kHalves; ++half)
+              tma_load_2d(v_at(j) + half * 8192 + lane * psize * 128, &tv, v_full(j), half * 64, row_v);
+          }
+        }
+        row_v = row;
+        row = next;
       }
     } else if (lane == 0) {
       const int kcol = (p.H + hk) * D, vcol = (p.H + p.Hkv + hk) * D;
-      for (int j = 0; j < nit; ++j) {
-        const int s = j & 1;
-        mbar_wait(kv_empty0 + 8 * s, (((uint32_t)j >> 1) & 1u) ^ 1u);
-        mbar_arrive_expect_tx(kv_full0 + 8 * s, 2 * L::kStage);
-        const int r = row_base + j * kTcBN;
-        for (int half = 0; half < kHalves; ++half) {
-          tma_load_2d(sbase + L::kK + s * L::kStage + half * 8192, &tk, kv_full0 + 8 * s, kcol + half * 64, r);
-          tma_load_2d(sbase + L::kV + s * L::kStage + half * 8192, &tv, kv_full0 + 8 * s, vcol + half * 64, r);
+      for (int j = 0; j <= nit; ++j) {
+        if (j < nit) {
+          mbar_wait(k_empty(j), k_phase(j) ^ 1u);
+          mbar_arrive_expect_tx(k_full(j), L::kStage);
+          for (int half = 0; half < kHalves; ++half)
+            tma_load_2d(k_at(j) + half * 8192, &tk, k_full(j), kcol + half * 64, row_base + j * kTcBN);
+        }
+        if (j > 0) {
+          mbar_wait(v_empty(j - 1), v_phase(j - 1) ^ 1u);
+          mbar_arrive_expect_tx(v_full(j - 1), L::kStage);
+          for (int half = 0; half < kHalves; ++half)
+            tma_load_2d(v_at(j - 1) + half * 8192, &tv, v_full(j - 1), vcol + half * 64, row_base + (j - 1) * kTcBN);
         }
       }
     }
@@ -254,7 +295,7 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
       const uint32_t qlo = ((sbase + L::kQ) >> 4) | kLoK;
       auto issue_qk = [&](int j) {
         const int s = j & 1;
-        const uint32_t klo = ((sbase + L::kK + s * L::kStage) >> 4) | kLoK;
+        const uint32_t klo = (k_at(j) >> 4) | kLoK;
 #pragma unroll
         for (int half = 0; half < kHalves; ++half)
 #pragma unroll
@@ -262,27 +303,29 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
             umma_f16_w(tS + s * kTcBN, desc(qlo + half * (16384u >> 4) + ks * 2u), desc(klo + half * (8192u >> 4) + ks * 2u),
                      idesc_qk, (half | ks) ? 1u : 0u);
         umma_commit_w(s_full0 + 8 * s);
+        umma_commit_w(k_empty(j));
       };
       mbar_wait_spin(q_full, 0);
-      mbar_wait_spin(kv_full0, 0);
+      mbar_wait_spin(k_full(0), 0);
       tc_fence_after();
       issue_qk(0);
       for (int j = 0; j < nit; ++j) {
         const int s = j & 1;
         if (j + 1 < nit) {
-          mbar_wait_spin(kv_full0 + 8 * ((j + 1) & 1), ((uint32_t)(j + 1) >> 1) & 1u);
+          mbar_wait_spin(k_full(j + 1), k_phase(j + 1));
           // S buffer (j+1)&1 last held block j-1: P(j-1) sat in it and PV(j-1) was issued before this UMMA, the pipe runs in order
           tc_fence_after();
           issue_qk(j + 1);
         }
-        mbar_wait_spin(p_full, (uint32_t)j & 1u);               // P(j) is written (and O rescaled where a row needed it)
+        mbar_wait_spin(v_full(j), v_phase(j));
+        mbar_wait_spin(p_full0 + 8 * s, ((uint32_t)j >> 1) & 1u);       // P(j) is written (and O rescaled where a row needed it)
         tc_fence_after();
-        const uint32_t vlo = ((sbase + L::kV + s * L::kStage) >> 4) | kLoMN;
+        const uint32_t vlo = (v_at(j) >> 4) | kLoMN;
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks)
           umma_f16_ts_w(tO, tS + s * kTcBN + ks * 8, desc(vlo + ks * (2048u >> 4)), idesc_pv, (j | ks) ? 1u : 0u);
         umma_commit_w(o_done);
-        umma_commit_w(kv_empty0 + 8 * s);
+        umma_commit_w(v_empty(j));
       }
     }
   } else if (warp < 4) {
@@ -335,15 +378,18 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
           for (int i = 0; i < 64; ++i) v[i] = __float_as_uint(large ? tanh_any(__uint_as_float(v[i])) : tanh_small(__uint_as_float(v[i])));
         }
       }
-      float mx = -INFINITY;
       if (need_mask) {
 #pragma unroll
         for (int i = 0; i < 64; ++i) {
           if (hidden(kv0 + i)) v[i] = 0xff800000u;        // -inf
         }
       }
+      float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};   // four chains: two warps per scheduler hide little
 #pragma unroll
-      for (int i = 0; i < 64; ++i) mx = fmaxf(mx, __uint_as_float(v[i]));
+      for (int i = 0; i < 64; i += 8)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) m4[c] = max3(m4[c], __uint_as_float(v[i + 2 * c]), __uint_as_float(v[i + 2 * c + 1]));
+      const float mx = fmaxf(max3(m4[0], m4[1], m4[2]), m4[3]);
       const float m_new = fmaxf(m_ref, mx * sl);
       const bool raise = m_new > m_ref + kSlack;
       float alpha = 1.f;
@@ -370,21 +416,22 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
         }
       }
       l *= alpha;
-      float rs0 = 0.f, rs1 = 0.f;
-      const float nm = -m_use;
+      float2 rs[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+      const float2 nm = make_float2(-m_use, -m_use), sl2 = make_float2(sl, sl);
       uint32_t w[32];
 #pragma unroll
       for (int i = 0; i < 32; ++i) {
-        const float p0 = ex2f(fmaf(__uint_as_float(v[2 * i]), sl, nm)), p1 = ex2f(fmaf(__uint_as_float(v[2 * i + 1]), sl, nm));
-        rs0 += p0; rs1 += p1;
-        w[i] = pack16<BF16>(p0, p1);
+        float2 e = __ffma2_rn(make_float2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])), sl2, nm);
+        e.x = ex2f(e.x); e.y = ex2f(e.y);
+        rs[i & 1] = __fadd2_rn(rs[i & 1], e);
+        w[i] = pack16<BF16>(e.x, e.y);
       }
       tmem_st_32x32(tS + sb * kTcBN, w);
       if (kv0 + kTcBN > limit) {                          // the sequence's last block: V rows that are not its own become zeros
-        mbar_wait_warp(kv_full0 + 8 * sb, ((uint32_t)j >> 1) & 1u);
+        mbar_wait_warp(v_full(j), v_phase(j));
         for (int i = threadIdx.x; i < (kv0 + kTcBN - limit) * 8 * kHalves; i += 128) {
           const int row = limit - kv0 + i / (8 * kHalves), c = i % (8 * kHalves);
-          asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(sbase + L::kV + sb * L::kStage + (c >> 3) * 8192 + row * 128 + (c & 7) * 16),
+          asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(v_at(j) + (c >> 3) * 8192 + row * 128 + (c & 7) * 16),
                        "r"(0) : "memory");
         }
         fence_proxy_async_smem();                         // generic-proxy stores -> visible to tcgen05.mma
@@ -392,8 +439,8 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(p_full);
-      l += rs0 + rs1;
+      if (lane == 0) mbar_arrive(p_full0 + 8 * sb);
+      l += (rs[0].x + rs[0].y) + (rs[1].x + rs[1].y);
     }
     // ---- finish: O / l -> 16 bit through shared memory (the Q tile is dead: every QK product has completed) ----
     mbar_wait_warp(o_done, (uint32_t)(nit - 1) & 1u);
@@ -425,7 +472,7 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
       }
     }
     if (MODE == kTcDense && p.lse && live)
-      p.lse[((long long)blockIdx.z * p.H + h) * p.S + grow] = m_ref * 0.6931471805599453f + __logf(l);
+      p.lse[((long long)blockIdx.y * p.H + h) * p.S + grow] = m_ref * 0.6931471805599453f + __logf(l);
     __syncwarp();
     // each warp copies ITS 32 rows out (written by its own lanes): CH lanes cover the bytes of a row
     uint16_t* obase = reinterpret_cast<uint16_t*>(p.out);
@@ -495,7 +542,7 @@ using namespace b200;
 static int tc_check(const void* qkv, const void* out, int B, int S, int H, int Hkv, int D, float scale, int dtype) {
   if ((D != 64 && D != 128) || (dtype != B200_DT_BF16 && dtype != B200_DT_FP16) || !(scale > 0.f)) return B200_ERR_UNSUPPORTED;
   if (B < 1 || S < 1 || H < 1 || Hkv < 1 || H % Hkv) return B200_ERR_BAD_SHAPE;
-  if (H > 65535 || B > 65535) return B200_ERR_UNSUPPORTED;
+  if (H > 65535 || B > 65535 || (S + kTcBM - 1) / kTcBM > 65535) return B200_ERR_UNSUPPORTED;
   if ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(out)) & 15) return B200_ERR_BAD_ALIGN;
   return 0;
 }
@@ -509,7 +556,7 @@ B200_API int b200_flash_attn_fwd_tc(const void* qkv, void* out, float* lse, int 
   FlashTcParams p = {};
   p.out = out; p.lse = lse; p.S = S; p.H = H; p.Hkv = Hkv; p.out_rs = (long long)H * D;
   p.scale_log2 = scale * kTcLog2e; p.causal = causal;
-  return fused_qkv<kTcDense>(qkv, (long long)B * S, p, D, dtype, dim3((S + kTcBM - 1) / kTcBM, H, B), stream);
+  return fused_qkv<kTcDense>(qkv, (long long)B * S, p, D, dtype, dim3(H, B, (S + kTcBM - 1) / kTcBM), stream);
 }
 
 // The packed form (see b200_flash_attn_varlen_fwd): `tokens` rows hold n_seqs sequences back to back, the longest of max_seqlen rows.
@@ -520,7 +567,7 @@ B200_API int b200_flash_attn_varlen_fwd_tc(const void* qkv, void* out, const int
   FlashTcParams p = {};
   p.out = out; p.cu = cu_seqlens; p.S = max_seqlen; p.H = H; p.Hkv = Hkv; p.out_rs = (long long)H * D;
   p.scale_log2 = scale * kTcLog2e; p.causal = causal;
-  return fused_qkv<kTcVarlen>(qkv, tokens, p, D, dtype, dim3((max_seqlen + kTcBM - 1) / kTcBM, H, n_seqs), stream);
+  return fused_qkv<kTcVarlen>(qkv, tokens, p, D, dtype, dim3(H, n_seqs, (max_seqlen + kTcBM - 1) / kTcBM), stream);
 }
 
 // Prompt pieces over a paged cache, one map, key and value rows of one size (arguments as in b200_multimap_attn_mma_ex; `tokens`: rows
