@@ -205,21 +205,26 @@ __device__ __forceinline__ void mbar_wait_sleep(uint32_t bar, uint32_t parity, u
   }
 }
 
-// Spin on the non-blocking test_wait (try_wait may park the thread for a system-dependent time).
-__device__ __forceinline__ void mbar_wait_spin(uint32_t bar, uint32_t parity) {
+// Spin on the non-blocking test_wait (try_wait may park the thread for a system-dependent time). The clock is read only where the first
+// test fails: these waits are on the critical path of the attention kernels' hand-offs, and most of them find the phase complete.
+__device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ void mbar_wait_spin(uint32_t bar, uint32_t parity) {
+  if (mbar_test_wait(bar, parity)) return;
   const long long t0 = clock64();
-  do {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    if (!ok && clock64() - t0 > B200_MBAR_TIMEOUT_CYCLES) {
+  while (!mbar_test_wait(bar, parity)) {
+    if (clock64() - t0 > B200_MBAR_TIMEOUT_CYCLES) {
       printf("b200: mbarrier wait timed out (block %d thread %d bar 0x%x parity %u)\n", blockIdx.x, threadIdx.x, bar, parity);
       __trap();
     }
-  } while (!ok);
+  }
 }
 
 // Whole-warp wait with one polling lane: 32 lanes spinning on try_wait steal issue slots and shared-memory

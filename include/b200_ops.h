@@ -409,8 +409,8 @@ int b200_paged_attn_tc(const void* q, long long tokens, const void* ck, const vo
                        int block_size, float scale, int window, int keep_first, float post, const struct b200_attn_opts* opts, int dtype,
                        void* stream);
 
-/* Backward on the same tensor cores (csrc/flash_bwd_tc.cu): a dK/dV pass (K, V resident per 128-key block, query tiles
- * stream) and a dQ pass (Q, dO resident per 128-row tile, key blocks stream), every product a tcgen05.mma with TMEM
+/* Backward on the same tensor cores (csrc/flash_bwd_tc.cu): a dQ pass (Q, dO resident per 128-row tile, key blocks stream; it
+ * also forms delta) and a dK/dV pass (K, V resident per 128-key block, query tiles stream), every product a tcgen05.mma with TMEM
  * accumulators; no atomics and no fp32 staging buffer (delta [B, H, S] is the only work buffer). head_dim 64 or 128, 16-bit,
  * scale > 0, no dropout; B200_ERR_UNSUPPORTED otherwise. */
 int b200_flash_attn_bwd_tc(const void* qkv, const void* out, const void* dout, const float* lse, float* delta, void* dqkv,

@@ -65,7 +65,7 @@ class _FlashAttentionFn(torch.autograd.Function):
                     float(scale), nv.dtype_code(qkv.dtype), nv.stream())
             if rc != 10006:
                 nv.check(rc, "flash_attn_bwd_tc")
-                nv.count_launch(3)   # delta, dK/dV pass, dQ pass
+                nv.count_launch(2)   # dQ pass (with delta), dK/dV pass
                 return dqkv, None, None, None, None, None, None, None, None, None
         dqkv32 = torch.empty(qkv.shape, dtype=torch.float32, device=qkv.device)
         fn = nv.proto("b200_flash_attn_bwd", [vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, f32, f32, u64, i32, vp])
