@@ -1144,6 +1144,19 @@ B200_API int b200_gemm(const b200_gemm_args* a, void* stream_) {
   return 0;
 }
 
+B200_API int b200_gemm_2d(const void* A, const void* B, void* D, const void* bias, const float* beta_rows, const void* A2, const void* B2,
+                          void* workspace, long long workspace_bytes, int M, int N, int K, int K2, long long a_rs, long long b_rs,
+                          long long d_rs, long long a2_rs, long long b2_rs, int a_mn, int b_mn, int in_dtype, int out_dtype, int bias_dtype,
+                          float alpha, float beta, void* stream) {
+  b200_gemm_args a = {};
+  a.A = A; a.B = B; a.D = D; a.bias = bias; a.beta_rows = beta_rows; a.A2 = A2; a.B2 = B2;
+  a.M = M; a.N = N; a.K = K; a.K2 = K2; a.batch = a.nb0 = a.b_div = 1;
+  a.a_rs = a_rs; a.b_rs = b_rs; a.d_rs = d_rs; a.a2_rs = a2_rs; a.b2_rs = b2_rs;
+  a.a_mn = a_mn; a.b_mn = b_mn; a.in_dtype = in_dtype; a.out_dtype = out_dtype; a.bias_dtype = bias_dtype;
+  a.alpha = alpha; a.beta = beta; a.workspace = workspace; a.workspace_bytes = workspace_bytes;
+  return b200_gemm(&a, stream);
+}
+
 B200_API int b200_gemm_w4(const b200_gemm_args* a, const b200_w4_desc* w, void* stream_) {
   cudaStream_t stream = (cudaStream_t)stream_;
   constexpr int ES = 2, EPR = 64, ctas = 2, bn = 256, bn_cta = 128;

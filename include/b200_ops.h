@@ -108,6 +108,11 @@ typedef struct b200_gemm_allreduce {
 long long b200_gemm_workspace_bytes(void);
 
 int b200_gemm(const b200_gemm_args* args, void* stream);
+/* b200_gemm of two matrices (batch 1) with plain arguments, for callers to whom filling the structure costs more than the launch. */
+int b200_gemm_2d(const void* A, const void* B, void* D, const void* bias, const float* beta_rows, const void* A2, const void* B2,
+                 void* workspace, long long workspace_bytes, int M, int N, int K, int K2, long long a_rs, long long b_rs, long long d_rs,
+                 long long a2_rs, long long b2_rs, int a_mn, int b_mn, int in_dtype, int out_dtype, int bias_dtype, float alpha, float beta,
+                 void* stream);
 
 /* The same GEMM with the B operand expanded from 4-bit codes inside the kernel: NF4 (QLoRA base,
  * Fine-Tuning/qwen3-14b-qlora-dist-deepspeed.py:101-106) or GPTQ/AWQ W4A16 weights

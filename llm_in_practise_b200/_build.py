@@ -11,9 +11,11 @@ under ``llm_in_practise_b200/_lib`` so they travel with the source tree.
 from __future__ import annotations
 
 import os
+import platform
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -123,6 +125,21 @@ def build_host(force: bool = False) -> Path:
     hdrs = list((CSRC / "host").glob("*.h")) + list((ROOT / "include").glob("*.h"))
     if force or _stale(out, srcs + hdrs):
         _run(["g++", *CXX_FLAGS, "-shared", "-o", str(out), *map(str, srcs)])
+    build_fastcall(force)
+    return out
+
+
+def build_fastcall(force: bool = False):
+    """The Python extension that calls the C ABI (``ops._native``); None where Python's headers or the ABI it relies on are missing:
+    calls then go through ctypes."""
+    include = sysconfig.get_paths()["include"]
+    src, out = CSRC / "host" / "python" / "fastcall.cpp", LIBDIR / "_b200_fastcall.so"
+    if not Path(include, "Python.h").exists() or platform.machine() != "x86_64" or sys.platform != "linux":
+        return None
+    if force or _stale(out, [src]):
+        tmp = out.with_suffix(".so.tmp%d" % os.getpid())
+        _run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-I", include, str(src), "-o", str(tmp)])
+        os.replace(tmp, out)
     return out
 
 

@@ -16,6 +16,7 @@ import os
 from dataclasses import dataclass
 from typing import List, Optional, Sequence, Tuple
 
+import numpy as np
 import torch
 
 from ..ops.gemm import ensure_graph_workspace
@@ -125,8 +126,6 @@ class RaggedGenerator(Generator):
                 and all(len(e[2]) == 1 and list(e[3]) == [0] for e in entries)):
             return self.decode([e[2][0] for e in entries], [e[1] for e in entries], [e[0] for e in entries], cache)
         ids: List[int] = []
-        pos: List[int] = []
-        slot: List[int] = []
         want: List[int] = []
         runs: List[List[int]] = []
         max_pos = 0
@@ -138,22 +137,22 @@ class RaggedGenerator(Generator):
                 raise ValueError(f"sequence of {pos0 + n} tokens does not fit the cache rows of {cache.max_len}")
             self._check_position(pos0 + n - 1)
             base = len(ids)
-            ids.extend(int(t) for t in toks)
-            pos.extend(range(pos0, pos0 + n))
-            slot.extend([row] * n)
+            ids.extend(map(int, toks))
             want.extend(base + int(w) for w in wanted)
             runs.append([base, n, pos0, row])
             max_pos = max(max_pos, pos0 + n - 1)
         if not ids:
             return None
-        meta = torch.tensor(pos + slot, dtype=torch.int32).view(2, -1)
+        # token t of a run is at its first position + (t - its first row): built by numpy, not token by token, and what goes to the device
+        # goes in two copies from pinned memory (a copy from pageable memory waits for the work queued before it)
+        first, count, start, rows = np.asarray(runs, dtype=np.int64).T
+        meta = torch.from_numpy(np.stack([np.arange(len(ids)) + np.repeat(start - first, count), np.repeat(rows, count)]).astype(np.int32))
+        long = torch.from_numpy(np.asarray(ids + (want or [0]), dtype=np.int64))
         if dev.type == "cuda":
             meta = meta.pin_memory().to(dev, non_blocking=True)
-            ids_t = torch.tensor(ids, dtype=torch.long).pin_memory().to(dev, non_blocking=True)
-        else:
-            ids_t = torch.tensor(ids, dtype=torch.long)
+            long = long.pin_memory().to(dev, non_blocking=True)
+        ids_t, want_t = long[:len(ids)], long[len(ids):]
         pieces = make_pieces(runs, dev)
-        want_t = torch.tensor(want, dtype=torch.long, device=dev) if want else torch.zeros(1, dtype=torch.long, device=dev)
         logits = self.model.forward_ragged(ids_t, meta[0], meta[1], cache, want_t, max_pos=max_pos, pieces=pieces,
                                            layer_outputs=layer_outputs)
         return logits if want else None

@@ -8,6 +8,7 @@ numerical oracles of the GPU tests.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 from pathlib import Path
 
@@ -16,6 +17,9 @@ import torch
 _LIBDIR = Path(__file__).resolve().parent.parent / "_lib"
 _lib = None
 _host_lib = None
+# the mapping behind os.environ, whose own look-up encodes the key each time (0.5 us, once or twice an op)
+_environ = getattr(os.environ, "_data", os.environ)
+_FORCE_KEY, _FORCE_ON = ("B200_FORCE_TORCH", "1") if _environ is os.environ else (os.environ.encodekey("B200_FORCE_TORCH"), os.environ.encodevalue("1"))
 launch_count = 0  # number of kernel launches issued through this binding (bench.py reports it)
 
 DT_BF16, DT_FP16, DT_FP32 = 0, 1, 2
@@ -61,9 +65,10 @@ def use_native(*tensors) -> bool:
     library is fatal there); CPU tensors go to the PyTorch reference path."""
     if not tensors or not tensors[0].is_cuda:
         return False
-    if os.environ.get("B200_FORCE_TORCH") == "1":
+    if _environ.get(_FORCE_KEY) == _FORCE_ON:
         return False
-    lib()  # raises if missing
+    if _lib is None:
+        lib()  # raises if missing
     return True
 
 
@@ -167,14 +172,40 @@ def _declare(L: ctypes.CDLL) -> None:
     # remaining prototypes are declared next to their Python wrappers via `proto`
 
 
-_declared = set()
+_KINDS = {ctypes.c_void_p: "p", ctypes.c_float: "f", **{t: "i" for t in (ctypes.c_int, ctypes.c_longlong, ctypes.c_int32, ctypes.c_int64,
+                                                                              ctypes.c_uint32, ctypes.c_uint64, ctypes.c_ulonglong)}}
 
 
-def proto(name: str, argtypes) -> ctypes._CFuncPtr:
-    """Fetch an entry point and (once) attach its argument types."""
-    fn = getattr(lib(), name)
-    if name not in _declared:
+def _fastcall():
+    """``make`` of the extension that calls the C ABI (csrc/host/python/fastcall.cpp), or None: calls then go through ctypes."""
+    p = _LIBDIR / "_b200_fastcall.so"
+    if not p.exists():
+        return None
+    try:
+        spec = importlib.util.spec_from_file_location("_b200_fastcall", p)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        return module.make
+    except ImportError:                      # built for another Python
+        return None
+
+
+_make_entry = _fastcall()
+
+
+def proto(name: str, argtypes):
+    """An entry point of the library as a callable with these argument types; made once per library. The ctypes function, or where all
+    its arguments are numbers and pointers a callable without ctypes' 2 us a call, which falls back on it for any other argument."""
+    L = _lib if _lib is not None else lib()
+    made = L.__dict__.get("_b200_entries")
+    if made is None:
+        made = L._b200_entries = {}
+    fn = made.get(name)
+    if fn is None:
+        fn = getattr(L, name)
         fn.argtypes = argtypes
         fn.restype = ctypes.c_int
-        _declared.add(name)
+        if _make_entry is not None and all(t in _KINDS for t in argtypes):
+            fn = _make_entry(ctypes.cast(fn, ctypes.c_void_p).value, "".join(_KINDS[t] for t in argtypes), fn) or fn
+        made[name] = fn
     return fn

@@ -60,7 +60,7 @@ def _stream_k_workspace(device: torch.device) -> Optional[torch.Tensor]:
     """Per (device, stream) scratch for stream-K GEMMs: zeroed once, then owned by that stream."""
     if _overlapped_collectives:
         return None
-    if torch.cuda.is_current_stream_capturing():
+    if torch._C._cuda_isCurrentStreamCapturing():
         return _sk_workspaces.get((device.index, "graph"))       # None: captured without stream-K
     index = device.index if device.index is not None else torch._C._cuda_getDevice()
     key = (index, torch._C._cuda_getCurrentRawStream(index))
@@ -138,6 +138,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         a = a.contiguous()
     if b.stride(-1) != 1:
         b = b.contiguous()
+    if ar is None and a.dim() == 2 and b.dim() == 2:
+        return _gemm_2d(a, b, a_mn, b_mn, out, out_dtype, alpha, beta, bias, lora, beta_rows)
     a4, b4 = _as4d(a), _as4d(b)
     if a_mn:
         K, M = a4.shape[-2], a4.shape[-1]
@@ -204,6 +206,41 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     nv.check(rc, f"gemm M={M} N={N} K={K} batch={batch}")
     nv.count_launch()
     del keep
+    return out
+
+
+_GEMM_2D = [ctypes.c_void_p] * 8 + [ctypes.c_longlong] + [ctypes.c_int] * 4 + [ctypes.c_longlong] * 5 + [ctypes.c_int] * 5 + \
+    [ctypes.c_float] * 2 + [ctypes.c_void_p]
+
+
+def _gemm_2d(a, b, a_mn, b_mn, out, out_dtype, alpha, beta, bias, lora, beta_rows):
+    """``gemm`` of two matrices, the common case: plain arguments instead of the structure with its batch strides (25 us a call with them,
+    14 without, of which the launch is 5)."""
+    K, M = a.shape if a_mn else a.shape[::-1]
+    Kb, N = b.shape if b_mn else b.shape[::-1]
+    if K != Kb:
+        raise ValueError(f"contraction mismatch: {K} vs {Kb}")
+    if out is None:
+        out = torch.empty(M, N, dtype=out_dtype, device=a.device)
+    elif tuple(out.shape) != (M, N) or out.stride(1) != 1:
+        raise ValueError(f"`out` must have shape {(M, N)} with a contiguous last dim")
+    a2 = b2 = None
+    k2 = a2_rs = b2_rs = 0
+    if lora is not None:
+        a2, b2 = lora
+        if a2.dtype != a.dtype or b2.dtype != a.dtype:
+            raise TypeError("lora operands must match the main dtype")
+        a2 = a2 if a2.stride(-1) == 1 else a2.contiguous()
+        b2 = b2 if b2.stride(-1) == 1 else b2.contiguous()
+        k2, a2_rs, b2_rs = a2.shape[-1], a2.stride(0), b2.stride(0)
+    ws = _stream_k_workspace(a.device)
+    fn = nv.proto("b200_gemm_2d", _GEMM_2D)
+    rc = fn(a.data_ptr(), b.data_ptr(), out.data_ptr(), nv.ptr(bias), nv.ptr(beta_rows), nv.ptr(a2), nv.ptr(b2), nv.ptr(ws),
+            0 if ws is None else ws.numel(), M, N, K, k2, a.stride(0), b.stride(0), out.stride(0), a2_rs, b2_rs, int(a_mn), int(b_mn),
+            nv.dtype_code(a.dtype), nv.dtype_code(out.dtype), nv.dtype_code(bias.dtype) if bias is not None else 0, alpha, beta, nv.stream())
+    if rc:
+        nv.check(rc, f"gemm M={M} N={N} K={K} batch=1")
+    nv.count_launch()
     return out
 
 
