@@ -15,12 +15,13 @@
 //                             c_i and r_64,j -> workspace. Chunks do not wait for one another.
 //   delta_chunk_scan_kernel   a CTA per (run, head, block of 16 value columns) walks the chunks with its columns of S in registers
 //                             and, for the products, in shared memory: [K; Q] S_0, U = T R, O += P U, S += K^T U. What the next
-//                             chunk needs is on its way (cp.async) meanwhile.
+//                             chunk needs is on its way (bulk copies) meanwhile.
 // All in fp32 FMAs (two per instruction), no tensor cores: the state is fp32 by definition, and splitting fp32 operands for bf16 or
 // tf32 mma.sync takes as many cycles as the FMAs do. r_ij is a product taken from j upwards, the roundings a walk makes too;
-// sums of logarithms would lose digits to cancellation. Bound: the latency of the sums across lanes with two warps per scheduler
-// (44 % of the issue slots are used), then the FMA rate. One prompt of 2048 tokens, 16 heads of 128 x 128 over 4 q/k heads: 502 us token
-// by token, 18 + 207 here; 2048 and 513 tokens: 586 -> 285 (6 more with the test for infinities and NaN); error of the state against 64 bits 2e-7 both ways.
+// sums of logarithms would lose digits to cancellation. Bound: a packed FMA with three register operands takes 2.7 cycles of a scheduler, not
+// 2 (95 FMAs a cycle and SM of 128, measured alone), 5500 of a chunk's 11 800 cycles; then the latency of the sums across lanes and the
+// three barriers of a chunk. One prompt of 2048 tokens, 16 heads of 128 x 128 over 4 q/k heads: 502 us token by token, 18 + 194 here; 2048 and
+// 513 tokens: 586 -> 272 (the shorter run's CTAs fill in behind the longer one's); error of the state against 64 bits 2e-7 both ways.
 #include "common.cuh"
 #include "../include/b200_ops.h"
 
@@ -37,12 +38,9 @@ struct DeltaChunkArgs {
   int n_runs, H, G, Dv, tile_lo, tile_hi;                 // chunks [tile_lo, tile_hi) of all the step's chunks, counted run by run
 };
 
-// 16 (4) bytes on their way to shared memory; zeros where `live` is false
+// 16 bytes on their way to shared memory; zeros where `live` is false
 __device__ __forceinline__ void dc_copy16(float* dst, const float* src, bool live) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(live ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ void dc_copy4(float* dst, const float* src, bool live) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(live ? 4 : 0) : "memory");
 }
 __device__ __forceinline__ void dc_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ float2 lo2(const float4& v) { return make_float2(v.x, v.y); }
@@ -163,8 +161,8 @@ template <int D> struct DcSmem {                          // float offsets
   static constexpr int NC = kDcNC;
   static constexpr int DP = D + 4;
   static constexpr int K = 0, Q = K + 2 * kDcC * DP, T = Q + kDcC * DP, P = T + kDcC * kDcCP, V = P + 2 * kDcC * kDcCP, S = V + 2 * kDcC * NC,
-                       R = S + D * NC, U = R + kDcC * NC, UD = U + kDcC * NC, O = UD + kDcC * NC, X = O + kDcC * NC,
-                       kTotal = X + 2 * 3 * kDcC;         // X: c | r_64 | beta, twice
+                       R = S + D * NC, U = R + kDcC * NC, UD = U + kDcC * NC, X = UD + kDcC * NC,
+                       Bar = X + 2 * 3 * kDcC, kTotal = Bar + 8;       // X: c | r_64 | beta, twice; Bar: K, V, P, X of each buffer, Q and T
 };
 
 // Where columns c, c + 1 (c even) of the pair of rows pr lie in a [rows / 2][16][2] array: 16 bytes, the two halves of 32 changing places
@@ -219,16 +217,28 @@ __device__ __forceinline__ float lower_dot(const float* row, const float* X, int
 }
 __device__ __forceinline__ bool not_finite(float x) { return !(fabsf(x) <= 3.402823466e38f); }
 
+// an "or" over the 256 threads of the chain's warps, and a barrier for them
+__device__ __forceinline__ int chain_or(int x) {
+  int r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\t"
+      "barrier.cta.red.or.pred q, 1, 256, p;\n\tselp.s32 %0, 1, 0, q;\n\t}" : "=r"(r) : "r"(x) : "memory");
+  return r;
+}
+
 // What limits the walk is shared memory, 128 bytes a cycle into registers against 128 FMAs: a tile of 4 x 4 outputs per thread would
 // take two bytes per FMA. So the small side of every product but the last stays in registers — S_0 with 16 rows of four columns in
 // every lane of every warp, R and U with eight — and a row of the other side costs one byte per FMA; the lanes' parts of
 // a row meet in four shuffles. Shared layouts: S, R and U hold pairs of neighbouring rows of one column side by side
 // ([rows / 2][16][2], pair_at), the pairs a packed FMA takes.
+// What the next chunk waits for is only K S_0, U = T R and S += K^T U. Warps 0-7, the chain, do these; warps 8-15 read out beside them: Q S_0
+// while the chain is at K S_0 and T R, then P U while it is at K^T U. Eight warps for all of it one after the other and copies of 16 bytes
+// by all of them: 262 us for runs of 2048 and 513 tokens, 245 now; the halves alone, with those copies, gave nothing (264).
 template <int D>
-__global__ void __launch_bounds__(256, 1)
+__global__ void __launch_bounds__(512, 1)
 delta_chunk_scan_kernel(const DeltaChunkArgs p) {
   using L = DcSmem<D>;
-  constexpr int NC = kDcNC, DP = L::DP, NT = 256, DT = D / 32;     // DT: state rows of a thread
+  constexpr int NC = kDcNC, DP = L::DP, DT = D / 32;     // DT: state rows of a thread
   extern __shared__ __align__(16) float sm[];
   const int h = blockIdx.y, col0 = blockIdx.x * NC, run = blockIdx.z;
   int tb = 0;
@@ -236,54 +246,64 @@ delta_chunk_scan_kernel(const DeltaChunkArgs p) {
   const int first = p.runs[4 * run], len = p.runs[4 * run + 1], p0 = p.runs[4 * run + 2], slot = p.runs[4 * run + 3];
   const int t_lo = max(tb, p.tile_lo), t_hi = min(tb + (len + kDcC - 1) / kDcC, p.tile_hi);
   if (t_lo >= t_hi) return;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31, warp = (tid >> 5) & 7;    // the warp's place in its half
+  const bool chain = tid < 256;
   const int rl = lane >> 2, cb = (lane & 3) * 4;          // this thread's four columns
   const int cg = cb + (lane >> 4) * 2 + (lane >> 3 & 1);  // and the one whose sum over the warp it ends up with (gather4)
-  const int kvh = h / (p.H / p.G);
+  const int kvh = h / (p.H / p.G), t8 = warp * 8;         // a warp's eight tokens of a chunk
 
-  auto fetch_kvp = [&](int tile, int buf) {
-    const int at = (tile - tb) * kDcC, n = min(kDcC, len - at);
-    for (int i = tid; i < kDcC * (D / 4); i += NT) {
-      const int t = i / (D / 4), d = i % (D / 4) * 4;
-      dc_copy16(sm + L::K + (buf * kDcC + t) * DP + d, p.k + (long long)(first + at + min(t, n - 1)) * p.ldk + (long long)kvh * D + d, t < n);
-    }
-    for (int i = tid; i < kDcC * (NC / 4); i += NT) {
-      const int t = i / (NC / 4), c = i % (NC / 4) * 4;
-      dc_copy16(sm + L::V + (buf * kDcC + t) * NC + c, p.v + (long long)(first + at + min(t, n - 1)) * p.ldv + (long long)h * p.Dv + col0 + c, t < n);
-    }
+  // What a chunk needs comes a row at a time by bulk copies, one to a thread of the reading half: cp.async pieces of 16 bytes took all warps
+  // 2400 of a chunk's 12 700 cycles to ask for. A barrier is armed one barrier of the CTA before its copies are asked for.
+  const uint32_t bar = smem_u32(sm + L::Bar);
+  auto kvp_bar = [&](int tile) { return bar + 8u * (tile & 1); };
+  const uint32_t qt_bar = bar + 16;
+  auto rows_of = [&](int tile) { return min(kDcC, len - (tile - tb) * kDcC); };
+  auto arm_kvp = [&](int tile) { mbar_arrive_expect_tx(kvp_bar(tile), (uint32_t)(rows_of(tile) * (D + NC) + kDcC * kDcC + 2 * kDcC) * 4u); };
+  auto arm_qt = [&](int tile) { mbar_arrive_expect_tx(qt_bar, (uint32_t)(rows_of(tile) * D + kDcC * kDcC) * 4u); };
+  const int ri = tid - 256;                               // place in the reading half
+  auto row_copy = [&](float* dst, const float* src, int floats, bool there, uint32_t b) {
+    if (there) bulk_load_1d(smem_u32(dst), src, floats * 4, b);
+    else
+      for (int i = 0; i < floats; i += 4) *reinterpret_cast<float4*>(dst + i) = make_float4(0.f, 0.f, 0.f, 0.f);     // tokens past the end
+  };
+  auto ask_kvp = [&](int tile) {
+    const int buf = tile & 1, n = rows_of(tile), j = ri & 63;
+    const long long row = first + (tile - tb) * kDcC + min(j, n - 1);
     const float* w = p.ws + ((long long)(tile - p.tile_lo) * p.H + h) * kDcWs + kDcC * kDcC;
-    for (int i = tid; i < kDcC * (kDcC / 4); i += NT) {
-      const int t = i / (kDcC / 4), c = i % (kDcC / 4) * 4;
-      dc_copy16(sm + L::P + (buf * kDcC + t) * kDcCP + c, w + t * kDcC + c, true);
-    }
-    float* x = sm + L::X + buf * 3 * kDcC;
-    if (tid < 2 * kDcC / 4) dc_copy16(x + tid * 4, w + kDcC * kDcC + tid * 4, true);
-    if (tid < kDcC) dc_copy4(x + 2 * kDcC + tid, p.beta + (long long)(first + at + min(tid, n - 1)) * p.ldb + h, tid < n);
-  };
-  auto fetch_q = [&](int tile) {
-    const int at = (tile - tb) * kDcC, n = min(kDcC, len - at);
-    for (int i = tid; i < kDcC * (D / 4); i += NT) {
-      const int t = i / (D / 4), d = i % (D / 4) * 4;
-      dc_copy16(sm + L::Q + t * DP + d, p.q + (long long)(first + at + min(t, n - 1)) * p.ldq + (long long)kvh * D + d, t < n);
+    if (ri < 64) row_copy(sm + L::K + (buf * kDcC + j) * DP, p.k + row * p.ldk + (long long)kvh * D, D, j < n, kvp_bar(tile));
+    else if (ri < 128) row_copy(sm + L::V + (buf * kDcC + j) * NC, p.v + row * p.ldv + (long long)h * p.Dv + col0, NC, j < n, kvp_bar(tile));
+    else if (ri < 192) row_copy(sm + L::P + (buf * kDcC + j) * kDcCP, w + j * kDcC, kDcC, true, kvp_bar(tile));
+    else {
+      if (j == 0) row_copy(sm + L::X + buf * 3 * kDcC, w + kDcC * kDcC, 2 * kDcC, true, kvp_bar(tile));
+      sm[L::X + buf * 3 * kDcC + 2 * kDcC + j] = j < n ? p.beta[row * p.ldb + h] : 0.f;
     }
   };
-  auto fetch_t = [&](int tile) {
+  auto ask_qt = [&](int tile) {
+    const int n = rows_of(tile), j = ri & 63;
+    const long long row = first + (tile - tb) * kDcC + min(j, n - 1);
     const float* w = p.ws + ((long long)(tile - p.tile_lo) * p.H + h) * kDcWs;
-    for (int i = tid; i < kDcC * (kDcC / 4); i += NT) {
-      const int t = i / (kDcC / 4), c = i % (kDcC / 4) * 4;
-      dc_copy16(sm + L::T + t * kDcCP + c, w + t * kDcC + c, true);
-    }
+    if (ri < 64) row_copy(sm + L::Q + j * DP, p.q + row * p.ldq + (long long)kvh * D, D, j < n, qt_bar);
+    else if (ri < 128) row_copy(sm + L::T + j * kDcCP, w + j * kDcC, kDcC, true, qt_bar);
   };
-  fetch_kvp(t_lo, t_lo & 1);
-  fetch_q(t_lo);
-  fetch_t(t_lo);
+  if (tid == 256) {
+    for (int i = 0; i < 3; ++i) mbar_init(bar + 8 * i, 1);
+    fence_mbar_init();
+    arm_kvp(t_lo);
+    arm_qt(t_lo);
+    if (t_lo + 1 < t_hi) arm_kvp(t_lo + 1);
+  }
+  __syncthreads();
+  if (!chain) {
+    ask_kvp(t_lo);
+    ask_qt(t_lo);
+  }
 
-  // the state: rows d0 .. d0 + DT of four columns, in pairs of rows, kept by the first four warps; the other four add up the second
+  // the state: rows d0 .. d0 + DT of four columns, in pairs of rows, kept by the first four warps; the chain's other four add up the second
   // half of each chunk's tokens
   const int d0 = ((warp & 3) * 8 + rl) * DT;
   float* sp = p.state + (((long long)slot * p.H + h) * D) * p.Dv + col0 + cb;
   float2 S[DT / 2][4];
-  const bool from_state = p0 > 0 || t_lo > tb, owner = warp < 4;
+  const bool from_state = p0 > 0 || t_lo > tb, owner = tid < 128;
 #pragma unroll
   for (int x = 0; x < DT / 2; ++x) {
     float4 s0 = make_float4(0.f, 0.f, 0.f, 0.f), s1 = s0;
@@ -302,112 +322,113 @@ delta_chunk_scan_kernel(const DeltaChunkArgs p) {
   };
   if (owner) publish_state();
 
+  // N pairs of pairs of rows of S, R or U, every eighth of them the lane's own
+  auto hold = [&](const float* X, auto& B) {
+    constexpr int N = sizeof(B) / sizeof(B[0]);
+#pragma unroll
+    for (int x = 0; x < N; ++x) {
+      const int pr = ((x >> 1) * 8 + rl) * 2 + (x & 1);
+      const float4 b0 = *reinterpret_cast<const float4*>(X + pair_at(pr, cb)), b1 = *reinterpret_cast<const float4*>(X + pair_at(pr, cb + 2));
+      B[x][0] = lo2(b0); B[x][1] = hi2(b0); B[x][2] = lo2(b1); B[x][3] = hi2(b1);
+    }
+  };
+  // eight rows of a [64, D] tile times the state: column cg of rows t8 .. t8 + 7
+  auto times_state = [&](const float* rows, float (&y)[8]) {
+    float2 s0[D / 16][4];
+    hold(sm + L::S, s0);
+#pragma unroll
+    for (int i = 0; i < 8; i += 2) {
+      float4 z[2];
+      dot_rows<2, D / 32>(rows + (t8 + i) * DP + rl * 4, DP, s0, z);
+      y[i] = gather4(z[0], lane);
+      y[i + 1] = gather4(z[1], lane);
+    }
+  };
+  // eight rows of a lower triangle times X (R or U); `odd`: X holds an infinity or NaN
+  auto times_lower = [&](const float* rows, const float* X, int odd, float (&y)[8]) {
+    float2 B[4][4];
+    hold(X, B);
+#pragma unroll
+    for (int i = 0; i < 8; i += 4) {
+      float4 z[4];
+      dot_rows<4, 2>(rows + (t8 + i) * kDcCP + rl * 4, kDcCP, B, z);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) y[i + e] = gather4(z[e], lane);
+    }
+    if (odd) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) y[i] = lower_dot(rows + (t8 + i) * kDcCP, X, t8 + i, cg);
+    }
+  };
+
   for (int tile = t_lo; tile < t_hi; ++tile) {
     const int buf = tile & 1;
     const int at = (tile - tb) * kDcC, n = min(kDcC, len - at);
-    const bool more = tile + 1 < t_hi;
-    dc_wait_all();
-    __syncthreads();
-    if (more) fetch_kvp(tile + 1, buf ^ 1);
+    const bool more = tile + 1 < t_hi, live = t8 < n;
+    mbar_wait(kvp_bar(tile), (uint32_t)((tile - t_lo) >> 1) & 1u);
+    mbar_wait(qt_bar, (uint32_t)(tile - t_lo) & 1u);
+    __syncthreads();                                      // and S, and beta
+    if (!chain && more) {
+      if (ri == 0) {
+        arm_qt(tile + 1);
+        if (tile + 2 < t_hi) arm_kvp(tile + 2);           // this chunk's barrier: all have waited for it
+      }
+      ask_kvp(tile + 1);
+    }
     const float* Ks = sm + L::K + buf * kDcC * DP;
     const float* cs = sm + L::X + buf * 3 * kDcC;         // c | r_64 | beta
     int odd = 0;                                          // an infinity or NaN among this thread's part of R, then of U
-    // ---- [K; Q] S_0: a warp holds S_0 whole in registers, D / 8 rows of four columns per lane ----
-    {
-      float2 s0[D / 16][4];
+    float y[8];
 #pragma unroll
-      for (int x = 0; x < D / 16; ++x) {
-        const int pr = ((x >> 1) * 8 + rl) * 2 + (x & 1);
-        const float4 b0 = *reinterpret_cast<const float4*>(sm + L::S + pair_at(pr, cb)), b1 = *reinterpret_cast<const float4*>(sm + L::S + pair_at(pr, cb + 2));
-        s0[x][0] = lo2(b0); s0[x][1] = hi2(b0); s0[x][2] = lo2(b1); s0[x][3] = hi2(b1);
-      }
+    for (int i = 0; i < 8; ++i) y[i] = 0.f;
+    if (chain) {
+      if (live) {
+        times_state(Ks, y);                               // K S_0
 #pragma unroll
-      for (int b = 0; b < 2; ++b) {
-        const int t = b * 32 + warp * 4;                   // four tokens of K, then of Q
-        float sk[4] = {0.f, 0.f, 0.f, 0.f}, sq[4];
-        if (t < n) {
-          float4 y[4];
-          dot_rows<4, D / 32>(Ks + t * DP + rl * 4, DP, s0, y);
-#pragma unroll
-          for (int i = 0; i < 4; ++i) sk[i] = gather4(y[i], lane);
-          dot_rows<4, D / 32>(sm + L::Q + t * DP + rl * 4, DP, s0, y);
-#pragma unroll
-          for (int i = 0; i < 4; ++i) sq[i] = gather4(y[i], lane);
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            sk[i] = cs[2 * kDcC + t + i] * (sm[L::V + (buf * kDcC + t + i) * NC + cg] - cs[t + i] * sk[i]);
-            odd |= not_finite(sk[i]);
-            if (!(lane & 4)) sm[L::O + (t + i) * NC + cg] = cs[t + i] * sq[i];
-          }
+        for (int i = 0; i < 8; ++i) {
+          y[i] = cs[2 * kDcC + t8 + i] * (sm[L::V + (buf * kDcC + t8 + i) * NC + cg] - cs[t8 + i] * y[i]);
+          odd |= not_finite(y[i]);
         }
-        if (!(lane & 4)) {
-#pragma unroll
-          for (int i = 0; i < 4; i += 2)
-            *reinterpret_cast<float2*>(sm + L::R + pair_at((t + i) / 2, cg) + (cg & 1) * 2) = make_float2(sk[i], sk[i + 1]);
-        }
-      }
-    }
-    odd = __syncthreads_or(odd);
-    if (more) fetch_q(tile + 1);
-    // a lower triangle times [64, NC], the right side held in registers (eight rows of four columns per lane)
-    float2 B[4][4];
-    auto hold = [&](const float* X) {
-#pragma unroll
-      for (int x = 0; x < 4; ++x) {
-        const int pr = ((x >> 1) * 8 + rl) * 2 + (x & 1);
-        const float4 b0 = *reinterpret_cast<const float4*>(X + pair_at(pr, cb)), b1 = *reinterpret_cast<const float4*>(X + pair_at(pr, cb + 2));
-        B[x][0] = lo2(b0); B[x][1] = hi2(b0); B[x][2] = lo2(b1); B[x][3] = hi2(b1);
-      }
-    };
-    hold(sm + L::R);
-    {
-      const int t = warp * 8;
-      float u[8];
-      if (t < n) {
-        float4 y[8];
-        dot_rows<8, 2>(sm + L::T + t * kDcCP + rl * 4, kDcCP, B, y);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) u[i] = gather4(y[i], lane);
-        if (odd) {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) u[i] = lower_dot(sm + L::T + (t + i) * kDcCP, sm + L::R, t + i, cg);
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) odd |= not_finite(u[i]);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) u[i] = 0.f;
       }
       if (!(lane & 4)) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) sm[L::UD + (t + i) * NC + cg] = cs[kDcC + t + i] * u[i];
-#pragma unroll
-        for (int i = 0; i < 8; i += 2) *reinterpret_cast<float2*>(sm + L::U + pair_at((t + i) / 2, cg) + (cg & 1) * 2) = make_float2(u[i], u[i + 1]);
+        for (int i = 0; i < 8; i += 2) *reinterpret_cast<float2*>(sm + L::R + pair_at((t8 + i) / 2, cg) + (cg & 1) * 2) = make_float2(y[i], y[i + 1]);
       }
+      odd = chain_or(odd);
+      float u[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) u[i] = 0.f;
+      if (live) {
+        times_lower(sm + L::T, sm + L::R, odd, u);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) odd |= not_finite(u[i]);
+      }
+      if (!(lane & 4)) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sm[L::UD + (t8 + i) * NC + cg] = cs[kDcC + t8 + i] * u[i];
+#pragma unroll
+        for (int i = 0; i < 8; i += 2) *reinterpret_cast<float2*>(sm + L::U + pair_at((t8 + i) / 2, cg) + (cg & 1) * 2) = make_float2(u[i], u[i + 1]);
+      }
+    } else if (live) {
+      times_state(sm + L::Q, y);                          // Q S_0
+#pragma unroll
+      for (int i = 0; i < 8; ++i) y[i] *= cs[t8 + i];
     }
     odd = __syncthreads_or(odd);
-    if (more) fetch_t(tile + 1);
-    // ---- the read-out ----
-    hold(sm + L::U);
-    float* orow = p.o + ((long long)(first + at) * p.H + h) * p.Dv + col0 + cg;
-    {
-      const int t = warp * 8;
-      if (t < n) {
-        float4 y[8];
-        dot_rows<8, 2>(sm + L::P + (buf * kDcC + t) * kDcCP + rl * 4, kDcCP, B, y);
+    if (!chain) {
+      if (more) ask_qt(tile + 1);
+      // ---- the read-out ----
+      if (live) {
         float z[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) z[i] = gather4(y[i], lane);
-        if (odd) {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) z[i] = lower_dot(sm + L::P + (buf * kDcC + t + i) * kDcCP, sm + L::U, t + i, cg);
-        }
+        times_lower(sm + L::P + buf * kDcC * kDcCP, sm + L::U, odd, z);
+        float* orow = p.o + ((long long)(first + at) * p.H + h) * p.Dv + col0 + cg;
         if (!(lane & 4)) {
 #pragma unroll
           for (int i = 0; i < 8; ++i)
-            if (t + i < n) orow[(long long)(t + i) * p.H * p.Dv] = sm[L::O + (t + i) * NC + cg] + z[i];
+            if (t8 + i < n) orow[(long long)(t8 + i) * p.H * p.Dv] = y[i] + z[i];
         }
       }
+      continue;
     }
     // ---- S = c_64 S + K^T (r_64 U) ----
     const float2 ce = make_float2(cs[kDcC - 1], cs[kDcC - 1]);
@@ -430,8 +451,8 @@ delta_chunk_scan_kernel(const DeltaChunkArgs p) {
         S[x][2] = __ffma2_rn(a[x], make_float2(u.z, u.z), S[x][2]); S[x][3] = __ffma2_rn(a[x], make_float2(u.w, u.w), S[x][3]);
       }
     }
-    if (!owner) publish_state();                          // the products with the old S ended two barriers ago
-    __syncthreads();
+    if (!owner) publish_state();                          // the products with the old S ended in front of the last barrier
+    asm volatile("bar.sync 1, 256;" ::: "memory");
     if (owner) {
 #pragma unroll
       for (int x = 0; x < DT / 2; ++x) {
@@ -463,7 +484,7 @@ static int run_windows(DeltaChunkArgs p, int bound, int window, cudaStream_t st)
     p.tile_hi = lo + window < bound ? lo + window : bound;
     prep<<<dim3(p.tile_hi - lo, p.G), 256, smem, st>>>(p);
     B200_LAUNCH_CHECK();
-    scan<<<dim3(p.Dv / kDcNC, p.H, p.n_runs), 256, scan_smem, st>>>(p);
+    scan<<<dim3(p.Dv / kDcNC, p.H, p.n_runs), 512, scan_smem, st>>>(p);
     B200_LAUNCH_CHECK();
   }
   return 0;
