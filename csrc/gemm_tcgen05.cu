@@ -744,14 +744,16 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
       const float beta = (p.beta_rows != nullptr && row_ok) ? p.beta_rows[row] : p.beta;
       if (sg.kb0 > 0) {
         // ---- stream-K contributor: publish this CTA's fp32 partial, the tile's owner finishes it ----
-        float* slot = p.sk_ws + ((long long)blockIdx.x * kBM + (q * 32 + lane)) * kAccStride;
+        // laid out [16-byte piece][row], so that a warp's store or load is whole lines (a row to a lane is 32 lines an instruction:
+        // 2048 x 5120 x 34816 625 us, now 596; 490 x 4096 x 12288 76, now 68)
+        uint4* slot = reinterpret_cast<uint4*>(p.sk_ws + (long long)blockIdx.x * kBM * kAccStride) + q * 32 + lane;
         for (int c = 0; c < nchunks; ++c) {
           uint32_t r[32];
           tmem_ld_32x32(t0 + c * 32, r);
           tmem_ld_wait();
 #pragma unroll
           for (int j = 0; j < 8; ++j)
-            reinterpret_cast<uint4*>(slot + c * 32)[j] = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+            slot[(c * 8 + j) * kBM] = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
         }
         __threadfence();
         asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -782,10 +784,10 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
         tmem_ld_32x32(t0 + c * 32, r);
         tmem_ld_wait();
         for (int v = 1; v <= ncontrib; ++v) {
-          const float* slot = p.sk_ws + ((long long)((unit + v * sk_g) * CTAS + rank) * kBM + (q * 32 + lane)) * kAccStride + c * 32;
+          const float4* slot = reinterpret_cast<const float4*>(p.sk_ws + (long long)((unit + v * sk_g) * CTAS + rank) * kBM * kAccStride) + q * 32 + lane;
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            const float4 w = reinterpret_cast<const float4*>(slot)[j];
+            const float4 w = slot[(c * 8 + j) * kBM];
             r[4 * j] = __float_as_uint(__uint_as_float(r[4 * j]) + w.x);
             r[4 * j + 1] = __float_as_uint(__uint_as_float(r[4 * j + 1]) + w.y);
             r[4 * j + 2] = __float_as_uint(__uint_as_float(r[4 * j + 2]) + w.z);
@@ -906,8 +908,16 @@ static int device_props() {
 static double kblock_cost(int ctas, int bn) {
   const double t_mma = 2.0 * bn;
   const double t_smem = 256.0 + 2.0 * bn / ctas;
-  return (t_mma > t_smem ? t_mma : t_smem) + 40.0;
+  return (t_mma > t_smem ? t_mma : t_smem) + 85.0;
 }
+
+// What a launch costs beside its k-blocks, in the same cycles: the last tile's epilogue for each 32 columns; a pair of CTAs (a cluster's
+// launch, and its barriers at both ends); stream-K's publish and wait; and, for each 32 columns and each unit that holds a part of the owner's
+// tile, one more trip to L2 in the owner's sum. Fitted over 50 shapes (M 20 to 8192, N 16 to 34816, K 512 to 34816) with every tile timed:
+// the choice is 2% above the best tile in the mean, 9% with ten k-blocks for all of stream-K. Narrow tiles in one wave now win where
+// stream-K cut few wide ones into many parts: 549 x 2048 x 2048 33 -> 23 us, 490 x 4096 x 4096 42 -> 34, 64 x 8192 x 2048 35 -> 21;
+// or tiles in fewer parts do: 64 x 5120 x 17408 80 -> 60.
+constexpr double kEpilogueChunk = 1200.0, kPairLaunch = 3000.0, kStreamK = 4000.0, kStreamKPart = 500.0;
 
 struct GemmConfig {
   int ctas, bn, stream_k;
@@ -928,14 +938,16 @@ static GemmConfig pick_config(int M, int N, int batch, int nkt, int b_mn, int EP
       const long long tiles = (long long)batch * ceil_div(M, kBM * ctas) * ceil_div(N, bn);
       const long long waves = (tiles + units - 1) / units;
       const double per = kblock_cost(ctas, bn);
-      const double classic = (double)waves * nkt * per;
+      const int chunks = ceil_div(bn, 32);
+      const double fixed = chunks * kEpilogueChunk + (ctas == 2 ? kPairLaunch : 0.0);
+      const double classic = (double)waves * nkt * per + fixed;
       if (classic < best.cost * 0.999) best = {ctas, bn, 0, classic};
       if (allow_sk && !no_sk && tiles % units != 0 && tiles * nkt >= 4ll * units) {
-        // equal k-block ranges per unit; ~10 k-blocks' worth of partial-tile write/read/wait per unit
-        const double sk = ((double)tiles * nkt / units + 10.0) * per;
-        // measured: worth it only when classic scheduling wastes a large part of a wave (few tiles);
+        // equal k-block ranges per unit
+        const double parts = tiles < units ? (double)units / tiles : 1.0;
+        const double sk = (double)tiles * nkt / units * per + fixed + kStreamK + kStreamKPart * parts * chunks;
         // with many waves the uneven k-ranges cost more L2 locality than the tail they recover
-        if (waves <= 4 && sk < classic * 0.85 && sk < best.cost * 0.97) best = {ctas, bn, 1, sk};
+        if (waves <= 4 && sk < classic * 0.9 && sk < best.cost * 0.999) best = {ctas, bn, 1, sk};
       }
     }
   }
