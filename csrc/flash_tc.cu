@@ -131,8 +131,9 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
   constexpr int kHalves = L::kHalves, NK = L::NK, NV = L::NV;
   // How far a row's maximum may run ahead of the one its weights refer to before O is scaled (an exponent of two). With none the largest
   // weight is 1 and has no rounding error, as in the mma.sync kernels: error of the result against 64 bits 0.00196 (six packed prompts,
-  // bf16) and 0.00199 (pieces over pages); with a slack of 8 it was 0.00200 and 0.00206, at 108 and 57 us instead of 114 and 61. Dense
-  // batches with heads of 128 never were on mma.sync here and keep the slack that their kernel was written with.
+  // bf16) and 0.00199 (pieces over pages); with a slack of 8 it was 0.00200 and 0.00206, at 108 and 57 us instead of 114 and 61
+  // (before keys and values had rings of their own; with none now 105 and 57). Dense batches with heads of 128 never were on mma.sync here
+  // and keep the slack that their kernel was written with.
   constexpr float kSlack = MODE == kTcDense && D == 128 ? 8.f : 0.f;
   extern __shared__ __align__(1024) uint8_t smem_tc[];
   const uint32_t sbase = smem_u32(smem_tc);
