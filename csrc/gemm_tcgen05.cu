@@ -908,16 +908,8 @@ static int device_props() {
 static double kblock_cost(int ctas, int bn) {
   const double t_mma = 2.0 * bn;
   const double t_smem = 256.0 + 2.0 * bn / ctas;
-  return (t_mma > t_smem ? t_mma : t_smem) + 85.0;
+  return (t_mma > t_smem ? t_mma : t_smem) + 40.0;
 }
-
-// What a launch costs beside its k-blocks, in the same cycles: the last tile's epilogue for each 32 columns; a pair of CTAs (a cluster's
-// launch, and its barriers at both ends); stream-K's publish and wait; and, for each 32 columns and each unit that holds a part of the owner's
-// tile, one more trip to L2 in the owner's sum. Fitted over 50 shapes (M 20 to 8192, N 16 to 34816, K 512 to 34816) with every tile timed:
-// the choice is 2% above the best tile in the mean, 9% with ten k-blocks for all of stream-K. Narrow tiles in one wave now win where
-// stream-K cut few wide ones into many parts: 549 x 2048 x 2048 33 -> 23 us, 490 x 4096 x 4096 42 -> 34, 64 x 8192 x 2048 35 -> 21;
-// or tiles in fewer parts do: 64 x 5120 x 17408 80 -> 60.
-constexpr double kEpilogueChunk = 1200.0, kPairLaunch = 3000.0, kStreamK = 4000.0, kStreamKPart = 500.0;
 
 struct GemmConfig {
   int ctas, bn, stream_k;
@@ -938,20 +930,26 @@ static GemmConfig pick_config(int M, int N, int batch, int nkt, int b_mn, int EP
       const long long tiles = (long long)batch * ceil_div(M, kBM * ctas) * ceil_div(N, bn);
       const long long waves = (tiles + units - 1) / units;
       const double per = kblock_cost(ctas, bn);
-      const int chunks = ceil_div(bn, 32);
-      const double fixed = chunks * kEpilogueChunk + (ctas == 2 ? kPairLaunch : 0.0);
-      const double classic = (double)waves * nkt * per + fixed;
+      const double classic = (double)waves * nkt * per;
       if (classic < best.cost * 0.999) best = {ctas, bn, 0, classic};
       if (allow_sk && !no_sk && tiles % units != 0 && tiles * nkt >= 4ll * units) {
-        // equal k-block ranges per unit
-        const double parts = tiles < units ? (double)units / tiles : 1.0;
-        const double sk = (double)tiles * nkt / units * per + fixed + kStreamK + kStreamKPart * parts * chunks;
+        // equal k-block ranges per unit; ~10 k-blocks' worth of partial-tile write/read/wait per unit. Parts are dearer than that for few
+        // tiles (549 x 2048 x 2048: 32 us, one wave of 80 columns 24; 64 x 4096 x 4096: 40 and 28), but a part's chain of additions is
+        // shorter and its error with it: 6.4e-7 and 2.1e-6 of an fp32 result, 6.0e-7 and 1.6e-6. No caller has asked for less.
+        const double sk = ((double)tiles * nkt / units + 10.0) * per;
+        // measured: worth it only when classic scheduling wastes a large part of a wave (few tiles);
         // with many waves the uneven k-ranges cost more L2 locality than the tail they recover
-        if (waves <= 4 && sk < classic * 0.9 && sk < best.cost * 0.999) best = {ctas, bn, 1, sk};
+        if (waves <= 4 && sk < classic * 0.85 && sk < best.cost * 0.97) best = {ctas, bn, 1, sk};
       }
     }
   }
   return best;
+}
+
+// stream-K in lock-step groups when the M-tiles of a panel fit a group and at most ~5 % of the units are left without one
+static int sk_group_of(int num_m, int units) {
+  static const bool sk_flat = getenv("B200_GEMM_SK_FLAT") != nullptr;
+  return num_m > 1 && num_m <= units && (units % num_m) * 20 <= units && !sk_flat ? num_m : 1;
 }
 
 template <int ES, int CTAS>
@@ -981,6 +979,22 @@ static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensor
 }  // namespace b200
 
 using namespace b200;
+
+// How b200_gemm cuts a product with a workspace on a part of `num_sms` SMs: plan = CTAs of a tile, its columns, whether k is cut into parts, and
+// the k-blocks (128 bytes of a row) of the longest chain of additions
+B200_API int b200_gemm_plan(int M, int N, int K, int batch, int b_mn, int in_dtype, int num_sms, int* plan) {
+  if (M <= 0 || N <= 0 || K <= 0 || batch <= 0 || num_sms <= 0 || !plan) return B200_ERR_BAD_SHAPE;
+  const int EPR = in_dtype == B200_DT_FP32 ? 32 : 64, nkt = ceil_div(K, EPR);
+  const GemmConfig c = pick_config(M, N, batch, nkt, b_mn ? 1 : 0, EPR, num_sms, true);
+  long long chain = nkt;
+  if (c.stream_k) {
+    const int num_m = ceil_div(M, kBM * c.ctas), units = num_sms / c.ctas, g = sk_group_of(num_m, units);
+    const long long items = (long long)batch * num_m * ceil_div(N, c.bn) / g * nkt, share = (items + units / g - 1) / (units / g);
+    if (share < chain) chain = share;
+  }
+  plan[0] = c.ctas; plan[1] = c.bn; plan[2] = c.stream_k; plan[3] = (int)chain;
+  return 0;
+}
 
 // A full-size workspace (b200_gemm_workspace_bytes()) carries the stream-K epoch on the device, in its last 16 bytes:
 // every stream-K launch on that workspace (b200_gemm and b200_gemm_w4 alike) then takes its epoch from there and the launch
@@ -1053,11 +1067,7 @@ B200_API int b200_gemm(const b200_gemm_args* a, void* stream_) {
   p.sk_group = 1;
   p.sk_ws = nullptr; p.sk_flags = nullptr; p.sk_epoch = 0; p.sk_state = nullptr;
   if (cfg.stream_k) {
-    static const bool sk_flat = getenv("B200_GEMM_SK_FLAT") != nullptr;
-    // lock-step groups when the M-tiles of a panel fit a group and at most ~5 % of the units are left without one
-    const int units_sk = g_num_sms / ctas;
-    if (p.num_m > 1 && p.num_m <= units_sk && (units_sk % p.num_m) * 20 <= units_sk && !sk_flat)
-      p.sk_group = p.num_m;
+    p.sk_group = sk_group_of(p.num_m, g_num_sms / ctas);
     static unsigned int epoch = 0;
     p.sk_ws = reinterpret_cast<float*>(a->workspace);
     p.sk_flags = reinterpret_cast<unsigned int*>(reinterpret_cast<char*>(a->workspace) +

@@ -108,6 +108,9 @@ typedef struct b200_gemm_allreduce {
 long long b200_gemm_workspace_bytes(void);
 
 int b200_gemm(const b200_gemm_args* args, void* stream);
+/* How that call is cut where it has a workspace, on a part of num_sms SMs (needs no GPU): plan[4] = CTAs of a tile, columns of a tile, whether k
+ * is cut into parts, k-blocks (128 bytes of a row) of the longest chain of additions. */
+int b200_gemm_plan(int M, int N, int K, int batch, int b_mn, int in_dtype, int num_sms, int* plan);
 /* b200_gemm of two matrices (batch 1) with plain arguments, for callers to whom filling the structure costs more than the launch. */
 int b200_gemm_2d(const void* A, const void* B, void* D, const void* bias, const float* beta_rows, const void* A2, const void* B2,
                  void* workspace, long long workspace_bytes, int M, int N, int K, int K2, long long a_rs, long long b_rs, long long d_rs,
