@@ -2,9 +2,12 @@
 // w = lin_a scale (code - lin_off) - zs, groups of 128, K a multiple of 512 (b200_w4_gemv_linear; other forms stay in gemv.cu).
 //
 // The weights are the 128-row operand of tcgen05.mma and come from TMEM; the tokens are its N. A code enters as the exact 16-bit value
-// 128 + code (1024 + code for fp16: the nibble OR-ed into the mantissa), one logic op per pair, and the affine map is applied in fp32 to
-// a group's sums:  sum_k w_k x_k = A (sum_k (b + c_k) x_k) - (A (b + lin_off) + zs) sum_k x_k.  sum_k x_k needs no pass over x: lane 31
-// of every warp's 32 rows carries codes of zero, so its sums are b sum_k x_k, and it hands them to the warp's other rows.
+// b + code with b = 16 (64 for fp16): the nibble OR-ed into the mantissa of b, one logic op per pair. The affine map is applied in fp32 to a
+// group's sums:  sum_k w_k x_k = A (sum_k (b + c_k) x_k) - (A (b + lin_off) + zs) sum_k x_k.  sum_k x_k needs no pass over x: lane 31
+// of every warp's 32 rows carries codes of zero, so its sums are b sum_k x_k, and it hands them to the warp's other rows. The two
+// sums cancel, and their error grows with b; 16 is the smallest that holds a code, and 64 saves fp16 a shift (16: up to 1.2 of 33 us).
+// Results that are not the 16-bit number next to the 64-bit one, 64 tokens, N 24576, K 4096: bf16 0.03 %, fp16 1 % (2 % where the
+// activations have a mean of 2); with 128 (bf16) and 1024, at the same time: 0.19, 15 and 84 %; mma.sync 0.12, 9 and 38 %.
 //
 // CTA (one per SM): a slice of k of a tile of R = 4 x (at most 31) rows, tile after tile, two groups (a pair) at a time.
 //   warp 0       TMA: codes of a pair (a box of [R rows x 128 bytes]) through a ring as long as fits; scales and zeros of four groups
@@ -251,7 +254,8 @@ w4_tc_kernel(const __grid_constant__ CUtensorMap tw, const __grid_constant__ CUt
     // ================= codes -> 16-bit values in TMEM, thread = row =================
     const int set = ((warp - kWtExp) >> 2) & 1, b = (warp - kWtExp) >> 3, q = warp & 3, row = q * p.rpw + lane;      // group 2 b + set of every unit
     const bool live = lane < p.rpw;
-    uint32_t magic = BF16 ? 0x43004300u : 0x64006400u, mask = 0x000F000Fu;
+    constexpr int kUp = BF16 ? 3 : 4;                     // where a nibble lies in the mantissa of 16 or 64
+    uint32_t magic = BF16 ? 0x41804180u : 0x54005400u, mask = 0x000F000Fu << kUp;
     asm volatile("" : "+r"(magic), "+r"(mask));           // both stay in registers (one LOP3 per pair of codes)
     const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + b * 128 + set * 64;
     uint32_t at[4];                                       // where the group's 64 bytes lie in a stage; other lanes read zeros
@@ -282,10 +286,10 @@ w4_tc_kernel(const __grid_constant__ CUtensorMap tw, const __grid_constant__ CUt
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
           const uint32_t x = w[hf * 8 + c];
-          o[4 * c] = wt_and_or(x >> 4, mask, magic);
-          o[4 * c + 1] = wt_and_or(x, mask, magic);
-          o[4 * c + 2] = wt_and_or(x >> 12, mask, magic);
-          o[4 * c + 3] = wt_and_or(x >> 8, mask, magic);
+          o[4 * c] = wt_and_or(x >> (4 - kUp), mask, magic);
+          o[4 * c + 1] = wt_and_or(x << kUp, mask, magic);
+          o[4 * c + 2] = wt_and_or(x >> (12 - kUp), mask, magic);
+          o[4 * c + 3] = wt_and_or(x >> (8 - kUp), mask, magic);
         }
         tmem_st_32x32(ta + hf * 32, o);
       }
@@ -300,7 +304,7 @@ w4_tc_kernel(const __grid_constant__ CUtensorMap tw, const __grid_constant__ CUt
     const int q = warp & 3, row = q * p.rpw + lane, t0 = ((warp - kWtSum) >> 2) * MH;
     const int mh = p.M - t0;                              // tokens of this half
     const bool live = lane < p.rpw;
-    constexpr float kB0 = BF16 ? 128.f : 1024.f;
+    constexpr float kBase = BF16 ? 16.f : 64.f;
     const uint32_t td = tmem + ((uint32_t)(q * 32) << 16) + 256 + t0;
     const uint32_t xs = sb + L.xs + (warp - kWtSum) * 256;
     int ss = 0;
@@ -331,7 +335,7 @@ w4_tc_kernel(const __grid_constant__ CUtensorMap tw, const __grid_constant__ CUt
           constexpr int CH = 16;
 #pragma unroll
           for (int k = 0; k < 2; ++k) {
-            const float A = a[2 * j + k] * p.lin_a, C = -fmaf(A, kB0 + p.lin_off, z[2 * j + k]) * (1.f / kB0);
+            const float A = a[2 * j + k] * p.lin_a, C = -fmaf(A, kBase + p.lin_off, z[2 * j + k]) * (1.f / kBase);
             const float2 A2 = make_float2(A, A), C2 = make_float2(C, C);
 #pragma unroll
             for (int c = 0; c < MH / CH; ++c) {
