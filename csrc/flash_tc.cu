@@ -41,6 +41,7 @@ constexpr int kTcBM = 128, kTcBN = 64;
 constexpr int kTcThreads = 256;
 constexpr uint32_t kTcTmemCols = 256, kTcTmemO = 128;
 constexpr float kTcLog2e = 1.4426950408889634f;
+constexpr int kTcGridY = 65535;          // largest second (and third) dimension of a grid
 enum { kTcDense = 0, kTcVarlen = 1, kTcPaged = 2 };
 
 // shared memory: Q [128 rows] as D / 64 swizzled halves of 16 KiB, the rings of K and of V [64 rows] as halves of 8 KiB, barriers. K and V
@@ -57,7 +58,9 @@ struct FlashTcParams {
   void* out;
   float* lse;         // [B, H, S] natural-log log-sum-exp of the scaled scores (what the backward kernel reads), may be null
   const int* cu;      // varlen: sequence b is rows [cu[b], cu[b + 1])
-  int S, H, Hkv;
+  int B, S, H, Hkv;
+  int group;          // dense, varlen: heads (of all sequences) whose tiles are taken together, see head_group; 0: all
+  unsigned h_inv;     // 2^32 / H, rounded up
   long long out_rs;   // elements between output rows
   float scale_log2;   // softmax scale * log2(e) (capped: cap * log2(e))
   int causal;
@@ -140,7 +143,7 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   // ---- where this CTA's rows and keys are ----
-  int h = blockIdx.y, hk, row_base, q0, limit;            // limit: keys of the sequence; q0: position of row 0; row_base: its row 0
+  int h = blockIdx.y, b = 0, hk, row_base, q0, limit;           // limit: keys of the sequence; q0: position of row 0; row_base: its row 0
   int nit, nA = 0, bB = 0;                                // key blocks: [0, nA), then bB, bB + 1, ...
   int nrows = kTcBM, low_max = 0, keepW = 0;
   bool solo = false;                                      // paged: the second half of the rows is the same head's next tile
@@ -171,10 +174,24 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
     nit = nA + (limit + kTcBN - 1) / kTcBN - bB;
     low_max = low_of(q0 + (solo ? kTcBM : kTcBN) - 1);
   } else {
-    // The tile is the slowest grid dimension, heavy (late) query tiles of all heads and sequences first: under the causal mask tile t has
+    // Heavy (late) query tiles of all heads and sequences first, or of a group of heads (see head_group): under the causal mask tile t has
     // t + 1 times the work of tile 0, and the short ones fill the end.
-    const int qt = (int)gridDim.z - 1 - (int)blockIdx.z, b = blockIdx.y;
-    h = blockIdx.x;
+    int qt;
+    if (p.group == 0) {
+      h = blockIdx.x; b = blockIdx.y;
+      qt = (int)gridDim.z - 1 - (int)blockIdx.z;
+    } else {
+      int x = blockIdx.x;
+      qt = (p.S + kTcBM - 1) / kTcBM - 1 - (int)blockIdx.y;
+      if (qt >= kTcGridY) {                               // more tiles than the second dimension holds: the first takes the rest
+        qt -= x / p.group * kTcGridY;
+        x %= p.group;
+      }
+      const int hb = (int)blockIdx.z * p.group + x;
+      b = p.H == 1 ? hb : (int)__umulhi((unsigned)hb, p.h_inv);
+      if (b >= p.B || qt < 0) return;
+      h = hb - b * p.H;
+    }
     hk = h / (p.H / p.Hkv);
     row_base = MODE == kTcVarlen ? p.cu[b] : b * p.S;
     limit = MODE == kTcVarlen ? p.cu[b + 1] - row_base : p.S;
@@ -473,7 +490,7 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
       }
     }
     if (MODE == kTcDense && p.lse && live)
-      p.lse[((long long)blockIdx.y * p.H + h) * p.S + grow] = m_ref * 0.6931471805599453f + __logf(l);
+      p.lse[((long long)b * p.H + h) * p.S + grow] = m_ref * 0.6931471805599453f + __logf(l);
     __syncwarp();
     // each warp copies ITS 32 rows out (written by its own lanes): CH lanes cover the bytes of a row
     uint16_t* obase = reinterpret_cast<uint16_t*>(p.out);
@@ -524,8 +541,41 @@ static int bind_device() {
   return 0;
 }
 
+// Tiles of dense and packed calls go out tile by tile, and a tile of every head reads its keys and values: with heads of 128 they are wanted
+// at 9 TB/s, which only L2 has. So where those of all heads are more than its 126 MB, the heads go in groups whose keys and values stay
+// there from one tile's turn to the next: 48 MB, less than half of it, since the queries and the results go through it too.
+// 16 x 4096, 32 heads of 128 (1.07 GB), causal / full / packed: 2172 / 3949 / 2745 us, in one group 2873 / 5412 / 3231, head by head
+// 2701 / 4734 / 2895; 2 x 8192: 1008 / 1916 / 1309, 1127 / 2519 / 1344 and 1346 / 2414 / 1445. 24 to 64 MB differ by 3 %. Heads of 64
+// want 3.6 TB/s and stay one group: 64 x 4096, 12 heads (0.8 GB) 3331 us, 3330 in groups; below 126 MB groups gain nothing: 48 x 512
+// packed, 40 / 8 heads of 128 (100 MB) 304 us, 310 in groups.
+// Sequences of more tiles than a grid's second and third dimension hold (8.4 million rows) take the grouped form as well.
+constexpr long long kTcL2Bytes = 126ll << 20, kTcGroupBytes = 48ll << 20;
+static int head_group(long long rows, FlashTcParams& p, int D, dim3& grid) {
+  const long long tiles = (p.S + kTcBM - 1) / kTcBM, heads = (long long)p.H * p.B, rep = p.H / p.Hkv;
+  const long long kv = (rows * D * 4 + p.B - 1) / p.B;    // keys and values of one head of a sequence (packed: of the mean one)
+  const bool divides = heads * p.H < (1ll << 32);         // what the kernel's quotient by H takes
+  p.group = 0;
+  grid = dim3(p.H, p.B, (unsigned)tiles);
+  if (tiles <= kTcGridY && (D == 64 || !divides || kv * (heads / rep) <= kTcL2Bytes)) return 0;
+  if (!divides) return B200_ERR_UNSUPPORTED;
+  const long long over = (tiles + kTcGridY - 1) / kTcGridY;
+  long long group = kTcGroupBytes / kv * rep;
+  if (group < rep) group = rep;
+  if (group * kTcGridY < heads) group = (heads + kTcGridY - 1) / kTcGridY;
+  if (group > heads) group = heads;
+  const long long groups = (heads + group - 1) / group;
+  group = ((heads + groups - 1) / groups + rep - 1) / rep * rep;          // of one size, heads of the same keys together
+  if (group * over > 0x7fffffffLL) return B200_ERR_UNSUPPORTED;
+  p.group = (int)group;
+  p.h_inv = p.H == 1 ? 0 : (unsigned)((1ll << 32) / p.H + 1);
+  grid = dim3((unsigned)(group * over), (unsigned)(tiles < kTcGridY ? tiles : kTcGridY), (unsigned)groups);
+  return 0;
+}
+
 template <int MODE>
-static int fused_qkv(const void* qkv, long long rows, FlashTcParams& p, int D, int dtype, dim3 grid, void* stream) {
+static int fused_qkv(const void* qkv, long long rows, FlashTcParams& p, int D, int dtype, void* stream) {
+  dim3 grid;
+  if (int rc = head_group(rows, p, D, grid)) return rc;
   if (int rc = bind_device()) return rc;
   CUtensorMap tm;
   if (int rc = rows_map(&tm, qkv, (uint64_t)(p.H + 2 * p.Hkv) * D, (uint64_t)rows, 64)) return rc;
@@ -543,9 +593,17 @@ using namespace b200;
 static int tc_check(const void* qkv, const void* out, int B, int S, int H, int Hkv, int D, float scale, int dtype) {
   if ((D != 64 && D != 128) || (dtype != B200_DT_BF16 && dtype != B200_DT_FP16) || !(scale > 0.f)) return B200_ERR_UNSUPPORTED;
   if (B < 1 || S < 1 || H < 1 || Hkv < 1 || H % Hkv) return B200_ERR_BAD_SHAPE;
-  if (H > 65535 || B > 65535 || (S + kTcBM - 1) / kTcBM > 65535) return B200_ERR_UNSUPPORTED;
+  if (H > 65535 || B > 65535) return B200_ERR_UNSUPPORTED;
   if ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(out)) & 15) return B200_ERR_BAD_ALIGN;
   return 0;
+}
+
+// Heads (of all sequences) whose tiles a dense (rows = B * S) or packed call takes together, 0 where it is refused
+B200_API int b200_flash_tc_group(long long rows, int B, int S, int H, int Hkv, int D) {
+  FlashTcParams p = {};
+  dim3 grid;
+  p.B = B; p.S = S; p.H = H; p.Hkv = Hkv;
+  return rows < 1 || B < 1 || S < 1 || H < 1 || Hkv < 1 || H % Hkv || D < 1 || head_group(rows, p, D, grid) ? 0 : p.group ? p.group : p.H * p.B;
 }
 
 // Causal (or full) attention forward on the tcgen05 path. head_dim 64 or 128, 16-bit, no dropout, scale > 0. qkv [B*S, (H + 2 Hkv) * D],
@@ -555,9 +613,9 @@ B200_API int b200_flash_attn_fwd_tc(const void* qkv, void* out, float* lse, int 
                                     float scale, int dtype, void* stream) {
   if (int rc = tc_check(qkv, out, B, S, H, Hkv, D, scale, dtype)) return rc;
   FlashTcParams p = {};
-  p.out = out; p.lse = lse; p.S = S; p.H = H; p.Hkv = Hkv; p.out_rs = (long long)H * D;
+  p.out = out; p.lse = lse; p.B = B; p.S = S; p.H = H; p.Hkv = Hkv; p.out_rs = (long long)H * D;
   p.scale_log2 = scale * kTcLog2e; p.causal = causal;
-  return fused_qkv<kTcDense>(qkv, (long long)B * S, p, D, dtype, dim3(H, B, (S + kTcBM - 1) / kTcBM), stream);
+  return fused_qkv<kTcDense>(qkv, (long long)B * S, p, D, dtype, stream);
 }
 
 // The packed form (see b200_flash_attn_varlen_fwd): `tokens` rows hold n_seqs sequences back to back, the longest of max_seqlen rows.
@@ -566,9 +624,9 @@ B200_API int b200_flash_attn_varlen_fwd_tc(const void* qkv, void* out, const int
   if (int rc = tc_check(qkv, out, n_seqs, max_seqlen, H, Hkv, D, scale, dtype)) return rc;
   if (!cu_seqlens || tokens < 1) return B200_ERR_BAD_SHAPE;
   FlashTcParams p = {};
-  p.out = out; p.cu = cu_seqlens; p.S = max_seqlen; p.H = H; p.Hkv = Hkv; p.out_rs = (long long)H * D;
+  p.out = out; p.cu = cu_seqlens; p.B = n_seqs; p.S = max_seqlen; p.H = H; p.Hkv = Hkv; p.out_rs = (long long)H * D;
   p.scale_log2 = scale * kTcLog2e; p.causal = causal;
-  return fused_qkv<kTcVarlen>(qkv, tokens, p, D, dtype, dim3(H, n_seqs, (max_seqlen + kTcBM - 1) / kTcBM), stream);
+  return fused_qkv<kTcVarlen>(qkv, tokens, p, D, dtype, stream);
 }
 
 // Prompt pieces over a paged cache, one map, key and value rows of one size (arguments as in b200_multimap_attn_mma_ex; `tokens`: rows

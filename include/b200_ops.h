@@ -406,6 +406,9 @@ int b200_flash_attn_bwd(const void* qkv, const void* out, const void* dout, cons
  * of qkv must be addressable as one 2-D tensor map (row stride (H + 2 Hkv) * D elements, 16-byte aligned base). */
 int b200_flash_attn_fwd_tc(const void* qkv, void* out, float* lse, int B, int S, int H, int Hkv, int D, int causal,
                            float scale, int dtype, void* stream);
+/* Heads, of all sequences, whose tiles that call (rows = B * S) or the packed one (rows of qkv, B sequences of at most S) takes together;
+ * 0: it is refused. Needs no GPU. */
+int b200_flash_tc_group(long long rows, int B, int S, int H, int Hkv, int D);
 /* The packed form (arguments as in b200_flash_attn_varlen_fwd; tokens: rows of qkv) and prompt pieces over a paged cache (one map,
  * D = Dv, arguments as in b200_multimap_attn_mma_ex; tokens: rows of q, pool_rows: blocks * G * block_size;
  * tile_of [n_tiles, 4] = (run, place in the run, tiles of the run, its first tile), wanted where H / G is odd), head_dim 64 or 128. */

@@ -35,3 +35,25 @@ def test_chains_of_few_tiles_stay_short(m, n, k, chain):
     out = (ctypes.c_int * 4)()
     assert nv.proto("b200_gemm_plan", [ctypes.c_int] * 7 + [ctypes.c_void_p])(m, n, k, 1, 0, nv.DT_BF16, 148, ctypes.addressof(out)) == 0
     assert out[3] <= chain
+
+
+@library
+@pytest.mark.parametrize("B,S,H,Hkv,D", [(16, 4096, 32, 32, 128), (2, 8192, 32, 8, 128), (64, 1024, 12, 12, 128), (1, 1 << 20, 8, 2, 128), (3, 70000, 5, 5, 128), (1, 16 << 20, 8, 2, 64)])
+def test_keys_of_a_group_of_heads_fit_the_cache(B, S, H, Hkv, D):
+    """The forward's tiles of heads of 128 go out by groups of heads whose keys and values stay in L2 (126 MB) while the group's tiles read them."""
+    group = nv.proto("b200_flash_tc_group", [ctypes.c_longlong] + [ctypes.c_int] * 5)(B * S, B, S, H, Hkv, D)
+    rep, kv = H // Hkv, S * D * 4
+    if B * Hkv * kv <= 126 << 20:
+        assert group == H * B
+    else:
+        assert group % rep == 0 and (group == rep or group // rep * kv <= 48 << 20)
+        assert group == rep or 3 * group * kv >= rep * (48 << 20)                   # and no fewer than need be
+
+
+@library
+def test_small_batches_are_one_group():
+    call = nv.proto("b200_flash_tc_group", [ctypes.c_longlong] + [ctypes.c_int] * 5)
+    assert call(4 * 512, 4, 512, 40, 8, 128) == 160 and call(4096, 1, 4096, 32, 8, 128) == 32
+    assert call(64 * 1024, 64, 1024, 12, 12, 64) == 768                    # heads of 64 do not wait for memory
+    assert call(64, 2, 65535 * 128 + 1, 4, 2, 64) == 8                     # more tiles than a grid's second dimension
+    assert call(64, 2, 512, 4, 3, 64) == 0
