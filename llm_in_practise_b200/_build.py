@@ -16,6 +16,7 @@ import shutil
 import subprocess
 import sys
 import sysconfig
+import warnings
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -112,8 +113,10 @@ def build_cuda(force: bool = False, verbose: bool = False, sources=None) -> Path
 
 def ensure_built(sources) -> Path:
     """Make sure libb200ops.so exists, is up to date and contains ``sources`` (stems of csrc/*.cu); compiles only what is
-    missing. The call a command-line entry point makes before it touches the GPU in a fresh checkout."""
-    return build_cuda(sources=list(sources))
+    missing, and the extension that calls it. What a command-line entry point calls before it touches the GPU in a fresh checkout."""
+    out = build_cuda(sources=list(sources))
+    build_fastcall()
+    return out
 
 
 def build_host(force: bool = False) -> Path:
@@ -129,16 +132,26 @@ def build_host(force: bool = False) -> Path:
     return out
 
 
+def fastcall_path() -> Path:
+    """The extension that calls the C ABI, under the name of the Python that it is built for: another one finds no file of its own."""
+    return LIBDIR / ("_b200_fastcall" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
+
+
 def build_fastcall(force: bool = False):
-    """The Python extension that calls the C ABI (``ops._native``); None where Python's headers or the ABI it relies on are missing:
-    calls then go through ctypes."""
+    """The Python extension that calls the C ABI (``ops._native``); None where Python's headers, the ABI it relies on or a compiler that
+    takes it are missing: calls then go through ctypes."""
     include = sysconfig.get_paths()["include"]
-    src, out = CSRC / "host" / "python" / "fastcall.cpp", LIBDIR / "_b200_fastcall.so"
+    src, out = CSRC / "host" / "python" / "fastcall.cpp", fastcall_path()
     if not Path(include, "Python.h").exists() or platform.machine() != "x86_64" or sys.platform != "linux":
         return None
     if force or _stale(out, [src]):
         tmp = out.with_suffix(".so.tmp%d" % os.getpid())
-        _run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-I", include, str(src), "-o", str(tmp)])
+        out.unlink(missing_ok=True)
+        try:
+            _run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-I", include, str(src), "-o", str(tmp)])
+        except (RuntimeError, OSError) as e:
+            warnings.warn(f"no extension for calls of the kernels, they go through ctypes: {e}")
+            return None
         os.replace(tmp, out)
     return out
 

@@ -10,6 +10,7 @@ from __future__ import annotations
 import ctypes
 import importlib.util
 import os
+import sysconfig
 from pathlib import Path
 
 import torch
@@ -73,7 +74,7 @@ def use_native(*tensors) -> bool:
 
 
 def lib() -> ctypes.CDLL:
-    global _lib
+    global _lib, _make_entry
     if _lib is None:
         p = lib_path()
         if not p.exists():
@@ -81,6 +82,8 @@ def lib() -> ctypes.CDLL:
                 f"{p} is missing: run `python -m llm_in_practise_b200._build` (or __graft_entry__.build()) first")
         _lib = ctypes.CDLL(str(p))
         _declare(_lib)
+        if _make_entry is None:              # built since this module was imported (_build.ensure_built)
+            _make_entry = _fastcall()
     return _lib
 
 
@@ -178,7 +181,8 @@ _KINDS = {ctypes.c_void_p: "p", ctypes.c_float: "f", **{t: "i" for t in (ctypes.
 
 def _fastcall():
     """``make`` of the extension that calls the C ABI (csrc/host/python/fastcall.cpp), or None: calls then go through ctypes."""
-    p = _LIBDIR / "_b200_fastcall.so"
+    # the name says for which Python it was built: the module uses its object layouts, and a loader by path does not check them
+    p = _LIBDIR / ("_b200_fastcall" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
     if not p.exists():
         return None
     try:
@@ -186,7 +190,7 @@ def _fastcall():
         module = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(module)
         return module.make
-    except ImportError:                      # built for another Python
+    except ImportError:                      # not a module, or one for another system
         return None
 
 

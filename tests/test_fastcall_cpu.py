@@ -2,9 +2,12 @@
 import ctypes
 import shutil
 import subprocess
+import sysconfig
+from pathlib import Path
 
 import pytest
 
+from llm_in_practise_b200 import _build
 from llm_in_practise_b200.ops import _native as nv
 
 vp, i32, i64, u64, f32 = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_ulonglong, ctypes.c_float
@@ -56,3 +59,35 @@ def test_what_is_not_made():
         pytest.skip("no extension here")
     assert nv._make_entry(16, "i" * 33, len) is None and nv._make_entry(16, "f" * 9, len) is None
     assert nv._make_entry(0, "i", len) is None and nv._make_entry(16, "d", len) is None
+
+
+def test_only_the_file_of_this_python_is_loaded(tmp_path, monkeypatch):
+    suffix = sysconfig.get_config_var("EXT_SUFFIX")
+    assert _build.fastcall_path().name == "_b200_fastcall" + suffix and "cpython" in suffix
+    monkeypatch.setattr(nv, "_LIBDIR", tmp_path)
+    (tmp_path / ("_b200_fastcall" + suffix)).write_bytes(b"not a module")
+    assert nv._fastcall() is None
+    if _build.fastcall_path().exists():
+        (tmp_path / ("_b200_fastcall" + suffix)).unlink()
+        shutil.copy(_build.fastcall_path(), tmp_path / "_b200_fastcall.so")
+        shutil.copy(_build.fastcall_path(), tmp_path / "_b200_fastcall.cpython-39-x86_64-linux-gnu.so")
+        assert nv._fastcall() is None
+        shutil.copy(_build.fastcall_path(), tmp_path / ("_b200_fastcall" + suffix))
+        assert nv._fastcall() is not None
+
+
+def test_no_compiler_leaves_ctypes(tmp_path, monkeypatch):
+    monkeypatch.setattr(_build, "LIBDIR", tmp_path)
+    monkeypatch.setenv("PATH", str(tmp_path))
+    if not Path(sysconfig.get_paths()["include"], "Python.h").exists():
+        pytest.skip("no headers here")
+    with pytest.warns(UserWarning, match="ctypes"):
+        assert _build.build_fastcall() is None
+    assert not list(tmp_path.iterdir())
+
+
+def test_a_fresh_checkout_builds_it(monkeypatch):
+    built = []
+    monkeypatch.setattr(_build, "build_cuda", lambda **kw: "library")
+    monkeypatch.setattr(_build, "build_fastcall", lambda: built.append(1))
+    assert _build.ensure_built(["gemv"]) == "library" and built
