@@ -11,7 +11,8 @@ from llm_in_practise_b200.ops.flash import flash_attention, flash_attention_varl
 @pytest.mark.parametrize("B,S,H,Hkv,D", [(5, 130, 40, 8, 128),      # three rounds of query tiles, one of key blocks; two rows in the last tile
                                          (24, 70, 8, 8, 64),        # a round and a part of one of single-tile items
                                          (3, 513, 24, 24, 64),      # items of one to nine pairs
-                                         (38, 64, 4, 4, 128)])      # four items more than SMs, a pair each
+                                         (38, 64, 4, 4, 128),       # four items more than SMs, a pair each
+                                         (20, 321, 16, 8, 128)])    # keys that stay in shared memory: 480 items of 2 to 12 pairs, a third one for some
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("causal", [True, False])
 def test_backward_items(B, S, H, Hkv, D, dtype, causal):
