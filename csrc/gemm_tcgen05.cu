@@ -911,13 +911,27 @@ static double kblock_cost(int ctas, int bn) {
   return (t_mma > t_smem ? t_mma : t_smem) + 40.0;
 }
 
+// What a launch of whole tiles costs beside that, in the same cycles: 45 more for each k-block; the last tile's epilogue for each 32 columns,
+// and for half of 32 more than a whole one (the loads and stores of the rest are not by whole lines); a pair of CTAs (a cluster's launch,
+// and its barriers at both ends). Over 624 products (M 20 to 8192, N 16 to 30522, K 512 to 12288, B along K and along N) with every tile timed
+// the choice is 0.8% above the best tile, by the k-blocks alone 4.5%, and nowhere slower than by these. Epilogues of 300 to 600 cycles do;
+// with 1200 and no more for halves (2.8%) one in twelve was slower than by the k-blocks, 4096 x 1536 x 512 17 -> 23 us.
+constexpr double kPerBlock = 45.0, kEpilogueChunk = 500.0, kHalfChunk = 3000.0, kPairLaunch = 3000.0;
+
 struct GemmConfig {
   int ctas, bn, stream_k;
   double cost;
 };
 
+// Two questions, since only one of them is about time alone.
+//   Whether a product of few tiles is cut along k: by the k-blocks, with ten of them for the hand-over. That is dearer than it counts (549 x
+//   2048 x 2048 32 us, in one wave of 80 columns 24; 64 x 4096 x 4096 40 and 28), but a part's chain of additions is shorter and its
+//   error with it: 6.4e-7 and 2.1e-6 of an fp32 result, 6.0e-7 and 1.6e-6. No caller has asked for less. Products of more than a wave are cut
+//   only where whole tiles waste much of one: 2345 x 5120 x 17408 takes 314 us whole, 488 in parts.
+//   Which tile, where it is not cut: the sums are the same bits whatever the tile, and the fitted cost takes the fastest. B along N, 300 x 5120 x
+//   2048: 23 us, 29 by the k-blocks alone; 512 x 768 x 768 13 and 16, 1024 x 3072 x 768 17 and 20.
 static GemmConfig pick_config(int M, int N, int batch, int nkt, int b_mn, int EPR, int num_sms, bool allow_sk) {
-  GemmConfig best = {1, 256, 0, 1e30};
+  GemmConfig cut = {1, 256, 0, 1e30}, best = cut;
   static const bool no_sk = getenv("B200_GEMM_NO_STREAMK") != nullptr;     // tuning switches are read once per process
   for (int ctas = 2; ctas >= 1; --ctas) {
     if (g_force_ctas && ctas != g_force_ctas) continue;
@@ -929,21 +943,20 @@ static GemmConfig pick_config(int M, int N, int batch, int nkt, int b_mn, int EP
       if (bn > 32 && bn > 2 * ((N + 15) / 16 * 16)) continue;  // do not pick tiles far wider than N
       const long long tiles = (long long)batch * ceil_div(M, kBM * ctas) * ceil_div(N, bn);
       const long long waves = (tiles + units - 1) / units;
-      const double per = kblock_cost(ctas, bn);
-      const double classic = (double)waves * nkt * per;
-      if (classic < best.cost * 0.999) best = {ctas, bn, 0, classic};
+      const double per = kblock_cost(ctas, bn), classic = (double)waves * nkt * per;
+      if (classic < cut.cost * 0.999) cut = {ctas, bn, 0, classic};
       if (allow_sk && !no_sk && tiles % units != 0 && tiles * nkt >= 4ll * units) {
-        // equal k-block ranges per unit; ~10 k-blocks' worth of partial-tile write/read/wait per unit. Parts are dearer than that for few
-        // tiles (549 x 2048 x 2048: 32 us, one wave of 80 columns 24; 64 x 4096 x 4096: 40 and 28), but a part's chain of additions is
-        // shorter and its error with it: 6.4e-7 and 2.1e-6 of an fp32 result, 6.0e-7 and 1.6e-6. No caller has asked for less.
+        // equal k-block ranges per unit. Worth it only when whole tiles waste a large part of a wave (few tiles); with many waves the
+        // uneven k-ranges cost more L2 locality than the tail they recover
         const double sk = ((double)tiles * nkt / units + 10.0) * per;
-        // measured: worth it only when classic scheduling wastes a large part of a wave (few tiles);
-        // with many waves the uneven k-ranges cost more L2 locality than the tail they recover
-        if (waves <= 4 && sk < classic * 0.85 && sk < best.cost * 0.97) best = {ctas, bn, 1, sk};
+        if (waves <= 4 && sk < classic * 0.85 && sk < cut.cost * 0.97) cut = {ctas, bn, 1, sk};
       }
+      const double whole = (double)waves * nkt * (per + kPerBlock) + ceil_div(bn, 32) * kEpilogueChunk +
+                           (bn % 32 && bn < N ? kHalfChunk : 0.0) + (ctas == 2 ? kPairLaunch : 0.0);
+      if (whole < best.cost * 0.999) best = {ctas, bn, 0, whole};
     }
   }
-  return best;
+  return cut.stream_k ? cut : best;
 }
 
 // stream-K in lock-step groups when the M-tiles of a panel fit a group and at most ~5 % of the units are left without one

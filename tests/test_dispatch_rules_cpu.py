@@ -38,6 +38,26 @@ def test_chains_of_few_tiles_stay_short(m, n, k, chain):
 
 
 @library
+@pytest.mark.parametrize("m,n,k,b_mn", [
+    (4096, 1536, 512, 0), (2345, 1536, 512, 0), (2345, 2048, 512, 0), (4096, 1000, 640, 0), (1024, 768, 768, 0), (1024, 3072, 768, 0), (300, 768, 768, 0),
+    (549, 1024, 1024, 0), (300, 5120, 2048, 0), (512, 768, 768, 1), (549, 16, 2048, 0), (8192, 8192, 8192, 0)])
+def test_whole_tiles(m, n, k, b_mn):
+    """Products that are not cut take tiles of whole 32 columns, unless the matrix is narrower: half of them cost more than the columns saved."""
+    out = (ctypes.c_int * 4)()
+    assert nv.proto("b200_gemm_plan", [ctypes.c_int] * 7 + [ctypes.c_void_p])(m, n, k, 1, b_mn, nv.DT_BF16, 148, ctypes.addressof(out)) == 0
+    assert not out[2] and (out[1] % 32 == 0 or out[1] >= n)
+
+
+@library
+@pytest.mark.parametrize("m,n,k", [(2345, 5120, 17408), (4096, 4096, 12288), (300, 24576, 4096)])
+def test_more_than_a_wave_is_not_cut(m, n, k):
+    """Parts of 17408 values in more than one wave read all of A and B from memory again: 488 us for the first, 314 by whole tiles."""
+    out = (ctypes.c_int * 4)()
+    assert nv.proto("b200_gemm_plan", [ctypes.c_int] * 7 + [ctypes.c_void_p])(m, n, k, 1, 0, nv.DT_BF16, 148, ctypes.addressof(out)) == 0
+    assert out[2] == 0
+
+
+@library
 @pytest.mark.parametrize("B,S,H,Hkv,D", [(16, 4096, 32, 32, 128), (2, 8192, 32, 8, 128), (64, 1024, 12, 12, 128), (1, 1 << 20, 8, 2, 128), (3, 70000, 5, 5, 128), (1, 16 << 20, 8, 2, 64)])
 def test_keys_of_a_group_of_heads_fit_the_cache(B, S, H, Hkv, D):
     """The forward's tiles of heads of 128 go out by groups of heads whose keys and values stay in L2 (126 MB) while the group's tiles read them."""
