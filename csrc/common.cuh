@@ -40,7 +40,8 @@
 // math) goes between the two calls. Captured into CUDA graphs as programmatic edges.
 // Measured on B200 (Qwen3-8B W4A16 decode replayed from a CUDA graph): 4.52 ms per token with the attribute vs 3.93 ms
 // without at batch 1, 5.62 vs 4.51 ms at batch 8 — the early-resident dependents cost more than the hidden launch gaps,
-// so the attribute is OFF by default (B200_PDL=1 turns it on); the device-side calls stay in the kernels as no-ops.
+// so the attribute is OFF by default (B200_PDL=1 turns it on); the device-side calls stay in the kernels as no-ops. w4_tc.cu launches its
+// own pair of kernels with it always: there the second one's weights are on their way while the first one orders the tokens.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -18,10 +18,11 @@
 //                             chunk needs is on its way (bulk copies) meanwhile.
 // All in fp32 FMAs (two per instruction), no tensor cores: the state is fp32 by definition, and splitting fp32 operands for bf16 or
 // tf32 mma.sync takes as many cycles as the FMAs do. r_ij is a product taken from j upwards, the roundings a walk makes too;
-// sums of logarithms would lose digits to cancellation. Bound: a packed FMA with three register operands takes 2.7 cycles of a scheduler, not
-// 2 (95 FMAs a cycle and SM of 128, measured alone), 5500 of a chunk's 11 800 cycles; then the latency of the sums across lanes and the
-// three barriers of a chunk. One prompt of 2048 tokens, 16 heads of 128 x 128 over 4 q/k heads: 502 us token by token, 18 + 194 here; 2048 and
-// 513 tokens: 586 -> 272 (the shorter run's CTAs fill in behind the longer one's); error of the state against 64 bits 2e-7 both ways.
+// sums of logarithms would lose digits to cancellation. Bound: a packed FMA takes 3.0 cycles of a scheduler with three operands of its own and
+// 2.3 where one is the last one's too, as here, not 2 (85 and 109 FMAs a cycle and SM of 128, measured alone, two to four warps per
+// scheduler), 4800 of a chunk's 11 800 cycles; then the latency of the sums across lanes and the four barriers of a chunk. One prompt
+// of 2048 tokens, 16 heads of 128 x 128 over 4 q/k heads: 502 us token by token, 18 + 194 here; 2048 and 513 tokens: 586 -> 272 (the
+// shorter run's CTAs fill in behind the longer one's); error of the state against 64 bits 2e-7 both ways.
 #include "common.cuh"
 #include "../include/b200_ops.h"
 

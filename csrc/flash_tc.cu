@@ -26,7 +26,7 @@
 //
 // Takes the place of the mma.sync kernels of flash_attn.cu (other head sizes, other scales and dropout stay there) and
 // multimap_attn_mma.cu (other sizes, two maps). Measured against them, bf16: six packed prompts of 77 - 2048 tokens, 32 / 8 heads
-// of 128: 237 -> 106 us, 16 / 8 heads of 64: 80 -> 57; pages of 64, 16 / 4 heads of 128, pieces of 2048 and 700 (at 512) tokens beside
+// of 128: 237 -> 107 us, 16 / 8 heads of 64: 86 -> 51; pages of 64, 16 / 4 heads of 128, pieces of 2048 and 700 (at 512) tokens beside
 // two that decode: 171 -> 57 us, window of 1024: 128 -> 42, chunks with capped scores: 194 -> 80; eight packed prompts of 30 - 250
 // tokens (fp16): 19.1 -> 16.4.
 // Reference call sites: SDPA behind nn.MultiheadAttention (LLM_Distributed_Trainning/PyTorch/ddp_basics/ddp_gpt_wikitext2.py:89-96),

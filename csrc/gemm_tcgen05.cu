@@ -912,8 +912,8 @@ static double kblock_cost(int ctas, int bn) {
 }
 
 // What a launch of whole tiles costs beside that, in the same cycles: 45 more for each k-block; the last tile's epilogue for each 32 columns,
-// and for half of 32 more than a whole one (the loads and stores of the rest are not by whole lines); a pair of CTAs (a cluster's launch,
-// and its barriers at both ends). Over 624 products (M 20 to 8192, N 16 to 30522, K 512 to 12288, B along K and along N) with every tile timed
+// and for half of 32 more than a whole one (its columns are stored one at a time); a pair of CTAs (a cluster's launch, and its barriers at
+// both ends). Over 624 products (M 20 to 8192, N 16 to 30522, K 512 to 12288, B along K and along N) with every tile timed
 // the choice is 0.8% above the best tile, by the k-blocks alone 4.5%, and nowhere slower than by these. Epilogues of 300 to 600 cycles do;
 // with 1200 and no more for halves (2.8%) one in twelve was slower than by the k-blocks, 4096 x 1536 x 512 17 -> 23 us.
 constexpr double kPerBlock = 45.0, kEpilogueChunk = 500.0, kHalfChunk = 3000.0, kPairLaunch = 3000.0;

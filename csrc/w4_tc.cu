@@ -497,6 +497,7 @@ static const int* wt_resident() {
 // The cut with the shortest time by what a unit (four groups) and the end of a tile take, us: 1.8 (up to 32 tokens) or 2.9, and 0.5, or 3.6
 // where parts meet; a unit takes half as long again in clusters of four, whose CTAs wait for one another. From N 24576 and 34816 at K 4096
 // and 5120, N 4096 at K 12288 and N 12288 at K 2048, each cut timed: N 24576, 64 tokens: 48 / 50 / 69 with 1 / 2 / 4 CTAs, N 4096: 64 / 38 / 42.
+// It takes two CTAs for both: the shortest of the second, 2 us above the shortest of the first.
 static W4TcCut w4_tc_cut(int M, long long N, int K, int group) {
   W4TcCut cut;
   if (M < 17 || M > 64 || N < 1 || N > (1 << 30) || K < 512 || K % 512 || group != 128) return cut;

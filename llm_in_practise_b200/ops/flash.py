@@ -59,7 +59,7 @@ class _FlashAttentionFn(torch.autograd.Function):
         dqkv = torch.empty_like(qkv)
         delta = torch.empty(B, H, S, dtype=torch.float32, device=qkv.device)
         if _TC_BWD and D in (64, 128) and dropout_p == 0.0:
-            # tcgen05 backward (csrc/flash_bwd_tc.cu): dK/dV pass + dQ pass, no atomics, no fp32 staging buffer
+            # tcgen05 backward (csrc/flash_bwd_tc.cu): dQ pass (with delta) + dK/dV pass, no atomics, no fp32 staging buffer
             ft = nv.proto("b200_flash_attn_bwd_tc", [vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, f32, i32, vp])
             rc = ft(nv.ptr(qkv), nv.ptr(out), nv.ptr(dout), nv.ptr(lse), nv.ptr(delta), nv.ptr(dqkv), B, S, H, Hkv, D, int(causal),
                     float(scale), nv.dtype_code(qkv.dtype), nv.stream())

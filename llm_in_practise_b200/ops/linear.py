@@ -45,8 +45,8 @@ def weight_workspace(device, dtype, numel: int, slot: int = 0) -> torch.Tensor:
     return buf[:numel]
 
 
-# largest token count served by the 4-bit GEMV instead of dequant + GEMM (measured, profiles/inference.md: at batch 48 the
-# table-free GEMV gives 12.4 ms per token vs 14.3 ms for dequant + GEMM, at batch 64 14.1 vs 14.7 ms)
+# Largest token count served by the 4-bit product instead of dequant + GEMM. 64 tokens (csrc/w4_tc.cu): N 24576, K 4096 56 us against 55,
+# N 4096, K 12288 45 against 67, N 6144, K 4096 28 against 48, N = K = 4096 26 against 40; 17 and 32 tokens of the first shape 38 against 54
 _W4_GEMV_MAX_M = int(__import__("os").environ.get("B200_W4_GEMV_MAX_M", "64"))   # integer-code weights (table-free kernel); NF4: 32
 
 class _LinearFn(torch.autograd.Function):

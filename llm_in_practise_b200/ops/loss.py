@@ -109,7 +109,8 @@ _VOCAB_CHUNK_MIN_BYTES = int(__import__("os").environ.get("B200_CE_VOCAB_MIN_MB"
 
 def _vocab_chunked(x, w, t, ignore_index, row_scale, gscale, need_dx, dw):
     """lm_head + CE over vocabulary chunks of ``_VOCAB_CHUNK`` columns (csrc/loss.cu, K8). The [M, C] chunk of logits
-    (32 MB for 2048 tokens x 8192 columns) lives in L2 between its GEMM and the kernels that consume it.
+    (64 MB for 2048 tokens x 16 384 columns) exists only between its GEMM and the kernels that consume it; beside the chunk's rows of
+    W (168 MB for K 5120) it does not stay in L2 whole.
 
     Frozen head (``dw is None``): ONE pass, flash-attention style — per chunk the kernel turns the logits into
     p = exp(l - running max) and returns the row rescale alpha; ``acc = alpha * acc + p @ W_chunk`` runs as a GEMM with

@@ -1,5 +1,5 @@
 """Every keyword argument the reference's scripts pass to the HF / PEFT / quantisation entry points this framework mirrors is
-accepted by the mirror (an AST scan of /root/reference; skipped where that tree is absent or empty)."""
+accepted by the mirror (an AST scan of the reference tree; skipped where that tree is absent or empty)."""
 import ast
 import dataclasses
 import glob

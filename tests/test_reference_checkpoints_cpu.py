@@ -13,7 +13,7 @@ _REF = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
 def _ref_module(fname):
     path = os.path.join(_REF, fname)
     if not os.path.exists(path):
-        pytest.skip(f"{path} is not present (created by __graft_entry__.build() where /root/reference exists)")
+        pytest.skip(f"{path} is not present (created by __graft_entry__.build() where the reference tree is)")
     spec = importlib.util.spec_from_file_location("ref_" + fname.replace(".", "_").replace("-", "_"), path)
     mod = importlib.util.module_from_spec(spec)
     spec.loader.exec_module(mod)
