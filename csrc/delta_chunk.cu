@@ -10,26 +10,38 @@
 //   O_i = c_i S_0^T q_i + sum_(j <= i) r_ij (q_i . k_j) u_j,   S = c_64 S_0 + sum_j r_64,j k_j u_j^T
 //
 // (the chunked form of the gated delta rule, Yang, Kautz and Hatamizadeh 2024), products of small matrices without a chain inside.
-//   delta_chunk_prep_kernel   a CTA per (chunk, q/k head): K K^T and Q K^T; then per head, 64 threads each: T = (I + A)^-1 by forward
-//                             substitution (a thread owns a column, rows of A are read as broadcasts), P_ij = r_ij (q_i . k_j),
-//                             c_i and r_64,j -> workspace. Chunks do not wait for one another.
+//   delta_chunk_prep_kernel   a CTA per (chunk, q/k head): K K^T and Q K^T; then per head, 64 threads each: T = (I + A)^-1 by blocks of 16,
+//                             P_ij = r_ij (q_i . k_j), c_i and r_64,j -> workspace, with K and Q. Chunks do not wait for one another.
 //   delta_chunk_scan_kernel   a CTA per (run, head, block of 16 value columns) walks the chunks with its columns of S in registers
 //                             and, for the products, in shared memory: [K; Q] S_0, U = T R, O += P U, S += K^T U. What the next
 //                             chunk needs is on its way (bulk copies) meanwhile.
-// All in fp32 FMAs (two per instruction), no tensor cores: the state is fp32 by definition, and splitting fp32 operands for bf16 or
-// tf32 mma.sync takes as many cycles as the FMAs do. r_ij is a product taken from j upwards, the roundings a walk makes too;
-// sums of logarithms would lose digits to cancellation. Bound: a packed FMA takes 3.0 cycles of a scheduler with three operands of its own and
-// 2.3 where one is the last one's too, as here, not 2 (85 and 109 FMAs a cycle and SM of 128, measured alone, two to four warps per
-// scheduler), 4800 of a chunk's 11 800 cycles; then the latency of the sums across lanes and the four barriers of a chunk. One prompt
-// of 2048 tokens, 16 heads of 128 x 128 over 4 q/k heads: 502 us token by token, 18 + 194 here; 2048 and 513 tokens: 586 -> 272 (the
-// shorter run's CTAs fill in behind the longer one's); error of the state against 64 bits 2e-7 both ways.
+// The products run on mma.sync with fp32 operands in three bf16 parts (split_mma.cuh), which has the error of fp32 or less: state against 64 bits,
+// 2048 and 513 tokens, 16 heads of 128: 1.9e-7 (by packed FMAs 2.2e-7, most of both from the keys). In two fp16 parts, with scales for each
+// column, the scan took 145 us instead of 170, with an error 5 to 15 % above that of the FMAs for heads of 64. r_ij is a product of the decays
+// themselves, roundings a walk makes too; sums of logarithms would lose digits to cancellation.
+// Bound of the scan: mma.sync and the instructions that split operands share the issue slots: a tile of 16 x 8 x 16 takes 48 cycles of a scheduler and
+// the split of its fp32 operand 28 more (measured apart: they do not overlap), 2800 + 2500 of a chunk's 6900 cycles; then its four
+// barriers. So Q, T and P come split, once for the eight column blocks and four heads; K, wanted in two forms, would not fit so.
+// One prompt of 2048 tokens, 16 heads of 128 x 128 over 4 q/k heads: 506 us token by token, 35 + 120 here (by FMAs, with T by substitution over
+// all 64 rows: 30 + 194); 2048 and 513 tokens: 35 + 170 (30 + 252; the shorter run's CTAs fill in behind the longer one's).
 #include "common.cuh"
+#include "split_mma.cuh"
 #include "../include/b200_ops.h"
 
 namespace b200 {
 
 constexpr int kDcC = 64, kDcCP = kDcC + 4;                // tokens of a chunk; padded row of a [64, 64] matrix
-constexpr long long kDcWs = 2 * kDcC * kDcC + 2 * kDcC;   // floats of workspace per (chunk, head): T, P, c, r_64
+// The workspace holds a chunk's matrices as the scan's products want them in shared memory, so that they are four bulk copies (a copy for each of their
+// rows: 320, and 200 us for a scan that takes 170). Q, T and P: operands of mma.sync in their three bf16 parts (split_mma.cuh), [8 rows x 16 columns][part][lane][2],
+// T and P without the blocks above the diagonal. K, which is read as it is and transposed: fp32, rows without padding, bits 3 and 4 of
+// the column turned by the row, so that pairs of columns of eight rows, and columns of four pairs of rows, are in different banks.
+__device__ __forceinline__ int dc_turn(int row) { return ((row >> 1) & 1) << 3 | ((row ^ (row >> 2)) & 1) << 4; }
+constexpr int kDcB = 3 * 64;                              // words of a block
+constexpr int dc_block(int j, int s) { return (j >> 1) * ((j >> 1) + 1) + (j & 1) * ((j >> 1) + 1) + s; }     // of T and P: rows 8 j .., columns 16 s ..
+constexpr int kDcT = 20 * kDcB, kDcPX = kDcT + 3 * kDcC, kDcHead = kDcT + kDcPX;      // words: T; P, c, r_64, beta
+constexpr int dc_q(int D) { return 8 * (D / 16) * kDcB; }
+constexpr int dc_kv(int D) { return kDcC * D + dc_q(D); } // K; Q
+constexpr int kDcWindow = 128;                            // chunks that the workspace holds
 
 struct DeltaChunkArgs {
   const float *q, *k, *v, *g, *beta;
@@ -37,32 +49,98 @@ struct DeltaChunkArgs {
   float *state, *o, *ws;
   const int* runs;
   int n_runs, H, G, Dv, tile_lo, tile_hi;                 // chunks [tile_lo, tile_hi) of all the step's chunks, counted run by run
+  long long kv_ws;                                        // where K and Q begin in ws
 };
 
-// 16 bytes on their way to shared memory; zeros where `live` is false
-__device__ __forceinline__ void dc_copy16(float* dst, const float* src, bool live) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(live ? 16 : 0) : "memory");
+template <int D> constexpr int prep_smem() {              // K | Q (later the four heads' A and T), K K^T | Q K^T, a of four heads
+  constexpr int tiles = 2 * kDcC * D, as = 4 * kDcC * kDcCP;
+  return ((tiles > as ? tiles : as) + 2 * kDcC * kDcCP + 4 * kDcC) * 4;
 }
-__device__ __forceinline__ void dc_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-__device__ __forceinline__ float2 lo2(const float4& v) { return make_float2(v.x, v.y); }
-__device__ __forceinline__ float2 hi2(const float4& v) { return make_float2(v.z, v.w); }
 
-template <int D> constexpr int prep_smem() {              // K | Q (later the four heads' A), K K^T | Q K^T, a | beta of four heads
-  constexpr int tiles = 2 * kDcC * (D + 4), as = 4 * kDcC * kDcCP;
-  return ((tiles > as ? tiles : as) + 2 * kDcC * kDcCP + 4 * 2 * kDcC) * 4;
+// In place: A [64, 64] strictly below the diagonal -> on and above it the transpose of T = (I + A)^-1 (zeros below it in the blocks of 16 it passes). 64 threads, thread j.
+// Blocks of 16: those on the diagonal by forward substitution, a column to a thread; then, the nearest to the diagonal first,
+// T_IJ = -T_II sum_(J <= M < I) A_IM T_MJ. The substitution of all 64 rows in registers was 2000 FMAs in a row of straight code, read once.
+__device__ __forceinline__ void invert_lower(float* As, int j, int barrier) {
+  const int blk = j >> 4, col = j & 15;
+  {
+    float x[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+      for (int m = 0; m < i; m += 2) {                    // x is zero above the column's diagonal
+        const float2 a = *reinterpret_cast<const float2*>(As + (blk * 16 + i) * kDcCP + blk * 16 + m);
+        s0 = fmaf(a.x, x[m], s0);
+        if (m + 1 < i) s1 = fmaf(a.y, x[m + 1], s1);
+      }
+      x[i] = (i == col ? 1.f : 0.f) - (s0 + s1);
+    }
+    asm volatile("bar.sync %0, 64;" ::"r"(barrier) : "memory");          // A's block is read: all of T's, transposed, takes its place
+#pragma unroll
+    for (int i = 0; i < 16; i += 4) *reinterpret_cast<float4*>(As + j * kDcCP + blk * 16 + i) = make_float4(x[i], x[i + 1], x[i + 2], x[i + 3]);
+  }
+  const int r0 = blk * 4;                                 // from here on: four rows of a block, column `col`
+#pragma unroll 1
+  for (int l = 1; l < 4; ++l) {
+    float y[3][4];
+    asm volatile("bar.sync %0, 64;" ::"r"(barrier) : "memory");
+#pragma unroll
+    for (int J = 0; J < 3; ++J) {
+      if (J + l > 3) break;
+      const float* Tc = As + (J * 16 + col) * kDcCP;      // column `col` of block column J of T, as a row
+      const float* Ar = As + ((J + l) * 16 + r0) * kDcCP;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) y[J][i] = 0.f;
+#pragma unroll 1
+      for (int M = J; M < J + l; ++M) {
+#pragma unroll
+        for (int k = 0; k < 16; k += 4) {
+          const float4 t = *reinterpret_cast<const float4*>(Tc + M * 16 + k);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float4 a = *reinterpret_cast<const float4*>(Ar + i * kDcCP + M * 16 + k);
+            y[J][i] = fmaf(a.x, t.x, y[J][i]); y[J][i] = fmaf(a.y, t.y, y[J][i]);
+            y[J][i] = fmaf(a.z, t.z, y[J][i]); y[J][i] = fmaf(a.w, t.w, y[J][i]);
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int J = 0; J < 3; ++J)
+      if (J + l < 4) *reinterpret_cast<float4*>(As + (J * 16 + col) * kDcCP + (J + l) * 16 + r0) = make_float4(y[J][0], y[J][1], y[J][2], y[J][3]);
+    asm volatile("bar.sync %0, 64;" ::"r"(barrier) : "memory");
+#pragma unroll
+    for (int J = 0; J < 3; ++J) {
+      if (J + l > 3) break;
+      const int I = (J + l) * 16;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) y[J][i] = 0.f;
+#pragma unroll
+      for (int k = 0; k < 16; ++k) {
+        const float4 t = *reinterpret_cast<const float4*>(As + (I + k) * kDcCP + I + r0);       // T_II's column k
+        const float v = As[(J * 16 + col) * kDcCP + I + k];
+        y[J][0] = fmaf(t.x, v, y[J][0]); y[J][1] = fmaf(t.y, v, y[J][1]); y[J][2] = fmaf(t.z, v, y[J][2]); y[J][3] = fmaf(t.w, v, y[J][3]);
+      }
+    }
+    asm volatile("bar.sync %0, 64;" ::"r"(barrier) : "memory");
+#pragma unroll
+    for (int J = 0; J < 3; ++J)
+      if (J + l < 4) *reinterpret_cast<float4*>(As + (J * 16 + col) * kDcCP + (J + l) * 16 + r0) = make_float4(-y[J][0], -y[J][1], -y[J][2], -y[J][3]);
+  }
+  asm volatile("bar.sync %0, 64;" ::"r"(barrier) : "memory");
 }
 
 template <int D>
 __global__ void __launch_bounds__(256, 2)
 delta_chunk_prep_kernel(const DeltaChunkArgs p) {
-  constexpr int DP = D + 4;
+  constexpr int KS = D / 16;
   extern __shared__ __align__(16) float sm[];
-  constexpr int kTiles = 2 * kDcC * DP, kAs = 4 * kDcC * kDcCP;
+  constexpr int kTiles = 2 * kDcC * D, kAs = 4 * kDcC * kDcCP;
   float* Ks = sm;
-  float* Qs = sm + kDcC * DP;
+  float* Qs = sm + kDcC * D;
   float* KK = sm + (kTiles > kAs ? kTiles : kAs);
   float* QK = KK + kDcC * kDcCP;
-  float* AB = QK + kDcC * kDcCP;                          // [4 heads][a 64 | beta 64]
+  float* AB = QK + kDcC * kDcCP;                          // [4 heads][a 64]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int tile = p.tile_lo + blockIdx.x, kvh = blockIdx.y, rep = p.H / p.G;
   int first = 0, n = 0;
@@ -72,174 +150,221 @@ delta_chunk_prep_kernel(const DeltaChunkArgs p) {
     at += nt;
   }
   if (n <= 0) return;                                     // the grid counts a chunk more per run than there may be
-  for (int i = tid; i < kDcC * (D / 4); i += 256) {
-    const int t = i / (D / 4), d = i % (D / 4) * 4;
-    const long long row = first + min(t, n - 1);
-    dc_copy16(Ks + t * DP + d, p.k + row * p.ldk + (long long)kvh * D + d, t < n);
-    dc_copy16(Qs + t * DP + d, p.q + row * p.ldq + (long long)kvh * D + d, t < n);
+  float* kv = p.ws + p.kv_ws + ((long long)blockIdx.x * p.G + kvh) * dc_kv(D);
+  {
+    constexpr int N = kDcC * (D / 4) / 256;
+    float4 x[N], y[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int t = (tid + 256 * i) / (D / 4), d = (tid + 256 * i) % (D / 4) * 4;
+      x[i] = y[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (t < n) {
+        x[i] = *reinterpret_cast<const float4*>(p.k + (long long)(first + t) * p.ldk + (long long)kvh * D + d);
+        y[i] = *reinterpret_cast<const float4*>(p.q + (long long)(first + t) * p.ldq + (long long)kvh * D + d);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int t = (tid + 256 * i) / (D / 4), d = (tid + 256 * i) % (D / 4) * 4;
+      const int at = t * D + (d ^ dc_turn(t));
+      *reinterpret_cast<float4*>(Ks + at) = x[i];
+      *reinterpret_cast<float4*>(Qs + at) = y[i];
+      *reinterpret_cast<float4*>(kv + at) = x[i];
+    }
   }
-  dc_wait_all();
   __syncthreads();
   {
-    const int rl = lane >> 2, cl = lane & 3, row0 = (warp & 1) * 32 + rl, col0 = (warp >> 1) * 16 + cl;
-    float2 ak[4][4], aq[4][4];
+    // 16 rows of K K^T or Q K^T to a warp, up to the diagonal; the two warps of a scheduler have ten tiles of eight columns together
+    const int g = lane >> 2, t2 = (lane & 3) * 2, mt = warp < 4 ? warp : 7 - warp, turn = dc_turn(g);
+    const float* rows = (warp < 4 ? Ks : Qs) + (mt * 16 + g) * D;
+    float* out = (warp < 4 ? KK : QK) + (mt * 16 + g) * kDcCP + t2;
+    SplitA a[KS];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int s = 0; s < KS; ++s)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) ak[i][j] = aq[i][j] = make_float2(0.f, 0.f);
-    if ((warp & 1) || warp < 4) {                         // rows 0 .. 31 x columns 32 .. 63 lie above the diagonal
-#pragma unroll 2
-      for (int d = 0; d < D; d += 4) {
-        float4 b[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(Ks + (col0 + 4 * j) * DP + d);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float4 x = *reinterpret_cast<const float4*>(Ks + (row0 + 8 * i) * DP + d);
-          const float4 y = *reinterpret_cast<const float4*>(Qs + (row0 + 8 * i) * DP + d);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            ak[i][j] = __ffma2_rn(lo2(x), lo2(b[j]), ak[i][j]);
-            aq[i][j] = __ffma2_rn(lo2(y), lo2(b[j]), aq[i][j]);
-            ak[i][j] = __ffma2_rn(hi2(x), hi2(b[j]), ak[i][j]);
-            aq[i][j] = __ffma2_rn(hi2(y), hi2(b[j]), aq[i][j]);
-          }
-        }
+      for (int x = 0; x < 4; ++x) {
+        const float2 v = *reinterpret_cast<const float2*>(rows + (x & 1) * 8 * D + ((16 * s + (x >> 1) * 8 + t2) ^ turn));
+        split3(v.x, v.y, a[s].p[0][x], a[s].p[1][x], a[s].p[2][x]);
       }
+    if (warp >= 4) {                                      // Q's operands for the scan: their rows are its columns
+      uint32_t* qw = reinterpret_cast<uint32_t*>(kv + kDcC * D);
+#pragma unroll
+      for (int s = 0; s < KS; ++s)
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+            *reinterpret_cast<uint2*>(qw + ((2 * mt + e) * KS + s) * kDcB + i * 64 + lane * 2) = make_uint2(a[s].p[i][e], a[s].p[i][2 + e]);
     }
+#pragma unroll 1
+    for (int j = 0; j < 2 * mt + 2; ++j) {
+      SplitAcc c;
+      const float* col = Ks + (8 * j + g) * D;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        KK[(row0 + 8 * i) * kDcCP + col0 + 4 * j] = ak[i][j].x + ak[i][j].y;
-        QK[(row0 + 8 * i) * kDcCP + col0 + 4 * j] = aq[i][j].x + aq[i][j].y;
+      for (int s = 0; s < KS; ++s) {
+        const float2 v = *reinterpret_cast<const float2*>(col + ((16 * s + t2) ^ turn)), w = *reinterpret_cast<const float2*>(col + ((16 * s + 8 + t2) ^ turn));
+        mma_split(a[s], split_b(v.x, v.y, w.x, w.y), c);
       }
+      *reinterpret_cast<float2*>(out + 8 * j) = make_float2(c.sum(0), c.sum(1));
+      *reinterpret_cast<float2*>(out + 8 * kDcCP + 8 * j) = make_float2(c.sum(2), c.sum(3));
+    }
   }
   __syncthreads();                                        // K and Q are read: their place takes the heads' A
-  const int grp = tid >> 6, j = tid & 63;
+  const int grp = tid >> 6, i = tid & 63;                 // a head, a row
   float* As = sm + grp * kDcC * kDcCP;
-  float* a_ = AB + grp * 2 * kDcC;
-  float* b_ = a_ + kDcC;
+  float* a_ = AB + grp * kDcC;
+  const int lane0 = (i & 7) * 4, s_end = (i >> 5) * 2 + 2;         // steps of 16 columns: the same in a warp, of whose rows the last ends at i | 31
   for (int hh = grp; hh < rep; hh += 4) {
     const int h = kvh * rep + hh;
-    a_[j] = j < n ? p.g[(long long)(first + j) * p.ldg + h] : 1.f;
-    b_[j] = j < n ? p.beta[(long long)(first + j) * p.ldb + h] : 0.f;
-    asm volatile("bar.sync %0, 64;" ::"r"(1 + grp) : "memory");
-    float* T = p.ws + ((long long)(tile - p.tile_lo) * p.H + h) * kDcWs;
-    float* P = T + kDcC * kDcC;
-    float r = 1.f, c = 1.f;
-    for (int i = 0; i < kDcC; ++i) {
-      const float a = a_[i];
-      if (i <= j) c *= a;
-      if (i > j) r *= a;
-      As[i * kDcCP + j] = i > j ? b_[i] * r * KK[i * kDcCP + j] : 0.f;
-      P[i * kDcC + j] = i >= j ? r * QK[i * kDcCP + j] : 0.f;
-    }
-    P[kDcC * kDcC + j] = c;
-    P[kDcC * kDcC + kDcC + j] = r;
-    asm volatile("bar.sync %0, 64;" ::"r"(1 + grp) : "memory");
-    float x[kDcC];                                        // column j of the inverse
+    const float b_i = i < n ? p.beta[(long long)(first + i) * p.ldb + h] : 0.f;
+    a_[i] = i < n ? p.g[(long long)(first + i) * p.ldg + h] : 1.f;
+    uint32_t* T = reinterpret_cast<uint32_t*>(p.ws + ((long long)blockIdx.x * p.H + h) * kDcHead);
+    uint32_t* P = T + kDcT;
+    float* X = reinterpret_cast<float*>(P + kDcT);
+    // 16 columns of row i as the operand's words: pairs 2 t, 2 t + 1 and 2 t + 8, + 9 are lane t's
+    auto store_row = [&](uint32_t* m, int s, const float (&x)[16]) {
+      uint32_t w[3][8];
 #pragma unroll
-    for (int i = 0; i < kDcC; ++i) x[i] = 0.f;
-#pragma unroll
-    for (int i = 0; i < kDcC; ++i) {
-      float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-#pragma unroll
-      for (int m = 0; m < i; m += 4) {                    // A is zero from the diagonal on, x from i on
-        const float4 a4 = *reinterpret_cast<const float4*>(As + i * kDcCP + m);
-        s0 = fmaf(a4.x, x[m], s0); s1 = fmaf(a4.y, x[m + 1], s1); s2 = fmaf(a4.z, x[m + 2], s2); s3 = fmaf(a4.w, x[m + 3], s3);
+      for (int t = 0; t < 4; ++t) {
+        split3(x[2 * t], x[2 * t + 1], w[0][2 * t], w[1][2 * t], w[2][2 * t]);
+        split3(x[2 * t + 8], x[2 * t + 9], w[0][2 * t + 1], w[1][2 * t + 1], w[2][2 * t + 1]);
       }
-      x[i] = (i == j ? 1.f : 0.f) - ((s0 + s1) + (s2 + s3));
-      T[i * kDcC + j] = x[i];
+      if (s > (i >> 4)) return;                           // above the diagonal
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        uint4* at = reinterpret_cast<uint4*>(m + dc_block(i >> 3, s) * kDcB + k * 64 + lane0 * 2);
+        at[0] = make_uint4(w[k][0], w[k][1], w[k][2], w[k][3]);
+        at[1] = make_uint4(w[k][4], w[k][5], w[k][6], w[k][7]);
+      }
+    };
+    asm volatile("bar.sync %0, 64;" ::"r"(1 + grp) : "memory");
+    float r = 1.f;                                        // r_ij, from the row's token to the ones before it
+#pragma unroll 1
+    for (int s = s_end - 1; s >= 0; --s) {
+      float x[16];
+#pragma unroll
+      for (int e0 = 12; e0 >= 0; e0 -= 4) {
+        const int j0 = 16 * s + e0;
+        const float4 k4 = *reinterpret_cast<const float4*>(KK + i * kDcCP + j0), q4 = *reinterpret_cast<const float4*>(QK + i * kDcCP + j0);
+        const float4 a4 = *reinterpret_cast<const float4*>(a_ + j0);
+        const float ka[4] = {k4.x, k4.y, k4.z, k4.w}, qa[4] = {q4.x, q4.y, q4.z, q4.w}, aa[4] = {a4.x, a4.y, a4.z, a4.w};
+        float A[4];
+#pragma unroll
+        for (int e = 3; e >= 0; --e) {
+          const bool on = j0 + e <= i;
+          x[e0 + e] = on ? r * qa[e] : 0.f;
+          A[e] = j0 + e < i ? b_i * (r * ka[e]) : 0.f;
+          if (on) r *= aa[e];
+        }
+        *reinterpret_cast<float4*>(As + i * kDcCP + j0) = make_float4(A[0], A[1], A[2], A[3]);
+      }
+      store_row(P, s, x);
     }
-    asm volatile("bar.sync %0, 64;" ::"r"(1 + grp) : "memory");   // the next head's a, beta and A overwrite these
+    X[i] = r;                                             // c_i
+    r = 1.f;                                              // r_64 of token i
+#pragma unroll 4
+    for (int j0 = kDcC - 4; j0 >= (i & 32); j0 -= 4) {
+      const float4 a4 = *reinterpret_cast<const float4*>(a_ + j0);
+      if (j0 + 3 > i) r *= a4.w;
+      if (j0 + 2 > i) r *= a4.z;
+      if (j0 + 1 > i) r *= a4.y;
+      if (j0 > i) r *= a4.x;
+    }
+    X[kDcC + i] = r;
+    X[2 * kDcC + i] = b_i;
+    asm volatile("bar.sync %0, 64;" ::"r"(1 + grp) : "memory");
+    invert_lower(As, i, 1 + grp);
+#pragma unroll 1
+    for (int s = 0; s < s_end; ++s) {
+      float x[16];
+#pragma unroll
+      for (int e = 0; e < 16; ++e) x[e] = 16 * s + e <= i ? As[(16 * s + e) * kDcCP + i] : 0.f;
+      store_row(T, s, x);
+    }
+    asm volatile("bar.sync %0, 64;" ::"r"(1 + grp) : "memory");   // the next head's a and A overwrite these
   }
 }
 
+template <int N> struct IntC { static constexpr int value = N; };
 constexpr int kDcNC = 16;                                 // value columns of a CTA: 128 CTAs for 16 heads of 128
 
 template <int D> struct DcSmem {                          // float offsets
-  static constexpr int NC = kDcNC;
-  static constexpr int DP = D + 4;
-  static constexpr int K = 0, Q = K + 2 * kDcC * DP, T = Q + kDcC * DP, P = T + kDcC * kDcCP, V = P + 2 * kDcC * kDcCP, S = V + 2 * kDcC * NC,
-                       R = S + D * NC, U = R + kDcC * NC, UD = U + kDcC * NC, X = UD + kDcC * NC,
-                       Bar = X + 2 * 3 * kDcC, kTotal = Bar + 8;       // X: c | r_64 | beta, twice; Bar: K, V, P, X of each buffer, Q and T
+  static constexpr int NC = kDcNC, KS = D / 16, kThreads = 2 * KS * 32;   // two warps to 16 rows of the state
+  static constexpr int K = 0, Q = K + 2 * kDcC * D, T = Q + dc_q(D), P = T + kDcT, Red = P + 2 * kDcPX, S = Red + KS * kDcC * NC,
+                       R = S + KS * 3 * 128, U = R + 4 * 3 * 128, UD = U + 4 * 3 * 128, Bar = UD + 4 * 3 * 128, kTotal = Bar + 8;
+  static_assert(kTotal * 4 <= 227 * 1024, "shared memory");
 };
 
-// Where columns c, c + 1 (c even) of the pair of rows pr lie in a [rows / 2][16][2] array: 16 bytes, the two halves of 32 changing places
-// with every other two pairs so that the eight lane groups of a warp read and write different banks
-__device__ __forceinline__ int pair_at(int pr, int c) { return pr * (2 * kDcNC) + (((c >> 1) ^ (pr >> 1 & 1)) << 2); }
-
-// NR rows' sums over 4 N2 elements (every eighth group of four, the lane's own) times four columns held as pairs of rows: with two warps per scheduler it is the rows beside one
-// another that keep the FMA pipe busy
-template <int NR, int N2>
-__device__ __forceinline__ void dot_rows(const float* rows, int stride, const float2 (&m)[2 * N2][4], float4 (&out)[NR]) {
-  float2 acc[NR][4];
+// half an operand A from an accumulator: columns 2 t, 2 t + 1 of rows g and g + 8 are what the lane holds of either
+__device__ __forceinline__ void store_half_a(float* at, int lane, int half, const float (&x)[4]) {
+  uint32_t p[3][2];
+  split3(x[0], x[1], p[0][0], p[1][0], p[2][0]);
+  split3(x[2], x[3], p[0][1], p[1][1], p[2][1]);
 #pragma unroll
-  for (int r = 0; r < NR; ++r)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) acc[r][c] = make_float2(0.f, 0.f);
-#pragma unroll
-  for (int x = 0; x < N2; ++x) {
-    float4 a[NR];
-#pragma unroll
-    for (int r = 0; r < NR; ++r) a[r] = *reinterpret_cast<const float4*>(rows + r * stride + 32 * x);
-#pragma unroll
-    for (int r = 0; r < NR; ++r)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) acc[r][c] = __ffma2_rn(lo2(a[r]), m[2 * x][c], acc[r][c]);
-#pragma unroll
-    for (int r = 0; r < NR; ++r)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) acc[r][c] = __ffma2_rn(hi2(a[r]), m[2 * x + 1][c], acc[r][c]);
-  }
-#pragma unroll
-  for (int r = 0; r < NR; ++r)
-    out[r] = make_float4(acc[r][0].x + acc[r][0].y, acc[r][1].x + acc[r][1].y, acc[r][2].x + acc[r][2].y, acc[r][3].x + acc[r][3].y);
+  for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(at + i * 128 + lane * 4 + half * 2) = make_uint2(p[i][0], p[i][1]);
 }
 
-// Four columns' parts in the eight lanes that share them (lane bits 2, 3, 4) -> the sum of column 2 (bit 4) + (bit 3): each step hands
-// half of what is left to the lane across
-__device__ __forceinline__ float gather4(const float4& v, int lane) {
-  const bool b4 = lane & 16, b3 = lane & 8;
-  const float x = (b4 ? v.z : v.x) + __shfl_xor_sync(0xffffffffu, b4 ? v.x : v.z, 16);
-  const float y = (b4 ? v.w : v.y) + __shfl_xor_sync(0xffffffffu, b4 ? v.y : v.w, 16);
-  const float z = (b3 ? y : x) + __shfl_xor_sync(0xffffffffu, b3 ? x : y, 8);
-  return z + __shfl_xor_sync(0xffffffffu, z, 4);
-}
-
-// Row t of a lower triangle times column c of X, in the layout of R and U: the columns above the diagonal are zero, and here they are not
-// multiplied either. dot_rows multiplies them, which is the same unless X holds an infinity or NaN: then it would reach rows, tokens, that
-// come before its own. So a chunk with such an R or U takes this one (a vote with the barriers that are there anyway).
-__device__ __forceinline__ float lower_dot(const float* row, const float* X, int t, int c) {
-  float s = 0.f;
-  for (int j = 0; j <= t; ++j) s = fmaf(row[j], X[pair_at(j >> 1, c) + (c & 1) * 2 + (j & 1)], s);
-  return s;
-}
-__device__ __forceinline__ bool not_finite(float x) { return !(fabsf(x) <= 3.402823466e38f); }
-
-// an "or" over the 256 threads of the chain's warps, and a barrier for them
-__device__ __forceinline__ int chain_or(int x) {
+// an "or" over the first N threads, and a barrier for them
+template <int N>
+__device__ __forceinline__ int half_or(int x) {
   int r;
   asm volatile(
       "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\t"
-      "barrier.cta.red.or.pred q, 1, 256, p;\n\tselp.s32 %0, 1, 0, q;\n\t}" : "=r"(r) : "r"(x) : "memory");
+      "barrier.cta.red.or.pred q, 1, %2, p;\n\tselp.s32 %0, 1, 0, q;\n\t}" : "=r"(r) : "r"(x), "n"(N) : "memory");
   return r;
 }
 
-// What limits the walk is shared memory, 128 bytes a cycle into registers against 128 FMAs: a tile of 4 x 4 outputs per thread would
-// take two bytes per FMA. So the small side of every product but the last stays in registers — S_0 with 16 rows of four columns in
-// every lane of every warp, R and U with eight — and a row of the other side costs one byte per FMA; the lanes' parts of
-// a row meet in four shuffles. Shared layouts: S, R and U hold pairs of neighbouring rows of one column side by side
-// ([rows / 2][16][2], pair_at), the pairs a packed FMA takes.
-// What the next chunk waits for is only K S_0, U = T R and S += K^T U. Warps 0-7, the chain, do these; warps 8-15 read out beside them: Q S_0
-// while the chain is at K S_0 and T R, then P U while it is at K^T U. Eight warps for all of it one after the other and copies of 16 bytes
-// by all of them: 262 us for runs of 2048 and 513 tokens, 245 now; the halves alone, with those copies, gave nothing (264).
+// Tokens [at, len) of a run one by one, from S [16 columns][D] in shared memory (`sm` has room for D x 16 and 2 x 16 x 16 floats more): what a chunk with an infinity or NaN in R, U
+// or Q S_0 takes, since a product with zeros above a diagonal, or of parts of an infinity, would carry it to tokens before its own.
 template <int D>
-__global__ void __launch_bounds__(512, 1)
+__device__ __noinline__ void walk_on(const DeltaChunkArgs& p, float* sm, int h, int col0, int first, int at, int len, float* state) {
+  const int tid = threadIdx.x, e = tid & 15, part = tid >> 4, kvh = h / (p.H / p.G);
+  constexpr int RPT = D / 16;                             // rows of a thread of the first 256
+  float s[RPT];
+  float* red = sm + D * 16;
+  if (tid < 256)
+    for (int i = 0; i < RPT; ++i) s[i] = sm[(part * RPT + i) * 16 + e];
+  for (int t = at; t < len; ++t) {
+    const long long row = first + t;
+    float d = 0.f, o = 0.f;
+    if (tid < 256) {
+      const float a = p.g[row * p.ldg + h];
+      const float* kr = p.k + row * p.ldk + (long long)kvh * D + part * RPT;
+      for (int i = 0; i < RPT; ++i) { s[i] *= a; d = fmaf(s[i], kr[i], d); }
+      red[part * 16 + e] = d;
+    }
+    __syncthreads();
+    if (tid < 256) {
+      float y = 0.f;
+      for (int i = 0; i < 16; ++i) y += red[i * 16 + e];
+      const float u = p.beta[row * p.ldb + h] * (p.v[row * p.ldv + (long long)h * p.Dv + col0 + e] - y);
+      const float* kr = p.k + row * p.ldk + (long long)kvh * D + part * RPT;
+      const float* qr = p.q + row * p.ldq + (long long)kvh * D + part * RPT;
+      for (int i = 0; i < RPT; ++i) { s[i] = fmaf(kr[i], u, s[i]); o = fmaf(s[i], qr[i], o); }
+      red[256 + part * 16 + e] = o;
+    }
+    __syncthreads();
+    if (tid < 16) {
+      float y = 0.f;
+      for (int i = 0; i < 16; ++i) y += red[256 + i * 16 + e];
+      p.o[(row * p.H + h) * p.Dv + col0 + e] = y;
+    }
+  }
+  if (tid < 256)
+    for (int i = 0; i < RPT; ++i) state[(long long)(part * RPT + i) * p.Dv + col0 + e] = s[i];
+}
+
+// The state of 16 columns, transposed, is the 16 rows of an mma.sync tile: S^T K^T, R^T T^T, U^T P^T, S^T Q^T have the chunk's tokens as columns,
+// U^T K the state's rows, and every accumulator is, lane by lane, half an operand of the next product. The operands are fp32 in three bf16 parts
+// (split_mma.cuh). A warp keeps eight rows of the state, fp32, in its accumulator.
+// What the next chunk waits for is only K S_0, U = T R and S += K^T U. All warps do the first, 16 rows of the state and half of the tokens each; their
+// parts meet in shared memory, where the first half of the warps forms R and U while the other half reads out Q S_0; all do the last, and
+// the second half P U after it.
+template <int D>
+__global__ void __launch_bounds__(DcSmem<D>::kThreads, 1)
 delta_chunk_scan_kernel(const DeltaChunkArgs p) {
   using L = DcSmem<D>;
-  constexpr int NC = kDcNC, DP = L::DP, DT = D / 32;     // DT: state rows of a thread
+  constexpr int NC = kDcNC, KS = L::KS, TW = 8 / KS;      // TW: tiles of eight tokens to a warp of one half
   extern __shared__ __align__(16) float sm[];
   const int h = blockIdx.y, col0 = blockIdx.x * NC, run = blockIdx.z;
   int tb = 0;
@@ -247,229 +372,209 @@ delta_chunk_scan_kernel(const DeltaChunkArgs p) {
   const int first = p.runs[4 * run], len = p.runs[4 * run + 1], p0 = p.runs[4 * run + 2], slot = p.runs[4 * run + 3];
   const int t_lo = max(tb, p.tile_lo), t_hi = min(tb + (len + kDcC - 1) / kDcC, p.tile_hi);
   if (t_lo >= t_hi) return;
-  const int tid = threadIdx.x, lane = tid & 31, warp = (tid >> 5) & 7;    // the warp's place in its half
-  const bool chain = tid < 256;
-  const int rl = lane >> 2, cb = (lane & 3) * 4;          // this thread's four columns
-  const int cg = cb + (lane >> 4) * 2 + (lane >> 3 & 1);  // and the one whose sum over the warp it ends up with (gather4)
-  const int kvh = h / (p.H / p.G), t8 = warp * 8;         // a warp's eight tokens of a chunk
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, half = warp / KS, w = warp % KS;
+  const int g = lane >> 2, t2 = (lane & 3) * 2;           // the lane's row and first column of an accumulator
+  const int kvh = h / (p.H / p.G), turn = dc_turn(g);
 
-  // What a chunk needs comes a row at a time by bulk copies, one to a thread of the reading half: cp.async pieces of 16 bytes took all warps
-  // 2400 of a chunk's 12 700 cycles to ask for. A barrier is armed one barrier of the CTA before its copies are asked for.
+  // What a chunk needs, as delta_chunk_prep_kernel laid it out: K and P | c | r_64 | beta a chunk ahead, Q and T half of one. One thread asks; all have
+  // waited for a barrier's last phase when it does.
   const uint32_t bar = smem_u32(sm + L::Bar);
-  auto kvp_bar = [&](int tile) { return bar + 8u * (tile & 1); };
+  auto kp_bar = [&](int tile) { return bar + 8u * (tile & 1); };
   const uint32_t qt_bar = bar + 16;
-  auto rows_of = [&](int tile) { return min(kDcC, len - (tile - tb) * kDcC); };
-  auto arm_kvp = [&](int tile) { mbar_arrive_expect_tx(kvp_bar(tile), (uint32_t)(rows_of(tile) * (D + NC) + kDcC * kDcC + 2 * kDcC) * 4u); };
-  auto arm_qt = [&](int tile) { mbar_arrive_expect_tx(qt_bar, (uint32_t)(rows_of(tile) * D + kDcC * kDcC) * 4u); };
-  const int ri = tid - 256;                               // place in the reading half
-  auto row_copy = [&](float* dst, const float* src, int floats, bool there, uint32_t b) {
-    if (there) bulk_load_1d(smem_u32(dst), src, floats * 4, b);
-    else
-      for (int i = 0; i < floats; i += 4) *reinterpret_cast<float4*>(dst + i) = make_float4(0.f, 0.f, 0.f, 0.f);     // tokens past the end
-  };
-  auto ask_kvp = [&](int tile) {
-    const int buf = tile & 1, n = rows_of(tile), j = ri & 63;
-    const long long row = first + (tile - tb) * kDcC + min(j, n - 1);
-    const float* w = p.ws + ((long long)(tile - p.tile_lo) * p.H + h) * kDcWs + kDcC * kDcC;
-    if (ri < 64) row_copy(sm + L::K + (buf * kDcC + j) * DP, p.k + row * p.ldk + (long long)kvh * D, D, j < n, kvp_bar(tile));
-    else if (ri < 128) row_copy(sm + L::V + (buf * kDcC + j) * NC, p.v + row * p.ldv + (long long)h * p.Dv + col0, NC, j < n, kvp_bar(tile));
-    else if (ri < 192) row_copy(sm + L::P + (buf * kDcC + j) * kDcCP, w + j * kDcC, kDcC, true, kvp_bar(tile));
-    else {
-      if (j == 0) row_copy(sm + L::X + buf * 3 * kDcC, w + kDcC * kDcC, 2 * kDcC, true, kvp_bar(tile));
-      sm[L::X + buf * 3 * kDcC + 2 * kDcC + j] = j < n ? p.beta[row * p.ldb + h] : 0.f;
-    }
+  auto copy = [&](int dst, const float* src, int floats, uint32_t b) { bulk_load_1d(smem_u32(sm + dst), src, floats * 4, b); };
+  auto head_ws = [&](int tile) { return p.ws + ((long long)(tile - p.tile_lo) * p.H + h) * kDcHead; };
+  auto kv_ws = [&](int tile) { return p.ws + p.kv_ws + ((long long)(tile - p.tile_lo) * p.G + kvh) * dc_kv(D); };
+  auto ask_kp = [&](int tile) {
+    mbar_arrive_expect_tx(kp_bar(tile), (kDcC * D + kDcPX) * 4u);
+    copy(L::K + (tile & 1) * kDcC * D, kv_ws(tile), kDcC * D, kp_bar(tile));
+    copy(L::P + (tile & 1) * kDcPX, head_ws(tile) + kDcT, kDcPX, kp_bar(tile));
   };
   auto ask_qt = [&](int tile) {
-    const int n = rows_of(tile), j = ri & 63;
-    const long long row = first + (tile - tb) * kDcC + min(j, n - 1);
-    const float* w = p.ws + ((long long)(tile - p.tile_lo) * p.H + h) * kDcWs;
-    if (ri < 64) row_copy(sm + L::Q + j * DP, p.q + row * p.ldq + (long long)kvh * D, D, j < n, qt_bar);
-    else if (ri < 128) row_copy(sm + L::T + j * kDcCP, w + j * kDcC, kDcC, true, qt_bar);
+    mbar_arrive_expect_tx(qt_bar, (dc_q(D) + kDcT) * 4u);
+    copy(L::Q, kv_ws(tile) + kDcC * D, dc_q(D), qt_bar);
+    copy(L::T, head_ws(tile), kDcT, qt_bar);
   };
-  if (tid == 256) {
+  const bool asks = tid == KS * 32;
+  if (asks) {
     for (int i = 0; i < 3; ++i) mbar_init(bar + 8 * i, 1);
     fence_mbar_init();
-    arm_kvp(t_lo);
-    arm_qt(t_lo);
-    if (t_lo + 1 < t_hi) arm_kvp(t_lo + 1);
-  }
-  __syncthreads();
-  if (!chain) {
-    ask_kvp(t_lo);
+    ask_kp(t_lo);
     ask_qt(t_lo);
   }
+  __syncthreads();
 
-  // the state: rows d0 .. d0 + DT of four columns, in pairs of rows, kept by the first four warps; the chain's other four add up the second
-  // half of each chunk's tokens
-  const int d0 = ((warp & 3) * 8 + rl) * DT;
-  float* sp = p.state + (((long long)slot * p.H + h) * D) * p.Dv + col0 + cb;
-  float2 S[DT / 2][4];
-  const bool from_state = p0 > 0 || t_lo > tb, owner = tid < 128;
+  // columns g, g + 8 of the state's rows 16 w + 8 half + t2, + 1
+  float S[4];
+  float* const sp = p.state + (((long long)slot * p.H + h) * D) * p.Dv;
+  auto s_at = [&](int x) { return (long long)(16 * w + 8 * half + t2 + (x & 1)) * p.Dv + col0 + g + (x >> 1) * 8; };
 #pragma unroll
-  for (int x = 0; x < DT / 2; ++x) {
-    float4 s0 = make_float4(0.f, 0.f, 0.f, 0.f), s1 = s0;
-    if (from_state && owner) {
-      s0 = *reinterpret_cast<const float4*>(sp + (long long)(d0 + 2 * x) * p.Dv);
-      s1 = *reinterpret_cast<const float4*>(sp + (long long)(d0 + 2 * x + 1) * p.Dv);
-    }
-    S[x][0] = make_float2(s0.x, s1.x); S[x][1] = make_float2(s0.y, s1.y); S[x][2] = make_float2(s0.z, s1.z); S[x][3] = make_float2(s0.w, s1.w);
-  }
-  auto publish_state = [&]() {
-#pragma unroll
-    for (int x = 0; x < DT / 2; ++x) {
-      *reinterpret_cast<float4*>(sm + L::S + pair_at(d0 / 2 + x, cb)) = make_float4(S[x][0].x, S[x][0].y, S[x][1].x, S[x][1].y);
-      *reinterpret_cast<float4*>(sm + L::S + pair_at(d0 / 2 + x, cb + 2)) = make_float4(S[x][2].x, S[x][2].y, S[x][3].x, S[x][3].y);
-    }
-  };
-  if (owner) publish_state();
-
-  // N pairs of pairs of rows of S, R or U, every eighth of them the lane's own
-  auto hold = [&](const float* X, auto& B) {
-    constexpr int N = sizeof(B) / sizeof(B[0]);
-#pragma unroll
-    for (int x = 0; x < N; ++x) {
-      const int pr = ((x >> 1) * 8 + rl) * 2 + (x & 1);
-      const float4 b0 = *reinterpret_cast<const float4*>(X + pair_at(pr, cb)), b1 = *reinterpret_cast<const float4*>(X + pair_at(pr, cb + 2));
-      B[x][0] = lo2(b0); B[x][1] = hi2(b0); B[x][2] = lo2(b1); B[x][3] = hi2(b1);
-    }
-  };
-  // eight rows of a [64, D] tile times the state: column cg of rows t8 .. t8 + 7
-  auto times_state = [&](const float* rows, float (&y)[8]) {
-    float2 s0[D / 16][4];
-    hold(sm + L::S, s0);
-#pragma unroll
-    for (int i = 0; i < 8; i += 2) {
-      float4 z[2];
-      dot_rows<2, D / 32>(rows + (t8 + i) * DP + rl * 4, DP, s0, z);
-      y[i] = gather4(z[0], lane);
-      y[i + 1] = gather4(z[1], lane);
-    }
-  };
-  // eight rows of a lower triangle times X (R or U); `odd`: X holds an infinity or NaN
-  auto times_lower = [&](const float* rows, const float* X, int odd, float (&y)[8]) {
-    float2 B[4][4];
-    hold(X, B);
-#pragma unroll
-    for (int i = 0; i < 8; i += 4) {
-      float4 z[4];
-      dot_rows<4, 2>(rows + (t8 + i) * kDcCP + rl * 4, kDcCP, B, z);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) y[i + e] = gather4(z[e], lane);
-    }
-    if (odd) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) y[i] = lower_dot(rows + (t8 + i) * kDcCP, X, t8 + i, cg);
-    }
-  };
+  for (int x = 0; x < 4; ++x) S[x] = p0 > 0 || t_lo > tb ? sp[s_at(x)] : 0.f;
+  store_half_a(sm + L::S + w * 384, lane, half, S);
 
   for (int tile = t_lo; tile < t_hi; ++tile) {
     const int buf = tile & 1;
     const int at = (tile - tb) * kDcC, n = min(kDcC, len - at);
-    const bool more = tile + 1 < t_hi, live = t8 < n;
-    mbar_wait(kvp_bar(tile), (uint32_t)((tile - t_lo) >> 1) & 1u);
+    const bool more = tile + 1 < t_hi;
+    float v[TW][4];                                       // first half: the values of the tokens whose R this warp forms
+    if (half == 0) {
+#pragma unroll
+      for (int i = 0; i < TW; ++i)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          const int t = 8 * (w + i * KS) + t2 + (x & 1);
+          v[i][x] = t < n ? p.v[(long long)(first + at + t) * p.ldv + (long long)h * p.Dv + col0 + g + (x >> 1) * 8] : 0.f;
+        }
+    }
+    mbar_wait(kp_bar(tile), (uint32_t)((tile - t_lo) >> 1) & 1u);
     mbar_wait(qt_bar, (uint32_t)(tile - t_lo) & 1u);
-    __syncthreads();                                      // and S, and beta
-    if (!chain && more) {
-      if (ri == 0) {
-        arm_qt(tile + 1);
-        if (tile + 2 < t_hi) arm_kvp(tile + 2);           // this chunk's barrier: all have waited for it
+    __syncthreads();                                      // and S; the other K and P are read
+    if (asks && more) ask_kp(tile + 1);
+    const float* Ks = sm + L::K + buf * kDcC * D;
+    const float* Ps = sm + L::P + buf * kDcPX;
+    const float* cs = Ps + kDcT;                   // c | r_64 | beta
+    int odd = 0;                                          // an infinity or NaN among this thread's part of R, then of U, or of Q S_0
+    auto load_b = [&](const float* at) {                  // [part][lane][2]
+      SplitB b;
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        const uint2 u = *reinterpret_cast<const uint2*>(at + i * 64 + lane * 2);
+        b.p[i][0] = u.x; b.p[i][1] = u.y;
       }
-      ask_kvp(tile + 1);
+      return b;
+    };
+    // eight rows of a lower triangle [64, 64] (from row 8 j) times R or U. The number of steps is chosen by one branch: a branch in front of each
+    // step kept the steps apart
+    auto times_lower = [&](const float* tri, const float* X, int j, float (&z)[4]) {
+      auto steps = [&](auto n) {
+        SplitAcc c[2];
+#pragma unroll
+        for (int s = 0; s < n.value; ++s) {
+          const SplitA a = load_a(X + s * 384, lane);
+          const SplitB b = load_b(tri + (dc_block(j, 0) + s) * kDcB);
+          if (s < 2) mma_split<true>(a, b, c[s & 1]);
+          else mma_split(a, b, c[s & 1]);
+        }
+#pragma unroll
+        for (int x = 0; x < 4; ++x) z[x] = n.value > 1 ? c[0].sum(x) + c[1].sum(x) : c[0].sum(x);
+      };
+      if (j < 2) steps(IntC<1>());
+      else if (j < 4) steps(IntC<2>());
+      else if (j < 6) steps(IntC<3>());
+      else steps(IntC<4>());
+    };
+    {
+      // ---- 16 rows of S in K S_0, half of the tokens ----
+      const SplitA a = load_a(sm + L::S + w * 384, lane);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int j = half * 4 + i;
+        SplitAcc c;
+        const float* row = Ks + (8 * j + g) * D;
+        const float2 x = *reinterpret_cast<const float2*>(row + ((16 * w + t2) ^ turn)), y = *reinterpret_cast<const float2*>(row + ((16 * w + 8 + t2) ^ turn));
+        mma_split<true>(a, split_b(x.x, x.y, y.x, y.y), c);
+        *reinterpret_cast<float4*>(sm + L::Red + (w * 8 + j) * 128 + lane * 4) = make_float4(c.sum(0), c.sum(1), c.sum(2), c.sum(3));
+      }
     }
-    const float* Ks = sm + L::K + buf * kDcC * DP;
-    const float* cs = sm + L::X + buf * 3 * kDcC;         // c | r_64 | beta
-    int odd = 0;                                          // an infinity or NaN among this thread's part of R, then of U
-    float y[8];
+    __syncthreads();
+    float y[TW][4];                                       // second half: columns g, g + 8 of tokens t2, t2 + 1 of the read-out
+    if (half == 0) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) y[i] = 0.f;
-    if (chain) {
-      if (live) {
-        times_state(Ks, y);                               // K S_0
+      for (int i = 0; i < TW; ++i) {
+        const int j = w + i * KS;
+        float z[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          y[i] = cs[2 * kDcC + t8 + i] * (sm[L::V + (buf * kDcC + t8 + i) * NC + cg] - cs[t8 + i] * y[i]);
-          odd |= not_finite(y[i]);
+        for (int k = 0; k < KS; ++k) {
+          const float4 r = *reinterpret_cast<const float4*>(sm + L::Red + (k * 8 + j) * 128 + lane * 4);
+          z[0] += r.x; z[1] += r.y; z[2] += r.z; z[3] += r.w;
+        }
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          const int t = 8 * j + t2 + (x & 1);
+          z[x] = cs[2 * kDcC + t] * (v[i][x] - cs[t] * z[x]);
+          odd |= not_finite(z[x]);
+        }
+        store_half_a(sm + L::R + (j >> 1) * 384, lane, j & 1, z);
+      }
+      odd = half_or<KS * 32>(odd);
+#pragma unroll
+      for (int i = 0; i < TW; ++i) {
+        const int j = w + i * KS;
+        float z[4];
+        times_lower(sm + L::T, sm + L::R, j, z);
+#pragma unroll
+        for (int x = 0; x < 4; ++x) odd |= not_finite(z[x]);
+        store_half_a(sm + L::U + (j >> 1) * 384, lane, j & 1, z);
+#pragma unroll
+        for (int x = 0; x < 4; ++x) z[x] *= cs[kDcC + 8 * j + t2 + (x & 1)];
+        store_half_a(sm + L::UD + (j >> 1) * 384, lane, j & 1, z);
+      }
+    } else {
+      // ---- Q S_0 ----
+      SplitAcc c[TW][2];
+#pragma unroll
+      for (int s = 0; s < KS; ++s) {
+        const SplitA a = load_a(sm + L::S + s * 384, lane);
+#pragma unroll
+        for (int i = 0; i < TW; ++i) {
+          const SplitB b = load_b(sm + L::Q + ((w + i * KS) * KS + s) * kDcB);
+          if (s < 2) mma_split<true>(a, b, c[i][s & 1]);
+          else mma_split(a, b, c[i][s & 1]);
         }
       }
-      if (!(lane & 4)) {
 #pragma unroll
-        for (int i = 0; i < 8; i += 2) *reinterpret_cast<float2*>(sm + L::R + pair_at((t8 + i) / 2, cg) + (cg & 1) * 2) = make_float2(y[i], y[i + 1]);
-      }
-      odd = chain_or(odd);
-      float u[8];
+      for (int i = 0; i < TW; ++i)
 #pragma unroll
-      for (int i = 0; i < 8; ++i) u[i] = 0.f;
-      if (live) {
-        times_lower(sm + L::T, sm + L::R, odd, u);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) odd |= not_finite(u[i]);
-      }
-      if (!(lane & 4)) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) sm[L::UD + (t8 + i) * NC + cg] = cs[kDcC + t8 + i] * u[i];
-#pragma unroll
-        for (int i = 0; i < 8; i += 2) *reinterpret_cast<float2*>(sm + L::U + pair_at((t8 + i) / 2, cg) + (cg & 1) * 2) = make_float2(u[i], u[i + 1]);
-      }
-    } else if (live) {
-      times_state(sm + L::Q, y);                          // Q S_0
-#pragma unroll
-      for (int i = 0; i < 8; ++i) y[i] *= cs[t8 + i];
+        for (int x = 0; x < 4; ++x) {
+          y[i][x] = c[i][0].sum(x) + c[i][1].sum(x);
+          odd |= not_finite(y[i][x]);
+          y[i][x] *= cs[8 * (w + i * KS) + t2 + (x & 1)];
+        }
     }
-    odd = __syncthreads_or(odd);
-    if (!chain) {
-      if (more) ask_qt(tile + 1);
+    if (__syncthreads_or(odd)) {                          // S is still the one in front of the chunk
+#pragma unroll
+      for (int x = 0; x < 4; ++x) sm[L::Red + (16 * w + 8 * half + t2 + (x & 1)) * 16 + g + (x >> 1) * 8] = S[x];
+      if (more) mbar_wait(kp_bar(tile + 1), (uint32_t)((tile + 1 - t_lo) >> 1) & 1u);      // what is on its way arrives before the CTA leaves
+      __syncthreads();
+      walk_on<D>(p, sm + L::Red, h, col0, first, at, min(len, (t_hi - tb) * kDcC), sp);
+      return;
+    }
+    if (asks && more) ask_qt(tile + 1);
+    {
+      // ---- S = c_64 S + K^T (r_64 U) ----
+      SplitAcc c[2];
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        const int d = 16 * w + 8 * half + g, r = 16 * s + t2;
+        const float* kc = Ks + r * D;
+        const int e0 = d ^ dc_turn(t2), e1 = d ^ dc_turn(t2 + 1);
+        const SplitB b = split_b(kc[e0], kc[D + e1], kc[8 * D + e0], kc[9 * D + e1]);
+        const SplitA a = load_a(sm + L::UD + s * 384, lane);
+        if (s < 2) mma_split<true>(a, b, c[s & 1]);
+        else mma_split(a, b, c[s & 1]);
+      }
+      const float ce = cs[kDcC - 1];
+#pragma unroll
+      for (int x = 0; x < 4; ++x) S[x] = fmaf(S[x], ce, c[0].sum(x) + c[1].sum(x));
+      store_half_a(sm + L::S + w * 384, lane, half, S);
+    }
+    if (half == 1) {
       // ---- the read-out ----
-      if (live) {
-        float z[8];
-        times_lower(sm + L::P + buf * kDcC * kDcCP, sm + L::U, odd, z);
-        float* orow = p.o + ((long long)(first + at) * p.H + h) * p.Dv + col0 + cg;
-        if (!(lane & 4)) {
 #pragma unroll
-          for (int i = 0; i < 8; ++i)
-            if (t8 + i < n) orow[(long long)(t8 + i) * p.H * p.Dv] = y[i] + z[i];
+      for (int i = 0; i < TW; ++i) {
+        const int t8 = 8 * (w + i * KS);
+        float z[4];
+        times_lower(Ps, sm + L::U, w + i * KS, z);
+        float* orow = p.o + ((long long)(first + at + t8) * p.H + h) * p.Dv + col0 + g;
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          const int t = t2 + (x & 1);
+          if (t8 + t < n) orow[(long long)t * p.H * p.Dv + (x >> 1) * 8] = y[i][x] + z[x];
         }
       }
-      continue;
-    }
-    // ---- S = c_64 S + K^T (r_64 U) ----
-    const float2 ce = make_float2(cs[kDcC - 1], cs[kDcC - 1]);
-#pragma unroll
-    for (int x = 0; x < DT / 2; ++x)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) S[x][c] = owner ? __fmul2_rn(S[x][c], ce) : make_float2(0.f, 0.f);
-    const int t_end = owner ? min(n, kDcC / 2) : n;
-#pragma unroll 8
-    for (int t = owner ? 0 : kDcC / 2; t < t_end; ++t) {
-      float2 a[DT / 2];
-      if (DT == 4) {
-        const float4 a4 = *reinterpret_cast<const float4*>(Ks + t * DP + d0);
-        a[0] = lo2(a4); a[DT / 2 - 1] = hi2(a4);
-      } else a[0] = *reinterpret_cast<const float2*>(Ks + t * DP + d0);
-      const float4 u = *reinterpret_cast<const float4*>(sm + L::UD + t * NC + cb);
-#pragma unroll
-      for (int x = 0; x < DT / 2; ++x) {
-        S[x][0] = __ffma2_rn(a[x], make_float2(u.x, u.x), S[x][0]); S[x][1] = __ffma2_rn(a[x], make_float2(u.y, u.y), S[x][1]);
-        S[x][2] = __ffma2_rn(a[x], make_float2(u.z, u.z), S[x][2]); S[x][3] = __ffma2_rn(a[x], make_float2(u.w, u.w), S[x][3]);
-      }
-    }
-    if (!owner) publish_state();                          // the products with the old S ended in front of the last barrier
-    asm volatile("bar.sync 1, 256;" ::: "memory");
-    if (owner) {
-#pragma unroll
-      for (int x = 0; x < DT / 2; ++x) {
-        const float4 a = *reinterpret_cast<const float4*>(sm + L::S + pair_at(d0 / 2 + x, cb)), b = *reinterpret_cast<const float4*>(sm + L::S + pair_at(d0 / 2 + x, cb + 2));
-        S[x][0].x += a.x; S[x][0].y += a.y; S[x][1].x += a.z; S[x][1].y += a.w;
-        S[x][2].x += b.x; S[x][2].y += b.y; S[x][3].x += b.z; S[x][3].y += b.w;
-      }
-      publish_state();
     }
   }
-  if (!owner) return;
 #pragma unroll
-  for (int x = 0; x < DT / 2; ++x) {
-    *reinterpret_cast<float4*>(sp + (long long)(d0 + 2 * x) * p.Dv) = make_float4(S[x][0].x, S[x][1].x, S[x][2].x, S[x][3].x);
-    *reinterpret_cast<float4*>(sp + (long long)(d0 + 2 * x + 1) * p.Dv) = make_float4(S[x][0].y, S[x][1].y, S[x][2].y, S[x][3].y);
-  }
+  for (int x = 0; x < 4; ++x) sp[s_at(x)] = S[x];
 }
 
 template <int D>
@@ -485,7 +590,7 @@ static int run_windows(DeltaChunkArgs p, int bound, int window, cudaStream_t st)
     p.tile_hi = lo + window < bound ? lo + window : bound;
     prep<<<dim3(p.tile_hi - lo, p.G), 256, smem, st>>>(p);
     B200_LAUNCH_CHECK();
-    scan<<<dim3(p.Dv / kDcNC, p.H, p.n_runs), 512, scan_smem, st>>>(p);
+    scan<<<dim3(p.Dv / kDcNC, p.H, p.n_runs), DcSmem<D>::kThreads, scan_smem, st>>>(p);
     B200_LAUNCH_CHECK();
   }
   return 0;
@@ -493,10 +598,10 @@ static int run_windows(DeltaChunkArgs p, int bound, int window, cudaStream_t st)
 }  // namespace b200
 
 // Workspace (floats) for a step of `tokens` tokens in n_runs runs: chunks are taken in windows of at most 128, however long the step is.
-B200_API long long b200_delta_chunk_workspace(int tokens, int n_runs, int H) {
+B200_API long long b200_delta_chunk_workspace(int tokens, int n_runs, int H, int G, int D) {
   using namespace b200;
   const long long bound = (long long)tokens / kDcC + n_runs;
-  return (bound < 128 ? bound : 128) * H * kDcWs;
+  return (bound < kDcWindow ? bound : kDcWindow) * ((long long)H * kDcHead + (long long)G * dc_kv(D));
 }
 
 // Arguments as in b200_linear_scan (mode 3), `runs` present; `ws`: b200_delta_chunk_workspace floats. B200_ERR_UNSUPPORTED: the caller
@@ -510,9 +615,10 @@ B200_API int b200_delta_chunk_scan(const float* q, long long ldq, const float* k
   auto al = [](const void* x, long long ld) { return !(reinterpret_cast<uintptr_t>(x) & 15) && ld % 4 == 0; };
   if ((D != 64 && D != 128) || Dv % 16 || !al(q, ldq) || !al(k, ldk) || !al(v, ldv) || !al(state, 0) || !al(o, 0) || !al(ws, 0) || !runs)
     return B200_ERR_UNSUPPORTED;
-  DeltaChunkArgs p = {q, k, v, g, beta, ldq, ldk, ldv, ldg, ldb, state, o, ws, runs, n_runs, H, G, Dv, 0, 0};
+  DeltaChunkArgs p = {q, k, v, g, beta, ldq, ldk, ldv, ldg, ldb, state, o, ws, runs, n_runs, H, G, Dv, 0, 0, 0};
   const long long bound = (long long)tokens / kDcC + n_runs;      // a run of n tokens has at most n / 64 + 1 chunks
   if (bound > 0x7fffffffLL) return B200_ERR_TOO_LARGE;
-  const int window = bound < 128 ? (int)bound : 128;
+  const int window = bound < kDcWindow ? (int)bound : kDcWindow;
+  p.kv_ws = (long long)window * H * kDcHead;
   return D == 64 ? run_windows<64>(p, (int)bound, window, (cudaStream_t)stream) : run_windows<128>(p, (int)bound, window, (cudaStream_t)stream);
 }

@@ -240,25 +240,28 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.
 def _chunks_pay(T: int, n_runs: int, pieces, H: int, G: int, D: int, Dv: int) -> bool:
     """Whether prompts of the delta rule with one decay per head take less time 64 tokens at a time (csrc/delta_chunk.cu) than token by
     token. Both as measured (us): the walk moves 0.24 per token of the longest run, or, with more (run, head, 16 columns) than about
-    320 (445 for keys of 64) at once, in proportion; a chunk is 6.5 (4.8) on one of 148 SMs, after the inverses. One run of 2048 tokens,
-    16 heads of 128: 225 against 502; three of 150: 74 against 56. The constants are fits to 16 heads and a few lengths; other head
+    320 (445 for keys of 64) at once, in proportion; a chunk is 3.9 (2.8) on one of 148 SMs, which take the (run, head, 16 columns) in
+    rounds, after the inverses. 16 heads of 128 over 4: one run of 2048 tokens 155 against 506, four of 512 163 against 218, three of 150 73
+    against 60, eight of 1000 534 against 732; 32 heads, one of 200: 64 against 65; 16 heads of 64, one of 150: 32 against 44. Other head
     counts rest on the proportions. Without ``pieces`` the runs count as equally long."""
     blocks = H * (Dv // 16)
     longest, tiles = (pieces.longest, pieces.n_tiles) if pieces is not None else (T / max(n_runs, 1), T / 64 + n_runs)
-    walk = 0.24 * max(longest, T * blocks / (320 if D == 128 else 445))
-    chunks = 17 * max(1.0, tiles * G / 200) + (6.5 if D == 128 else 4.8) * max(longest / 64, tiles * blocks / 148)
+    walk = 8 + 0.24 * max(longest, T * blocks / (320 if D == 128 else 445))
+    rounds = max(-(-longest // 64) + 0.5, -(-n_runs * blocks // 148) * (tiles / max(n_runs, 1) + 0.5))
+    chunks = (31 if D == 128 else 23.5) * max(1.0, tiles * G / 160) + (3.85 if D == 128 else 2.8) * rounds
     return chunks < 0.9 * walk
 
 
 def _delta_chunks(q, k, v, g, beta, state, runs, n_runs, o, H, G, D, Dv) -> bool:
-    """Mode "head_delta" over the runs of a step in chunks of 64 tokens; False: rows the kernels do not take. The workspace is 33 KB per
-    chunk and head for at most 128 chunks at a time (136 MB at 32 heads), which the walk does without."""
+    """Mode "head_delta" over the runs of a step in chunks of 64 tokens; False: rows the kernels do not take. The workspace is 31 KB per
+    chunk and head and 80 KB (keys of 64: 41) per chunk and q/k head for at most 128 chunks at a time (211 MB at 32 heads over 8), which the walk
+    does without."""
     T = q.shape[0]
     if not nv.has("b200_delta_chunk_scan"):               # a library linked for a model without this mode
         return False
     size = nv.lib().b200_delta_chunk_workspace
     size.restype = i64
-    ws = torch.empty(size(T, n_runs, H), dtype=torch.float32, device=q.device)
+    ws = torch.empty(size(T, n_runs, H, G, D), dtype=torch.float32, device=q.device)
     fn = nv.proto("b200_delta_chunk_scan", [vp, i64, vp, i64, vp, i64, vp, i64, vp, i64, vp, vp, i32, vp, vp, i32, i32, i32, i32, i32, vp])
     rc = fn(nv.ptr(q), q.stride(0), nv.ptr(k), k.stride(0), nv.ptr(v), v.stride(0), nv.ptr(g), g.stride(0), nv.ptr(beta), beta.stride(0),
             nv.ptr(state), nv.ptr(runs), n_runs, nv.ptr(o), nv.ptr(ws), T, H, G, D, Dv, nv.stream())
