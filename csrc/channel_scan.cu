@@ -13,13 +13,14 @@
 //   pass 1  every tile but a run's last forms its local state (from zero) and the product of its decays,
 //   carry   per element of S, the tiles of a run are chained: incoming state of tile j + 1 = decay_j * incoming_j + local_j,
 //   pass 2  every tile is walked again from its incoming state and writes its outputs; the last one leaves the run's state.
-// Runs of at most one tile (decode batches, short pieces) take pass 0: one walk from and to the state row.
+// Runs of at most one tile (decode batches, short pieces) take pass 0: one walk from and to the state row. Passes 1 and 2 of square states (64 or
+// 128) on whole vectors go by products of matrices (channel_tile_kernel), other sizes token by token.
 //
 // Columns of S are independent. A thread owns R rows of CPT columns, LPC lanes share a column and reduce their parts of an
 // output by shuffles (each step halves the columns a lane still carries), a CTA owns a block of columns of one (run or tile,
 // head). k, q, g and v of a chunk of tokens are staged through shared memory by cp.async, one chunk ahead.
 #include "common.cuh"
-#include "mma_sync.cuh"
+#include "split_mma.cuh"
 #include "../include/b200_ops.h"
 
 namespace b200 {
@@ -290,6 +291,275 @@ channel_scan_kernel(const ChannelScanArgs a) {
   }
 }
 
+// ---- tiles of a prompt by products of matrices: D = Dv, 64 or 128, 16-byte rows -------------------------------------------------
+// 16 tokens at a time. With A_i the decays' product over a block's tokens up to i (bonus: up to the one before), B_j that over those after j
+// and E that over all 16, per key channel,
+//   o_i = (A_i q_i)^T S + sum_(j <= i) W_ij v_j ,  W_ij = sum_d q_id k_jd prod_(j < s <= i) g_sd (bonus: s < i, and u_d for j = i) ,
+//   S <- diag(E) S + sum_j (B_j k_j) v_j^T ,
+// where every decay is a product of those a walk multiplies too: nothing is divided, and products that underflow do so in a walk as well.
+// W is formed by the threads that have the block's q, k and g in registers (two channels each), 120 products running down its columns and nine
+// sums over a warp; the rest are products on mma.sync in split bf16 (split_mma.cuh), transposed: 16 columns of S are a warp's 16 rows,
+// the state's rows its accumulators, which are an operand of the next product as they lie. The other operand, A q and B k, is split once
+// for all columns and read in the order of its lanes.
+// A tile with an infinity or NaN, or a product that grows to one, is walked (walk_tile): a product with W's zeros would carry it to tokens before its
+// own.
+// Bound: the issue slots, which mma.sync and the splits share (split_mma.cuh): of pass 2's 26 000 cycles a tile and head 11 500 are mma.sync, 2800 splits of S,
+// 3500 W; pass 1 reads and writes 1.2 TB/s beside it. Two CTAs per SM by registers. Passes 1 / 2, token by token before: 2345 tokens in
+// three runs, 16 heads of 128 with a bonus 75 + 146 -> 54 + 104 us (all of the mixer 257 -> 204); 790 tokens, 32 heads of 64: 99 -> 68. Error
+// against 64 bits, 500 tokens, decays in 0.9 .. 1 / 0.99 .. 1: state 8.2e-8 / 1.9e-7 (walk 8.6e-8 / 2.3e-7), outputs 1.2e-7 / 1.8e-7 (1.2e-7 / 2.2e-7).
+template <int D> struct TileSmem {                        // offsets in 32-bit words
+  static constexpr int kWarps = D / 16, KS = D / 16, NT = D / 8, QS = 200, KT = 202, WR = 18;
+  static constexpr int E = 0, K = 4 * D, Q = K + 4 * NT * KT, W = Q + 8 * KS * QS, kBoth = W + (D / 64) * 64 * WR, kFirst = K + 4 * NT * KT;
+  static constexpr int kWalk = D * D + 2 * D;
+  static constexpr int bytes(int pass) { return (pass == 1 ? (kFirst > kWalk ? kFirst : kWalk) : (kBoth > kWalk ? kBoth : kWalk)) * 4; }
+};
+
+// 16 values a lane, summed over the warp: lane l keeps the sum of value l / 2
+__device__ __forceinline__ float gather16(float (&v)[16], int lane) {
+#pragma unroll
+  for (int w = 8; w >= 1; w >>= 1) {
+    const bool up = lane & (2 * w);
+#pragma unroll
+    for (int i = 0; i < w; ++i) {
+      const float mine = up ? v[w + i] : v[i], theirs = up ? v[i] : v[w + i];
+      v[i] = mine + __shfl_xor_sync(0xffffffffu, theirs, 2 * w);
+    }
+  }
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+// Tokens [c0, n) of a tile one by one, from the S [D][D] in shared memory
+template <int PASS, int D, bool BONUS>
+__device__ __noinline__ void walk_tile(const ChannelScanArgs& a, float* S, int h, int first, int c0, int n) {
+  const int e = threadIdx.x % D, half = threadIdx.x / D, kvh = h / (a.H / a.G);
+  float* red = S + D * D;
+  for (int t = c0; t < n; ++t) {
+    const long long row = first + t;
+    const float *k = a.k + row * a.ldk + (long long)kvh * D, *q = a.q + row * a.ldq + (long long)kvh * D, *g = a.g + row * a.ldg + (long long)h * D;
+    const float v = a.v[row * a.ldv + (long long)h * D + e];
+    float o = 0.f;
+    for (int d = half * (D / 2); d < (half + 1) * (D / 2); ++d) {
+      const float s = S[d * D + e], kv = k[d] * v;
+      if (PASS != 1 && BONUS) o = fmaf(fmaf(a.u[h * D + d], kv, s), q[d], o);
+      const float x = fmaf(g[d], s, kv);
+      if (PASS != 1 && !BONUS) o = fmaf(x, q[d], o);
+      S[d * D + e] = x;
+    }
+    if (PASS == 1) continue;
+    red[half * D + e] = o;
+    __syncthreads();
+    if (half == 0) a.o[(row * a.H + h) * D + e] = red[e] + red[D + e];
+    __syncthreads();
+  }
+  __syncthreads();
+}
+
+template <int PASS, int D, bool BONUS>
+__global__ void __launch_bounds__(TileSmem<D>::kWarps * 32, D == 64 ? 3 : 2)
+channel_tile_kernel(const ChannelScanArgs a) {
+  using L = TileSmem<D>;
+  constexpr int KS = L::KS, NT = L::NT;
+  extern __shared__ __align__(16) float sm[];
+  uint32_t* smw = reinterpret_cast<uint32_t*>(sm);
+  const int b_ = blockIdx.x, h = blockIdx.y, kvh = h / (a.H / a.G);
+  const int place = a.tile_of[4 * b_ + 1], count = a.tile_of[4 * b_ + 2];
+  if (PASS == 1 && place + 1 == count) return;           // nobody asks for the last tile's local state
+  const int first = a.tiles[4 * b_], n = a.tiles[4 * b_ + 1], slot = a.tiles[4 * b_ + 3];
+  const bool keep = PASS == 1 || place + 1 == count;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t2 = (lane & 3) * 2;
+  float* part = a.part + ((long long)b_ * a.H + h) * D * D;
+  float* dst = PASS == 1 ? part : a.state + ((long long)slot * a.H + h) * D * D;
+
+  float S[NT][4];                                         // S^T: columns 16 warp + g and + 8 of the state's rows 8 j + t2, + 1
+  auto each = [&](auto f) {
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int x = 0; x < 4; ++x) f(S[j][x], (8 * j + t2 + (x & 1)) * D + warp * 16 + g + (x >> 1) * 8);
+  };
+  float dec = 1.f;                                        // pass 1: the tile's decay product of channel tid
+  for (int c0 = 0; c0 < n; c0 += 64) {
+    const int cn = min(64, n - c0);
+    int odd = 0;
+    // ---- this thread's two channels of one block of 16 tokens ----
+    {
+      const int blk = tid / (D / 2), c = tid % (D / 2);
+      float2 gg[16], kk[16], qq[PASS == 1 ? 1 : 16];
+      const long long row0 = first + c0 + blk * 16;
+      const float* gp = a.g + row0 * a.ldg + (long long)h * D + 2 * c;
+      const float* kp = a.k + row0 * a.ldk + (long long)kvh * D + 2 * c;
+      const float* qp = a.q + row0 * a.ldq + (long long)kvh * D + 2 * c;
+#pragma unroll
+      for (int x = 0; x < 16; ++x) {
+        const bool live = blk * 16 + x < cn;
+        gg[x] = live ? *reinterpret_cast<const float2*>(gp + x * a.ldg) : make_float2(1.f, 1.f);
+        kk[x] = live ? *reinterpret_cast<const float2*>(kp + x * a.ldk) : make_float2(0.f, 0.f);
+        if (PASS != 1) qq[PASS == 1 ? 0 : x] = live ? *reinterpret_cast<const float2*>(qp + x * a.ldq) : make_float2(0.f, 0.f);
+      }
+      if constexpr (PASS != 1) {
+        float* Ws = sm + L::W + ((c >> 5) * 4 + blk) * 16 * L::WR;       // each warp of a block its sums
+        float v[16];
+        const float2 u = BONUS ? *reinterpret_cast<const float2*>(a.u + h * D + 2 * c) : make_float2(1.f, 1.f);
+#pragma unroll
+        for (int x = 0; x < 16; ++x) v[x] = fmaf(qq[x].x * u.x, kk[x].x, qq[x].y * u.y * kk[x].y);
+        float w = gather16(v, lane);
+        const int s = lane >> 1;
+        odd |= not_finite(w);
+        if (!(lane & 1)) Ws[s * L::WR + s] = w;
+        // columns j and 15 - j of W together: 15 - j and j elements below the diagonal
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          v[j] = 0.f;
+          float2 p = kk[j];
+#pragma unroll
+          for (int i = j + 1; i < 16; ++i) {
+            if (!BONUS) p = __fmul2_rn(p, gg[i]);
+            v[i] = fmaf(qq[i].x, p.x, qq[i].y * p.y);
+            if (BONUS) p = __fmul2_rn(p, gg[i]);
+          }
+          p = kk[15 - j];
+#pragma unroll
+          for (int i = 16 - j; i < 16; ++i) {
+            if (!BONUS) p = __fmul2_rn(p, gg[i]);
+            v[i - 16 + j] = fmaf(qq[i].x, p.x, qq[i].y * p.y);
+            if (BONUS) p = __fmul2_rn(p, gg[i]);
+          }
+          w = gather16(v, lane);
+          odd |= not_finite(w);
+          if (!(lane & 1) && s != j) Ws[s > j ? s * L::WR + j : (16 - j + s) * L::WR + 15 - j] = w;
+        }
+        // A q: pairs of channels of a token
+        uint32_t* Qs = smw + L::Q + (blk * 2 * KS + (c >> 3)) * L::QS + (c & 3) * 2 + ((c >> 2) & 1);
+        float2 p = make_float2(1.f, 1.f);
+#pragma unroll
+        for (int x = 0; x < 16; ++x) {
+          if (!BONUS) p = __fmul2_rn(p, gg[x]);
+          const float2 y = __fmul2_rn(qq[x], p);
+          if (BONUS) p = __fmul2_rn(p, gg[x]);
+          odd |= not_finite(y.x) | not_finite(y.y);
+          uint32_t* at = Qs + (x >> 3) * KS * L::QS + (x & 7) * 8;
+          split3(y.x, y.y, at[0], at[64], at[128]);
+        }
+      }
+      // B k: pairs of tokens of a channel
+      uint32_t* Kb = smw + L::K + (blk * NT + (c >> 2)) * L::KT + (c & 3) * 16;
+      float2 p = make_float2(1.f, 1.f);
+#pragma unroll
+      for (int x = 14; x >= 0; x -= 2) {
+        const float2 y1 = __fmul2_rn(kk[x + 1], p);
+        p = __fmul2_rn(p, gg[x + 1]);
+        const float2 y0 = __fmul2_rn(kk[x], p);
+        p = __fmul2_rn(p, gg[x]);
+        odd |= not_finite(y0.x) | not_finite(y0.y) | not_finite(y1.x) | not_finite(y1.y);
+        uint32_t* at = Kb + ((x >> 1) & 3) * 2 + (x >> 3);
+        split3(y0.x, y1.x, at[0], at[64], at[128]);
+        split3(y0.y, y1.y, at[8], at[72], at[136]);
+      }
+      odd |= not_finite(p.x) | not_finite(p.y);
+      *reinterpret_cast<float2*>(sm + L::E + blk * D + 2 * c) = p;
+    }
+    // the values: 16 columns of this warp
+    const float* vp = a.v + (long long)(first + c0) * a.ldv + (long long)h * D + warp * 16 + g;
+    auto value = [&](int t, int hi) { return t < cn ? vp[(long long)t * a.ldv + hi * 8] : 0.f; };
+    each([&](float& s, int at) { s = PASS == 1 && c0 == 0 ? 0.f : part[at]; });
+    __syncthreads();
+    const float before = dec;
+    if (PASS == 1 && tid < D) dec *= (sm[L::E + tid] * sm[L::E + D + tid]) * (sm[L::E + 2 * D + tid] * sm[L::E + 3 * D + tid]);
+    const int nb = (cn + 15) / 16;
+#pragma unroll 1
+    for (int blk = 0; blk < nb; ++blk) {
+      SplitA va;
+      {
+        const int t = blk * 16 + t2;
+        split3(value(t, 0), value(t + 1, 0), va.p[0][0], va.p[1][0], va.p[2][0]);
+        split3(value(t, 1), value(t + 1, 1), va.p[0][1], va.p[1][1], va.p[2][1]);
+        split3(value(t + 8, 0), value(t + 9, 0), va.p[0][2], va.p[1][2], va.p[2][2]);
+        split3(value(t + 8, 1), value(t + 9, 1), va.p[0][3], va.p[1][3], va.p[2][3]);
+      }
+      auto load_b = [&](const uint32_t* at) {
+        SplitB b;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          const uint2 v = *reinterpret_cast<const uint2*>(at + i * 64 + lane * 2);
+          b.p[i][0] = v.x; b.p[i][1] = v.y;
+        }
+        return b;
+      };
+      if (PASS != 1) {
+        SplitAcc oa[2];
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          float w[4];
+          const int i = 8 * m + g;
+#pragma unroll
+          for (int x = 0; x < 4; ++x) {                   // W_ij of token i, j = t2, t2 + 1, t2 + 8, t2 + 9
+            const int j = t2 + (x & 1) + (x >> 1) * 8;
+            const float* at = sm + L::W + (blk * 16 + i) * L::WR + j;
+            w[x] = j > i ? 0.f : (D == 128 ? at[0] + at[64 * L::WR] : at[0]);
+          }
+          mma_split<true>(va, split_b(w[0], w[1], w[2], w[3]), oa[m]);
+        }
+#pragma unroll
+        for (int s = 0; s < KS; ++s) {
+          SplitA sa;
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            split3(S[2 * s + j][0], S[2 * s + j][1], sa.p[0][2 * j], sa.p[1][2 * j], sa.p[2][2 * j]);
+            split3(S[2 * s + j][2], S[2 * s + j][3], sa.p[0][2 * j + 1], sa.p[1][2 * j + 1], sa.p[2][2 * j + 1]);
+          }
+#pragma unroll
+          for (int m = 0; m < 2; ++m) mma_split(sa, load_b(smw + L::Q + ((blk * 2 + m) * KS + s) * L::QS), oa[m]);
+        }
+        float* orow = a.o + ((long long)(first + c0 + blk * 16) * a.H + h) * D + warp * 16 + g;
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+          for (int x = 0; x < 4; ++x) {
+            const int t = 8 * m + t2 + (x & 1);
+            const float o = oa[m].sum(x);
+            odd |= not_finite(o);
+            if (blk * 16 + t < cn) orow[(long long)t * a.H * D + (x >> 1) * 8] = o;
+          }
+      }
+      if (!keep && c0 + (blk + 1) * 16 >= n) break;       // nobody asks for this state
+#pragma unroll
+      for (int j = 0; j < NT; ++j) {
+        SplitAcc sa;
+        mma_split<true>(va, load_b(smw + L::K + (blk * NT + j) * L::KT), sa);
+        const float2 e = *reinterpret_cast<const float2*>(sm + L::E + blk * D + 8 * j + t2);
+#pragma unroll
+        for (int x = 0; x < 4; ++x) S[j][x] = fmaf(x & 1 ? e.y : e.x, S[j][x], sa.sum(x));
+      }
+    }
+    if (keep) each([&](float& s, int) { odd |= not_finite(s); });
+    if (__syncthreads_or(odd)) {                          // from the state in front of these tokens, which still lies there, again
+      each([&](float&, int at) { sm[at] = PASS == 1 && c0 == 0 ? 0.f : part[at]; });
+      if (PASS == 1 && tid < D) {
+        dec = before;
+        for (int t = c0; t < n; ++t) dec *= a.g[(long long)(first + t) * a.ldg + (long long)h * D + tid];
+        a.pdec[((long long)b_ * a.H + h) * D + tid] = dec;
+      }
+      __syncthreads();
+      walk_tile<PASS, D, BONUS>(a, sm, h, first, c0, n);
+      if (keep)
+        for (int i = tid; i < D * D; i += L::kWarps * 32) dst[i] = sm[i];
+      return;
+    }
+    if (c0 + 64 < n) each([&](float& s, int at) { part[at] = s; });       // a longer tile: its state waits where it came from
+  }
+  if (keep) each([&](float& s, int at) { dst[at] = s; });
+  if (PASS == 1 && tid < D) a.pdec[((long long)b_ * a.H + h) * D + tid] = dec;
+}
+
+template <int PASS, int D, bool BONUS>
+static int launch_tiles(const ChannelScanArgs& a, int n_tiles, cudaStream_t st) {
+  auto kern = channel_tile_kernel<PASS, D, BONUS>;
+  constexpr int smem = TileSmem<D>::bytes(PASS);
+  B200_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  kern<<<dim3(n_tiles, a.H), TileSmem<D>::kWarps * 32, smem, st>>>(a);
+  return 0;
+}
+
 // Chains the tiles of every run: part[tile] (local state) becomes the tile's incoming state. A thread owns V neighbouring
 // elements of one head's state; the loads do not depend on the chain, so four tiles are in flight.
 template <int V>
@@ -514,13 +784,18 @@ B200_API int b200_channel_scan(const float* q, long long ldq, const float* k, lo
   if (n_tiles <= 0) {
     CS_L(0, n_runs);
   } else {
-    CS_L(1, n_tiles);
+    // runs of several tiles where a head's state is square and rows are whole vectors: by products; else token by token
+    const bool mat = (D == 64 || D == 128) && Dv == D && a.vec && a.vecv && (!u || al(u, 4));
+    if (mat) { if (int rc = D == 64 ? launch_tiles<1, 64, false>(a, n_tiles, st) : launch_tiles<1, 128, false>(a, n_tiles, st)) return rc; }
+    else CS_L(1, n_tiles);
     const int V = Dv % 4 == 0 && al(part, 4) ? 4 : 1;
     const long long n = (long long)D * Dv / V;
     dim3 grid((unsigned)((n + 127) / 128), H, n_runs);
     if (V == 4) channel_scan_carry_kernel<4><<<grid, 128, 0, st>>>(part, pdec, state, runs, run_tiles, H, D, Dv);
     else channel_scan_carry_kernel<1><<<grid, 128, 0, st>>>(part, pdec, state, runs, run_tiles, H, D, Dv);
-    CS_L(2, n_tiles);
+    if (!mat) CS_L(2, n_tiles);
+    else if (int rc = D == 64 ? (u ? launch_tiles<2, 64, true>(a, n_tiles, st) : launch_tiles<2, 64, false>(a, n_tiles, st))
+                              : (u ? launch_tiles<2, 128, true>(a, n_tiles, st) : launch_tiles<2, 128, false>(a, n_tiles, st))) return rc;
   }
 #undef CS_L
 #undef CS_B
