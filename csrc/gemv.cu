@@ -521,6 +521,7 @@ w4_units_kernel(const GemvParams p, const int split) {
   const int T = (int)((ntiles - 1 - cl) / ncl) + 1;       // the grid has no more clusters than tiles
   const int upt = (cnt + 3) / 4;                          // units of a tile
   const long long U = (long long)T * upt;
+  const int dt = kWsWarps / upt, dp = kWsWarps % upt;     // a round further: tiles and units of one (no division per unit)
   const int gpr = p.K / p.group;
   const bool sv = p.group == 128 && gpr % 4 == 0 &&
                   !((reinterpret_cast<uintptr_t>(p.scale) | reinterpret_cast<uintptr_t>(p.zs)) & 15);
@@ -543,9 +544,12 @@ w4_units_kernel(const GemvParams p, const int split) {
   uint4 wa[4], wb[4];
   const uint8_t *pa = nullptr, *pb = nullptr;             // rows g and g + 8 of the next unit
   int left = 0;                                           // and the chunks it has
-  auto aim = [&](long long u, int buf) {
-    const int tl = (int)(u / upt), c = (int)(u - (long long)tl * upt) * 4;
-    const long long row0 = (cl + (long long)tl * ncl) * 16;
+  int tl_next = warp / upt, part_next = warp % upt;       // the unit to ask for
+  auto aim = [&](int buf) {
+    const int c = part_next * 4;
+    const long long row0 = (cl + (long long)tl_next * ncl) * 16;
+    tl_next += dt; part_next += dp;
+    if (part_next >= upt) { part_next -= upt; ++tl_next; }
     const uint8_t* w = reinterpret_cast<const uint8_t*>(p.w) + (c0 + c) * 64 + t * 16;
     pa = w + min(row0 + g, p.N - 1) * (p.K / 2);
     pb = w + min(row0 + g + 8, p.N - 1) * (p.K / 2);
@@ -556,8 +560,9 @@ w4_units_kernel(const GemvParams p, const int split) {
     *reinterpret_cast<float4*>(scales + lane * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
     *reinterpret_cast<float4*>(scales + 128 + lane * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
   }
+  int part = part_next;                                   // of this warp's unit in its tile
   if (warp < U) {
-    aim(warp, 0);
+    aim(0);
 #pragma unroll
     for (int j = 0; j < 4; ++j)
       if (j < left) { wa[j] = ld_nc_v4(pa + j * 64); wb[j] = ld_nc_v4(pb + j * 64); }
@@ -565,33 +570,39 @@ w4_units_kernel(const GemvParams p, const int split) {
   cp_async_commit();
 
   // ---- the activations of this CTA's chunks, and their sums
-  for (int u = warp; u < cnt * TG; u += kWsWarps) {
-    const int c = u / TG, tok = (u - c * TG) * 8 + g;
-    uint4 v[4];
+  // two chunks of a warp's at a time: a trip to memory each
+  for (int u0 = warp; u0 < cnt * TG; u0 += 2 * kWsWarps) {
+    uint4 v[2][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] = make_uint4(0, 0, 0, 0);
-    if (tok < p.M) {
+    for (int b = 0; b < 2; ++b) {
+      const int u = u0 + b * kWsWarps, c = u / TG, tok = (u - c * TG) * 8 + g;
       const uint4* px = reinterpret_cast<const uint4*>(p.x + (long long)tok * p.x_rs + (c0 + c) * 128 + t * 32);
+      const bool live = u < cnt * TG && tok < p.M;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) v[i] = __ldg(px + i);
+      for (int i = 0; i < 4; ++i) v[b][i] = live ? __ldg(px + i) : make_uint4(0, 0, 0, 0);
     }
-    float s = 0.f;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint32_t w[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+    for (int b = 0; b < 2; ++b) {
+      const int u = u0 + b * kWsWarps;
+      if (u >= cnt * TG) break;
+      float s = 0.f;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        float2 f;
-        if (BF16) f = unpack_bf16x2(w[j]);
-        else f = __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
-        s += f.x + f.y;
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t w[4] = {v[b][i].x, v[b][i].y, v[b][i].z, v[b][i].w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float2 f;
+          if (BF16) f = unpack_bf16x2(w[j]);
+          else f = __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
+          s += f.x + f.y;
+        }
+        *reinterpret_cast<uint4*>(xs + ((u * 4 + i) * 32 + lane) * 16) =
+            make_uint4(__byte_perm(w[0], w[2], 0x5410), __byte_perm(w[0], w[2], 0x7632), __byte_perm(w[1], w[3], 0x5410), __byte_perm(w[1], w[3], 0x7632));
       }
-      *reinterpret_cast<uint4*>(xs + ((u * 4 + i) * 32 + lane) * 16) =
-          make_uint4(__byte_perm(w[0], w[2], 0x5410), __byte_perm(w[0], w[2], 0x7632), __byte_perm(w[1], w[3], 0x5410), __byte_perm(w[1], w[3], 0x7632));
+      s += __shfl_xor_sync(0xffffffffu, s, 1);
+      s += __shfl_xor_sync(0xffffffffu, s, 2);
+      if (t == 0) xsum[u * 8 + g] = s;
     }
-    s += __shfl_xor_sync(0xffffffffu, s, 1);
-    s += __shfl_xor_sync(0xffffffffu, s, 2);
-    if (t == 0) xsum[u * 8 + g] = s;
   }
   __syncthreads();
 
@@ -599,7 +610,7 @@ w4_units_kernel(const GemvParams p, const int split) {
   asm volatile("" : "+r"(magic), "+r"(mask));            // both stay in registers (one LOP3 per pair of codes)
   const float b0 = (BF16 ? 128.f : 1024.f) + p.lin_off;
   const int rounds = (int)((U + kWsWarps - 1) / kWsWarps);
-  int part = warp % upt;                                  // of this warp's unit in its tile
+  int tl0 = 0, up0 = 0;                                   // of the round's first unit
   for (int rd = 0; rd < rounds; ++rd) {
     const long long u = (long long)rd * kWsWarps + warp;
     float* rb = red + (rd & 1) * kWsWarps * TG * 128;     // the other buffer may still be read
@@ -614,7 +625,8 @@ w4_units_kernel(const GemvParams p, const int split) {
       *reinterpret_cast<float4*>(zb) = *reinterpret_cast<const float4*>(sc + g * 4 + 96);
       const int c = part * 4, here = cnt - c;
       left = 0;
-      if (u + kWsWarps < U) aim(u + kWsWarps, (rd + 1) & 1);
+      const int next = part_next;
+      if (u + kWsWarps < U) aim((rd + 1) & 1);
       cp_async_commit();
       float sum[TG][4];
 #pragma unroll
@@ -656,7 +668,7 @@ w4_units_kernel(const GemvParams p, const int split) {
           }
         }
       }
-      part = (part + kWsWarps) % upt;
+      part = next;
 #pragma unroll
       for (int tg = 0; tg < TG; ++tg)
         *reinterpret_cast<float4*>(rb + (warp * TG + tg) * 128 + lane * 4) = make_float4(sum[tg][0], sum[tg][1], sum[tg][2], sum[tg][3]);
@@ -667,7 +679,7 @@ w4_units_kernel(const GemvParams p, const int split) {
     if (e >= 0 && e < TG * 128) {
       const long long u0 = (long long)rd * kWsWarps;
       const int n = (int)min((long long)kWsWarps, U - u0);
-      int tl = (int)(u0 / upt), up = (int)(u0 - (long long)tl * upt);
+      int tl = tl0, up = up0;
       float s = up ? carry[e] : 0.f;
       float v[kWsWarps];
 #pragma unroll
@@ -685,6 +697,8 @@ w4_units_kernel(const GemvParams p, const int split) {
       }
       carry[e] = s;
     }
+    tl0 += dt; up0 += dp;
+    if (up0 >= upt) { up0 -= upt; ++tl0; }
   }
   if (split == 1) return;
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
