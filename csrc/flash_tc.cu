@@ -3,7 +3,8 @@
 // row (TMEM lane = row, so row max and row sum need no shuffles).
 //
 //   CTA = 128 query rows; 256 threads: warps 0-3 softmax, warp 4 TMA producer, warp 5 tcgen05 issuer (the whole warp runs the
-//   issue loop, elect.sync picks the lane).
+//   issue loop, elect.sync picks the lane); where a CTA goes on from tile to tile (RUN below), warp 6 finds the next one and warp 7
+//   writes results out.
 //   TMEM (256 columns, two CTAs per SM): S(even j) [0, 64), S(odd j) [64, 128), O [128, 128 + D).
 //   per 64-key block j:   S_j = Q K_j^T          (M 128 x N 64 x K D), issued one block AHEAD of the softmax
 //                         softmax warps: tcgen05.ld S_j (64 registers), running max, P = exp2(S c - m c) -> 16 bit,
@@ -26,7 +27,7 @@
 //
 // Takes the place of the mma.sync kernels of flash_attn.cu (other head sizes, other scales and dropout stay there) and
 // multimap_attn_mma.cu (other sizes, two maps). Measured against them, bf16: six packed prompts of 77 - 2048 tokens, 32 / 8 heads
-// of 128: 237 -> 107 us, 16 / 8 heads of 64: 86 -> 51; pages of 64, 16 / 4 heads of 128, pieces of 2048 and 700 (at 512) tokens beside
+// of 128: 237 -> 103 us, 16 / 8 heads of 64: 86 -> 51; pages of 64, 16 / 4 heads of 128, pieces of 2048 and 700 (at 512) tokens beside
 // two that decode: 171 -> 57 us, window of 1024: 128 -> 42, chunks with capped scores: 194 -> 80; eight packed prompts of 30 - 250
 // tokens (fp16): 19.1 -> 16.4.
 // Reference call sites: SDPA behind nn.MultiheadAttention (LLM_Distributed_Trainning/PyTorch/ddp_basics/ddp_gpt_wikitext2.py:89-96),
@@ -51,7 +52,7 @@ enum { kTcDense = 0, kTcVarlen = 1, kTcPaged = 2 };
 template <int D> struct TcSmem {
   static constexpr uint32_t kHalves = D / 64, kStage = 8192 * kHalves;
   static constexpr int NK = D == 64 ? 4 : 3, NV = D == 64 ? 4 : 2;      // two CTAs fit an SM
-  static constexpr uint32_t kQ = 0, kK = 16384 * kHalves, kV = kK + NK * kStage, kBar = kV + NV * kStage, kBytes = kBar + 192;
+  static constexpr uint32_t kQ = 0, kK = 16384 * kHalves, kV = kK + NK * kStage, kBar = kV + NV * kStage, kBytes = kBar + 512;
 };
 
 struct FlashTcParams {
@@ -126,10 +127,17 @@ __device__ __forceinline__ float tanh_small(float x) {
 }
 __device__ __forceinline__ float tanh_any(float x) { return 1.f - __fdividef(2.f, 1.f + ex2f(x * 2.8853900817779268f)); }
 
-template <int MODE, int D, bool BF16, bool CAP>
+// RUN: a CTA goes on to the tiles of CTAs that have not started (clusterlaunchcontrol). The next tile's Q and keys come, and its first scores are taken,
+// while the softmax warps finish the one before; a warp of its own writes that out by TMA. Set-up, the wait for the first scores and the
+// end were 13 000 of a CTA's 26 000 cycles for sequences of 512 (8000 or 4600 of them the wait, in the first round and after it). One tile to a CTA
+// before: 4 x 512, 40 / 8 heads of 128: packed 37.9 -> 33.9 us, dense with its backward 115 -> 113; six packed prompts of 77 to 2048
+// tokens, 32 / 8 heads: 106 -> 102 (99 where the SM clock held); eleven of 17 to 1000, 40 / 8 heads: 52 -> 46; eight of 1000, 16 heads of 64: 59 -> 56; one of 4096
+// or 8192: the same. A piece of a paged prompt starts with its page numbers either way and gained nothing (102 us for 5596 tokens), with capped scores
+// it lost a fifth to registers spilled in the loop; so pieces, and calls that are resident at once, keep a tile to a CTA.
+template <int MODE, int D, bool BF16, bool CAP, bool RUN>
 __global__ void __launch_bounds__(kTcThreads, 2)
 flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
-                    const FlashTcParams p) {
+                    const __grid_constant__ CUtensorMap to, const FlashTcParams p) {
   using L = TcSmem<D>;
   constexpr int kHalves = L::kHalves, NK = L::NK, NV = L::NV;
   // How far a row's maximum may run ahead of the one its weights refer to before O is scaled (an exponent of two). With none the largest
@@ -142,84 +150,96 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
   const uint32_t sbase = smem_u32(smem_tc);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-  // ---- where this CTA's rows and keys are ----
-  int h = blockIdx.y, b = 0, hk, row_base, q0, limit;           // limit: keys of the sequence; q0: position of row 0; row_base: its row 0
-  int nit, nA = 0, bB = 0;                                // key blocks: [0, nA), then bB, bB + 1, ...
-  int nrows = kTcBM, low_max = 0, keepW = 0;
-  bool solo = false;                                      // paged: the second half of the rows is the same head's next tile
-  const int* trow = nullptr;
+  // ---- a tile: its rows and keys ----
+  struct Tile {
+    int h, b, hk, row_base, q0, limit;                    // limit: keys of the sequence; q0: position of row 0; row_base: its row 0
+    int nit, nA, bB;                                      // key blocks: [0, nA), then bB, bB + 1, ...; nit 0: no tile any more
+    int nrows, low_max, slot;                             // paged
+  };
+  const int keepW = MODE == kTcPaged && p.window > 0 ? max(p.keep_first, 0) : 0;
+  const bool solo = MODE == kTcPaged && ((p.H / p.Hkv) & 1);              // paged: the second half of the rows is the same head's next tile
   auto low_of = [&](int pos) {
     return p.opt.chunk > 0 ? pos / p.opt.chunk * p.opt.chunk : (p.window > 0 ? max(0, pos + 1 - p.window) : 0);
   };
-  if (MODE == kTcPaged) {
-    const int tile = (int)gridDim.x - 1 - (int)blockIdx.x, rep = p.H / p.Hkv;
-    const int* tl = p.tiles + 4 * tile;
-    row_base = tl[0]; nrows = tl[1]; q0 = tl[2];
-    solo = rep & 1;
-    if (solo) {
-      const int place = p.tile_of[4 * tile + 1];
-      if (place & 1) return;                              // the tile before it takes both
-      if (place + 1 < p.tile_of[4 * tile + 2]) nrows += tl[5];
-      hk = h / rep;
-    } else {
-      hk = h / (rep / 2);
-      h *= 2;
-    }
-    trow = p.table + (long long)tl[3] * p.max_blocks;
-    limit = q0 + nrows;
-    const int lo0 = low_of(q0);
-    keepW = p.window > 0 ? max(p.keep_first, 0) : 0;
-    nA = (min(keepW, lo0) + kTcBN - 1) / kTcBN;
-    bB = max(lo0 / kTcBN, nA);
-    nit = nA + (limit + kTcBN - 1) / kTcBN - bB;
-    low_max = low_of(q0 + (solo ? kTcBM : kTcBN) - 1);
-  } else {
-    // Heavy (late) query tiles of all heads and sequences first, or of a group of heads (see head_group): under the causal mask tile t has
-    // t + 1 times the work of tile 0, and the short ones fill the end.
-    int qt;
-    if (p.group == 0) {
-      h = blockIdx.x; b = blockIdx.y;
-      qt = (int)gridDim.z - 1 - (int)blockIdx.z;
-    } else {
-      int x = blockIdx.x;
-      qt = (p.S + kTcBM - 1) / kTcBM - 1 - (int)blockIdx.y;
-      if (qt >= kTcGridY) {                               // more tiles than the second dimension holds: the first takes the rest
-        qt -= x / p.group * kTcGridY;
-        x %= p.group;
+  // the tile that a CTA with this index is for; false: none (a sequence's end, the half of a pair that its other half takes)
+  auto tile_of = [&](int bx, int by, int bz, Tile& t) {
+    t.h = by; t.b = 0; t.nA = t.bB = 0; t.nrows = kTcBM; t.low_max = 0; t.slot = 0;
+    if (MODE == kTcPaged) {
+      const int tile = (int)gridDim.x - 1 - bx, rep = p.H / p.Hkv;
+      const int* tl = p.tiles + 4 * tile;
+      t.row_base = tl[0]; t.nrows = tl[1]; t.q0 = tl[2];
+      if (solo) {
+        const int place = p.tile_of[4 * tile + 1];
+        if (place & 1) return false;                      // the tile before it takes both
+        if (place + 1 < p.tile_of[4 * tile + 2]) t.nrows += tl[5];
+        t.hk = t.h / rep;
+      } else {
+        t.hk = t.h / (rep / 2);
+        t.h *= 2;
       }
-      const int hb = (int)blockIdx.z * p.group + x;
-      b = p.H == 1 ? hb : (int)__umulhi((unsigned)hb, p.h_inv);
-      if (b >= p.B || qt < 0) return;
-      h = hb - b * p.H;
+      t.slot = tl[3];
+      t.limit = t.q0 + t.nrows;
+      const int lo0 = low_of(t.q0);
+      t.nA = (min(keepW, lo0) + kTcBN - 1) / kTcBN;
+      t.bB = max(lo0 / kTcBN, t.nA);
+      t.nit = t.nA + (t.limit + kTcBN - 1) / kTcBN - t.bB;
+      t.low_max = low_of(t.q0 + (solo ? kTcBM : kTcBN) - 1);
+    } else {
+      // Heavy (late) query tiles of all heads and sequences first, or of a group of heads (see head_group): under the causal mask tile t has
+      // t + 1 times the work of tile 0, and the short ones fill the end.
+      int qt;
+      if (p.group == 0) {
+        t.h = bx; t.b = by;
+        qt = (int)gridDim.z - 1 - bz;
+      } else {
+        int x = bx;
+        qt = (p.S + kTcBM - 1) / kTcBM - 1 - by;
+        if (qt >= kTcGridY) {                             // more tiles than the second dimension holds: the first takes the rest
+          qt -= x / p.group * kTcGridY;
+          x %= p.group;
+        }
+        const int hb = bz * p.group + x;
+        t.b = p.H == 1 ? hb : (int)__umulhi((unsigned)hb, p.h_inv);
+        if (t.b >= p.B || qt < 0) return false;
+        t.h = hb - t.b * p.H;
+      }
+      t.hk = t.h / (p.H / p.Hkv);
+      t.row_base = MODE == kTcVarlen ? p.cu[t.b] : t.b * p.S;
+      t.limit = MODE == kTcVarlen ? p.cu[t.b + 1] - t.row_base : p.S;
+      t.q0 = qt * kTcBM;
+      if (MODE == kTcVarlen && t.q0 >= t.limit) return false;
+      const int kv_end = p.causal ? min(t.limit, t.q0 + kTcBM) : t.limit;
+      t.nit = (kv_end + kTcBN - 1) / kTcBN;
     }
-    hk = h / (p.H / p.Hkv);
-    row_base = MODE == kTcVarlen ? p.cu[b] : b * p.S;
-    limit = MODE == kTcVarlen ? p.cu[b + 1] - row_base : p.S;
-    q0 = qt * kTcBM;
-    if (MODE == kTcVarlen && q0 >= limit) return;
-    const int kv_end = p.causal ? min(limit, q0 + kTcBM) : limit;
-    nit = (kv_end + kTcBN - 1) / kTcBN;
-  }
-  auto block_of = [&](int it) { return MODE == kTcPaged ? (it < nA ? it : bB + (it - nA)) : it; };
+    return true;
+  };
+  Tile t0;
+  if (!RUN && !tile_of(blockIdx.x, blockIdx.y, blockIdx.z, t0)) return;
 
   const uint32_t bar = sbase + L::kBar;
-  // P has two barriers: the softmax may be a block ahead of the issuing warp (S(j + 1) is asked for before V(j) and P(j) are waited for)
-  const uint32_t q_full = bar, s_full0 = bar + 8, p_full0 = bar + 24, o_done = bar + 40, tmem_slot = bar + 48;
-  auto k_full = [&](int j) { return bar + 56 + 8u * (j % NK); };
-  auto k_empty = [&](int j) { return bar + 56 + 8u * (NK + j % NK); };
-  auto v_full = [&](int j) { return bar + 56 + 8u * (2 * NK + j % NV); };
-  auto v_empty = [&](int j) { return bar + 56 + 8u * (2 * NK + NV + j % NV); };
-  auto k_phase = [&](int j) { return (uint32_t)(j / NK) & 1u; };
-  auto v_phase = [&](int j) { return (uint32_t)(j / NV) & 1u; };
-  auto k_at = [&](int j) { return sbase + L::kK + (uint32_t)(j % NK) * L::kStage; };
-  auto v_at = [&](int j) { return sbase + L::kV + (uint32_t)(j % NV) * L::kStage; };
+  // P has two barriers: the softmax may be a block ahead of the issuing warp (S(j + 1) is asked for before V(j) and P(j) are waited for).
+  // Blocks are counted through all tiles of the CTA (g): buffers, stages and phases go by that.
+  const uint32_t q_full = bar, q_empty = bar + 8, s_full0 = bar + 16, p_full0 = bar + 32, o_done = bar + 48, tmem_slot = bar + 56, st_free = bar + 64,
+                 tile_full0 = bar + 72, tile_empty0 = bar + 88, ask = bar + 104, clc = bar + 112, clc_at = bar + 256, o_staged = bar + 400;
+  auto k_full = [&](int j) { return bar + 120 + 8u * ((uint32_t)j % NK); };
+  auto k_empty = [&](int j) { return bar + 120 + 8u * (NK + (uint32_t)j % NK); };
+  auto v_full = [&](int j) { return bar + 120 + 8u * (2 * NK + (uint32_t)j % NV); };
+  auto v_empty = [&](int j) { return bar + 120 + 8u * (2 * NK + NV + (uint32_t)j % NV); };
+  auto k_phase = [&](int j) { return ((uint32_t)j / NK) & 1u; };
+  auto v_phase = [&](int j) { return ((uint32_t)j / NV) & 1u; };
+  auto k_at = [&](int j) { return sbase + L::kK + ((uint32_t)j % NK) * L::kStage; };
+  auto v_at = [&](int j) { return sbase + L::kV + ((uint32_t)j % NV) * L::kStage; };
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tq);
+    if (RUN) tma_prefetch_desc(&to);
     if (MODE == kTcPaged) { tma_prefetch_desc(&tk); tma_prefetch_desc(&tv); }
-    mbar_init(q_full, 1);
+    mbar_init(q_full, 1); mbar_init(q_empty, 1); mbar_init(st_free, 1); mbar_init(o_staged, 4); mbar_init(ask, 1); mbar_init(clc, 1);
     for (int s = 0; s < NK; ++s) { mbar_init(k_full(s), 1); mbar_init(k_empty(s), 1); }
     for (int s = 0; s < NV; ++s) { mbar_init(v_full(s), 1); mbar_init(v_empty(s), 1); }
-    for (int s = 0; s < 2; ++s) { mbar_init(s_full0 + 8 * s, 1); mbar_init(p_full0 + 8 * s, 4); }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(s_full0 + 8 * s, 1); mbar_init(p_full0 + 8 * s, 4);
+      if (RUN) { mbar_init(tile_full0 + 8 * s, 1); mbar_init(tile_empty0 + 8 * s, 7); }   // producer, issuer, four softmax warps, the one that writes out
+    }
     mbar_init(o_done, 1);
     fence_mbar_init();
   }
@@ -230,76 +250,189 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
   uint32_t tmem_base;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
 
-  if (warp == 4) {
-    // ---- Q: D / 64 column halves, each 128 rows (two 64-row boxes stacked = one K-major 128B-swizzled tile) ----
+  // The n-th tile of this CTA, for a whole warp; false: there are no more. done_with: its place may be written again
+  auto tile_part = [&](int n, int part) {
+    int4 x;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w) : "r"(bar + 272 + (n & 1) * 32 + part * 16) : "memory");
+    return x;
+  };
+  auto take_tile = [&](int n, Tile& t) {
+    if (!RUN) { t = t0; return n == 0; }
+    mbar_wait_warp(tile_full0 + 8 * (n & 1), ((uint32_t)n >> 1) & 1u);
+    const int4 a = tile_part(n, 0), b = tile_part(n, 1);
+    t.h = a.x; t.b = a.y; t.hk = a.z; t.row_base = a.w; t.q0 = b.x; t.limit = b.y; t.nit = b.z;
+    return t.nit > 0;
+  };
+  auto done_with = [&](int n) {
+    if (!RUN) return;
+    __syncwarp();
+    if (lane == 0) mbar_arrive(tile_empty0 + 8 * (n & 1));
+  };
+
+  if (RUN && warp == 6) {
+    // ---- tiles: this CTA's own, then those of CTAs that have not started, which need not any more (clusterlaunchcontrol). The next one is taken
+    //      when the producer is at the last blocks of the one before: taken early, long tiles would find their turn behind long tiles ----
     if (lane == 0) {
-      mbar_arrive_expect_tx(q_full, 16384 * kHalves);
-      for (int half = 0; half < kHalves; ++half)
-        for (int rb = 0; rb < 2; ++rb) {
-          const int col = (MODE == kTcPaged && !solo ? h + rb : h) * D + half * 64;
-          const int row = MODE == kTcPaged ? row_base + (solo ? rb * 64 : 0) : row_base + q0 + rb * 64;
-          tma_load_2d(sbase + L::kQ + half * 16384 + rb * 8192, &tq, q_full, col, row);
-        }
+      int bx = blockIdx.x, by = blockIdx.y, bz = blockIdx.z;
+      uint32_t clc_phase = 0;
+      bool more = true;
+      auto next = [&]() {
+        mbar_arrive_expect_tx(clc, 16);
+        asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(clc_at), "r"(clc) : "memory");
+        mbar_wait(clc, clc_phase);
+        clc_phase ^= 1u;
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t.reg .b128 r;\n\t"
+            "ld.shared.b128 r, [%4];\n\t"
+            "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\t"
+            "selp.u32 %3, 1, 0, p;\n\t"
+            "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%0, %1, %2, _}, r;\n\t}"
+            : "+r"(bx), "+r"(by), "+r"(bz), "=r"(ok) : "r"(clc_at) : "memory");
+        fence_proxy_async_smem();                         // the answer is read: the next one may be written there
+        return ok != 0;
+      };
+      for (int n = 0;; ++n) {
+        Tile t = {};
+        while (more && !tile_of(bx, by, bz, t)) more = next();
+        mbar_wait(tile_empty0 + 8 * (n & 1), (((uint32_t)n >> 1) & 1u) ^ 1u);
+        int4* at = reinterpret_cast<int4*>(smem_tc + L::kBar + 272 + (n & 1) * 32);
+        at[0] = make_int4(t.h, t.b, t.hk, t.row_base);
+        at[1] = make_int4(t.q0, t.limit, more ? t.nit : 0, 0);
+        mbar_arrive(tile_full0 + 8 * (n & 1));
+        if (!more) break;
+        mbar_wait(ask, (uint32_t)n & 1u);
+        more = next();
+      }
     }
-    if (MODE == kTcPaged) {
-      // a block is `pieces` boxes of `psize` rows; lane i looks up and fetches piece i, its page number one block ahead
-      const int psl = min(p.bs_log2, 6), psize = 1 << psl, pieces = kTcBN >> psl;
-      auto row_of = [&](int it) {
-        const int kp = block_of(it) * kTcBN + lane * psize;
-        return (it < nit && lane < pieces && kp < limit)
-                   ? ((trow[kp >> p.bs_log2] * p.Hkv + hk) << p.bs_log2) + (kp & ((1 << p.bs_log2) - 1)) : -1;
-      };
-      auto bytes_of = [&](int it) {
-        return (uint32_t)(min(pieces, (limit - block_of(it) * kTcBN + psize - 1) >> psl) * psize * 128 * kHalves);
-      };
-      // block it's keys, then the values of the block before it: a K stage is free long before a V stage
-      int row = row_of(0), row_v = -1;
-      for (int it = 0; it <= nit; ++it) {
-        if (it < nit) {
-          if (lane == 0) {
-            mbar_wait(k_empty(it), k_phase(it) ^ 1u);
-            mbar_arrive_expect_tx(k_full(it), bytes_of(it));
-          }
-          __syncwarp();
-          if (row >= 0) {
-#pragma unroll
+  }
+  if (RUN && warp == 7) {
+    // ---- out: the results that the softmax warps left in the ring of V, 32 rows (a warp's) at a time: by TMA where all of them are the tile's, else
+    //      16 bytes to a lane ----
+    Tile t;
+    for (int n = 0; take_tile(n, t); ++n) {
+      done_with(n);
+      mbar_wait_warp(o_staged, (uint32_t)n & 1u);
+      bool by_hand = false;
+#pragma unroll 1
+      for (int q = 0; q < 4; ++q) {
+        const int live = t.limit - t.q0 - q * 32, first = t.row_base + t.q0 + q * 32;
+        const uint32_t at = sbase + L::kV + q * 4096;
+        if (live >= 32) {
+          if (lane == 0)
             for (int half = 0; half < kHalves; ++half)
-              tma_load_2d(k_at(it) + half * 8192 + lane * psize * 128, &tk, k_full(it), half * 64, row);
+              asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(&to), "r"(at + half * 16384),
+                           "r"(t.h * D + half * 64), "r"(first) : "memory");
+        } else if (live > 0) {
+          by_hand = true;
+          for (int i = lane; i < live * (D / 8); i += 32) {
+            const int r = i / (D / 8), c = i % (D / 8);
+            uint4 x;
+            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w)
+                         : "r"(at + (c >> 3) * 16384 + r * 128 + (((c ^ r) & 7) << 4)));
+            *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) + (long long)(first + r) * p.out_rs + t.h * D + c * 8) = x;
           }
-        }
-        const int next = row_of(it + 1);
-        if (it > 0) {
-          const int j = it - 1;
-          if (lane == 0) {
-            mbar_wait(v_empty(j), v_phase(j) ^ 1u);
-            mbar_arrive_expect_tx(v_full(j), bytes_of(j));
-          }
-          __syncwarp();
-          if (row_v >= 0) {
-#pragma unroll
-            for (int half = 0; half < kHalves; ++half)
-              tma_load_2d(v_at(j) + half * 8192 + lane * psize * 128, &tv, v_full(j), half * 64, row_v);
-          }
-        }
-        row_v = row;
-        row = next;
-      }
-    } else if (lane == 0) {
-      const int kcol = (p.H + hk) * D, vcol = (p.H + p.Hkv + hk) * D;
-      for (int j = 0; j <= nit; ++j) {
-        if (j < nit) {
-          mbar_wait(k_empty(j), k_phase(j) ^ 1u);
-          mbar_arrive_expect_tx(k_full(j), L::kStage);
-          for (int half = 0; half < kHalves; ++half)
-            tma_load_2d(k_at(j) + half * 8192, &tk, k_full(j), kcol + half * 64, row_base + j * kTcBN);
-        }
-        if (j > 0) {
-          mbar_wait(v_empty(j - 1), v_phase(j - 1) ^ 1u);
-          mbar_arrive_expect_tx(v_full(j - 1), L::kStage);
-          for (int half = 0; half < kHalves; ++half)
-            tma_load_2d(v_at(j - 1) + half * 8192, &tv, v_full(j - 1), vcol + half * 64, row_base + (j - 1) * kTcBN);
         }
       }
+      if (lane == 0) {
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+      }
+      if (by_hand) fence_proxy_async_smem();              // the next tile's values come by TMA
+      __syncwarp();
+      if (lane == 0) mbar_arrive(st_free);
+    }
+  }
+  if (warp == 4) {
+    Tile t;
+    int g0 = 0;                                           // blocks of the tiles before
+    for (int n = 0; take_tile(n, t); g0 += t.nit, ++n) {
+      done_with(n);
+      const int h = t.h, hk = t.hk, nit = t.nit, limit = t.limit;
+      auto block_of = [&](int it) { return MODE == kTcPaged ? (it < t.nA ? it : t.bB + (it - t.nA)) : it; };
+      // ---- Q: D / 64 column halves, each 128 rows (two 64-row boxes stacked = one K-major 128B-swizzled tile). The scores before it are done:
+      //      with the tile before still in its softmax and its end ----
+      if (lane == 0) {
+        if (RUN) mbar_wait(q_empty, ((uint32_t)n & 1u) ^ 1u);
+        mbar_arrive_expect_tx(q_full, 16384 * kHalves);
+        for (int half = 0; half < kHalves; ++half)
+          for (int rb = 0; rb < 2; ++rb) {
+            const int col = (MODE == kTcPaged && !solo ? h + rb : h) * D + half * 64;
+            const int row = MODE == kTcPaged ? t.row_base + (solo ? rb * 64 : 0) : t.row_base + t.q0 + rb * 64;
+            tma_load_2d(sbase + L::kQ + half * 16384 + rb * 8192, &tq, q_full, col, row);
+          }
+      }
+      // the ring of V holds the tile before while it is written out
+      auto before_v = [&](int j) {
+        if (RUN && j == 0 && n > 0) mbar_wait(st_free, (uint32_t)(n - 1) & 1u);
+        mbar_wait(v_empty(g0 + j), v_phase(g0 + j) ^ 1u);
+      };
+      if (MODE == kTcPaged) {
+        // a block is `pieces` boxes of `psize` rows; lane i looks up and fetches piece i, its page number one block ahead
+        const int* trow = p.table + (long long)t.slot * p.max_blocks;
+        const int psl = min(p.bs_log2, 6), psize = 1 << psl, pieces = kTcBN >> psl;
+        auto row_of = [&](int it) {
+          const int kp = block_of(it) * kTcBN + lane * psize;
+          return (it < nit && lane < pieces && kp < limit)
+                     ? ((trow[kp >> p.bs_log2] * p.Hkv + hk) << p.bs_log2) + (kp & ((1 << p.bs_log2) - 1)) : -1;
+        };
+        auto bytes_of = [&](int it) {
+          return (uint32_t)(min(pieces, (limit - block_of(it) * kTcBN + psize - 1) >> psl) * psize * 128 * kHalves);
+        };
+        // block it's keys, then the values of the block before it: a K stage is free long before a V stage
+        int row = row_of(0), row_v = -1;
+        for (int it = 0; it <= nit; ++it) {
+          if (it < nit) {
+            const int g = g0 + it;
+            if (lane == 0) {
+                            mbar_wait(k_empty(g), k_phase(g) ^ 1u);
+              mbar_arrive_expect_tx(k_full(g), bytes_of(it));
+            }
+            __syncwarp();
+            if (row >= 0) {
+#pragma unroll
+              for (int half = 0; half < kHalves; ++half)
+                tma_load_2d(k_at(g) + half * 8192 + lane * psize * 128, &tk, k_full(g), half * 64, row);
+            }
+          }
+          const int next = row_of(it + 1);
+          if (it > 0) {
+            const int j = it - 1, g = g0 + j;
+            if (lane == 0) {
+              before_v(j);
+              mbar_arrive_expect_tx(v_full(g), bytes_of(j));
+            }
+            __syncwarp();
+            if (row_v >= 0) {
+#pragma unroll
+              for (int half = 0; half < kHalves; ++half)
+                tma_load_2d(v_at(g) + half * 8192 + lane * psize * 128, &tv, v_full(g), half * 64, row_v);
+            }
+          }
+          row_v = row;
+          row = next;
+        }
+      } else if (lane == 0) {
+        const int kcol = (p.H + hk) * D, vcol = (p.H + p.Hkv + hk) * D;
+        for (int j = 0; j <= nit; ++j) {
+          if (j < nit) {
+            const int g = g0 + j;
+            if (RUN && j == max(0, nit - 2)) mbar_arrive(ask);
+            mbar_wait(k_empty(g), k_phase(g) ^ 1u);
+            mbar_arrive_expect_tx(k_full(g), L::kStage);
+            for (int half = 0; half < kHalves; ++half)
+              tma_load_2d(k_at(g) + half * 8192, &tk, k_full(g), kcol + half * 64, t.row_base + j * kTcBN);
+          }
+          if (j > 0) {
+            const int g = g0 + j - 1;
+            before_v(j - 1);
+            mbar_arrive_expect_tx(v_full(g), L::kStage);
+            for (int half = 0; half < kHalves; ++half)
+              tma_load_2d(v_at(g) + half * 8192, &tv, v_full(g), vcol + half * 64, t.row_base + (j - 1) * kTcBN);
+          }
+        }
+      }
+      __syncwarp();
     }
   } else if (warp == 5) {
     {   // the whole warp runs this block (see umma_f16_w)
@@ -323,47 +456,60 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
         umma_commit_w(s_full0 + 8 * s);
         umma_commit_w(k_empty(j));
       };
-      mbar_wait_spin(q_full, 0);
-      mbar_wait_spin(k_full(0), 0);
-      tc_fence_after();
-      issue_qk(0);
-      for (int j = 0; j < nit; ++j) {
-        const int s = j & 1;
-        if (j + 1 < nit) {
-          mbar_wait_spin(k_full(j + 1), k_phase(j + 1));
-          // S buffer (j+1)&1 last held block j-1: P(j-1) sat in it and PV(j-1) was issued before this UMMA, the pipe runs in order
-          tc_fence_after();
-          issue_qk(j + 1);
-        }
-        mbar_wait_spin(v_full(j), v_phase(j));
-        mbar_wait_spin(p_full0 + 8 * s, ((uint32_t)j >> 1) & 1u);       // P(j) is written (and O rescaled where a row needed it)
+      Tile t;
+      int g0 = 0;
+      for (int n = 0; take_tile(n, t); g0 += t.nit, ++n) {
+        done_with(n);
+        const int nit = t.nit;
+        mbar_wait_spin(q_full, (uint32_t)n & 1u);
+        mbar_wait_spin(k_full(g0), k_phase(g0));
         tc_fence_after();
-        const uint32_t vlo = (v_at(j) >> 4) | kLoMN;
+        issue_qk(g0);                                     // into the buffer of the last block but one: its P has been read by products issued before
+        if (RUN && nit == 1) umma_commit_w(q_empty);
+        for (int j = 0; j < nit; ++j) {
+          const int g = g0 + j, s = g & 1;
+          if (j + 1 < nit) {
+            mbar_wait_spin(k_full(g + 1), k_phase(g + 1));
+            // S buffer (g+1)&1 last held block g-1: P(g-1) sat in it and PV(g-1) was issued before this UMMA, the pipe runs in order
+            tc_fence_after();
+            issue_qk(g + 1);
+            if (RUN && j + 2 == nit) umma_commit_w(q_empty);     // the tile's scores are done with Q
+          }
+          mbar_wait_spin(v_full(g), v_phase(g));
+          mbar_wait_spin(p_full0 + 8 * s, ((uint32_t)g >> 1) & 1u);     // P(g) is written (and O rescaled where a row needed it; and taken, the tile before)
+          tc_fence_after();
+          const uint32_t vlo = (v_at(g) >> 4) | kLoMN;
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          umma_f16_ts_w(tO, tS + s * kTcBN + ks * 8, desc(vlo + ks * (2048u >> 4)), idesc_pv, (j | ks) ? 1u : 0u);
-        umma_commit_w(o_done);
-        umma_commit_w(v_empty(j));
+          for (int ks = 0; ks < 4; ++ks)
+            umma_f16_ts_w(tO, tS + s * kTcBN + ks * 8, desc(vlo + ks * (2048u >> 4)), idesc_pv, (j | ks) ? 1u : 0u);
+          umma_commit_w(o_done);
+          umma_commit_w(v_empty(g));
+        }
       }
     }
   } else if (warp < 4) {
     // ================= softmax: thread = query row =================
     const int q = warp;                             // TMEM lane quarter this warp may touch (warp index mod 4)
     const int r = q * 32 + lane;                    // row inside the tile
-    const int rr = MODE == kTcPaged && !solo ? (r & 63) : r;      // two heads: rows 64 .. 127 are the second one's
-    const int grow = q0 + rr;                       // position in the sequence
+    const int rmask = MODE == kTcPaged && !solo ? 63 : 127;       // two heads: rows 64 .. 127 are the second one's
     const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
     const uint32_t tS = tmem_base + lane_addr, tO = tmem_base + lane_addr + kTcTmemO;
     const float sl = p.scale_log2;
+    Tile t;
+    int g0 = 0;
+    for (int n = 0; take_tile(n, t); g0 += t.nit, ++n) {
+    const int nit = t.nit, limit = t.limit, q0 = t.q0, nrows = t.nrows, low_max = t.low_max;
+    auto block_of = [&](int it) { return MODE == kTcPaged ? (it < t.nA ? it : t.bB + (it - t.nA)) : it; };
+    const int rr = r & rmask, grow = q0 + rr;       // row of the tile, position in the sequence
     const int lim = (MODE == kTcPaged || p.causal) ? min(grow, limit - 1) : limit - 1;      // last visible key of this row
     const int low = MODE == kTcPaged ? low_of(grow) : 0;                                    // first one, besides kept tokens
     float m_ref = -INFINITY, l = 0.f;
     uint32_t v[64];
     for (int j = 0; j < nit; ++j) {
-      const int kv0 = block_of(j) * kTcBN, sb = j & 1;
+      const int g = g0 + j, kv0 = block_of(j) * kTcBN, sb = g & 1;
       const bool need_mask = MODE == kTcPaged ? (kv0 + kTcBN - 1 > q0 || (kv0 < low_max && kv0 + kTcBN - 1 >= keepW))
                                               : ((p.causal && kv0 + kTcBN - 1 > q0) || (kv0 + kTcBN > limit));
-      mbar_wait_warp(s_full0 + 8 * sb, ((uint32_t)j >> 1) & 1u);
+      mbar_wait_warp(s_full0 + 8 * sb, ((uint32_t)g >> 1) & 1u);
       tc_fence_after();
       tmem_ld_32x32(tS + sb * kTcBN, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
       tmem_ld_32x32(tS + sb * kTcBN + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[32]));
@@ -419,7 +565,7 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
       // it must not reach the wait after the loop two phases behind, where the parity of "PV(nit-3) done" reads as
       // "PV(nit-1) done" and O would be taken before the last two products. So the last block always waits.
       if (j > 0 && (any_raise || j == nit - 1)) {
-        mbar_wait_warp(o_done, (uint32_t)(j - 1) & 1u);
+        mbar_wait_warp(o_done, (uint32_t)(g - 1) & 1u);
         tc_fence_after();
       }
       if (any_raise) {
@@ -446,10 +592,10 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
       }
       tmem_st_32x32(tS + sb * kTcBN, w);
       if (kv0 + kTcBN > limit) {                          // the sequence's last block: V rows that are not its own become zeros
-        mbar_wait_warp(v_full(j), v_phase(j));
+        mbar_wait_warp(v_full(g), v_phase(g));
         for (int i = threadIdx.x; i < (kv0 + kTcBN - limit) * 8 * kHalves; i += 128) {
           const int row = limit - kv0 + i / (8 * kHalves), c = i % (8 * kHalves);
-          asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(v_at(j) + (c >> 3) * 8192 + row * 128 + (c & 7) * 16),
+          asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(v_at(g) + (c >> 3) * 8192 + row * 128 + (c & 7) * 16),
                        "r"(0) : "memory");
         }
         fence_proxy_async_smem();                         // generic-proxy stores -> visible to tcgen05.mma
@@ -460,9 +606,11 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
       if (lane == 0) mbar_arrive(p_full0 + 8 * sb);
       l += rs.x + rs.y;
     }
-    // ---- finish: O / l -> 16 bit through shared memory (the Q tile is dead: every QK product has completed) ----
-    mbar_wait_warp(o_done, (uint32_t)(nit - 1) & 1u);
+    // ---- finish: O / l -> 16 bit through shared memory (the ring of V: every product has completed, and the next tile's values wait) ----
+    mbar_wait_warp(o_done, (uint32_t)(g0 + nit - 1) & 1u);
     tc_fence_after();
+    const int4 who = RUN ? tile_part(n, 0) : make_int4(t.h, t.b, 0, t.row_base);         // RUN: read again, registers are short in the loop
+    const int h = who.x, b = who.y, row_base = who.w;
     const int head = MODE == kTcPaged && !solo ? h + (r >> 6) : h;
     const bool live = MODE == kTcPaged ? rr < nrows : grow < limit;
     if (MODE == kTcPaged && p.opt.sink) l += ex2f(p.opt.sink[head] * kTcLog2e - m_ref);   // no key: not scaled, not capped
@@ -472,7 +620,8 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
       if (p.opt.gate && live) inv /= 1.f + expf(-p.opt.gate[(long long)(row_base + rr) * p.opt.ld_gate + head]);
     }
     constexpr int CH = D / 8;                             // 16-byte chunks of an output row
-    const uint32_t orow = sbase + L::kQ + (uint32_t)r * (D * 2u);
+    // RUN: in the ring of V, halves of 64 columns, 128 bytes a row, pieces turned by the row (the swizzle of TMA); else over Q, a whole row after another
+    const uint32_t orow = RUN ? sbase + L::kV + q * 4096 + lane * 128 : sbase + L::kQ + (uint32_t)r * (D * 2u);
 #pragma unroll 1
     for (int c = 0; c < D / 32; ++c) {
       uint32_t o[32];
@@ -485,26 +634,33 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
         for (int e = 0; e < 4; ++e)
           w[e] = pack16<BF16>(__uint_as_float(o[g * 8 + e * 2]) * inv, __uint_as_float(o[g * 8 + e * 2 + 1]) * inv);
         const uint32_t chunk = (uint32_t)(c * 4 + g);
-        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(orow + ((chunk ^ ((uint32_t)r & (CH - 1u))) << 4)), "r"(w[0]),
+        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(RUN ? orow + (chunk >> 3) * 16384 + (((chunk ^ (uint32_t)lane) & 7u) << 4)
+                                                                          : orow + ((chunk ^ ((uint32_t)r & (CH - 1u))) << 4)), "r"(w[0]),
                      "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
       }
     }
-    if (MODE == kTcDense && p.lse && live)
-      p.lse[((long long)b * p.H + h) * p.S + grow] = m_ref * 0.6931471805599453f + __logf(l);
+    if (RUN) fence_proxy_async_smem();                    // written here, read by TMA
     __syncwarp();
-    // each warp copies ITS 32 rows out (written by its own lanes): CH lanes cover the bytes of a row
-    uint16_t* obase = reinterpret_cast<uint16_t*>(p.out);
+    if (RUN && lane == 0) mbar_arrive(o_staged);
+    if (MODE == kTcDense && p.lse && live)
+      p.lse[((long long)b * p.H + h) * p.S + grow] = fmaf(__log2f(l), 0.6931471805599453f, __fmul_rn(m_ref, 0.6931471805599453f));
+    done_with(n);
+    if (!RUN) {
+      // each warp copies ITS 32 rows out (written by its own lanes): CH lanes cover the bytes of a row
+      uint16_t* obase = reinterpret_cast<uint16_t*>(p.out);
 #pragma unroll 4
-    for (int it = 0; it < CH; ++it) {
-      const int row = q * 32 + it * (32 / CH) + lane / CH, chunk = lane % CH;
-      uint32_t w0, w1, w2, w3;
-      asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w0), "=r"(w1), "=r"(w2), "=r"(w3)
-                   : "r"(sbase + L::kQ + (uint32_t)row * (D * 2u) + (((uint32_t)chunk ^ ((uint32_t)row & (CH - 1u))) << 4)));
-      const int rw = MODE == kTcPaged && !solo ? (row & 63) : row;
-      const bool keep = MODE == kTcPaged ? rw < nrows : q0 + rw < limit;
-      const long long at = (long long)(MODE == kTcPaged ? row_base + rw : row_base + q0 + rw) * p.out_rs +
-                           (MODE == kTcPaged && !solo ? h + (row >> 6) : h) * D + chunk * 8;
-      if (keep) *reinterpret_cast<uint4*>(obase + at) = make_uint4(w0, w1, w2, w3);
+      for (int it = 0; it < CH; ++it) {
+        const int row = q * 32 + it * (32 / CH) + lane / CH, chunk = lane % CH;
+        uint32_t w0, w1, w2, w3;
+        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w0), "=r"(w1), "=r"(w2), "=r"(w3)
+                     : "r"(sbase + L::kQ + (uint32_t)row * (D * 2u) + (((uint32_t)chunk ^ ((uint32_t)row & (CH - 1u))) << 4)));
+        const int rw = MODE == kTcPaged && !solo ? (row & 63) : row;
+        const bool keep = MODE == kTcPaged ? rw < nrows : q0 + rw < limit;
+        const long long at = (long long)(MODE == kTcPaged ? row_base + rw : row_base + q0 + rw) * p.out_rs +
+                             (MODE == kTcPaged && !solo ? h + (row >> 6) : h) * D + chunk * 8;
+        if (keep) *reinterpret_cast<uint4*>(obase + at) = make_uint4(w0, w1, w2, w3);
+      }
+    }
     }
   }
   tc_fence_before();
@@ -515,12 +671,12 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
   }
 }
 
-template <int MODE, int D, bool BF16, bool CAP>
-static int launch_tc(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FlashTcParams& p, dim3 grid, cudaStream_t st) {
-  auto kern = flash_fwd_tc_kernel<MODE, D, BF16, CAP>;
+template <int MODE, int D, bool BF16, bool CAP, bool RUN>
+static int launch_tc(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to, const FlashTcParams& p, dim3 grid, cudaStream_t st) {
+  auto kern = flash_fwd_tc_kernel<MODE, D, BF16, CAP, RUN>;
   // per call: the attribute belongs to the current device, and a process may use several
   B200_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcSmem<D>::kBytes));
-  kern<<<grid, kTcThreads, TcSmem<D>::kBytes, st>>>(tq, tk, tv, p);
+  kern<<<grid, kTcThreads, TcSmem<D>::kBytes, st>>>(tq, tk, tv, to, p);
   B200_LAUNCH_CHECK();
   return 0;
 }
@@ -581,8 +737,15 @@ static int fused_qkv(const void* qkv, long long rows, FlashTcParams& p, int D, i
   if (int rc = rows_map(&tm, qkv, (uint64_t)(p.H + 2 * p.Hkv) * D, (uint64_t)rows, 64)) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   const bool bf = dtype == B200_DT_BF16;
-  if (D == 64) return bf ? launch_tc<MODE, 64, true, false>(tm, tm, tm, p, grid, st) : launch_tc<MODE, 64, false, false>(tm, tm, tm, p, grid, st);
-  return bf ? launch_tc<MODE, 128, true, false>(tm, tm, tm, p, grid, st) : launch_tc<MODE, 128, false, false>(tm, tm, tm, p, grid, st);
+  // More tiles than two CTAs for each SM take: those go on from tile to tile. Fewer: nothing to go on to, and a tile's way through the other warps
+  // takes 1 us more (100 tokens, 32 heads of 128: 12.3 us, 14.3).
+  const bool run = (long long)grid.x * grid.y * grid.z > 2 * kNumSMs;
+  CUtensorMap to = tm;
+  if (run)
+    if (int rc = rows_map(&to, p.out, (uint64_t)p.H * D, (uint64_t)rows, 32)) return rc;
+#define TC_ROWS(DD, BB) (run ? launch_tc<MODE, DD, BB, false, true>(tm, tm, tm, to, p, grid, st) : launch_tc<MODE, DD, BB, false, false>(tm, tm, tm, to, p, grid, st))
+  return D == 64 ? (bf ? TC_ROWS(64, true) : TC_ROWS(64, false)) : (bf ? TC_ROWS(128, true) : TC_ROWS(128, false));
+#undef TC_ROWS
 }
 
 }  // namespace b200
@@ -661,8 +824,8 @@ B200_API int b200_paged_attn_tc(const void* q, long long tokens, const void* ck,
   cudaStream_t st = (cudaStream_t)stream;
   const bool bf = dtype == B200_DT_BF16;
 #define TC_PAGED(DD)                                                                                                           \
-  (capped ? (bf ? launch_tc<kTcPaged, DD, true, true>(tq, tk, tv, p, grid, st) : launch_tc<kTcPaged, DD, false, true>(tq, tk, tv, p, grid, st)) \
-          : (bf ? launch_tc<kTcPaged, DD, true, false>(tq, tk, tv, p, grid, st) : launch_tc<kTcPaged, DD, false, false>(tq, tk, tv, p, grid, st)))
+  (capped ? (bf ? launch_tc<kTcPaged, DD, true, true, false>(tq, tk, tv, tq, p, grid, st) : launch_tc<kTcPaged, DD, false, true, false>(tq, tk, tv, tq, p, grid, st)) \
+          : (bf ? launch_tc<kTcPaged, DD, true, false, false>(tq, tk, tv, tq, p, grid, st) : launch_tc<kTcPaged, DD, false, false, false>(tq, tk, tv, tq, p, grid, st)))
   return D == 64 ? TC_PAGED(64) : TC_PAGED(128);
 #undef TC_PAGED
 }
