@@ -161,15 +161,46 @@ struct SegmentIter {
   }
 };
 
+// tcgen05.mma from converged code: the whole warp runs the issue loop and elect.sync picks the lane, always the same one. From a branch of one thread
+// four products and a commit took 420 cycles whatever their size, and waiting for the stage 70 to 180 more, where the pipe takes 512 for
+// 256 x 256 x 64 on two SMs: the operands of an instruction went through the vector registers. Now 300 and 70. A x B^T of bf16, before -> now:
+// 2048 x 34816 x 5120 494 -> 459 us (1.59 PFLOP/s), 2048 x 5120 x 17408 267 -> 248, 2048 x 5120 x 5120 94 -> 88, 2345 x 3072 x 2048 42 -> 36.
+// A k-block is four products along k, their operands a step apart; `acc`: whether the first one accumulates.
+#define GEMM_MMA(KIND, PRED, A, B) "@q tcgen05.mma.cta_group::%7.kind::" KIND " [%0], " A ", " B ", %3, " PRED ";\n\t"
+#define GEMM_MMA4(KIND)                                                                                                                      \
+  asm volatile(                                                                                                                              \
+      "{\n\t.reg .pred q, t, f;\n\t.reg .b64 a1, a2, a3, b1, b2, b3;\n\t"                                                                    \
+      "elect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 f, %4, 0;\n\tsetp.eq.b32 t, %4, %4;\n\t"                                                   \
+      "add.u64 a1, %1, %5;\n\tadd.u64 a2, a1, %5;\n\tadd.u64 a3, a2, %5;\n\t"                                                                \
+      "add.u64 b1, %2, %6;\n\tadd.u64 b2, b1, %6;\n\tadd.u64 b3, b2, %6;\n\t"                                                                \
+      GEMM_MMA(KIND, "f", "%1", "%2") GEMM_MMA(KIND, "t", "a1", "b1") GEMM_MMA(KIND, "t", "a2", "b2") GEMM_MMA(KIND, "t", "a3", "b3") "}"    \
+      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(acc), "l"(a_step), "l"(b_step), "n"(CTAS) : "memory")
+#define GEMM_MMA1(KIND)                                                                                                                      \
+  asm volatile(                                                                                                                              \
+      "{\n\t.reg .pred q, f;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 f, %4, 0;\n\t"                                                    \
+      "@q tcgen05.mma.cta_group::%5.kind::" KIND " [%0], %1, %2, %3, f;\n\t}"                                                               \
+      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(acc), "n"(CTAS) : "memory")
 template <int ES, int CTAS>
-__device__ __forceinline__ void umma_issue(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-  if constexpr (CTAS == 1) {
-    if constexpr (ES == 2) umma_f16(d, a, b, idesc, acc);
-    else umma_tf32(d, a, b, idesc, acc);
-  } else {
-    if constexpr (ES == 2) umma_f16_2sm(d, a, b, idesc, acc);
-    else umma_tf32_2sm(d, a, b, idesc, acc);
-  }
+__device__ __forceinline__ void umma_kblock(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc, uint64_t a_step, uint64_t b_step) {
+  if constexpr (ES == 2) GEMM_MMA4("f16");
+  else GEMM_MMA4("tf32");
+}
+template <int ES, int CTAS>
+__device__ __forceinline__ void umma_kstep(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+  if constexpr (ES == 2) GEMM_MMA1("f16");
+  else GEMM_MMA1("tf32");
+}
+#undef GEMM_MMA
+#undef GEMM_MMA4
+#undef GEMM_MMA1
+// arrive, once the products of that lane are done, on the barrier (of both CTAs of a pair)
+template <int CTAS>
+__device__ __forceinline__ void umma_commit_elected(uint32_t bar) {
+  if constexpr (CTAS == 1)
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar) : "memory");
+  else
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+                 "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}" ::"r"(bar), "h"((uint16_t)3) : "memory");
 }
 
 template <typename OutT>
@@ -496,15 +527,13 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
       }
     }
   } else if (warp == 1) {
-    // ================= MMA issuer (one thread of the leader CTA) =================
-    if (lane == 0 && leader) {
+    // ================= MMA issuer (a warp of the leader CTA, see umma_kblock) =================
+    if (leader) {
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
       uint32_t acc_phase = 0;
-      // Shared-memory descriptors, split so that the per-UMMA work is ONE 32-bit add per operand.
-      // (Building each 64-bit descriptor from scratch costs ~45 dependent uniform-datapath ops per
-      // k-block, ~540 cycles, which made this thread — not the tensor pipe — the bottleneck.)
+      // Shared-memory descriptors, split so that a stage or a step along k is one add.
       //   hi word: stride-byte-offset 1024 (8-row groups) | version 1 | 128-byte swizzle
       //   lo word: (address >> 4) | (leading-byte-offset >> 4) << 16
       // K-major: rows of 128 B, k-step = +32 B inside the swizzle row, LBO unused (16).
@@ -533,24 +562,16 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
           if (kb < p.num_k) {
             const uint32_t a_lo = a_lo_main + (uint32_t)stage * a_stage16;
             const uint32_t b_lo = b_lo_main + (uint32_t)stage * b_stage16;
-            umma_issue<ES, CTAS>(d_tmem, desc(a_lo), desc(b_lo), p.idesc_main, kb != sg.kb0 ? 1u : 0u);
-#pragma unroll
-            for (int k = 1; k < EPR / UK; ++k)
-              umma_issue<ES, CTAS>(d_tmem, desc(a_lo + k * a_step_main), desc(b_lo + k * b_step_main), p.idesc_main, 1u);
+            umma_kblock<ES, CTAS>(d_tmem, desc(a_lo), desc(b_lo), p.idesc_main, kb != sg.kb0 ? 1u : 0u, a_step_main, b_step_main);
           } else {
             const uint32_t a_lo = a_lo_lora + (uint32_t)stage * a_stage16;
             const uint32_t b_lo = b_lo_lora + (uint32_t)stage * b_stage16;
             for (int k = 0; k < lora_ksteps; ++k)
-              umma_issue<ES, CTAS>(d_tmem, desc(a_lo + k * kStepK), desc(b_lo + k * kStepK), p.idesc_lora,
+              umma_kstep<ES, CTAS>(d_tmem, desc(a_lo + k * kStepK), desc(b_lo + k * kStepK), p.idesc_lora,
                                    (kb != sg.kb0 || k != 0) ? 1u : 0u);
           }
-          if constexpr (CTAS == 1) {
-            umma_commit(empty_bar(stage));
-            if (kb == sg.kb1 - 1) umma_commit(tfull_bar(acc));
-          } else {
-            umma_commit_2sm(empty_bar(stage), 3);
-            if (kb == sg.kb1 - 1) umma_commit_2sm(tfull_bar(acc), 3);
-          }
+          umma_commit_elected<CTAS>(empty_bar(stage));
+          if (kb == sg.kb1 - 1) umma_commit_elected<CTAS>(tfull_bar(acc));
           if (++stage == p.stages) { stage = 0; phase ^= 1u; }
         }
         acc ^= 1;
