@@ -7,7 +7,7 @@
 // The pair halves the B traffic per flop, which matters because at 128 x 256 tiles the kernel is
 // bound by L2->SM bandwidth (~12.5 TB/s), not by the tensor pipe: 85 flop/B caps a single-CTA
 // kernel near 1.0 PFLOP/s, 128 flop/B lifts the cap to ~1.6 (measured; see profiles/).
-// Per unit: warp 0 feeds a ring of shared-memory stages with TMA (128-byte swizzle), warp 1 issues
+// Per unit: warps 0 and 6 feed a ring of shared-memory stages with TMA (128-byte swizzle; A and B), warp 1 issues
 // tcgen05.mma into one of two TMEM accumulators, warps 2-5 drain the other accumulator with
 // tcgen05.ld and write D, so the epilogue of tile i overlaps the main loop of tile i+1. BN
 // (16..256), the CTA-group size and the stage count are run-time choices: the host picks the
@@ -27,6 +27,7 @@
 #include "../include/b200_ops.h"
 
 #include <stdio.h>
+#include <type_traits>
 #include <stdlib.h>
 #include <string.h>
 
@@ -34,7 +35,7 @@ namespace b200 {
 
 constexpr int kBM = 128;             // rows per CTA = TMEM lanes
 constexpr int kStageABytes = 16384;  // 128 rows x 128 B
-constexpr int kGemmThreads = 192;    // producer, mma, 4 epilogue warps
+constexpr int kGemmThreads = 224;    // producer of A, mma, 4 epilogue warps, producer of B
 constexpr int kAccStride = 256;      // TMEM columns between the two accumulators
 
 struct GemmKernelParams {
@@ -201,6 +202,23 @@ __device__ __forceinline__ void umma_commit_elected(uint32_t bar) {
   else
     asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
                  "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}" ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
+
+// the same for the producer's loads and its arrival
+template <int CTAS>
+__device__ __forceinline__ void tma_load_4d_elected(uint32_t dst, const CUtensorMap* tm, uint32_t bar, int c0, int c1, int c2, int c3) {
+  if constexpr (CTAS == 1)
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+                 "@q cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];\n\t}"
+                 ::"r"(dst), "l"(reinterpret_cast<uint64_t>(tm)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
+  else
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+                 "@q cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];\n\t}"
+                 ::"r"(dst), "l"(reinterpret_cast<uint64_t>(tm)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx_elected(uint32_t bar, uint32_t bytes) {
+  asm volatile("{\n\t.reg .pred q;\n\t.reg .b64 st;\n\telect.sync _|q, 0xffffffff;\n\t@q mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}"
+               ::"r"(bar), "r"(bytes) : "memory");
 }
 
 template <typename OutT>
@@ -426,8 +444,8 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
       tma_prefetch_desc(&tmB2);
     }
     for (int s = 0; s < p.stages; ++s) {
-      // one arrival per CTA's producer (+ the TMA transaction bytes) (+ W4: the dequant warps of every CTA)
-      mbar_init(full_bar(s), (W4 && !W4DBG(128)) ? CTAS * 2 : CTAS);   // W4: + one arrival per CTA from its dequant warps
+      // the leader's producer, which expects the bytes of the unit's CTAs (+ W4: the dequant warps of every CTA)
+      mbar_init(full_bar(s), 1 + ((W4 && !W4DBG(128)) ? CTAS : 0));
       mbar_init(empty_bar(s), 1);     // tcgen05.commit (multicast to both CTAs of a pair)
     }
     for (int s = 0; s < raw_stages; ++s) {
@@ -468,64 +486,74 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
   const int total_tiles = tiles_per_batch * p.batch;
   const int num_k_total = p.num_k + (p.K2 > 0 ? 1 : 0);
 
-  if (warp == 0) {
-    // ================= TMA producer (every CTA loads its own rows of A and its share of B) =========
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      const uint32_t tx_full = (uint32_t)CTAS * (kStageABytes + stage_b_bytes);
-      const uint32_t tx_a_only = (uint32_t)CTAS * kStageABytes;
-      const uint32_t box_bytes = EPR * 128;  // MN-major operands: one box = EPR k-rows x 128 B
-      SegmentIter it(p, unit, nunits, total_tiles, num_k_total);
-      Segment sg;
-      while (it.next(sg)) {
-        const int tile = sg.tile;
-        const int bt = tile / tiles_per_batch;
-        const int rem = tile - bt * tiles_per_batch;
-        const int n_blk = rem / p.num_m;
-        const int m_blk = rem - n_blk * p.num_m;
-        const int m0 = m_blk * (kBM * CTAS) + (int)rank * kBM;
-        const int n0 = n_blk * p.bn + (int)rank * bn_cta;
-        const int ab0 = bt % p.nb0, ab1 = bt / p.nb0;
-        const int btb = p.b_map ? p.b_map[bt] : bt / p.b_div;
-        if (btb < 0) continue;                       // grouped GEMM: unused row tile
-        const int bb0 = btb % p.nb0_b, bb1 = btb / p.nb0_b;
-        for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
-          mbar_wait(empty_bar(stage), phase ^ 1u);
-          const uint32_t fb_local = full_bar(stage);
-          const uint32_t fb = leader ? fb_local : mapa_shared(fb_local, 0);  // the leader's barrier
-          const bool dbg_b = W4 && W4DBG(64);   // timing experiment: also stream a (dummy) B tile through TMA
-          if (leader) mbar_arrive_expect_tx(fb_local, (W4 && kb < p.num_k && !dbg_b) ? tx_a_only : tx_full);
-          else mbar_arrive_cluster(fb);
-          const uint32_t sa = sA0 + (uint32_t)stage * kStageABytes;
-          const uint32_t sb = sB0 + (uint32_t)stage * stage_b_bytes;
-          auto load = [&](uint32_t dst, const CUtensorMap* tm, int c0, int c1, int c2, int c3) {
-            if constexpr (CTAS == 1) tma_load_4d(dst, tm, fb, c0, c1, c2, c3);
-            else tma_load_4d_2sm(dst, tm, fb, c0, c1, c2, c3);
-          };
-          if (kb < p.num_k) {
-            const int k0 = kb * EPR;
+  // ================= TMA producers (every CTA: its own rows of A and its share of B) =========
+  // A warp for each operand: one warp for both took 90 cycles to see that a stage is free, 200 for A's box and 120 to 180 for each box of B, 530 a
+  // k-block with B K-major (two boxes) and 690 with B MN-major (three) where the products take 512. So the next stage's barrier is also looked at
+  // before this one's loads, by the issuer too. 2048 x 5120 x 16384 with B MN-major 287 -> 249 us, K-major 2048 x 34816 x 5120 459 -> 444,
+  // 2048 x 16384 x 5120 215 -> 208. Converged code alone changed nothing here.
+  // The bytes of both operands and CTAs arrive on the leader's barrier; some may come before the leader expects them, but not before the phase
+  // that they belong to: a producer waits for `empty`, which follows the last use of the stage.
+  auto produce = [&](auto of_a, auto of_b) {
+    constexpr bool A = decltype(of_a)::value, B = decltype(of_b)::value;
+    int stage = 0;
+    uint32_t phase = 0;
+    const uint32_t tx_full = (uint32_t)CTAS * (kStageABytes + stage_b_bytes);
+    const uint32_t tx_a_only = (uint32_t)CTAS * kStageABytes;
+    const uint32_t box_bytes = EPR * 128;  // MN-major operands: one box = EPR k-rows x 128 B
+    const uint32_t fb0 = leader ? full_bar(0) : mapa_shared(full_bar(0), 0);   // the leader's barriers
+    bool free = false;
+    SegmentIter it(p, unit, nunits, total_tiles, num_k_total);
+    Segment sg;
+    while (it.next(sg)) {
+      const int tile = sg.tile;
+      const int bt = tile / tiles_per_batch;
+      const int rem = tile - bt * tiles_per_batch;
+      const int n_blk = rem / p.num_m;
+      const int m_blk = rem - n_blk * p.num_m;
+      const int m0 = m_blk * (kBM * CTAS) + (int)rank * kBM;
+      const int n0 = n_blk * p.bn + (int)rank * bn_cta;
+      const int ab0 = bt % p.nb0, ab1 = bt / p.nb0;
+      const int btb = p.b_map ? p.b_map[bt] : bt / p.b_div;
+      if (btb < 0) continue;                       // grouped GEMM: unused row tile
+      const int bb0 = btb % p.nb0_b, bb1 = btb / p.nb0_b;
+      for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
+        if (!free) mbar_wait(empty_bar(stage), phase ^ 1u);
+        const uint32_t fb = fb0 + 8u * stage;
+        const uint32_t sa = sA0 + (uint32_t)stage * kStageABytes;
+        const uint32_t sb = sB0 + (uint32_t)stage * stage_b_bytes;
+        if (++stage == p.stages) { stage = 0; phase ^= 1u; }
+        free = mbar_test_wait(empty_bar(stage), phase ^ 1u);
+        if (A && leader) mbar_expect_tx_elected(fb, (W4 && kb < p.num_k) ? tx_a_only : tx_full);
+        if (kb < p.num_k) {
+          const int k0 = kb * EPR;
+          if constexpr (A) {
             if (!p.a_mn) {
-              load(sa, &tmA, k0, m0, ab0, ab1);
+              tma_load_4d_elected<CTAS>(sa, &tmA, fb, k0, m0, ab0, ab1);
             } else {
-              for (int j = 0; j < kBM / EPR; ++j) load(sa + j * box_bytes, &tmA, m0 + j * EPR, k0, ab0, ab1);
+#pragma unroll
+              for (int j = 0; j < kBM / EPR; ++j) tma_load_4d_elected<CTAS>(sa + j * box_bytes, &tmA, fb, m0 + j * EPR, k0, ab0, ab1);
             }
-            if constexpr (W4) { if (dbg_b) load(sb, &tmB, k0, (n0 % 512), bb0, bb1); }
-            if constexpr (!W4) {
-              if (!p.b_mn) {
-                load(sb, &tmB, k0, n0, bb0, bb1);
-              } else {
-                for (int j = 0; j < bn_cta / EPR; ++j) load(sb + j * box_bytes, &tmB, n0 + j * EPR, k0, bb0, bb1);
-              }
-            }
-          } else {
-            load(sa, &tmA2, 0, m0, 0, 0);
-            load(sb, &tmB2, 0, n0, 0, 0);
           }
-          if (++stage == p.stages) { stage = 0; phase ^= 1u; }
+          if constexpr (B && !W4) {
+            if (!p.b_mn) {
+              tma_load_4d_elected<CTAS>(sb, &tmB, fb, k0, n0, bb0, bb1);
+            } else {
+#pragma unroll 2
+              for (int j = 0; j < bn_cta / EPR; ++j) tma_load_4d_elected<CTAS>(sb + j * box_bytes, &tmB, fb, n0 + j * EPR, k0, bb0, bb1);
+            }
+          }
+        } else {
+          if constexpr (A) tma_load_4d_elected<CTAS>(sa, &tmA2, fb, 0, m0, 0, 0);
+          if constexpr (B) tma_load_4d_elected<CTAS>(sb, &tmB2, fb, 0, n0, 0, 0);
         }
       }
     }
+  };
+
+  if (warp == 0) {
+    produce(std::true_type{}, std::integral_constant<bool, W4>{});
+  } else if (!W4 && warp == 6) {
+    produce(std::false_type{}, std::true_type{});
   } else if (warp == 1) {
     // ================= MMA issuer (a warp of the leader CTA, see umma_kblock) =================
     if (leader) {
@@ -549,6 +577,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
       const uint32_t a_stage16 = kStageABytes >> 4, b_stage16 = stage_b_bytes >> 4;
       const int lora_ksteps = (p.K2 + UK - 1) / UK;
       auto desc = [](uint32_t lo) { return ((uint64_t)kDescHi << 32) | (uint64_t)lo; };
+      bool full = false;   // whether the stage that comes next was seen full, a k-block ahead
       SegmentIter it(p, unit, nunits, total_tiles, num_k_total);
       Segment sg;
       while (it.next(sg)) {
@@ -557,22 +586,24 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)acc * kAccStride;
         for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
-          mbar_wait(full_bar(stage), phase);
+          if (!full) mbar_wait(full_bar(stage), phase);
           tc_fence_after();
+          const int cur = stage;
+          if (++stage == p.stages) { stage = 0; phase ^= 1u; }
+          full = mbar_test_wait(full_bar(stage), phase);
           if (kb < p.num_k) {
-            const uint32_t a_lo = a_lo_main + (uint32_t)stage * a_stage16;
-            const uint32_t b_lo = b_lo_main + (uint32_t)stage * b_stage16;
+            const uint32_t a_lo = a_lo_main + (uint32_t)cur * a_stage16;
+            const uint32_t b_lo = b_lo_main + (uint32_t)cur * b_stage16;
             umma_kblock<ES, CTAS>(d_tmem, desc(a_lo), desc(b_lo), p.idesc_main, kb != sg.kb0 ? 1u : 0u, a_step_main, b_step_main);
           } else {
-            const uint32_t a_lo = a_lo_lora + (uint32_t)stage * a_stage16;
-            const uint32_t b_lo = b_lo_lora + (uint32_t)stage * b_stage16;
+            const uint32_t a_lo = a_lo_lora + (uint32_t)cur * a_stage16;
+            const uint32_t b_lo = b_lo_lora + (uint32_t)cur * b_stage16;
             for (int k = 0; k < lora_ksteps; ++k)
               umma_kstep<ES, CTAS>(d_tmem, desc(a_lo + k * kStepK), desc(b_lo + k * kStepK), p.idesc_lora,
                                    (kb != sg.kb0 || k != 0) ? 1u : 0u);
           }
-          umma_commit_elected<CTAS>(empty_bar(stage));
+          umma_commit_elected<CTAS>(empty_bar(cur));
           if (kb == sg.kb1 - 1) umma_commit_elected<CTAS>(tfull_bar(acc));
-          if (++stage == p.stages) { stage = 0; phase ^= 1u; }
         }
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1u;
