@@ -388,7 +388,7 @@ __device__ __noinline__ int ar_reduce(const GemmKernelParams& p, int next, int n
   return next;
 }
 
-template <int ES, int CTAS, bool W4, bool AR>
+template <int ES, int CTAS, bool W4>
 __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmA2,
                                           const CUtensorMap& tmB2, const GemmKernelParams& p, const W4Params* w4) {
   constexpr int EPR = 128 / ES;  // elements per 128-byte swizzle row = k-block depth
@@ -771,7 +771,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
     const long long sk_total = (long long)(total_tiles / sk_g) * num_k_total;
     // fused all-reduce: this CTA's reduction items are ar_next, ar_next + gridDim.x, ... < ar_items (see ar_reduce)
     const int ar_slabs = (kBM * CTAS) / kArSlabRows;
-    const int ar_items = AR ? ((total_tiles - p.ar_rank + p.ar_world - 1) / p.ar_world) * ar_slabs : 0;
+    const int ar_items = p.ar_world > 1 ? ((total_tiles - p.ar_rank + p.ar_world - 1) / p.ar_world) * ar_slabs : 0;
     int ar_next = blockIdx.x;
     const uint32_t ar_poll_slot = sk_epoch_slot;     // stream-K is off in this mode: the slot is free
     while (it.next(sg)) {
@@ -862,7 +862,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
       }
       acc ^= 1;
       if (acc == 0) acc_phase ^= 1u;
-      if constexpr (AR) {
+      if (!W4 && p.ar_world > 1) {
         // this CTA's rows of the tile are in D: one system-scope fence + release by one thread covers the stores the
         // other epilogue threads made before the barrier
         asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -875,7 +875,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
         ar_next = ar_reduce<CTAS>(p, ar_next, ar_items, 2, false, total_tiles, ar_poll_slot);
       }
     }
-    if constexpr (AR) {
+    if (!W4 && p.ar_world > 1) {
       // ---- the rest of this CTA's share of the reduction, then the cross-rank completion barrier ----
       ar_reduce<CTAS>(p, ar_next, ar_items, 1 << 30, true, total_tiles, ar_poll_slot);
       asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -915,13 +915,12 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
   }
 }
 
-// AR: with the all-reduce over ranks after it, which needs 230 registers a thread; without, 128, and other kernels find room beside a launch.
-template <int ES, int CTAS, bool AR>
+template <int ES, int CTAS>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ CUtensorMap tmA2, const __grid_constant__ CUtensorMap tmB2,
                     const __grid_constant__ GemmKernelParams p) {
-  gemm_body<ES, CTAS, false, AR>(tmA, tmB, tmA2, tmB2, p, nullptr);
+  gemm_body<ES, CTAS, false>(tmA, tmB, tmA2, tmB2, p, nullptr);
 }
 
 // Same pipeline with the B operand expanded from 4-bit codes inside the kernel (NF4 / GPTQ / AWQ weights, optionally
@@ -930,7 +929,7 @@ __global__ void __launch_bounds__(kW4Threads, 1)
 gemm_w4_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmA2,
                        const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ W4Params w4,
                        const __grid_constant__ GemmKernelParams p) {
-  gemm_body<2, 2, true, false>(tmA, tmA, tmA2, tmB2, p, &w4);
+  gemm_body<2, 2, true>(tmA, tmA, tmA2, tmB2, p, &w4);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1018,12 +1017,12 @@ static int sk_group_of(int num_m, int units) {
   return num_m > 1 && num_m <= units && (units % num_m) * 20 <= units && !sk_flat ? num_m : 1;
 }
 
-template <int ES, int CTAS, bool AR>
-static int launch_kernel(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmA2, const CUtensorMap& tmB2,
+template <int ES, int CTAS>
+static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmA2, const CUtensorMap& tmB2,
                   const GemmKernelParams& p, int grid, int smem, cudaStream_t stream) {
   static bool configured = false;
   if (!configured) {
-    B200_CHECK(cudaFuncSetAttribute(gemm_tcgen05_kernel<ES, CTAS, AR>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_max_smem));
+    B200_CHECK(cudaFuncSetAttribute(gemm_tcgen05_kernel<ES, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_max_smem));
     configured = true;
   }
   cudaLaunchConfig_t cfg = {};
@@ -1038,15 +1037,8 @@ static int launch_kernel(const CUtensorMap& tmA, const CUtensorMap& tmB, const C
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  B200_CHECK(cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<ES, CTAS, AR>, tmA, tmB, tmA2, tmB2, p));
+  B200_CHECK(cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<ES, CTAS>, tmA, tmB, tmA2, tmB2, p));
   return 0;
-}
-
-template <int ES, int CTAS>
-static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmA2, const CUtensorMap& tmB2,
-                  const GemmKernelParams& p, int grid, int smem, cudaStream_t stream) {
-  return p.ar_world > 1 ? launch_kernel<ES, CTAS, true>(tmA, tmB, tmA2, tmB2, p, grid, smem, stream)
-                        : launch_kernel<ES, CTAS, false>(tmA, tmB, tmA2, tmB2, p, grid, smem, stream);
 }
 
 }  // namespace b200

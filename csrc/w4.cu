@@ -73,63 +73,95 @@ struct W4Shards {
   int nshards;
 };
 
-// Expansion to [N, K] by kW4ExpandBlocks blocks an SM that go over the weights, so that it runs beside a GEMM: they and the persistent GEMM's block fit
-// on an SM together, in registers (24 warps of 40, 7 of 128) and shared memory, whichever of the two starts first. (A block for every 256 runs of 32
-// weights kept a GEMM out until the last one had started, and found no room beside one that ran.) A warp takes runs of 1024 weights of a row; lane l takes the 32-bit words l, l + 32, ..
-// (8 weights, always of one group): a load of a warp is 128 contiguous bytes, a store 512, four of each in flight. Bound by HBM: 34816 x 5120 to bf16 96 -> 91 us (5.0 TB/s), 5120 x 17408
-// 51 -> 48; one block of four warps with copies seven runs ahead 203. K % 32 == 0, group % 32 == 0.
-constexpr int kW4ExpandBlocks = 3;
+// Each thread expands 16 packed bytes (32 weights). K % 32 == 0, group % 32 == 0.
 template <typename T>
-__global__ void __launch_bounds__(256, 6)
-w4_dequant_kernel(W4Shards sh, T* __restrict__ out, long long N, int K, int group, int shift, const float* __restrict__ lut_g,
+__global__ void __launch_bounds__(256)
+w4_dequant_kernel(W4Shards sh, T* __restrict__ out, long long N, int K, int group, const float* __restrict__ lut_g,
                   long long out_rs) {
-  constexpr int U = 4, RUN = U * 256;
   __shared__ float lut[16];
   if (threadIdx.x < 16) lut[threadIdx.x] = lut_g ? lut_g[threadIdx.x] : kNF4[threadIdx.x];
   __syncthreads();
-  const int runs = (K + RUN - 1) / RUN, groups = K / group;
-  const int first = blockIdx.x * 8 + (threadIdx.x >> 5), step = gridDim.x * 8;
-  const int step_n = step / runs, step_r = step % runs;
-  long long n = first / runs;
-  int r = first % runs;
-#pragma unroll 1
-  while (n < N) {
-    const int k0 = r * RUN + (threadIdx.x & 31) * 8;
-    const int s = sh.nshards > 1 ? (int)(n / sh.rows_per_shard) : 0;
-    const long long nl = n - (long long)s * sh.rows_per_shard;
-    const uint8_t* codes = sh.packed[s] + nl * K / 2;
-    const float* scale = sh.scale[s] + nl * groups;
-    const float* zero = sh.zs[s] ? sh.zs[s] + nl * groups : nullptr;
-    uint32_t word[U];
-    float sc[U], zs[U];
+  const int chunks_per_row = K / 32;
+  const long long cid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (cid >= N * chunks_per_row) return;
+  const long long n = cid / chunks_per_row;
+  const int kc = (int)(cid - n * chunks_per_row);
+  const int s = sh.nshards > 1 ? (int)(n / sh.rows_per_shard) : 0;
+  const long long nl = n - (long long)s * sh.rows_per_shard;
+  const uint4 raw = *reinterpret_cast<const uint4*>(sh.packed[s] + (nl * K / 2) + kc * 16);
+  const int g = (kc * 32) / group;
+  const int groups_per_row = K / group;
+  const float sc = sh.scale[s][nl * groups_per_row + g];
+  const float zs = sh.zs[s] ? sh.zs[s][nl * groups_per_row + g] : 0.f;
+  const uint32_t words[4] = {raw.x, raw.y, raw.z, raw.w};
+  T* o = out + n * out_rs + kc * 32;
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int k = k0 + u * 256, g = shift >= 0 ? k >> shift : k / group;
-      const bool in = k < K;
-      word[u] = in ? *reinterpret_cast<const uint32_t*>(codes + k / 2) : 0u;
-      sc[u] = in ? scale[g] : 0.f;
-      zs[u] = in && zero ? zero[g] : 0.f;
+  for (int wi = 0; wi < 4; ++wi) {
+    float v[8];
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const uint32_t byte = (words[wi] >> (8 * b)) & 0xFFu;
+      v[2 * b] = lut[byte >> 4] * sc - zs;
+      v[2 * b + 1] = lut[byte & 15u] * sc - zs;
     }
-    T* o = out + n * out_rs + k0;
+    uint4 ov;
+    T* oe = reinterpret_cast<T*>(&ov);
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      uint4 ov;
-      T* oe = reinterpret_cast<T*>(&ov);
-#pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        const uint32_t byte = (word[u] >> (8 * b)) & 0xFFu;
-        oe[2 * b] = from_f32<T>(lut[byte >> 4] * sc[u] - zs[u]);
-        oe[2 * b + 1] = from_f32<T>(lut[byte & 15u] * sc[u] - zs[u]);
-      }
-      if (k0 + u * 256 < K) *reinterpret_cast<uint4*>(o + u * 256) = ov;
-    }
-    n += step_n;
-    r += step_r;
-    if (r >= runs) { r -= runs; ++n; }
+    for (int j = 0; j < 8; ++j) oe[j] = from_f32<T>(v[j]);
+    *reinterpret_cast<uint4*>(o + wi * 8) = ov;
   }
 }
 
-// Transposed expansion: out_t[k, n] = w[n, k] (out_t row stride out_rs elements), for callers that want W^T itself. One CTA (128 threads)
+// Same expansion with fully coalesced traffic: lane l of a warp takes the 32-bit word l of a 128-byte run of codes (8 weights)
+// and writes one 16-byte vector, so a warp reads 128 contiguous bytes and writes 512 contiguous bytes per step (the kernel
+// above gives every thread a 64-byte output run, i.e. 16-byte pieces at a 64-byte stride per store instruction). Four
+// independent steps per thread keep loads in flight. K % 8 == 0. Measured slower than the kernel above (see b200_w4_dequant): opt-in.
+template <typename T>
+__global__ void __launch_bounds__(256)
+w4_dequant_coalesced_kernel(W4Shards sh, T* __restrict__ out, long long N, int K, int group, const float* __restrict__ lut_g,
+                            long long out_rs) {
+  __shared__ float lut[16];
+  if (threadIdx.x < 16) lut[threadIdx.x] = lut_g ? lut_g[threadIdx.x] : kNF4[threadIdx.x];
+  __syncthreads();
+  constexpr int U = 4;
+  const long long nwords = N * (long long)K / 8;
+  const long long w0 = ((long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31)) * U + (threadIdx.x & 31);
+  const int groups_per_row = K / group;
+  uint32_t code[U];
+  float sc[U], zs[U];
+  long long oidx[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const long long w = w0 + u * 32;
+    oidx[u] = -1;
+    if (w < nwords) {
+      const long long e = w * 8, n = e / K;
+      const int k = (int)(e - n * K);
+      const int s = sh.nshards > 1 ? (int)(n / sh.rows_per_shard) : 0;
+      const long long nl = n - (long long)s * sh.rows_per_shard;
+      code[u] = *reinterpret_cast<const uint32_t*>(sh.packed[s] + (nl * K + k) / 2);
+      sc[u] = sh.scale[s][nl * groups_per_row + k / group];
+      zs[u] = sh.zs[s] ? sh.zs[s][nl * groups_per_row + k / group] : 0.f;
+      oidx[u] = n * out_rs + k;
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    if (oidx[u] < 0) continue;
+    uint4 ov;
+    T* oe = reinterpret_cast<T*>(&ov);
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const uint32_t byte = (code[u] >> (8 * b)) & 0xFFu;
+      oe[2 * b] = from_f32<T>(lut[byte >> 4] * sc[u] - zs[u]);
+      oe[2 * b + 1] = from_f32<T>(lut[byte & 15u] * sc[u] - zs[u]);
+    }
+    *reinterpret_cast<uint4*>(out + oidx[u]) = ov;
+  }
+}
+
+// Transposed expansion: out_t[k, n] = w[n, k] (out_t row stride out_rs elements). Used by the backward pass so that
+// dgrad (dY x W) reads W^T as a K-major tcgen05 operand instead of the slower MN-major path. One CTA (128 threads)
 // owns a 64(n) x 64(k) tile: each thread expands one 16-byte chunk (32 weights of one row) into a padded shared
 // tile t[k][n], then the tile is written out as 64 rows of 128 contiguous bytes. N % 64 == 0, K % 64 == 0.
 template <typename T>
@@ -407,14 +439,23 @@ B200_API int b200_w4_dequant(const void* const* packed, const void* const* scale
   }
   sh.rows_per_shard = rows_per_shard;
   sh.nshards = nshards;
-  int shift = -1;
-  if ((group & (group - 1)) == 0)
-    for (shift = 0; (1 << shift) < group;) ++shift;
-  const long long blocks = (N * ((K + 1023) / 1024) + 7) / 8;
-  const unsigned grid = (unsigned)(blocks < kNumSMs * kW4ExpandBlocks ? blocks : kNumSMs * kW4ExpandBlocks);
+  const long long chunks = N * (K / 32);
+  const unsigned grid = (unsigned)((chunks + 255) / 256);
   cudaStream_t st = (cudaStream_t)stream;
-  if (out_dtype == B200_DT_BF16) w4_dequant_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(sh, (__nv_bfloat16*)out, N, K, group, shift, lut, out_rs);
-  else if (out_dtype == B200_DT_FP16) w4_dequant_kernel<__half><<<grid, 256, 0, st>>>(sh, (__half*)out, N, K, group, shift, lut, out_rs);
+  // measured inside a training step (8-layer slice, ncu launch list): 63.5 us per call for the coalesced kernel vs 47.7 us for
+  // the one-chunk-per-thread kernel below (4x the load instructions, scale fetched per word) — kept as an option only
+  static const bool coalesced = getenv("B200_W4_DEQUANT_COALESCED") != nullptr;
+  if (coalesced && out_rs % 8 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
+    const long long nwords = N * (long long)K / 8;
+    const unsigned g2 = (unsigned)((nwords + 256 * 4 - 1) / (256 * 4));
+    if (out_dtype == B200_DT_BF16) w4_dequant_coalesced_kernel<__nv_bfloat16><<<g2, 256, 0, st>>>(sh, (__nv_bfloat16*)out, N, K, group, lut, out_rs);
+    else if (out_dtype == B200_DT_FP16) w4_dequant_coalesced_kernel<__half><<<g2, 256, 0, st>>>(sh, (__half*)out, N, K, group, lut, out_rs);
+    else return B200_ERR_UNSUPPORTED;
+    B200_LAUNCH_CHECK();
+    return 0;
+  }
+  if (out_dtype == B200_DT_BF16) w4_dequant_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(sh, (__nv_bfloat16*)out, N, K, group, lut, out_rs);
+  else if (out_dtype == B200_DT_FP16) w4_dequant_kernel<__half><<<grid, 256, 0, st>>>(sh, (__half*)out, N, K, group, lut, out_rs);
   else return B200_ERR_UNSUPPORTED;
   B200_LAUNCH_CHECK();
   return 0;

@@ -197,21 +197,14 @@ class FusedLinear(nn.Module):
         self.nf4 = q
         self.weight = None
 
-    def _ahead(self) -> bool:
-        return dq.ENABLED and self.nf4.packed.is_cuda and nv.available() and not torch.cuda.is_current_stream_capturing()
-
-    def _materialize_weight(self, dtype=None, backward: bool = False) -> torch.Tensor:
+    def _materialize_weight(self, dtype=None) -> torch.Tensor:
         if self.nf4 is not None:
             dtype = dtype or torch.bfloat16
-            if self._ahead():
-                return dq.pipeline(self.nf4.packed.device).get(self.nf4, dtype, backward)   # expanded one GEMM ahead
+            if dq.ENABLED and self.nf4.packed.is_cuda and nv.available() and not torch.cuda.is_current_stream_capturing():
+                return dq.pipeline(self.nf4.packed.device).get(self.nf4, dtype, False)   # expanded one GEMM ahead
             ws = weight_workspace(self.nf4.packed.device, dtype, self.out_features * self.in_features)
             return self.nf4.dequantize(dtype, out=ws.view(self.out_features, self.in_features))
         return self.weight
-
-    def _weight_done(self) -> None:
-        if self.nf4 is not None and self._ahead():
-            dq.pipeline(self.nf4.packed.device).done()
 
     def _fwd(self, x: torch.Tensor, lora=None) -> torch.Tensor:
         """y = x W^T (+ low-rank term) (+ bias); a 4-bit base goes through the dequant-fused tcgen05 GEMM."""
@@ -219,21 +212,23 @@ class FusedLinear(nn.Module):
             y = gemm_w4(x, self.nf4, lora=lora, bias=self.bias)
             if y is not None:
                 return y
-        y = gemm(x, self._materialize_weight(x.dtype), lora=lora, bias=self.bias)
-        self._weight_done()
-        return y
+        return gemm(x, self._materialize_weight(x.dtype), lora=lora, bias=self.bias)
 
     def _dgrad(self, dy: torch.Tensor, lora=None) -> torch.Tensor:
-        """dX = dY x W (+ low-rank term). W is read as it is stored, an MN-major operand: expanding a 4-bit base to W^T instead took
-        227 us a weight of the 5120-wide layer, W itself 90, and the product is a few per cent from the K-major one (2048 x 5120 x 16384:
-        249 us against 233)."""
-        if self.nf4 is not None:
-            dx = gemm_w4(dy, self.nf4, b_mn=True, lora=lora)   # codes expanded inside the GEMM (peer shards included)
+        """dX = dY x W (+ low-rank term). A 4-bit base is expanded straight into W^T so the GEMM reads two K-major
+        operands (the MN-major B path of the tcgen05 kernel is ~25 % slower)."""
+        q = self.nf4
+        if q is not None:
+            dx = gemm_w4(dy, q, b_mn=True, lora=lora)          # codes expanded inside the GEMM (peer shards included)
             if dx is not None:
                 return dx
-        dx = gemm(dy, self._materialize_weight(dy.dtype, True), b_mn=True, lora=lora)
-        self._weight_done()
-        return dx
+        if q is not None and dy.is_cuda and getattr(q, "can_transpose", lambda: False)() and dy.dtype != torch.float32:
+            if dq.ENABLED and nv.available() and not torch.cuda.is_current_stream_capturing():
+                return gemm(dy, dq.pipeline(q.packed.device).get(q, dy.dtype, True), lora=lora)
+            ws = weight_workspace(q.packed.device, dy.dtype, self.out_features * self.in_features)
+            wt = q.dequantize(dy.dtype, out=ws.view(self.in_features, self.out_features), transpose=True)
+            return gemm(dy, wt, lora=lora)
+        return gemm(dy, self._materialize_weight(dy.dtype), b_mn=True, lora=lora)
 
     def dense_weight(self) -> torch.Tensor:
         """A fresh dense copy of the base weight (for merging / export)."""
