@@ -216,7 +216,7 @@ class FusedLinear(nn.Module):
 
     def _dgrad(self, dy: torch.Tensor, lora=None) -> torch.Tensor:
         """dX = dY x W (+ low-rank term). A 4-bit base is expanded straight into W^T so the GEMM reads two K-major
-        operands (the MN-major B path of the tcgen05 kernel is ~25 % slower)."""
+        operands (the MN-major B path of the tcgen05 kernel is ~7 % slower)."""
         q = self.nf4
         if q is not None:
             dx = gemm_w4(dy, q, b_mn=True, lora=lora)          # codes expanded inside the GEMM (peer shards included)

@@ -31,6 +31,7 @@ for name, out_f, in_f in shapes:
     q = NF4Weight.quantize(w, True)
     del w
     ws = torch.empty(out_f, in_f, device=dev, dtype=torch.bfloat16)
+    wst = torch.empty(in_f, out_f, device=dev, dtype=torch.bfloat16)
     x = torch.randn(M, in_f, device=dev, dtype=torch.bfloat16)
     dy = torch.randn(M, out_f, device=dev, dtype=torch.bfloat16)
     y = torch.empty(M, out_f, device=dev, dtype=torch.bfloat16)
@@ -38,7 +39,7 @@ for name, out_f, in_f in shapes:
     fl = 2.0 * M * out_f * in_f
     for tag, fused, unfused, cublas in (
         ("fwd", lambda: G.gemm_w4(x, q, out=y, force=True), lambda: G.gemm(x, q.dequantize(out=ws), out=y), lambda: torch.matmul(x, ws.t(), out=y)),
-        ("dgrad", lambda: G.gemm_w4(dy, q, b_mn=True, out=dx, force=True), lambda: G.gemm(dy, q.dequantize(out=ws), b_mn=True, out=dx),
+        ("dgrad", lambda: G.gemm_w4(dy, q, b_mn=True, out=dx, force=True), lambda: G.gemm(dy, q.dequantize(out=wst, transpose=True), out=dx),
          lambda: torch.matmul(dy, ws, out=dx))):
         tf, tu, tc = timeit(fused), timeit(unfused), timeit(cublas)
         rows.append({"shape": f"{name} {tag}", "M": M, "out": out_f, "in": in_f, "fused_ms": round(tf, 4), "dequant+gemm_ms": round(tu, 4),
