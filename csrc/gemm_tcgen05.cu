@@ -518,6 +518,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
       const int bb0 = btb % p.nb0_b, bb1 = btb / p.nb0_b;
       for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
         if (!free) mbar_wait(empty_bar(stage), phase ^ 1u);
+        __syncwarp();
         const uint32_t fb = fb0 + 8u * stage;
         const uint32_t sa = sA0 + (uint32_t)stage * kStageABytes;
         const uint32_t sb = sB0 + (uint32_t)stage * stage_b_bytes;
@@ -587,6 +588,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
         const uint32_t d_tmem = tmem_base + (uint32_t)acc * kAccStride;
         for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
           if (!full) mbar_wait(full_bar(stage), phase);
+          __syncwarp();   // lanes may have seen the barrier at different times: one of all 32 is elected
           tc_fence_after();
           const int cur = stage;
           if (++stage == p.stages) { stage = 0; phase ^= 1u; }
