@@ -58,7 +58,7 @@ struct GemmKernelParams {
   float* sk_ws;
   unsigned int* sk_flags;
   unsigned int sk_epoch;      // host-provided epoch (used when sk_state is null)
-  unsigned int* sk_state;     // device epoch: [0] = epoch of the last stream-K launch, [1] = ticket counter (graph-replayable)
+  unsigned int* sk_state;     // device epoch: [0] = epoch of the last stream-K launch, [1] = units that have started (graph-replayable)
   // K16 (grouped GEMM): b_map[batch] = which B matrix (and bias row) batch entry `batch` multiplies with, -1 = skip the
   // entry. Read on the device, so the grouping (tokens sorted by expert) never visits the host.
   const int* b_map;
@@ -123,7 +123,7 @@ struct SegmentIter {
   long long item, end;  // stream-K: current / last work item of this unit
   int tile, stride, total_tiles, nkt, grp_size, member;
   bool stream_k;
-  __device__ SegmentIter(const GemmKernelParams& p, int unit, int nunits, int total_tiles_, int nkt_) {
+  __host__ __device__ SegmentIter(const GemmKernelParams& p, int unit, int nunits, int total_tiles_, int nkt_) {
     stream_k = p.stream_k != 0;
     total_tiles = total_tiles_;
     nkt = nkt_;
@@ -144,7 +144,7 @@ struct SegmentIter {
       item = end = 0;   // spare units beyond the last whole group
     }
   }
-  __device__ bool next(Segment& s) {
+  __host__ __device__ bool next(Segment& s) {
     if (!stream_k) {
       if (tile >= total_tiles) return false;
       s.tile = tile; s.kb0 = 0; s.kb1 = nkt;
@@ -161,6 +161,19 @@ struct SegmentIter {
     return true;
   }
 };
+
+// A tile's owner waits for units of higher numbers, which hold its later k-blocks. So the n-th unit to START takes the n-th number from the end: what it
+// waits for has been on an SM before it, waits in its turn only for what started earlier still, and the first one waits for nobody. Whatever else is
+// on the GPU, and however few units are there at once, a launch gets to its end. (By block index an owner waited for CTAs that nothing had yet
+// given an SM.)
+__host__ __device__ __forceinline__ int sk_unit_of(int started, int nunits) { return nunits - 1 - started; }
+// how many units after this one's group hold later k-blocks of a tile that it begins
+__host__ __device__ __forceinline__ int sk_parts_after(int tile, int group, int groups, int grp_size, long long total, int nkt) {
+  const long long tile_end = (long long)(tile / grp_size + 1) * nkt;
+  int n = 0;
+  for (int v = group + 1; v < groups && total * v / groups < tile_end; ++v) ++n;
+  return n;
+}
 
 // tcgen05.mma from converged code: the whole warp runs the issue loop and elect.sync picks the lane, always the same one. From a branch of one thread
 // four products and a commit took 420 cycles whatever their size, and waiting for the stage 70 to 180 more, where the pipe takes 512 for
@@ -404,38 +417,38 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
   const uint32_t raw0 = sB0 + (uint32_t)p.stages * stage_b_bytes;          // packed-code ring (W4 only)
   const uint32_t lut0 = raw0 + (uint32_t)raw_stages * kRawStageBytes;      // byte -> 2 x 16-bit table, one copy per lane
   const uint32_t bar0 = lut0 + (W4 ? (uint32_t)w4->lut_bytes : 0u);
-  // barrier block: full[stages] | empty[stages] | tmem_full[2] | tmem_empty[2] | tmem_ptr | raw_full[] | raw_empty[]
+  // barrier block: full[stages] | empty[stages] | tmem_full[2] | tmem_empty[2] | tmem_ptr | unit, epoch | raw_full[] | raw_empty[]
   auto full_bar = [&](int s) { return bar0 + 8u * s; };
   auto empty_bar = [&](int s) { return bar0 + 8u * (p.stages + s); };
   auto tfull_bar = [&](int a) { return bar0 + 8u * (2 * p.stages + a); };
   auto tempty_bar = [&](int a) { return bar0 + 8u * (2 * p.stages + 2 + a); };
   const uint32_t tmem_slot = bar0 + 8u * (2 * p.stages + 4);
-  auto rfull_bar = [&](int s) { return bar0 + 8u * (2 * p.stages + 5 + s); };
-  auto rempty_bar = [&](int s) { return bar0 + 8u * (2 * p.stages + 5 + raw_stages + s); };
+  auto rfull_bar = [&](int s) { return bar0 + 8u * (2 * p.stages + 6 + s); };
+  auto rempty_bar = [&](int s) { return bar0 + 8u * (2 * p.stages + 6 + raw_stages + s); };
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const uint32_t rank = CTAS == 2 ? cluster_ctarank() : 0u;
   const bool leader = rank == 0;
-  const int unit = blockIdx.x / CTAS, nunits = gridDim.x / CTAS;
+  const int nunits = gridDim.x / CTAS;
 
-  const uint32_t sk_epoch_slot = tmem_slot + 4u;   // second half of the 8-byte TMEM-pointer slot (no static shared memory: the
-                                                   // dynamic allocation already takes the whole 227 KB)
+  const uint32_t sk_unit_slot = tmem_slot + 8u;    // unit and epoch (no static shared memory: the dynamic allocation already takes the whole 227 KB)
   if (warp == 0 && lane == 0) {
-    if (p.stream_k) {
-      unsigned int e = p.sk_epoch;
+    if (p.stream_k && leader) {
+      unsigned int e = p.sk_epoch, started = blockIdx.x / CTAS;
       if (p.sk_state) {
-        // every CTA of the launch reads the old epoch, then takes a ticket; the last ticket publishes the new epoch for the
+        // every unit of the launch reads the old epoch, then counts itself; the last one publishes the new epoch for the
         // next launch on this stream. Nothing here comes from the host, so a captured launch can be replayed.
         e = *((volatile unsigned int*)p.sk_state) + 1u;
         __threadfence();
-        if (atomicAdd(p.sk_state + 1, 1u) == gridDim.x - 1) {
+        started = atomicAdd(p.sk_state + 1, 1u);
+        if (started == (unsigned)nunits - 1u) {
           p.sk_state[1] = 0u;
           __threadfence();
           *((volatile unsigned int*)p.sk_state) = e;
         }
-      }
-      asm volatile("st.shared.u32 [%0], %1;" ::"r"(sk_epoch_slot), "r"(e) : "memory");
+      }                                            // a workspace without the counter: blocks are given SMs in the order of their index
+      asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(sk_unit_slot), "r"(sk_unit_of((int)started, nunits)), "r"(e) : "memory");
     }
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
@@ -481,6 +494,12 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
   tc_fence_after();
   uint32_t tmem_base;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
+  int unit = blockIdx.x / CTAS;
+  unsigned int sk_epoch_v = 0;
+  if (p.stream_k) {                                // the leader's, which stays until its peer is done
+    if constexpr (CTAS == 1) asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(unit), "=r"(sk_epoch_v) : "r"(sk_unit_slot) : "memory");
+    else asm volatile("ld.shared::cluster.v2.u32 {%0, %1}, [%2];" : "=r"(unit), "=r"(sk_epoch_v) : "r"(mapa_shared(sk_unit_slot, 0)) : "memory");
+  }
 
   const int tiles_per_batch = p.num_m * p.num_n;
   const int total_tiles = tiles_per_batch * p.batch;
@@ -767,15 +786,13 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
     SegmentIter it(p, unit, nunits, total_tiles, num_k_total);
     Segment sg;
     const int sk_g = p.stream_k ? p.sk_group : 1;
-    unsigned int sk_epoch_v = 0;
-    if (p.stream_k) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(sk_epoch_v) : "r"(sk_epoch_slot) : "memory");
     const int sk_groups = nunits / sk_g, sk_grp = unit / sk_g;
     const long long sk_total = (long long)(total_tiles / sk_g) * num_k_total;
     // fused all-reduce: this CTA's reduction items are ar_next, ar_next + gridDim.x, ... < ar_items (see ar_reduce)
     const int ar_slabs = (kBM * CTAS) / kArSlabRows;
     const int ar_items = p.ar_world > 1 ? ((total_tiles - p.ar_rank + p.ar_world - 1) / p.ar_world) * ar_slabs : 0;
     int ar_next = blockIdx.x;
-    const uint32_t ar_poll_slot = sk_epoch_slot;     // stream-K is off in this mode: the slot is free
+    const uint32_t ar_poll_slot = sk_unit_slot;      // stream-K is off in this mode: the slot is free
     while (it.next(sg)) {
       const int tile = sg.tile;
       const int bt = tile / tiles_per_batch;
@@ -800,7 +817,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
         // ---- stream-K contributor: publish this CTA's fp32 partial, the tile's owner finishes it ----
         // laid out [16-byte piece][row], so that a warp's store or load is whole lines (a row to a lane is 32 lines an instruction:
         // 2048 x 5120 x 34816 625 us, now 596; 490 x 4096 x 12288 76, now 68)
-        uint4* slot = reinterpret_cast<uint4*>(p.sk_ws + (long long)blockIdx.x * kBM * kAccStride) + q * 32 + lane;
+        uint4* slot = reinterpret_cast<uint4*>(p.sk_ws + (long long)(unit * CTAS + (int)rank) * kBM * kAccStride) + q * 32 + lane;
         for (int c = 0; c < nchunks; ++c) {
           uint32_t r[32];
           tmem_ld_32x32(t0 + c * 32, r);
@@ -811,13 +828,12 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
         }
         __threadfence();
         asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (threadIdx.x == 64) asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p.sk_flags + blockIdx.x), "r"(sk_epoch_v) : "memory");
+        if (threadIdx.x == 64) asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p.sk_flags + unit * CTAS + (int)rank), "r"(sk_epoch_v) : "memory");
       } else {
         // number of following units that hold later k-blocks of this tile (0 unless stream-K split it)
         int ncontrib = 0;
         if (sg.kb1 < num_k_total) {
-          const long long tile_end = (long long)(tile / sk_g + 1) * num_k_total;
-          for (int v = sk_grp + 1; v < sk_groups && sk_total * v / sk_groups < tile_end; ++v) ++ncontrib;
+          ncontrib = sk_parts_after(tile, sk_grp, sk_groups, sk_g, sk_total, num_k_total);
           for (int v = 1; v <= ncontrib; ++v) {
             const unsigned int* f = p.sk_flags + (unit + v * sk_g) * CTAS + rank;   // same member of the next group
             unsigned int seen;
@@ -825,7 +841,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
             do {
               asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(f) : "memory");
               if (clock64() - tw > 20000000000ll) {
-                printf("b200 gemm: stream-K wait timed out (block %d waits for block %d)\n", blockIdx.x, (unit + v * sk_g) * CTAS + (int)rank);
+                printf("b200 gemm: stream-K wait timed out (unit %d waits for unit %d)\n", unit, unit + v * sk_g);
                 __trap();
               }
             } while (seen != sk_epoch_v);
@@ -1063,6 +1079,38 @@ B200_API int b200_gemm_plan(int M, int N, int K, int batch, int b_mn, int in_dty
   return 0;
 }
 
+// Which units of a product that is cut wait for which, by the order in which they start (0 first): pairs (waits, waited for), at most `cap` of
+// them into `pairs`; the return value is how many there are, 0 for a product of whole tiles, or minus a status. A launch gets to its end with any number of
+// units on the GPU at once as long as none waits for one that starts after it.
+B200_API int b200_gemm_streamk_waits(int M, int N, int K, int batch, int b_mn, int in_dtype, int num_sms, int* pairs, int cap) {
+  if (M <= 0 || N <= 0 || K <= 0 || batch <= 0 || num_sms <= 0 || cap < 0 || (cap > 0 && !pairs)) return -B200_ERR_BAD_SHAPE;
+  const int EPR = in_dtype == B200_DT_FP32 ? 32 : 64, nkt = ceil_div(K, EPR);
+  const GemmConfig c = pick_config(M, N, batch, nkt, b_mn ? 1 : 0, EPR, num_sms, true);
+  if (!c.stream_k) return 0;
+  GemmKernelParams p = {};
+  const int nunits = num_sms / c.ctas, num_m = ceil_div(M, kBM * c.ctas), tiles = batch * num_m * ceil_div(N, c.bn);
+  p.stream_k = 1;
+  p.sk_group = sk_group_of(num_m, nunits);
+  const int groups = nunits / p.sk_group;
+  int n = 0;
+  for (int started = 0; started < nunits; ++started) {
+    const int unit = sk_unit_of(started, nunits);
+    SegmentIter it(p, unit, nunits, tiles, nkt);
+    Segment sg;
+    while (it.next(sg)) {
+      if (sg.kb0 > 0 || sg.kb1 == nkt) continue;
+      const int parts = sk_parts_after(sg.tile, unit / p.sk_group, groups, p.sk_group, (long long)(tiles / p.sk_group) * nkt, nkt);
+      for (int v = 1; v <= parts; ++v, ++n) {
+        if (n >= cap) continue;
+        pairs[2 * n] = started;
+        for (int other = 0; other < nunits; ++other)
+          if (sk_unit_of(other, nunits) == unit + v * p.sk_group) pairs[2 * n + 1] = other;
+      }
+    }
+  }
+  return n;
+}
+
 // A full-size workspace (b200_gemm_workspace_bytes()) carries the stream-K epoch on the device, in its last 16 bytes:
 // every stream-K launch on that workspace (b200_gemm and b200_gemm_w4 alike) then takes its epoch from there and the launch
 // can be captured in a CUDA graph. A smaller workspace falls back to the host-side counters.
@@ -1223,7 +1271,7 @@ B200_API int b200_gemm(const b200_gemm_args* a, void* stream_) {
   }
   const int units = g_num_sms / ctas;
   const int grid = (cfg.stream_k ? units : (int)(total_tiles < units ? total_tiles : units)) * ctas;
-  const int smem = stages * stage_bytes + 8 * (2 * stages + 5) + 1024;
+  const int smem = stages * stage_bytes + 8 * (2 * stages + 6) + 1024;
   if (ES == 2) rc = ctas == 2 ? launch<2, 2>(tmA, tmB, tmA2, tmB2, p, grid, smem, stream)
                               : launch<2, 1>(tmA, tmB, tmA2, tmB2, p, grid, smem, stream);
   else rc = ctas == 2 ? launch<4, 2>(tmA, tmB, tmA2, tmB2, p, grid, smem, stream)
@@ -1305,7 +1353,7 @@ B200_API int b200_gemm_w4(const b200_gemm_args* a, const b200_w4_desc* w, void* 
   static const bool env_nolut = getenv("B200_W4_NOLUT") != nullptr;
   if (env_raw >= 0) raw_stages = env_raw;
   if (env_nolut) lut_bytes = 0;
-  int stages = (g_max_smem - 1024 - lut_bytes - raw_stages * kRawStageBytes - 8 * (2 * 8 + 5 + 2 * raw_stages)) / stage_bytes;
+  int stages = (g_max_smem - 1024 - lut_bytes - raw_stages * kRawStageBytes - 8 * (2 * 8 + 6 + 2 * raw_stages)) / stage_bytes;
   if (stages > 8) stages = 8;
   if (stages < 3) return B200_ERR_UNSUPPORTED;
   p.stages = stages;
@@ -1365,7 +1413,7 @@ B200_API int b200_gemm_w4(const b200_gemm_args* a, const b200_w4_desc* w, void* 
 #endif
 
   const int grid = (p.stream_k ? units : (int)(tiles < units ? tiles : units)) * ctas;
-  const int smem = stages * stage_bytes + raw_stages * kRawStageBytes + lut_bytes + 8 * (2 * stages + 5 + 2 * raw_stages) + 1024;
+  const int smem = stages * stage_bytes + raw_stages * kRawStageBytes + lut_bytes + 8 * (2 * stages + 6 + 2 * raw_stages) + 1024;
   static bool configured = false;
   if (!configured) {
     B200_CHECK(cudaFuncSetAttribute(gemm_w4_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, g_max_smem));

@@ -111,6 +111,8 @@ int b200_gemm(const b200_gemm_args* args, void* stream);
 /* How that call is cut where it has a workspace, on a part of num_sms SMs (needs no GPU): plan[4] = CTAs of a tile, columns of a tile, whether k
  * is cut into parts, k-blocks (128 bytes of a row) of the longest chain of additions. */
 int b200_gemm_plan(int M, int N, int K, int batch, int b_mn, int in_dtype, int num_sms, int* plan);
+/* Pairs (unit that waits, unit waited for) of such a product, units by the order in which they start; returns their number, or minus a status */
+int b200_gemm_streamk_waits(int M, int N, int K, int batch, int b_mn, int in_dtype, int num_sms, int* pairs, int cap);
 /* b200_gemm of two matrices (batch 1) with plain arguments, for callers to whom filling the structure costs more than the launch. */
 int b200_gemm_2d(const void* A, const void* B, void* D, const void* bias, const float* beta_rows, const void* A2, const void* B2,
                  void* workspace, long long workspace_bytes, int M, int N, int K, int K2, long long a_rs, long long b_rs, long long d_rs,

@@ -48,10 +48,10 @@ _overlapped_collectives = 0
 def overlapped_collectives(active: bool) -> None:
     """Called by the wrappers that run a peer-memory collective kernel on a side stream WHILE compute continues (DDP
     bucket all-reduce, FSDP reduce-scatter). Such a kernel spins on flags and has a grid barrier, i.e. it needs all of
-    its CTAs resident; a stream-K GEMM needs all of ITS CTAs resident too (tile owners wait for the partial sums of
-    other CTAs). Two kernels of that kind pending on one GPU can each get only part of their CTAs placed and then wait
-    for each other forever (seen as "stream-K wait timed out" in the 2-GPU DDP suite). While any such wrapper is alive,
-    GEMMs therefore run one CTA pair per tile (no cross-CTA dependency: their CTAs always drain)."""
+    its CTAs resident. Tile owners of a stream-K GEMM wait for the partial sums of other CTAs; when those were numbered by
+    their index, both kernels could get only part of their CTAs placed and wait for each other ("stream-K wait timed out"
+    in the 2-GPU DDP suite). Owners now wait only for CTAs that started before them, so a GEMM drains by itself, but no run
+    on several GPUs has shown the two side by side since: while any such wrapper is alive, GEMMs run one CTA pair per tile."""
     global _overlapped_collectives
     _overlapped_collectives = max(0, _overlapped_collectives + (1 if active else -1))
 

@@ -38,6 +38,23 @@ def test_chains_of_few_tiles_stay_short(m, n, k, chain):
 
 
 @library
+@pytest.mark.parametrize("sms", [148, 132, 7])
+@pytest.mark.parametrize("m,n,k", [(20, 4096, 2048), (64, 4096, 4096), (64, 5120, 17408), (300, 4096, 16384), (490, 6144, 4096), (549, 2048, 2048),
+                                   (1024, 72, 4096), (2048, 5120, 5120), (2048, 5120, 17408), (2345, 2048, 2048)])
+def test_parts_wait_only_for_what_started_before_them(m, n, k, sms):
+    """A tile's owner sums the parts of other units. Units that start in order, each kept on the GPU until what it waits for is there, all finish
+    whatever the number that fits at once, one included; they do not if one waits for a unit that starts after it."""
+    fn = nv.proto("b200_gemm_streamk_waits", [ctypes.c_int] * 7 + [ctypes.c_void_p, ctypes.c_int])
+    out = (ctypes.c_int * 4000)()
+    count = fn(m, n, k, 1, 0, nv.DT_BF16, sms, ctypes.addressof(out), 2000)
+    plan = (ctypes.c_int * 4)()
+    assert nv.proto("b200_gemm_plan", [ctypes.c_int] * 7 + [ctypes.c_void_p])(m, n, k, 1, 0, nv.DT_BF16, sms, ctypes.addressof(plan)) == 0
+    assert 0 <= count <= 2000 and (count > 0) == bool(plan[2])
+    waits = [(out[2 * i], out[2 * i + 1]) for i in range(count)]
+    assert all(0 <= other < unit < sms // plan[0] for unit, other in waits)
+
+
+@library
 @pytest.mark.parametrize("m,n,k,b_mn", [
     (4096, 1536, 512, 0), (2345, 1536, 512, 0), (2345, 2048, 512, 0), (4096, 1000, 640, 0), (1024, 768, 768, 0), (1024, 3072, 768, 0), (300, 768, 768, 0),
     (549, 1024, 1024, 0), (300, 5120, 2048, 0), (512, 768, 768, 1), (549, 16, 2048, 0), (8192, 8192, 8192, 0)])
