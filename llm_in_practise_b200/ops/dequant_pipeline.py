@@ -15,6 +15,7 @@ the ZeRO-3 shard prefetcher (parallel/zero.py) a single consumer stream.
 from __future__ import annotations
 
 import os
+import weakref
 from typing import Dict, Optional, Tuple
 
 import torch
@@ -23,13 +24,14 @@ ENABLED = os.environ.get("B200_DEQUANT_AHEAD", "1") != "0"
 
 
 class _Slot:
-    __slots__ = ("buf", "key", "ready", "used")
+    __slots__ = ("buf", "key", "ready", "used", "home", "stream")
 
     def __init__(self):
         self.buf: Optional[torch.Tensor] = None
         self.key = None
         self.ready = torch.cuda.Event()
         self.used = torch.cuda.Event()      # recorded on the compute stream once the consumer GEMM is enqueued
+        self.home = self.stream = None      # the streams whose pool the buffer is from, and that it was handed to
 
 
 class DequantPipeline:
@@ -38,34 +40,64 @@ class DequantPipeline:
         self.stream = torch.cuda.Stream(device)
         self.slots = [_Slot() for _ in range(nslots)]
         self.next_of: Dict[tuple, Tuple[object, torch.dtype, bool]] = {}
+        self.known: Dict[int, weakref.ref] = {}   # by id, the weights that the side stream has been ordered after
         self.prev_key = None
         self.cur = -1                       # slot handed out by the last request
         self.hits = self.misses = 0
 
-    def _expand(self, slot: _Slot, q, dtype, transpose: bool, key) -> None:
+    def release(self) -> None:
+        """Before the buffers go back to their pools: what runs there next comes after their last expansions and products."""
+        for slot in self.slots:
+            self._give_back(slot)
+
+    def _give_back(self, slot: _Slot) -> None:
+        if slot.buf is not None:
+            if slot.stream is not None:
+                slot.used.record(slot.stream)
+            slot.home.wait_event(slot.ready)
+            slot.home.wait_event(slot.used)
+            slot.buf = slot.key = None
+
+    def _expand(self, slot: _Slot, q, dtype, transpose: bool, key, comp) -> None:
         n = q.N * q.K
+        after = self.known.get(id(q))
+        behind = after is None or after() is not q                       # the weight may still be on its way on the compute stream
         if slot.buf is None or slot.buf.dtype != dtype or slot.buf.numel() < n:
+            self._give_back(slot)
             slot.buf = torch.empty(n, dtype=dtype, device=self.device)
+            slot.home = comp
+            behind = True                                                # and so may what had this memory before
+        if behind:
+            self.stream.wait_stream(comp)
         self.stream.wait_event(slot.used)                                # the GEMM that last read this buffer is done
         with torch.cuda.stream(self.stream):
             shape = (q.K, q.N) if transpose else (q.N, q.K)
             q.dequantize(dtype, out=slot.buf[:n].view(shape), transpose=transpose)
             slot.ready.record(self.stream)
+        if behind:
+            self.known[id(q)] = weakref.ref(q, lambda _, i=id(q): self._forget(i))
         slot.key = key
+
+    def _forget(self, i: int) -> None:
+        entry = self.known.get(i)
+        if entry is not None and entry() is None:
+            del self.known[i]
 
     def get(self, q, dtype: torch.dtype, transpose: bool) -> torch.Tensor:
         key = (id(q), dtype, transpose)
         comp = torch.cuda.current_stream(self.device)
         if self.cur >= 0:
-            self.slots[self.cur].used.record(comp)                       # previous consumer is enqueued before this point
+            last = self.slots[self.cur]
+            last.used.record(last.stream)                                # previous consumer is enqueued before this point
         hit = next((i for i, s in enumerate(self.slots) if s.key == key), None)
         if hit is None:
             self.misses += 1
             hit = (self.cur + 1) % len(self.slots)
-            self._expand(self.slots[hit], q, dtype, transpose, key)
+            self._expand(self.slots[hit], q, dtype, transpose, key, comp)
         else:
             self.hits += 1
         slot = self.slots[hit]
+        slot.stream = comp
         comp.wait_event(slot.ready)
         if self.prev_key is not None:
             self.next_of[self.prev_key] = (q, dtype, transpose)
@@ -76,7 +108,7 @@ class DequantPipeline:
             nkey = (id(nq), ndt, ntr)
             other = (hit + 1) % len(self.slots)
             if self.slots[other].key != nkey:
-                self._expand(self.slots[other], nq, ndt, ntr, nkey)
+                self._expand(self.slots[other], nq, ndt, ntr, nkey, comp)
         n = q.N * q.K
         return slot.buf[:n].view((q.K, q.N) if transpose else (q.N, q.K))
 
@@ -93,4 +125,6 @@ def pipeline(device: torch.device) -> DequantPipeline:
 
 
 def reset() -> None:
+    for p in _pipes.values():
+        p.release()
     _pipes.clear()
