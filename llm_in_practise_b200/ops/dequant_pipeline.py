@@ -23,15 +23,24 @@ import torch
 ENABLED = os.environ.get("B200_DEQUANT_AHEAD", "1") != "0"
 
 
+def _stamp(q) -> tuple:
+    """What changes when a weight's codes or scales are written or replaced."""
+    return tuple((t.data_ptr(), 0 if t.is_inference() else t._version) for t in vars(q).values() if isinstance(t, torch.Tensor))
+
+
 class _Slot:
-    __slots__ = ("buf", "key", "ready", "used", "home", "stream")
+    __slots__ = ("buf", "key", "ref", "stamp", "ready", "used", "home", "stream")
 
     def __init__(self):
         self.buf: Optional[torch.Tensor] = None
-        self.key = None
+        self.key = self.stamp = None
+        self.ref = lambda: None             # the weight it holds; an id alone may be another object's by now
         self.ready = torch.cuda.Event()
         self.used = torch.cuda.Event()      # recorded on the compute stream once the consumer GEMM is enqueued
         self.home = self.stream = None      # the streams whose pool the buffer is from, and that it was handed to
+
+    def holds(self, q, key, stamp) -> bool:
+        return self.key == key and self.ref() is q and self.stamp == stamp
 
 
 class DequantPipeline:
@@ -39,8 +48,8 @@ class DequantPipeline:
         self.device = device
         self.stream = torch.cuda.Stream(device)
         self.slots = [_Slot() for _ in range(nslots)]
-        self.next_of: Dict[tuple, Tuple[object, torch.dtype, bool]] = {}
-        self.known: Dict[int, weakref.ref] = {}   # by id, the weights that the side stream has been ordered after
+        self.next_of: Dict[tuple, Tuple[object, torch.dtype, bool]] = {}     # weakly: a model that is gone leaves nothing here
+        self.known: Dict[int, tuple] = {}   # id -> (weight, stamp) that the side stream has been ordered after
         self.prev_key = None
         self.cur = -1                       # slot handed out by the last request
         self.hits = self.misses = 0
@@ -58,10 +67,10 @@ class DequantPipeline:
             slot.home.wait_event(slot.used)
             slot.buf = slot.key = None
 
-    def _expand(self, slot: _Slot, q, dtype, transpose: bool, key, comp) -> None:
+    def _expand(self, slot: _Slot, q, dtype, transpose: bool, key, stamp, comp) -> None:
         n = q.N * q.K
         after = self.known.get(id(q))
-        behind = after is None or after() is not q                       # the weight may still be on its way on the compute stream
+        behind = after is None or after[0]() is not q or after[1] != stamp   # the weight may still be on its way on the compute stream
         if slot.buf is None or slot.buf.dtype != dtype or slot.buf.numel() < n:
             self._give_back(slot)
             slot.buf = torch.empty(n, dtype=dtype, device=self.device)
@@ -74,41 +83,42 @@ class DequantPipeline:
             shape = (q.K, q.N) if transpose else (q.N, q.K)
             q.dequantize(dtype, out=slot.buf[:n].view(shape), transpose=transpose)
             slot.ready.record(self.stream)
+        stamp = _stamp(q)                                                # a first expansion may add a table to the weight
         if behind:
-            self.known[id(q)] = weakref.ref(q, lambda _, i=id(q): self._forget(i))
-        slot.key = key
+            self.known[id(q)] = (weakref.ref(q, lambda _, i=id(q): self._forget(i)), stamp)
+        slot.key, slot.ref, slot.stamp = key, weakref.ref(q), stamp
 
     def _forget(self, i: int) -> None:
         entry = self.known.get(i)
-        if entry is not None and entry() is None:
+        if entry is not None and entry[0]() is None:
             del self.known[i]
 
     def get(self, q, dtype: torch.dtype, transpose: bool) -> torch.Tensor:
-        key = (id(q), dtype, transpose)
+        key, stamp = (id(q), dtype, transpose), _stamp(q)
         comp = torch.cuda.current_stream(self.device)
         if self.cur >= 0:
             last = self.slots[self.cur]
             last.used.record(last.stream)                                # previous consumer is enqueued before this point
-        hit = next((i for i, s in enumerate(self.slots) if s.key == key), None)
+        hit = next((i for i, s in enumerate(self.slots) if s.holds(q, key, stamp)), None)
         if hit is None:
             self.misses += 1
             hit = (self.cur + 1) % len(self.slots)
-            self._expand(self.slots[hit], q, dtype, transpose, key, comp)
+            self._expand(self.slots[hit], q, dtype, transpose, key, stamp, comp)
         else:
             self.hits += 1
         slot = self.slots[hit]
         slot.stream = comp
         comp.wait_event(slot.ready)
         if self.prev_key is not None:
-            self.next_of[self.prev_key] = (q, dtype, transpose)
+            self.next_of[self.prev_key] = (weakref.ref(q), dtype, transpose)
         self.prev_key, self.cur = key, hit
-        nxt = self.next_of.get(key)
-        if nxt is not None:
-            nq, ndt, ntr = nxt
-            nkey = (id(nq), ndt, ntr)
+        nref, ndt, ntr = self.next_of.get(key, (lambda: None, None, False))
+        nq = nref()
+        if nq is not None:
+            nkey, nstamp = (id(nq), ndt, ntr), _stamp(nq)
             other = (hit + 1) % len(self.slots)
-            if self.slots[other].key != nkey:
-                self._expand(self.slots[other], nq, ndt, ntr, nkey, comp)
+            if not self.slots[other].holds(nq, nkey, nstamp):
+                self._expand(self.slots[other], nq, ndt, ntr, nkey, nstamp, comp)
         n = q.N * q.K
         return slot.buf[:n].view((q.K, q.N) if transpose else (q.N, q.K))
 

@@ -1,5 +1,6 @@
 """Expansion of 4-bit weights ahead of their GEMMs: which work is ordered after which, on streams that only keep count."""
 import contextlib
+import gc
 
 import pytest
 import torch
@@ -89,3 +90,30 @@ def test_a_round_that_repeats_is_expanded_ahead(pipe):
             assert torch.equal(p.get(w, torch.float32, False), w.packed.view(4, 4))
             comp.work("product")
     assert p.misses == 4                                     # the first round, and the first step from its end to its beginning
+
+
+def test_a_weight_that_changed_is_expanded_again(pipe):
+    p, comp = pipe
+    w = Weight("a", comp)
+    p.get(w, torch.float32, False)
+    w.packed.fill_(7.0)
+    comp.work("filled")
+    assert bool((p.get(w, torch.float32, False) == 7.0).all()) and "filled" in w.runs[1]
+
+
+def test_an_id_is_not_a_weight(pipe):
+    p, comp = pipe
+    w = Weight("a", comp)
+    old = id(w)
+    p.get(w, torch.float32, False)
+    del w
+    gc.collect()
+    assert not p.known                                       # nothing is kept of what is gone
+    for _ in range(50):                                      # until one lies where the other did, on the same memory
+        w = Weight("bb", comp)
+        if id(w) == old:
+            break
+    assert bool((p.get(w, torch.float32, False) == 2.0).all())
+    q = Weight("ccc", comp)
+    p.slots[p.cur].key, p.slots[p.cur].stamp = (id(q), torch.float32, False), dq._stamp(q)
+    assert bool((p.get(q, torch.float32, False) == 3.0).all())
