@@ -302,6 +302,7 @@ flash_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_consta
           if (!RT) mbar_wait_spin(res_full0 + 8 * (ka & 1), ((uint32_t)ka >> 1) & 1u);
         }
         mbar_wait_spin(st_full0 + 8 * sa.s, sa.ph);
+        __syncwarp();                                      // each lane has looked for itself (see umma_row_ts)
         // buffer i & 1 last held pair i - 2, whose P and dS are read by products issued before this one: the pipe runs in order
         tc_fence_after();
         issue_sdp(ka, i, sa.s);
@@ -316,6 +317,7 @@ flash_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_consta
           if (!RT || n + 1 < t.n_iter) ahead(i + 1);
           // P and dS of the pair are in TMEM (and the accumulators of the item before have been read)
           mbar_wait_spin(ds_full0 + 8 * (i & 1), ((uint32_t)i >> 1) & 1u);
+          __syncwarp();
           tc_fence_after();
           const uint32_t buf = tmem_base + (uint32_t)(i & 1) * kBwTBuf, ring = sRing + st.s * L::kStage;
           const uint32_t first = (ring >> 4) | kLoMN, second = ((ring + L::kTile) >> 4) | kLoMN;

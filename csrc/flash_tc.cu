@@ -463,6 +463,7 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
         const int nit = t.nit;
         mbar_wait_spin(q_full, (uint32_t)n & 1u);
         mbar_wait_spin(k_full(g0), k_phase(g0));
+        __syncwarp();                                     // each lane has looked for itself (see umma_f16_w)
         tc_fence_after();
         issue_qk(g0);                                     // into the buffer of the last block but one: its P has been read by products issued before
         if (RUN && nit == 1) umma_commit_w(q_empty);
@@ -470,6 +471,7 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
           const int g = g0 + j, s = g & 1;
           if (j + 1 < nit) {
             mbar_wait_spin(k_full(g + 1), k_phase(g + 1));
+            __syncwarp();
             // S buffer (g+1)&1 last held block g-1: P(g-1) sat in it and PV(g-1) was issued before this UMMA, the pipe runs in order
             tc_fence_after();
             issue_qk(g + 1);
@@ -477,6 +479,7 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
           }
           mbar_wait_spin(v_full(g), v_phase(g));
           mbar_wait_spin(p_full0 + 8 * s, ((uint32_t)g >> 1) & 1u);     // P(g) is written (and O rescaled where a row needed it; and taken, the tile before)
+          __syncwarp();
           tc_fence_after();
           const uint32_t vlo = (v_at(g) >> 4) | kLoMN;
 #pragma unroll

@@ -805,6 +805,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
       if (bsel < 0) continue;                        // grouped GEMM: unused row tile
       const long long bias_off = (long long)bsel * p.bias_bs;
       mbar_wait_sleep(tfull_bar(acc), acc_phase, 128);
+      __syncwarp();                                  // each lane has looked for itself, tcgen05.ld takes them together
       tc_fence_after();
       const int row = m0 + q * 32 + lane;
       const bool row_ok = row < p.M;
@@ -846,6 +847,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
               }
             } while (seen != sk_epoch_v);
           }
+          __syncwarp();
         }
       for (int c = 0; c < nchunks; ++c) {
         const int col0 = n0 + c * 32;

@@ -243,6 +243,7 @@ w4_tc_kernel(const __grid_constant__ CUtensorMap tw, const __grid_constant__ CUt
       mbar_wait(x_full(b), ph);
       mbar_wait(d_empty(b), ph ^ 1u);
       mbar_wait(a_full(b), ph);
+      __syncwarp();                                        // each lane has looked for itself (see wt_group)
       tc_fence_after();
       const uint64_t bd = ((uint64_t)kHi << 32) | ((sb + L.x + b * kPair) >> 4) | kLo;
       wt_group<(MT * 128 >> 4)>(tmem + 256 + b * (2 * MT), tmem + b * 128, bd, idesc);
