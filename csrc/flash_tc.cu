@@ -740,9 +740,11 @@ static int fused_qkv(const void* qkv, long long rows, FlashTcParams& p, int D, i
   if (int rc = rows_map(&tm, qkv, (uint64_t)(p.H + 2 * p.Hkv) * D, (uint64_t)rows, 64)) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   const bool bf = dtype == B200_DT_BF16;
-  // More tiles than two CTAs for each SM take: those go on from tile to tile. Fewer: nothing to go on to, and a tile's way through the other warps
-  // takes 1 us more (100 tokens, 32 heads of 128: 12.3 us, 14.3).
-  const bool run = (long long)grid.x * grid.y * grid.z > 2 * kNumSMs;
+  // More tiles than two rounds of two CTAs for each SM: CTAs go on from tile to tile. With none to go on to, or one each, a tile's way through the other
+  // warps is not made up for. One tile to a CTA against tiles in turn, us, 8 heads: 400 tiles of 64 tokens, heads of 64: 11.0, 12.2; 352 of 256: 14.6, 16.5; 320 of
+  // 1024, heads of 128: 22.0, 22.8; 304 packed of 17: 12.4, 14.2; some are faster in turn (400 of 64, heads of 128: 13.1, 12.5). 592: within 6 % either
+  // way. From 640 on: 64 tokens 14.6, 14.5 (heads of 128: 18.7, 16.2), 512 26.9, 24.8 (29.8, 27.1); 896: 18.7, 16.6 (22.9, 18.8), 34.9, 32.1 (41.3, 37.1).
+  const bool run = (long long)grid.x * grid.y * grid.z > 4 * kNumSMs;
   CUtensorMap to = tm;
   if (run)
     if (int rc = rows_map(&to, p.out, (uint64_t)p.H * D, (uint64_t)rows, 32)) return rc;

@@ -1,4 +1,5 @@
-"""Forward attention of more tiles than are resident at once, where a CTA goes on from tile to tile, against the same sequences alone."""
+"""Forward attention of more tiles than are resident at once, against the same sequences alone. A CTA goes on from tile to tile where there are more
+than 592; the others here ([128] * 9) take a CTA each."""
 import pytest
 import torch
 
@@ -10,7 +11,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("H,Hkv,D", [(40, 8, 128), (48, 48, 64)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("causal", [True, False])
-@pytest.mark.parametrize("lens", [[1, 63, 700, 129, 65, 2, 300, 64], [128] * 9, [5, 1300]])
+@pytest.mark.parametrize("lens", [[1, 63, 700, 129, 65, 2, 300, 64], [128] * 9, [128] * 16, [5, 1300]])
 def test_packed_tiles_in_turn(H, Hkv, D, dtype, causal, lens):
     """Tiles past a sequence's end, of one row to 128, of one key block to twenty: the bits of a call that one CTA a tile takes."""
     g = torch.Generator(device="cuda").manual_seed(len(lens))
