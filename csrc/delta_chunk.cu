@@ -41,7 +41,9 @@ constexpr int dc_block(int j, int s) { return (j >> 1) * ((j >> 1) + 1) + (j & 1
 constexpr int kDcT = 20 * kDcB, kDcPX = kDcT + 3 * kDcC, kDcHead = kDcT + kDcPX;      // words: T; P, c, r_64, beta
 constexpr int dc_q(int D) { return 8 * (D / 16) * kDcB; }
 constexpr int dc_kv(int D) { return kDcC * D + dc_q(D); } // K; Q
-constexpr int kDcWindow = 128;                            // chunks that the workspace holds
+// What a step's workspace takes at most, for each head: 4.3 MB, 136 MB at 32 heads. That holds all a step needs up to 37 chunks (with a q/k head for each head and
+// keys of 128; 82 at four heads to one, 135 with keys of 64 as well); longer ones go by windows of chunks.
+constexpr long long kDcMost = 128ll * 8320;
 
 struct DeltaChunkArgs {
   const float *q, *k, *v, *g, *beta;
@@ -597,11 +599,11 @@ static int run_windows(DeltaChunkArgs p, int bound, int window, cudaStream_t st)
 }
 }  // namespace b200
 
-// Workspace (floats) for a step of `tokens` tokens in n_runs runs: chunks are taken in windows of at most 128, however long the step is.
-B200_API long long b200_delta_chunk_workspace(int tokens, int n_runs, int H, int G, int D) {
+// Workspace (floats) for a step of `tokens` tokens in n_runs runs, whatever its q/k heads and key size are; bounded, however long the step is.
+B200_API long long b200_delta_chunk_workspace(int tokens, int n_runs, int H) {
   using namespace b200;
-  const long long bound = (long long)tokens / kDcC + n_runs;
-  return (bound < kDcWindow ? bound : kDcWindow) * ((long long)H * kDcHead + (long long)G * dc_kv(D));
+  const long long all = ((long long)tokens / kDcC + n_runs) * (kDcHead + dc_kv(128));
+  return H * (all < kDcMost ? all : kDcMost);
 }
 
 // Arguments as in b200_linear_scan (mode 3), `runs` present; `ws`: b200_delta_chunk_workspace floats. B200_ERR_UNSUPPORTED: the caller
@@ -618,7 +620,9 @@ B200_API int b200_delta_chunk_scan(const float* q, long long ldq, const float* k
   DeltaChunkArgs p = {q, k, v, g, beta, ldq, ldk, ldv, ldg, ldb, state, o, ws, runs, n_runs, H, G, Dv, 0, 0, 0};
   const long long bound = (long long)tokens / kDcC + n_runs;      // a run of n tokens has at most n / 64 + 1 chunks
   if (bound > 0x7fffffffLL) return B200_ERR_TOO_LARGE;
-  const int window = bound < kDcWindow ? (int)bound : kDcWindow;
+  const long long holds = b200_delta_chunk_workspace(tokens, n_runs, H) / ((long long)H * kDcHead + (long long)G * dc_kv(D));
+  const long long windows = (bound + holds - 1) / holds;
+  const int window = (int)((bound + windows - 1) / windows);
   p.kv_ws = (long long)window * H * kDcHead;
   return D == 64 ? run_windows<64>(p, (int)bound, window, (cudaStream_t)stream) : run_windows<128>(p, (int)bound, window, (cudaStream_t)stream);
 }

@@ -698,7 +698,7 @@ int b200_linear_scan(const float* q, long long ldq, const float* k, long long ld
                      int ones, void* stream);
 /* Mode 3 of it over prompts, 64 tokens at a time (csrc/delta_chunk.cu): D 64 or 128, Dv % 16 == 0, 16-byte aligned rows; ws holds
  * b200_delta_chunk_workspace floats. B200_ERR_UNSUPPORTED otherwise. */
-long long b200_delta_chunk_workspace(int tokens, int n_runs, int H, int G, int D);
+long long b200_delta_chunk_workspace(int tokens, int n_runs, int H);
 int b200_delta_chunk_scan(const float* q, long long ldq, const float* k, long long ldk, const float* v, long long ldv, const float* g,
                           long long ldg, const float* beta, long long ldb, float* state, const int* runs, int n_runs, float* o, float* ws,
                           int tokens, int H, int G, int D, int Dv, void* stream);

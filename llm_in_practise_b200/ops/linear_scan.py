@@ -253,22 +253,22 @@ def _chunks_pay(T: int, n_runs: int, pieces, H: int, G: int, D: int, Dv: int) ->
 
 
 def _delta_chunks(q, k, v, g, beta, state, runs, n_runs, o, H, G, D, Dv) -> bool:
-    """Mode "head_delta" over the runs of a step in chunks of 64 tokens; False: rows the kernels do not take. The workspace is 31 KB per
-    chunk and head and 80 KB (keys of 64: 41) per chunk and q/k head for at most 128 chunks at a time (211 MB at 32 heads over 8), which the walk
-    does without."""
+    """Mode "head_delta" over the runs of a step in chunks of 64 tokens; False: rows the kernels do not take. The workspace is 113 KB per
+    chunk and head up to 4.3 MB per head (136 MB at 32), which the walk does without; a chunk takes 31 KB of it per head and 82 KB (keys of 64: 41)
+    per q/k head, and longer steps go by windows of as many chunks as it holds."""
     T = q.shape[0]
     if not nv.has("b200_delta_chunk_scan"):               # a library linked for a model without this mode
         return False
     size = nv.lib().b200_delta_chunk_workspace
     size.restype = i64
-    ws = torch.empty(size(T, n_runs, H, G, D), dtype=torch.float32, device=q.device)
+    ws = torch.empty(size(T, n_runs, H), dtype=torch.float32, device=q.device)
     fn = nv.proto("b200_delta_chunk_scan", [vp, i64, vp, i64, vp, i64, vp, i64, vp, i64, vp, vp, i32, vp, vp, i32, i32, i32, i32, i32, vp])
     rc = fn(nv.ptr(q), q.stride(0), nv.ptr(k), k.stride(0), nv.ptr(v), v.stride(0), nv.ptr(g), g.stride(0), nv.ptr(beta), beta.stride(0),
             nv.ptr(state), nv.ptr(runs), n_runs, nv.ptr(o), nv.ptr(ws), T, H, G, D, Dv, nv.stream())
     if rc == nv.ERR_UNSUPPORTED:
         return False
     nv.check(rc, "delta_chunk_scan")
-    nv.count_launch(2 * max(1, -(-(T // 64 + n_runs) // 128)))
+    nv.count_launch(2 * -(-(T // 64 + n_runs) // (ws.numel() // (7872 * H + 160 * D * G))))
     return True
 
 

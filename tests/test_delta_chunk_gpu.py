@@ -35,7 +35,7 @@ def took(monkeypatch):
 @pytest.mark.parametrize("lens,H,G,D,Dv", [
     ([64], 2, 1, 64, 16), ([65, 17, 63], 4, 4, 128, 48), ([1, 130, 1, 200], 4, 2, 128, 32), ([300], 6, 1, 64, 64),
     ([64, 128, 90], 20, 4, 128, 128),                     # more (run, head, column block)s than SMs
-    ([8300, 40], 1, 1, 64, 16),                           # more chunks than one window of 128
+    ([8300, 40], 1, 1, 64, 16), ([2500, 70], 2, 2, 128, 32),         # more chunks than the workspace holds: three windows, two
 ])
 @pytest.mark.parametrize("decay", [(0.9, 1.0), (0.0, 1.0), (1e-6, 1e-3)])
 def test_chunks(lens, H, G, D, Dv, decay, took):

@@ -25,6 +25,20 @@ def test_delta_rule_in_chunks(lens, H, G, D, chunks):
 
 
 @library
+@pytest.mark.parametrize("H", [1, 16, 32, 40])
+def test_workspace_of_the_delta_rule_is_bounded(H):
+    """At most 4.3 MB per head, however long the step and however many q/k heads it has; at least a chunk's matrices (7872 words per head, 20480 per
+    q/k head for keys of 128); and asked for as it always was, without the q/k heads."""
+    fn = nv.lib().b200_delta_chunk_workspace
+    fn.restype, fn.argtypes = ctypes.c_longlong, [ctypes.c_int] * 3
+    for tokens, runs in [(1, 1), (64, 1), (500, 3), (2368, 1), (8192, 1), (1 << 20, 64), ((1 << 31) - 1, 1)]:
+        words = fn(tokens, runs, H)
+        assert H * (7872 + 20480) <= words <= H * 128 * 8320
+        if tokens // 64 + runs <= 37:
+            assert words == (tokens // 64 + runs) * H * (7872 + 20480)
+
+
+@library
 @pytest.mark.parametrize("m,n,k,chain", [
     (20, 4096, 2048, 6), (64, 4096, 4096, 11), (128, 8192, 2048, 10), (64, 5120, 17408, 37), (200, 2048, 2048, 5), (200, 6144, 4096, 21),
     (490, 4096, 2048, 14), (490, 6144, 4096, 42), (549, 2048, 2048, 11), (549, 4096, 4096, 43), (1024, 2048, 4096, 29), (1500, 2048, 4096, 43),
