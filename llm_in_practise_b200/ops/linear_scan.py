@@ -240,15 +240,19 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.
 def _chunks_pay(T: int, n_runs: int, pieces, H: int, G: int, D: int, Dv: int) -> bool:
     """Whether prompts of the delta rule with one decay per head take less time 64 tokens at a time (csrc/delta_chunk.cu) than token by
     token. Both as measured (us): the walk moves 0.24 per token of the longest run, or, with more (run, head, 16 columns) than about
-    320 (445 for keys of 64) at once, in proportion; a chunk is 3.9 (2.8) on one of 148 SMs, which take the (run, head, 16 columns) in
-    rounds, after the inverses. 16 heads of 128 over 4: one run of 2048 tokens 155 against 506, four of 512 163 against 218, three of 150 73
-    against 60, eight of 1000 534 against 732; 32 heads, one of 200: 64 against 65; 16 heads of 64, one of 150: 32 against 44. Other head
-    counts rest on the proportions. Without ``pieces`` the runs count as equally long."""
+    320 (445 for keys of 64) at once, in proportion. In chunks there is the preparation, a CTA per chunk and q/k head; then a chunk is 4.05 (3.03) on one of
+    148 SMs, which take the (run, head, 16 columns) in rounds. 16 heads of 128 over 4: one run of 2048 tokens 153 against 506, four of 512 163 against
+    217, three of 150 71 against 59, eight of 1000 574 against 729; 16 over 16 179 and 506, 189 and 217, 75 and 59, 726 and 729; 32 over 32, 1000 tokens, 181
+    and 293; 16 over 16 of 64, four of 512, 85 and 131. Over 99 such steps (8 to 40 heads, 4 to 40 q/k heads, 100 to 8192 tokens) the time in chunks is
+    met to 4.5 % in the mean, 15 at most; none takes chunks where the walk is faster. Without ``pieces`` the runs count as equally long."""
     blocks = H * (Dv // 16)
     longest, tiles = (pieces.longest, pieces.n_tiles) if pieces is not None else (T / max(n_runs, 1), T / 64 + n_runs)
     walk = 8 + 0.24 * max(longest, T * blocks / (320 if D == 128 else 445))
     rounds = max(-(-longest // 64) + 0.5, -(-n_runs * blocks // 148) * (tiles / max(n_runs, 1) + 0.5))
-    chunks = (31 if D == 128 else 23.5) * max(1.0, tiles * G / 160) + (3.85 if D == 128 else 2.8) * rounds
+    if D == 128:
+        chunks = 6.4 + 18.9 * max(1.0, tiles * G / 200) + 4.05 * rounds
+    else:
+        chunks = 3.3 + 16.0 * max(1.0, tiles * G / 280) + 3.03 * rounds
     return chunks < 0.9 * walk
 
 

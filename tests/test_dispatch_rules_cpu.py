@@ -12,9 +12,12 @@ library = pytest.mark.skipif(not nv.lib_path().exists(), reason="no kernel libra
 
 @pytest.mark.parametrize("lens,H,G,D,chunks", [
     ([1] * 64, 16, 4, 128, False),                        # a decode batch
-    ([150] * 3, 16, 4, 128, False),                       # short runs beside one another: 74 us in chunks, 56 token by token
-    ([2048], 16, 4, 128, True),                           # 225 against 502
-    ([2048, 513], 16, 4, 128, True),                      # 285 against 586
+    ([150] * 3, 16, 4, 128, False),                       # short runs beside one another: 71 us in chunks, 59 token by token
+    ([2048], 16, 4, 128, True),                           # 153 against 506
+    ([2048, 513], 16, 4, 128, True),                      # 198 against 590
+    ([512] * 4, 16, 16, 64, True),                        # a q/k head for each head: 85 against 131
+    ([1000], 32, 32, 128, True),                          # 181 against 293
+    ([200] * 16, 32, 32, 128, False),                     # 759 against 561
 ])
 def test_delta_rule_in_chunks(lens, H, G, D, chunks):
     """With the runs known on the host, and without them, where they count as equally long."""
