@@ -531,7 +531,7 @@ channel_tile_kernel(const ChannelScanArgs a) {
         for (int x = 0; x < 4; ++x) S[j][x] = fmaf(x & 1 ? e.y : e.x, S[j][x], sa.sum(x));
       }
     }
-    if (keep) each([&](float& s, int) { odd |= not_finite(s); });
+    if (keep || c0 + 64 < n) each([&](float& s, int) { odd |= not_finite(s); });      // a state that is used
     if (__syncthreads_or(odd)) {                          // from the state in front of these tokens, which still lies there, again
       each([&](float&, int at) { sm[at] = PASS == 1 && c0 == 0 ? 0.f : part[at]; });
       if (PASS == 1 && tid < D) {

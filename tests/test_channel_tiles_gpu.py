@@ -3,6 +3,7 @@ blocks of 16 tokens, tiles of 64 and runs, and what is walked instead."""
 import pytest
 import torch
 
+from llm_in_practise_b200.inference import ragged
 from llm_in_practise_b200.inference.ragged import make_pieces
 from llm_in_practise_b200.ops.linear_scan import linear_scan
 
@@ -92,3 +93,48 @@ def test_not_finite_stays_behind_its_token(what, value, at, bonus):
             assert finite[cols.reshape(finite.shape)].all()
             finite &= cols.reshape(finite.shape)
         assert ((got.double() - want)[finite].abs().max() / want[finite].abs().max()).item() < 4 * (D + 64) * 2.0 ** -24
+
+
+@pytest.mark.parametrize("rows,lens,H,G,D", [(65, [66, 200], 2, 2, 64), (128, [129, 384], 2, 1, 128), (200, [433, 30, 201], 4, 4, 64)])
+@pytest.mark.parametrize("bonus", [False, True])
+@pytest.mark.parametrize("bad", [None, 3, 90, 190])
+def test_tiles_of_more_than_64_tokens(rows, lens, H, G, D, bonus, bad, monkeypatch):
+    """A caller's own tiles, whose state waits in the scratch between 64 tokens and the next; with a NaN in a later part of one, too."""
+    q, k, v, g, state, runs, u = case(lens, H, G, D, 0.9, bonus, seed=11)
+    if bad is not None:
+        k[bad, 1] = float("nan")
+    want_o, want_s = walk(q, k, v, state, runs, H, G, D, g, u)
+    monkeypatch.setattr(ragged, "TILE_Q", rows)
+    pieces = make_pieces(runs, "cuda")
+    pieces.tile_rows = rows
+    assert pieces.n_tiles == sum(-(-n // rows) for n in lens)
+    pos = slot = torch.zeros(q.shape[0], dtype=torch.int32, device="cuda")
+    o = linear_scan(q, k, v, state, pos, slot, pieces.runs, pieces.n_runs, H, G, D, D, "channel", g=g, pieces=pieces, u=u)
+    for got, want in ((o, want_o), (state, want_s)):
+        finite = want.isfinite()
+        assert torch.equal(got.isfinite(), finite)
+        assert ((got.double() - want)[finite].abs().max() / want[finite].abs().max()).item() < 4 * (D + 64) * 2.0 ** -24
+
+
+def test_a_state_that_only_the_products_lose(monkeypatch):
+    """The last 16 tokens before the state is put by take it from one end of fp32's range towards the other: their own sum is outside it."""
+    H = G = 1
+    D = 64
+    q, k, v, g, state, runs, u = case([256], H, G, D, 0.9, False, seed=12)
+    runs[0][2] = 3
+    g[:128, 5] = 1.0
+    q[:64, 5] = 0.0
+    q[64:, 5] = 1e-38
+    k[:, 5] = 0.0
+    k[48:64, 5] = 3.1e37
+    v[48:64] = 0.0
+    v[48:64, 9] = 1.0
+    state[0, 0, 5] = 0.0
+    state[0, 0, 5, 9] = -3e38
+    want = walk(q, k, v, state.clone(), runs, H, G, D, g, u)[0][64:128]
+    monkeypatch.setattr(ragged, "TILE_Q", 128)
+    pieces = make_pieces(runs, "cuda")
+    pieces.tile_rows = 128
+    pos = slot = torch.zeros(256, dtype=torch.int32, device="cuda")
+    got = linear_scan(q, k, v, state, pos, slot, pieces.runs, pieces.n_runs, H, G, D, D, "channel", g=g, pieces=pieces, u=u)[64:128]
+    assert bool(got.isfinite().all()) and ((got.double() - want).abs().max() / want.abs().max()).item() < 4 * (D + 64) * 2.0 ** -24
