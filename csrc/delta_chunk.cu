@@ -316,44 +316,69 @@ __device__ __forceinline__ int half_or(int x) {
   return r;
 }
 
-// Tokens [at, len) of a run one by one, from S [16 columns][D] in shared memory (`sm` has room for D x 16 and 2 x 16 x 16 floats more): what a chunk with an infinity or NaN in R, U
-// or Q S_0 takes, since a product with zeros above a diagonal, or of parts of an infinity, would carry it to tokens before its own.
+// Tokens [at, len) of a run one by one, from S [D][16 columns] in shared memory at `s0`: what a chunk with an infinity or NaN in R, U or Q S_0 takes,
+// since a product with zeros above a diagonal, or of parts of an infinity, would carry it to tokens before its own. A warp has one of the columns (keys of 64: two)
+// in registers, so that tokens follow one another without a barrier; their k, q and v come through the front of `sm`, 64 at a time. A NaN in the
+// first of 2048 tokens, 16 heads of 128: the mixer 292 -> 735 us (with S k summed over the CTA and k, q read where they lie, token by token, 2980).
 template <int D>
-__device__ __noinline__ void walk_on(const DeltaChunkArgs& p, float* sm, int h, int col0, int first, int at, int len, float* state) {
-  const int tid = threadIdx.x, e = tid & 15, part = tid >> 4, kvh = h / (p.H / p.G);
-  constexpr int RPT = D / 16;                             // rows of a thread of the first 256
-  float s[RPT];
-  float* red = sm + D * 16;
-  if (tid < 256)
-    for (int i = 0; i < RPT; ++i) s[i] = sm[(part * RPT + i) * 16 + e];
-  for (int t = at; t < len; ++t) {
-    const long long row = first + t;
-    float d = 0.f, o = 0.f;
-    if (tid < 256) {
-      const float a = p.g[row * p.ldg + h];
-      const float* kr = p.k + row * p.ldk + (long long)kvh * D + part * RPT;
-      for (int i = 0; i < RPT; ++i) { s[i] *= a; d = fmaf(s[i], kr[i], d); }
-      red[part * 16 + e] = d;
+__device__ __noinline__ void walk_on(const DeltaChunkArgs& p, float* sm, const float* s0, int h, int col0, int first, int at, int len, float* state) {
+  constexpr int NT = DcSmem<D>::kThreads, CPW = kDcNC * 32 / NT, RPL = D / 32;
+  static_assert(2 * kDcC * D + kDcC * (kDcNC + 2) <= DcSmem<D>::Red, "the staged tokens lie in front of S");
+  float *Ks = sm, *Qs = Ks + kDcC * D, *Vs = Qs + kDcC * D, *As = Vs + kDcC * kDcNC, *Bs = As + kDcC;
+  const int tid = threadIdx.x, lane = tid & 31, col = (tid >> 5) * CPW, kvh = h / (p.H / p.G);
+  float s[CPW][RPL];
+#pragma unroll
+  for (int c = 0; c < CPW; ++c)
+#pragma unroll
+    for (int i = 0; i < RPL; ++i) s[c][i] = s0[(lane + 32 * i) * kDcNC + col + c];
+  for (int t0 = at; t0 < len; t0 += kDcC) {
+    const int n = min(kDcC, len - t0);
+    const long long row = first + t0;
+    __syncthreads();                                      // the tokens before are read
+    for (int i = tid; i < n * (D / 4); i += NT) {
+      const int t = i / (D / 4), d = i % (D / 4) * 4;
+      *reinterpret_cast<float4*>(Ks + t * D + d) = *reinterpret_cast<const float4*>(p.k + (row + t) * p.ldk + (long long)kvh * D + d);
+      *reinterpret_cast<float4*>(Qs + t * D + d) = *reinterpret_cast<const float4*>(p.q + (row + t) * p.ldq + (long long)kvh * D + d);
     }
+    for (int i = tid; i < n * kDcNC; i += NT) Vs[i] = p.v[(row + i / kDcNC) * p.ldv + (long long)h * p.Dv + col0 + i % kDcNC];
+    if (tid < n) { As[tid] = p.g[(row + tid) * p.ldg + h]; Bs[tid] = p.beta[(row + tid) * p.ldb + h]; }
     __syncthreads();
-    if (tid < 256) {
-      float y = 0.f;
-      for (int i = 0; i < 16; ++i) y += red[i * 16 + e];
-      const float u = p.beta[row * p.ldb + h] * (p.v[row * p.ldv + (long long)h * p.Dv + col0 + e] - y);
-      const float* kr = p.k + row * p.ldk + (long long)kvh * D + part * RPT;
-      const float* qr = p.q + row * p.ldq + (long long)kvh * D + part * RPT;
-      for (int i = 0; i < RPT; ++i) { s[i] = fmaf(kr[i], u, s[i]); o = fmaf(s[i], qr[i], o); }
-      red[256 + part * 16 + e] = o;
-    }
-    __syncthreads();
-    if (tid < 16) {
-      float y = 0.f;
-      for (int i = 0; i < 16; ++i) y += red[256 + i * 16 + e];
-      p.o[(row * p.H + h) * p.Dv + col0 + e] = y;
+    for (int tb = 0; tb < n; tb += 16) {                  // the outputs' sums over the warp wait for one another's tokens
+      float o[CPW][16];
+#pragma unroll
+      for (int x = 0; x < 16; ++x) {
+        const int t = tb + x;
+#pragma unroll
+        for (int c = 0; c < CPW; ++c) o[c][x] = 0.f;
+        if (t >= n) continue;
+        const float a = As[t], b = Bs[t];
+        float k[RPL], q[RPL];
+#pragma unroll
+        for (int i = 0; i < RPL; ++i) { k[i] = Ks[t * D + lane + 32 * i]; q[i] = Qs[t * D + lane + 32 * i]; }
+#pragma unroll
+        for (int c = 0; c < CPW; ++c) {
+          float d = 0.f;
+#pragma unroll
+          for (int i = 0; i < RPL; ++i) { s[c][i] *= a; d = fmaf(s[c][i], k[i], d); }
+#pragma unroll
+          for (int w = 16; w >= 1; w >>= 1) d += __shfl_xor_sync(0xffffffffu, d, w);
+          const float u = b * (Vs[t * kDcNC + col + c] - d);
+#pragma unroll
+          for (int i = 0; i < RPL; ++i) { s[c][i] = fmaf(k[i], u, s[c][i]); o[c][x] = fmaf(s[c][i], q[i], o[c][x]); }
+        }
+      }
+      const int t = tb + (lane >> 1);
+#pragma unroll
+      for (int c = 0; c < CPW; ++c) {
+        const float y = gather16(o[c], lane);
+        if (!(lane & 1) && t < n) p.o[((row + t) * p.H + h) * p.Dv + col0 + col + c] = y;
+      }
     }
   }
-  if (tid < 256)
-    for (int i = 0; i < RPT; ++i) state[(long long)(part * RPT + i) * p.Dv + col0 + e] = s[i];
+#pragma unroll
+  for (int c = 0; c < CPW; ++c)
+#pragma unroll
+    for (int i = 0; i < RPL; ++i) state[(long long)(lane + 32 * i) * p.Dv + col0 + col + c] = s[c][i];
 }
 
 // The state of 16 columns, transposed, is the 16 rows of an mma.sync tile: S^T K^T, R^T T^T, U^T P^T, S^T Q^T have the chunk's tokens as columns,
@@ -537,7 +562,7 @@ delta_chunk_scan_kernel(const DeltaChunkArgs p) {
       for (int x = 0; x < 4; ++x) sm[L::Red + (16 * w + 8 * half + t2 + (x & 1)) * 16 + g + (x >> 1) * 8] = S[x];
       if (more) mbar_wait(kp_bar(tile + 1), (uint32_t)((tile + 1 - t_lo) >> 1) & 1u);      // what is on its way arrives before the CTA leaves
       __syncthreads();
-      walk_on<D>(p, sm + L::Red, h, col0, first, at, min(len, (t_hi - tb) * kDcC), sp);
+      walk_on<D>(p, sm, sm + L::Red, h, col0, first, at, min(len, (t_hi - tb) * kDcC), sp);
       return;
     }
     if (asks && more) ask_qt(tile + 1);
