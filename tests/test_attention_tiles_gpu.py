@@ -53,3 +53,30 @@ def test_dense_tiles_in_turn(B, S, H, Hkv, D):
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(again, out) and torch.equal(lse2, lse)
+
+
+@pytest.mark.parametrize("dtype,eps", [(torch.bfloat16, 2.0 ** -9), (torch.float16, 2.0 ** -12)])
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("lens,H,Hkv,D", [([30, 700, 129, 64], 28, 7, 128), ([256] * 30, 12, 12, 64)])
+def test_tiles_in_turn_against_fp64(lens, H, Hkv, D, dtype, eps, causal):
+    """Packed, and where the lengths are equal dense as well. Weights and results are rounded to 16 bits, each by at most eps of itself."""
+    g = torch.Generator(device="cuda").manual_seed(D)
+    qkv = torch.randn(sum(lens), (H + 2 * Hkv) * D, device="cuda", generator=g).to(dtype)
+    cu = torch.tensor([0] + lens, dtype=torch.int32).cumsum(0).to(torch.int32).cuda()
+    assert len(lens) * H * -(-max(lens) // 128) > 592
+    got = [flash_attention_varlen(qkv, cu, max(lens), H, Hkv, D, D ** -0.5, causal)]
+    if len(set(lens)) == 1:
+        got.append(_fwd(qkv, len(lens), lens[0], H, Hkv, D, causal, D ** -0.5)[0])
+    x, at = qkv.double().view(-1, H + 2 * Hkv, D).transpose(0, 1), 0
+    for n in lens:
+        q, k, v = x[:H, at:at + n], x[H:H + Hkv, at:at + n], x[H + Hkv:, at:at + n]
+        k, v = k.repeat_interleave(H // Hkv, 0), v.repeat_interleave(H // Hkv, 0)
+        s = q @ k.transpose(1, 2) * D ** -0.5
+        if causal:
+            s = s.masked_fill(torch.ones(n, n, device="cuda").triu(1).bool(), float("-inf"))
+        p = torch.softmax(s, -1)
+        ref, most = (p @ v).transpose(0, 1).reshape(n, -1), (p @ v.abs()).transpose(0, 1).reshape(n, -1)
+        for o in got:
+            # eps for each weight and for the result, and as much again for the exponentials and the sums in fp32
+            assert bool(((o[at:at + n].double() - ref).abs() <= 4 * eps * most + 2.0 ** -24).all())
+        at += n

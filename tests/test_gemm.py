@@ -106,6 +106,21 @@ def test_gemm_lora_extra_kblock(r):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K,r", [(300, 4096, 16384, 16), (549, 2048, 2048, 8), (2345, 2048, 512, 64), (256, 16, 640, 40), (128, 512, 640, 16), (1000, 5120, 1536, 24)])
+def test_gemm_lora_extra_kblock_mn_major(M, N, K, r):
+    """B along N (three boxes a k-block from a producer of its own), then a low-rank k-block of both operands: tiles of a pair of CTAs and of one, cut along k
+    (the first two) and whole, ragged rows, the smallest N."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x, w, t, lb = (torch.randn(*s, device="cuda", generator=g).bfloat16() for s in ((M, K), (K, N), (M, r), (N, r)))
+    d = torch.randn(M, N, device="cuda", generator=g)
+    ref = x.double() @ w.double() + t.double() @ lb.double().t() + 0.5 * d.double()
+    out = G.gemm(x, w, b_mn=True, out=d.clone(), beta=0.5, lora=(t, lb))
+    # any order of K + r + 1 fp32 additions, rounded or truncated: 2^-23 of the sum of magnitudes for each
+    bound = (K + r + 1) * 2.0 ** -23 * (x.abs().double() @ w.abs().double() + t.abs().double() @ lb.abs().double().t() + d.abs().double())
+    assert bool(((out.double() - ref).abs() <= bound).all())
+
+
+@pytest.mark.gpu
 def test_gemm_batched_gqa_strided():
     # attention-shaped: Q [B,S,H,D] view, K [B,S,Hkv,D] view, scores[b,h] = Q K^T; then P V (b_mn)
     B, S, H, Hkv, D = 2, 256, 8, 2, 128
