@@ -130,10 +130,10 @@ __device__ __forceinline__ float tanh_any(float x) { return 1.f - __fdividef(2.f
 // RUN: a CTA goes on to the tiles of CTAs that have not started (clusterlaunchcontrol). The next tile's Q and keys come, and its first scores are taken,
 // while the softmax warps finish the one before; a warp of its own writes that out by TMA. Set-up, the wait for the first scores and the
 // end were 13 000 of a CTA's 26 000 cycles for sequences of 512 (8000 or 4600 of them the wait, in the first round and after it). One tile to a CTA
-// before: 4 x 512, 40 / 8 heads of 128: packed 37.9 -> 33.9 us, dense with its backward 115 -> 113; six packed prompts of 77 to 2048
-// tokens, 32 / 8 heads: 106 -> 102 (99 where the SM clock held); eleven of 17 to 1000, 40 / 8 heads: 52 -> 46; eight of 1000, 16 heads of 64: 59 -> 56; one of 4096
+// before: 4 x 512, 40 / 8 heads of 128: packed 37.9 -> 33.9 us; six packed prompts of 77 to 2048
+// tokens, 32 / 8 heads: 105 -> 100; eleven of 17 to 1000, 40 / 8 heads: 52 -> 46; eight of 1000, 16 heads of 64: 59 -> 56; one of 4096
 // or 8192: the same. A piece of a paged prompt starts with its page numbers either way and gained nothing (102 us for 5596 tokens), with capped scores
-// it lost a fifth to registers spilled in the loop; so pieces, and calls that are resident at once, keep a tile to a CTA.
+// it lost a fifth to registers spilled in the loop; so pieces, and calls of few tiles (see fused_qkv), keep a tile to a CTA.
 template <int MODE, int D, bool BF16, bool CAP, bool RUN>
 __global__ void __launch_bounds__(kTcThreads, 2)
 flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,

@@ -986,8 +986,9 @@ static double kblock_cost(int ctas, int bn) {
 // What a launch of whole tiles costs beside that, in the same cycles: 45 more for each k-block; the last tile's epilogue for each 32 columns,
 // and for half of 32 more than a whole one (its columns are stored one at a time); a pair of CTAs (a cluster's launch, and its barriers at
 // both ends). Over 624 products (M 20 to 8192, N 16 to 30522, K 512 to 12288, B along K and along N) with every tile timed
-// the choice is 0.8% above the best tile, by the k-blocks alone 4.5%, and nowhere slower than by these. Epilogues of 300 to 600 cycles do;
-// with 1200 and no more for halves (2.8%) one in twelve was slower than by the k-blocks, 4096 x 1536 x 512 17 -> 23 us.
+// the choice is 0.8% above the best tile, by the k-blocks alone 5.3%, and nowhere slower than by these. (Fitted to the kernel whose products one thread issued, when the latter was 4.5%;
+// timed again since: MN-major B 0.1 to 0.6%, tiles of up to 64 columns 1.1%, at most 27% for 20 x 4096 x 2048, 19.3 us and 15.2.) Epilogues of 300 to 600 cycles do;
+// with 1200 and no more for halves (2.9%) one in fifteen was slower than by the k-blocks, 4096 x 1536 x 512 17 -> 22 us.
 constexpr double kPerBlock = 45.0, kEpilogueChunk = 500.0, kHalfChunk = 3000.0, kPairLaunch = 3000.0;
 
 struct GemmConfig {

@@ -65,7 +65,7 @@ template <int N_>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N_) : "memory"); }
 
 // (a & b) | c in ONE instruction: with b and c as immediates the compiler splits it into two LOP3s (the expansion of the
-// codes is 22 % of all issued instructions of this kernel, profiles/r2/gemv.md)
+// codes is 22 % of all issued instructions of this kernel)
 __device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t b, uint32_t c) {
   uint32_t d;
   asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
@@ -114,7 +114,7 @@ struct GemvParams {
 // the affine map is applied to the chunk's fp32 partial sum instead:  sum_k w_k x_k = A_row * (sum_k (bias + c_k) x_k -
 // B_row * sum_k x_k), with sum_k x_k produced by one more MMA per k-step whose weight operand is the constant 1.0. That
 // replaces 32 packed FMAs per lane and chunk by 8 MMAs and 8 scalar FMAs: the kernel is bound by instruction issue,
-// not by HBM (3.5 instructions per weight before; profiles/r2/gemv.md).
+// not by HBM (3.5 instructions per weight before).
 template <bool BF16, bool W4, int TG, int MINB, bool LIN = false, bool POST = false>
 __global__ void __launch_bounds__(256, MINB)
 gemv_mma_kernel(const GemvParams p) {
@@ -164,7 +164,7 @@ gemv_mma_kernel(const GemvParams p) {
   // Work item = (16-row tile, batch of U chunks per warp). All packed weights (and scales) of an item are requested
   // before any of them is used, so an item costs ONE trip to DRAM instead of U dependent ones; the activations come from
   // shared memory (staged once per CTA when they fit), so the only long-latency operation left inside an item is that
-  // one trip. (A cp.async prefetch ring in shared memory was measured 1.5x SLOWER than this: profiles/r2/gemv.md.)
+  // one trip. (A cp.async prefetch ring in shared memory was measured 1.5x SLOWER than this.)
   constexpr int U = MINB >= 3 ? 1 : 4;     // 3-4 CTAs per SM (<= 80 registers): one chunk at a time, occupancy hides the latency
   const int nb = (nchunks + 8 * U - 1) / (8 * U);
   const long long my_tiles = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;

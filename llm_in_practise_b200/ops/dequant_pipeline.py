@@ -2,7 +2,8 @@
 
 The dequant kernels are HBM-bound (4.5 TB/s for ~0.1 ms), the tcgen05 GEMMs are bound by the tensor pipe and the
 shared-memory port and leave most of the DRAM bandwidth idle — so the next weight is expanded *while* the current GEMM
-runs. Dequant blocks (256 threads, 64 B of shared memory) co-reside with the persistent GEMM CTAs on the same SMs.
+runs. An SM has room for one dequant block of 256 threads and 32 registers beside a GEMM CTA (224 threads of 234), for one of 42 registers
+none; the others wait for an SM that the GEMM has left. Only the next GEMM waits for them, and a GEMM's CTAs only for those that started before.
 
 The order of requests in a training step is the same every step (q|k|v, o, gate|up, down per layer, then the transposed
 ones in reverse), so the pipeline simply remembers which (weight, layout) followed which last time and expands that one

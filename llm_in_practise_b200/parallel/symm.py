@@ -156,7 +156,7 @@ def allreduce_(buf: SymmBuffer, flags: PeerFlags, offset: int, n: int, scale: fl
     vp, i32, i64, u32, f32 = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_uint, ctypes.c_float
     grid = max(1, min(grid, (n // 4 + 255) // 256))
     base = flags.take_grid_target(grid, 1)
-    # measured at 2 ranks (profiles/r2): the peer-pointer kernel moves the same bytes faster (0.44 vs 0.66 ms for 252 MiB);
+    # measured at 2 ranks: the peer-pointer kernel moves the same bytes faster (0.44 vs 0.66 ms for 252 MiB);
     # the switch only saves traffic from 3 ranks up (2 n / W instead of 2 n (W - 1) / W per rank)
     if nvls_enabled(buf, lowp, min_world=3) and (offset * 4) % 16 == 0:
         fn = nv.proto("b200_allreduce_nvls", [vp, vp, vp, i64, i32, i32, u32, f32, i32, vp, u32, i32, vp])
