@@ -314,6 +314,20 @@ template <int D> struct TileSmem {                        // offsets in 32-bit w
   static constexpr int bytes(int pass) { return (pass == 1 ? (kFirst > kWalk ? kFirst : kWalk) : (kBoth > kWalk ? kBoth : kWalk)) * 4; }
 };
 
+// 16 values a lane, summed over the warp: lane l keeps the sum of value l / 2
+__device__ __forceinline__ float gather16(float (&v)[16], int lane) {
+#pragma unroll
+  for (int w = 8; w >= 1; w >>= 1) {
+    const bool up = lane & (2 * w);
+#pragma unroll
+    for (int i = 0; i < w; ++i) {
+      const float mine = up ? v[w + i] : v[i], theirs = up ? v[i] : v[w + i];
+      v[i] = mine + __shfl_xor_sync(0xffffffffu, theirs, 2 * w);
+    }
+  }
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
 // Tokens [c0, n) of a tile one by one, from the S [D][D] in shared memory; a state that is kept goes to `dst`. A thread has half of a column in registers; k, q and g
 // of 16 tokens come through shared memory, where their halves of the outputs meet. A NaN in one channel of the first of 2345 tokens, 16 heads of 128:
 // the mixer 232 -> 336 us, in all channels 480 (with S in shared memory and k, q, g read where they lie, 754 and 1133).

@@ -316,15 +316,17 @@ __device__ __forceinline__ int half_or(int x) {
   return r;
 }
 
-// Tokens [at, len) of a run one by one, from S [D][16 columns] in shared memory at `s0`: what a chunk with an infinity or NaN in R, U or Q S_0 takes,
+// Tokens [at, len) of a run one by one, from S [D][16 columns] in shared memory (at Red): what a chunk with an infinity or NaN in R, U or Q S_0 takes,
 // since a product with zeros above a diagonal, or of parts of an infinity, would carry it to tokens before its own. A warp has one of the columns (keys of 64: two)
 // in registers, so that tokens follow one another without a barrier; their k, q and v come through the front of `sm`, 64 at a time. A NaN in the
-// first of 2048 tokens, 16 heads of 128: the mixer 292 -> 735 us (with S k summed over the CTA and k, q read where they lie, token by token, 2980).
+// first of 2048 tokens, 16 heads of 128: the mixer 292 -> 1010 us (with S k summed over the CTA and k, q read where they lie, token by token, 2980). Outputs of several tokens
+// summed at once take 735 to 780, but the longer code costs steps without a NaN 0.3 to 0.4% more (2048 and 513 tokens: 194.5 us of the two kernels, 195.1 to 195.3).
 template <int D>
-__device__ __noinline__ void walk_on(const DeltaChunkArgs& p, float* sm, const float* s0, int h, int col0, int first, int at, int len, float* state) {
+__device__ __noinline__ void walk_on(const DeltaChunkArgs& p, float* sm, int h, int col0, int first, int at, int len, float* state) {
   constexpr int NT = DcSmem<D>::kThreads, CPW = kDcNC * 32 / NT, RPL = D / 32;
   static_assert(2 * kDcC * D + kDcC * (kDcNC + 2) <= DcSmem<D>::Red, "the staged tokens lie in front of S");
   float *Ks = sm, *Qs = Ks + kDcC * D, *Vs = Qs + kDcC * D, *As = Vs + kDcC * kDcNC, *Bs = As + kDcC;
+  const float* s0 = sm + DcSmem<D>::Red;
   const int tid = threadIdx.x, lane = tid & 31, col = (tid >> 5) * CPW, kvh = h / (p.H / p.G);
   float s[CPW][RPL];
 #pragma unroll
@@ -343,35 +345,25 @@ __device__ __noinline__ void walk_on(const DeltaChunkArgs& p, float* sm, const f
     for (int i = tid; i < n * kDcNC; i += NT) Vs[i] = p.v[(row + i / kDcNC) * p.ldv + (long long)h * p.Dv + col0 + i % kDcNC];
     if (tid < n) { As[tid] = p.g[(row + tid) * p.ldg + h]; Bs[tid] = p.beta[(row + tid) * p.ldb + h]; }
     __syncthreads();
-    for (int tb = 0; tb < n; tb += 16) {                  // the outputs' sums over the warp wait for one another's tokens
-      float o[CPW][16];
+#pragma unroll 1
+    for (int t = 0; t < n; ++t) {
+      const float a = As[t], b = Bs[t];
+      float k[RPL], q[RPL];
 #pragma unroll
-      for (int x = 0; x < 16; ++x) {
-        const int t = tb + x;
-#pragma unroll
-        for (int c = 0; c < CPW; ++c) o[c][x] = 0.f;
-        if (t >= n) continue;
-        const float a = As[t], b = Bs[t];
-        float k[RPL], q[RPL];
-#pragma unroll
-        for (int i = 0; i < RPL; ++i) { k[i] = Ks[t * D + lane + 32 * i]; q[i] = Qs[t * D + lane + 32 * i]; }
-#pragma unroll
-        for (int c = 0; c < CPW; ++c) {
-          float d = 0.f;
-#pragma unroll
-          for (int i = 0; i < RPL; ++i) { s[c][i] *= a; d = fmaf(s[c][i], k[i], d); }
-#pragma unroll
-          for (int w = 16; w >= 1; w >>= 1) d += __shfl_xor_sync(0xffffffffu, d, w);
-          const float u = b * (Vs[t * kDcNC + col + c] - d);
-#pragma unroll
-          for (int i = 0; i < RPL; ++i) { s[c][i] = fmaf(k[i], u, s[c][i]); o[c][x] = fmaf(s[c][i], q[i], o[c][x]); }
-        }
-      }
-      const int t = tb + (lane >> 1);
+      for (int i = 0; i < RPL; ++i) { k[i] = Ks[t * D + lane + 32 * i]; q[i] = Qs[t * D + lane + 32 * i]; }
 #pragma unroll
       for (int c = 0; c < CPW; ++c) {
-        const float y = gather16(o[c], lane);
-        if (!(lane & 1) && t < n) p.o[((row + t) * p.H + h) * p.Dv + col0 + col + c] = y;
+        float d = 0.f, o = 0.f;
+#pragma unroll
+        for (int i = 0; i < RPL; ++i) { s[c][i] *= a; d = fmaf(s[c][i], k[i], d); }
+#pragma unroll
+        for (int w = 16; w >= 1; w >>= 1) d += __shfl_xor_sync(0xffffffffu, d, w);
+        const float u = b * (Vs[t * kDcNC + col + c] - d);
+#pragma unroll
+        for (int i = 0; i < RPL; ++i) { s[c][i] = fmaf(k[i], u, s[c][i]); o = fmaf(s[c][i], q[i], o); }
+#pragma unroll
+        for (int w = 16; w >= 1; w >>= 1) o += __shfl_xor_sync(0xffffffffu, o, w);
+        if (lane == 0) p.o[((row + t) * p.H + h) * p.Dv + col0 + col + c] = o;
       }
     }
   }
@@ -562,7 +554,7 @@ delta_chunk_scan_kernel(const DeltaChunkArgs p) {
       for (int x = 0; x < 4; ++x) sm[L::Red + (16 * w + 8 * half + t2 + (x & 1)) * 16 + g + (x >> 1) * 8] = S[x];
       if (more) mbar_wait(kp_bar(tile + 1), (uint32_t)((tile + 1 - t_lo) >> 1) & 1u);      // what is on its way arrives before the CTA leaves
       __syncthreads();
-      walk_on<D>(p, sm, sm + L::Red, h, col0, first, at, min(len, (t_hi - tb) * kDcC), sp);
+      walk_on<D>(p, sm, h, col0, first, at, min(len, (t_hi - tb) * kDcC), sp);
       return;
     }
     if (asks && more) ask_qt(tile + 1);

@@ -53,20 +53,6 @@ __device__ __forceinline__ SplitA load_a(const float* at, int lane) {        // 
   return a;
 }
 
-// 16 values a lane, summed over the warp: lane l keeps the sum of value l / 2
-__device__ __forceinline__ float gather16(float (&v)[16], int lane) {
-#pragma unroll
-  for (int w = 8; w >= 1; w >>= 1) {
-    const bool up = lane & (2 * w);
-#pragma unroll
-    for (int i = 0; i < w; ++i) {
-      const float mine = up ? v[w + i] : v[i], theirs = up ? v[i] : v[w + i];
-      v[i] = mine + __shfl_xor_sync(0xffffffffu, theirs, 2 * w);
-    }
-  }
-  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
-}
-
 // also where rounding to 16 bits may be an infinity
 __device__ __forceinline__ bool not_finite(float x) { return !(fabsf(x) <= 3.3e38f); }
 
